@@ -178,6 +178,7 @@ flash_core_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   const int T = p.nkt;
   // n counts key tiles over all work items of this CTA: every per-tile barrier completes one phase per n

@@ -16,7 +16,8 @@ template <bool F32IN>
 __global__ void __launch_bounds__(256)
 layernorm_rows_kernel(const void* __restrict__ x, __nv_bfloat16* __restrict__ y,
                       const float* __restrict__ w, const float* __restrict__ b, long long rows, int cols,
-                      float eps, int normalize, int silu, const void* __restrict__ x2 = nullptr, int cols1 = 0) {
+                      float eps, int normalize, int silu, const void* __restrict__ x2, int cols1) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int nvec = cols >> 3;
   const long long warp_global = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -102,6 +103,7 @@ template <bool F32IN, int L>
 __global__ void __launch_bounds__(256)
 layernorm_rows_narrow_kernel(const void* __restrict__ x, __nv_bfloat16* __restrict__ y, const float* __restrict__ w,
                              const float* __restrict__ b, long long rows, int cols, float eps, int normalize, int silu) {
+  pdl_wait();
   constexpr int RPW = 32 / L;
   const int lane = threadIdx.x & 31;
   const int sub = lane / L, l = lane % L;
@@ -158,6 +160,7 @@ layernorm_rows_narrow_kernel(const void* __restrict__ x, __nv_bfloat16* __restri
 __global__ void __launch_bounds__(256)
 pair_outer_sum_kernel(const float* __restrict__ a, const float* __restrict__ c, const float* __restrict__ extra,
                       float* __restrict__ z, int n_i, int n_j, int cols) {
+  pdl_wait();
   const int nvec = cols >> 3;
   const long long total = (long long)n_i * n_j * nvec;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -183,6 +186,7 @@ pair_outer_sum_kernel(const float* __restrict__ a, const float* __restrict__ c, 
 template <bool YF32>
 __global__ void __launch_bounds__(256)
 add_rows_kernel(const float* x, const void* __restrict__ y, float* out, long long rows, long long period, int cols) {
+  pdl_wait();
   const int nvec = cols >> 3;
   const long long total = rows * nvec;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -200,6 +204,7 @@ add_rows_kernel(const float* x, const void* __restrict__ y, float* out, long lon
 // h[r, j] = silu(h12[r, j]) * h12[r, H + j]   (bf16 in, bf16 out; H multiple of 8)
 __global__ void __launch_bounds__(256)
 swiglu_rows_kernel(const __nv_bfloat16* __restrict__ h12, __nv_bfloat16* __restrict__ h, long long rows, int H) {
+  pdl_wait();
   const int nvec = H >> 3;
   const long long total = rows * nvec;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -220,6 +225,7 @@ template <bool F32IN>
 __global__ void __launch_bounds__(256)
 adaln_rows_kernel(const void* __restrict__ x, const float* __restrict__ cond, int cw, int alpha_col, int beta_col,
                   float lns, __nv_bfloat16* __restrict__ y, long long rows, int cols, float eps) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int nvec = cols >> 3;
   const long long warp_global = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -271,6 +277,7 @@ template <bool XF32, bool HF32>
 __global__ void __launch_bounds__(256)
 gated_residual_rows_kernel(void* __restrict__ x, const void* __restrict__ h, const float* __restrict__ cond, int cw,
                            int gamma_col, long long rows, int cols) {
+  pdl_wait();
   const int nvec = cols >> 3;
   const long long total = rows * nvec;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -295,6 +302,7 @@ gated_residual_rows_kernel(void* __restrict__ x, const void* __restrict__ h, con
 __global__ void __launch_bounds__(256)
 masked_softmax_rows_kernel(const __nv_bfloat16* __restrict__ logits, const uint8_t* __restrict__ mask,
                            __nv_bfloat16* __restrict__ out, int H, int n_rows, int n, int pitch) {
+  pdl_wait();
   constexpr float kNegMasked = -1.0e6f * 1.4426950408889634f;
   const int lane = threadIdx.x & 31;
   const long long rows = (long long)H * n_rows;
@@ -345,6 +353,7 @@ masked_softmax_rows_kernel(const __nv_bfloat16* __restrict__ logits, const uint8
 __global__ void __launch_bounds__(256)
 pwa_gate_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ og,
                 int S, int n, int H) {
+  pdl_wait();
   const long long total = (long long)S * n * H * 4;
   const long long o_plane = (long long)n * S * 32;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -373,6 +382,7 @@ pwa_gate_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __rest
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, const float* __restrict__ w,
                   const float* __restrict__ b, long long rows, int cols, float eps, int normalize, int order) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long warp_global = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long warp_stride = (long long)gridDim.x * (blockDim.x >> 5);
@@ -425,6 +435,7 @@ split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, co
 __global__ void __launch_bounds__(256)
 gate_rows_f32_kernel(const float* __restrict__ a, long long a_pitch, const float* __restrict__ b, long long b_pitch,
                      const uint8_t* __restrict__ rowmask, float* __restrict__ out, long long rows, int cols, int mode) {
+  pdl_wait();
   const int nvec = cols >> 2;
   const long long total = rows * nvec;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -447,6 +458,7 @@ gate_rows_f32_kernel(const float* __restrict__ a, long long a_pitch, const float
 __global__ void __launch_bounds__(256)
 softmax_bias_f32_kernel(float* __restrict__ s, const float* __restrict__ bias, const uint8_t* __restrict__ keymask,
                         long long groups, int n, int H, int bias_div, int mask_div_heads) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long rows = groups * n;
   const long long warp_global = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

@@ -10,7 +10,6 @@
 #include <atomic>
 #include <mutex>
 #include <unordered_map>
-#include <unordered_set>
 
 #include "../../include/b200pair.h"
 
@@ -43,13 +42,6 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 
 // Kernels launched by this library since it was loaded (all threads, all devices).
 inline std::atomic<unsigned long long> g_launch_count{0};
-
-// After every kernel launch: count it and pick up a launch error.
-#define B200_AFTER_LAUNCH()                                   \
-  do {                                                        \
-    ::b200::g_launch_count.fetch_add(1, std::memory_order_relaxed); \
-    B200_CUDA(cudaGetLastError());                            \
-  } while (0)
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -133,22 +125,46 @@ inline int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const ui
   return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, rank, dims, strides_bytes, box, swz);
 }
 
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel, device) instead of on every launch.
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) when a (kernel, device) first asks for this much, not on every launch.
 inline int set_smem_once(const void* kernel, uint32_t bytes) {
   static std::mutex mu;
-  static std::unordered_set<uint64_t> done;
+  static std::unordered_map<uint64_t, uint32_t> granted;
   int dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
   const uint64_t key = reinterpret_cast<uint64_t>(kernel) * 64 + uint64_t(dev & 63);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (done.count(key)) return 0;
-  }
-  B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
   std::lock_guard<std::mutex> lock(mu);
-  done.insert(key);
+  uint32_t& have = granted[key];
+  if (have >= bytes) return 0;
+  B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  have = bytes;
   return 0;
 }
+
+// Every kernel launch goes through here.  Programmatic dependent launch: a kernel's CTAs start as soon as those of the
+// kernel before it in the stream have exited, so its launch latency and set-up (barriers, tensor-memory allocation,
+// descriptor prefetch) overlap the completion and memory flush of that kernel; see pdl_wait().
+template <class... Params, class... Args>
+inline int launch(void (*kernel)(Params...), int grid, int block, uint32_t smem, cudaStream_t stream, Args&&... args) {
+  if (smem > 48 * 1024)
+    if (int e = set_smem_once(reinterpret_cast<const void*>(kernel), smem)) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(unsigned(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+  g_launch_count.fetch_add(1, std::memory_order_relaxed);
+  return 0;
+}
+#define B200_LAUNCH(...)                                  \
+  do {                                                    \
+    if (int e__ = ::b200::launch(__VA_ARGS__)) return e__; \
+  } while (0)
 
 inline int sm_count() {
   static int n = 0;

@@ -18,17 +18,10 @@
 
 namespace b200 {
 
-template <class Kernel>
-static int set_smem(Kernel k, uint32_t bytes) {
-  return set_smem_once(reinterpret_cast<const void*>(k), bytes);
-}
-
 template <int DH>
 static int launch_window_attention(const WindowAttnParams& p, int BM, cudaStream_t st) {
   const uint32_t smem = uint32_t(2u * p.Hk * p.heads * DH * 2u + p.Hk + 16);
-  if (int e = set_smem(window_attention_kernel<DH>, smem)) return e;
-  window_attention_kernel<DH><<<BM * p.NW, p.heads * p.W, smem, st>>>(p);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(window_attention_kernel<DH>, BM * p.NW, p.heads * p.W, smem, st, p);
   return B200_OK;
 }
 
@@ -113,13 +106,10 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   const int total = p.tiles_m * p.tiles_n * a.batch;
   const int grid = total < sm_count() ? total : sm_count();
   if (BN == 256) {
-    if (int e = set_smem(bmm_nt_kernel<256>, BmmCfg<256>::SMEM_BYTES)) return e;
-    bmm_nt_kernel<256><<<grid, 192, BmmCfg<256>::SMEM_BYTES, stream>>>(tmA, tmB, tmC, p);
+    B200_LAUNCH(bmm_nt_kernel<256>, grid, 192, BmmCfg<256>::SMEM_BYTES, stream, tmA, tmB, tmC, p);
   } else {
-    if (int e = set_smem(bmm_nt_kernel<128>, BmmCfg<128>::SMEM_BYTES)) return e;
-    bmm_nt_kernel<128><<<grid, 192, BmmCfg<128>::SMEM_BYTES, stream>>>(tmA, tmB, tmC, p);
+    B200_LAUNCH(bmm_nt_kernel<128>, grid, 192, BmmCfg<128>::SMEM_BYTES, stream, tmA, tmB, tmC, p);
   }
-  B200_AFTER_LAUNCH();
   return 0;
 }
 
@@ -134,22 +124,24 @@ static int launch_rows_to_bf16(const void* x, bool f32, __nv_bfloat16* y, const 
   if (!x2 && cols <= 128) {  // narrow rows: several rows per warp
     const int nn = normalize, ss = silu;
     if (cols <= 64) {
-      if (f32) layernorm_rows_narrow_kernel<true, 8><<<int(blocks), warps * 32, 0, stream>>>(x, y, w, b, rows, cols, 1e-5f, nn, ss);
-      else layernorm_rows_narrow_kernel<false, 8><<<int(blocks), warps * 32, 0, stream>>>(x, y, w, b, rows, cols, 1e-5f, nn, ss);
+      if (f32) B200_LAUNCH(layernorm_rows_narrow_kernel<true, 8>, int(blocks), warps * 32, 0, stream, x, y, w, b, rows,
+                           cols, 1e-5f, nn, ss);
+      else B200_LAUNCH(layernorm_rows_narrow_kernel<false, 8>, int(blocks), warps * 32, 0, stream, x, y, w, b, rows, cols,
+                       1e-5f, nn, ss);
     } else {
-      if (f32) layernorm_rows_narrow_kernel<true, 16><<<int(blocks), warps * 32, 0, stream>>>(x, y, w, b, rows, cols, 1e-5f, nn, ss);
-      else layernorm_rows_narrow_kernel<false, 16><<<int(blocks), warps * 32, 0, stream>>>(x, y, w, b, rows, cols, 1e-5f, nn, ss);
+      if (f32) B200_LAUNCH(layernorm_rows_narrow_kernel<true, 16>, int(blocks), warps * 32, 0, stream, x, y, w, b, rows,
+                           cols, 1e-5f, nn, ss);
+      else B200_LAUNCH(layernorm_rows_narrow_kernel<false, 16>, int(blocks), warps * 32, 0, stream, x, y, w, b, rows,
+                       cols, 1e-5f, nn, ss);
     }
-    B200_AFTER_LAUNCH();
     return 0;
   }
   if (f32)
-    layernorm_rows_kernel<true><<<int(blocks), warps * 32, 0, stream>>>(x, y, w, b, rows, cols, 1e-5f, normalize, silu,
-                                                                       x2, cols1);
+    B200_LAUNCH(layernorm_rows_kernel<true>, int(blocks), warps * 32, 0, stream, x, y, w, b, rows, cols, 1e-5f, normalize,
+                silu, x2, cols1);
   else
-    layernorm_rows_kernel<false><<<int(blocks), warps * 32, 0, stream>>>(x, y, w, b, rows, cols, 1e-5f, normalize, silu,
-                                                                        x2, cols1);
-  B200_AFTER_LAUNCH();
+    B200_LAUNCH(layernorm_rows_kernel<false>, int(blocks), warps * 32, 0, stream, x, y, w, b, rows, cols, 1e-5f,
+                normalize, silu, x2, cols1);
   return 0;
 }
 
@@ -198,10 +190,8 @@ static int launch_flash_t(const FlashLaunch& a, cudaStream_t stream) {
     return fail(B200_ERR_INVALID_ARGUMENT, "attention supports at most %d tokens (got %d)", Cfg::MAX_T * 128, p.N);
   p.nqg = (p.nqt + G - 1) / G;
   p.total_work = p.Bt * p.H * p.nqg;
-  if (int e = set_smem(flash_core_kernel<DH, G>, Cfg::SMEM_BYTES)) return e;
   const int grid = p.total_work < sm_count() ? p.total_work : sm_count();
-  flash_core_kernel<DH, G><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(tmQ, tmQ, tmV, tmB, p);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(flash_core_kernel<DH, G>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, tmQ, tmQ, tmV, tmB, p);
   return 0;
 }
 
@@ -217,8 +207,6 @@ static int launch_pair_bias(const void* z, bool f32, const float* ln_w, const fl
   const uint64_t str[1] = {256};
   const uint32_t box[2] = {64, 16};
   if (int e = make_tmap_bf16(&tmW, w_z, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
-  if (int e = set_smem(pair_bias_kernel<true>, pair_bias::SMEM_BYTES)) return e;
-  if (int e = set_smem(pair_bias_kernel<false>, pair_bias::SMEM_BYTES)) return e;
   PairBiasParams p;
   p.z = z;
   p.ln_w = ln_w;
@@ -236,10 +224,9 @@ static int launch_pair_bias(const void* z, bool f32, const float* ln_w, const fl
   p.eps = 1e-5f;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
   if (f32)
-    pair_bias_kernel<true><<<grid, pair_bias::THREADS, pair_bias::SMEM_BYTES, stream>>>(tmW, p);
+    B200_LAUNCH(pair_bias_kernel<true>, grid, pair_bias::THREADS, pair_bias::SMEM_BYTES, stream, tmW, p);
   else
-    pair_bias_kernel<false><<<grid, pair_bias::THREADS, pair_bias::SMEM_BYTES, stream>>>(tmW, p);
-  B200_AFTER_LAUNCH();
+    B200_LAUNCH(pair_bias_kernel<false>, grid, pair_bias::THREADS, pair_bias::SMEM_BYTES, stream, tmW, p);
   return 0;
 }
 
@@ -340,9 +327,8 @@ int b200_layernorm_fwd(const void* x, void* y, const float* w, const float* b, i
   int64_t blocks = (rows + warps - 1) / warps;
   const int64_t cap = int64_t(sm_count()) * 16;
   if (blocks > cap) blocks = cap;
-  layernorm_rows_kernel<false><<<int(blocks), warps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      x, static_cast<__nv_bfloat16*>(y), w, b, rows, cols, eps, 1, 0);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(layernorm_rows_kernel<false>, int(blocks), warps * 32, 0, static_cast<cudaStream_t>(stream), x,
+              static_cast<__nv_bfloat16*>(y), w, b, rows, cols, eps, 1, 0, nullptr, 0);
   return B200_OK;
 }
 
@@ -393,8 +379,6 @@ static int launch_trimul_project(const void* z, const uint8_t* mask, __nv_bfloat
     if (int e = make_tmap_bf16(&tmA, a_buf, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
     if (int e = make_tmap_bf16(&tmB, b_buf, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
-  if (int e = set_smem(trimul_in_kernel<true>, trimul_in::SMEM_BYTES)) return e;
-  if (int e = set_smem(trimul_in_kernel<false>, trimul_in::SMEM_BYTES)) return e;
   TriMulInParams pi;
   pi.z = z;
   pi.mask = mask;
@@ -414,10 +398,9 @@ static int launch_trimul_project(const void* z, const uint8_t* mask, __nv_bfloat
   pi.eps = 1e-5f;
   const int grid = pi.num_tiles < sm_count() ? pi.num_tiles : sm_count();
   if (f32)
-    trimul_in_kernel<true><<<grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream>>>(tmWin, tmA, tmB, pi);
+    B200_LAUNCH(trimul_in_kernel<true>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
   else
-    trimul_in_kernel<false><<<grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream>>>(tmWin, tmA, tmB, pi);
-  B200_AFTER_LAUNCH();
+    B200_LAUNCH(trimul_in_kernel<false>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
   return 0;
 }
 
@@ -449,8 +432,6 @@ static int launch_trimul_output(const void* z, void* out, const __nv_bfloat16* t
                           str, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return e;
   }
-  if (int e = set_smem(trimul_out_kernel<true>, trimul_out::SMEM_BYTES)) return e;
-  if (int e = set_smem(trimul_out_kernel<false>, trimul_out::SMEM_BYTES)) return e;
   TriMulOutParams po;
   po.z = z;
   po.out = out;
@@ -469,10 +450,9 @@ static int launch_trimul_output(const void* z, void* out, const __nv_bfloat16* t
   po.eps = 1e-5f;
   const int grid = po.num_tiles < sm_count() ? po.num_tiles : sm_count();
   if (f32)
-    trimul_out_kernel<true><<<grid, trimul_out::THREADS, trimul_out::SMEM_BYTES, stream>>>(tmWout, tmT, tmO, po);
+    B200_LAUNCH(trimul_out_kernel<true>, grid, trimul_out::THREADS, trimul_out::SMEM_BYTES, stream, tmWout, tmT, tmO, po);
   else
-    trimul_out_kernel<false><<<grid, trimul_out::THREADS, trimul_out::SMEM_BYTES, stream>>>(tmWout, tmT, tmO, po);
-  B200_AFTER_LAUNCH();
+    B200_LAUNCH(trimul_out_kernel<false>, grid, trimul_out::THREADS, trimul_out::SMEM_BYTES, stream, tmWout, tmT, tmO, po);
   return 0;
 }
 
@@ -628,8 +608,6 @@ int b200_transition_fwd(const void* x, void* out, const void* w13, const void* w
                           box, CU_TENSOR_MAP_SWIZZLE_64B))
       return e;
   }
-  if (int e = set_smem(transition_kernel<true>, transition::SMEM_BYTES)) return e;
-  if (int e = set_smem(transition_kernel<false>, transition::SMEM_BYTES)) return e;
   TransitionParams p;
   p.x = x;
   p.out = out;
@@ -642,10 +620,9 @@ int b200_transition_fwd(const void* x, void* out, const void* w13, const void* w
   p.eps = 1e-5f;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
   if (x_dtype == B200_DTYPE_F32)
-    transition_kernel<true><<<grid, transition::THREADS, transition::SMEM_BYTES, stream>>>(tmW1, tmW3, tmO, p);
+    B200_LAUNCH(transition_kernel<true>, grid, transition::THREADS, transition::SMEM_BYTES, stream, tmW1, tmW3, tmO, p);
   else
-    transition_kernel<false><<<grid, transition::THREADS, transition::SMEM_BYTES, stream>>>(tmW1, tmW3, tmO, p);
-  B200_AFTER_LAUNCH();
+    B200_LAUNCH(transition_kernel<false>, grid, transition::THREADS, transition::SMEM_BYTES, stream, tmW1, tmW3, tmO, p);
   return B200_OK;
 }
 
@@ -740,8 +717,6 @@ static int opm_run(const void* m, const uint8_t* mask, int mask_ndim, void* out,
     const uint32_t box[2] = {64, 64};
     if (int e = make_tmap_bf16(&tmW, w->w_ab, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
-  if (int e = set_smem(opm_proj_kernel<true>, opm_proj::SMEM_BYTES)) return e;
-  if (int e = set_smem(opm_proj_kernel<false>, opm_proj::SMEM_BYTES)) return e;
   const size_t m_esz = m_dtype == B200_DTYPE_F32 ? 4 : 2;
   const size_t o_esz = out_dtype == B200_DTYPE_F32 ? 4 : 2;
 
@@ -761,14 +736,12 @@ static int opm_run(const void* m, const uint8_t* mask, int mask_ndim, void* out,
     pp.eps = 1e-5f;
     const int grid = pp.num_tiles < sm_count() ? pp.num_tiles : sm_count();
     if (m_dtype == B200_DTYPE_F32)
-      opm_proj_kernel<true><<<grid, opm_proj::THREADS, opm_proj::SMEM_BYTES, stream>>>(tmW, pp);
+      B200_LAUNCH(opm_proj_kernel<true>, grid, opm_proj::THREADS, opm_proj::SMEM_BYTES, stream, tmW, pp);
     else
-      opm_proj_kernel<false><<<grid, opm_proj::THREADS, opm_proj::SMEM_BYTES, stream>>>(tmW, pp);
-    B200_AFTER_LAUNCH();
+      B200_LAUNCH(opm_proj_kernel<false>, grid, opm_proj::THREADS, opm_proj::SMEM_BYTES, stream, tmW, pp);
     const float* scale_ptr = ext_scale;
     if (mask_ndim == 3 && !ext_scale) {
-      opm_inv_row_count_kernel<<<1, 1024, 0, stream>>>(pp.mask, S, N, inv);
-      B200_AFTER_LAUNCH();
+      B200_LAUNCH(opm_inv_row_count_kernel, 1, 1024, 0, stream, pp.mask, S, N, inv);
       scale_ptr = inv;
     }
     for (int i0 = 0; i0 < N; i0 += CI) {
@@ -1084,8 +1057,6 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
     const uint32_t box[2] = {64, 8};
     if (int e = make_tmap_bf16(&tmWB, w->w_b, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
-  if (int e = set_smem(triatt_proj_kernel<true>, triatt_proj::SMEM_BYTES)) return e;
-  if (int e = set_smem(triatt_proj_kernel<false>, triatt_proj::SMEM_BYTES)) return e;
   TriAttProjParams pp;
   pp.z = z;
   pp.ln_w = w->ln_w;
@@ -1107,10 +1078,11 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
   pp.bias_scale = 1.4426950408889634f;
   const int grid = pp.num_tiles < sm_count() ? pp.num_tiles : sm_count();
   if (f32)
-    triatt_proj_kernel<true><<<grid, triatt_proj::THREADS, triatt_proj::SMEM_BYTES, stream>>>(tmW, tmQKG, tmVT, tmWB, pp);
+    B200_LAUNCH(triatt_proj_kernel<true>, grid, triatt_proj::THREADS, triatt_proj::SMEM_BYTES, stream, tmW, tmQKG, tmVT,
+                tmWB, pp);
   else
-    triatt_proj_kernel<false><<<grid, triatt_proj::THREADS, triatt_proj::SMEM_BYTES, stream>>>(tmW, tmQKG, tmVT, tmWB, pp);
-  B200_AFTER_LAUNCH();
+    B200_LAUNCH(triatt_proj_kernel<false>, grid, triatt_proj::THREADS, triatt_proj::SMEM_BYTES, stream, tmW, tmQKG, tmVT,
+                tmWB, pp);
   {
     FlashLaunch a;
     a.qk = qkg;
@@ -1260,9 +1232,8 @@ int b200_window_bias_fwd(const void* z, const float* ln_w, const float* ln_b, co
   while (lpr * 4 < c_z) lpr *= 2;  // lanes per pair: four channels each
   const int grid = grid_for(p.pairs * lpr, 256);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (z_dtype == B200_DTYPE_F32) window_bias_kernel<true><<<grid, 256, 0, st>>>(p, lpr);
-  else window_bias_kernel<false><<<grid, 256, 0, st>>>(p, lpr);
-  B200_AFTER_LAUNCH();
+  if (z_dtype == B200_DTYPE_F32) B200_LAUNCH(window_bias_kernel<true>, grid, 256, 0, st, p, lpr);
+  else B200_LAUNCH(window_bias_kernel<false>, grid, 256, 0, st, p, lpr);
   return B200_OK;
 }
 
@@ -1294,9 +1265,8 @@ int b200_pair_outer_sum(const float* a, const float* c, const float* extra, floa
   B200_CHECK_ARG(aligned(a, 32) && aligned(c, 32) && aligned(z, 32) && (!extra || aligned(extra, 32)),
                  "a/c/extra/z must be 32-byte aligned");
   if (n_i == 0 || n_j == 0) return B200_OK;
-  pair_outer_sum_kernel<<<grid_for((int64_t)n_i * n_j * (cols / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      a, c, extra, z, n_i, n_j, cols);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(pair_outer_sum_kernel, grid_for((int64_t)n_i * n_j * (cols / 8), 256), 256, 0,
+              static_cast<cudaStream_t>(stream), a, c, extra, z, n_i, n_j, cols);
   return B200_OK;
 }
 
@@ -1310,9 +1280,8 @@ int b200_add_rows(const float* x, const void* y, float* out, int64_t rows, int64
   if (rows == 0) return B200_OK;
   const int grid = grid_for(rows * (cols / 8), 256);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (y_dtype == B200_DTYPE_F32) add_rows_kernel<true><<<grid, 256, 0, st>>>(x, y, out, rows, period, cols);
-  else add_rows_kernel<false><<<grid, 256, 0, st>>>(x, y, out, rows, period, cols);
-  B200_AFTER_LAUNCH();
+  if (y_dtype == B200_DTYPE_F32) B200_LAUNCH(add_rows_kernel<true>, grid, 256, 0, st, x, y, out, rows, period, cols);
+  else B200_LAUNCH(add_rows_kernel<false>, grid, 256, 0, st, x, y, out, rows, period, cols);
   return B200_OK;
 }
 
@@ -1339,9 +1308,8 @@ int b200_swiglu_fwd(const void* h12, void* h, int64_t rows, int hidden, b200_str
   B200_CHECK_ARG(rows >= 0 && hidden > 0 && hidden % 8 == 0, "hidden=%d must be a positive multiple of 8", hidden);
   B200_CHECK_ARG(aligned(h12, 16) && aligned(h, 16), "h12/h must be 16-byte aligned");
   if (rows == 0) return B200_OK;
-  swiglu_rows_kernel<<<grid_for(rows * (hidden / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(h12), static_cast<__nv_bfloat16*>(h), rows, hidden);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(swiglu_rows_kernel, grid_for(rows * (hidden / 8), 256), 256, 0, static_cast<cudaStream_t>(stream),
+              static_cast<const __nv_bfloat16*>(h12), static_cast<__nv_bfloat16*>(h), rows, hidden);
   return B200_OK;
 }
 
@@ -1358,12 +1326,11 @@ int b200_adaln_fwd(const void* x, const float* cond, int cond_width, int alpha_c
   const int grid = grid_for(rows, 8);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (x_dtype == B200_DTYPE_F32)
-    adaln_rows_kernel<true><<<grid, 256, 0, st>>>(x, cond, cond_width, alpha_col, beta_col, lns,
-                                                  static_cast<__nv_bfloat16*>(y), rows, cols, 1e-5f);
+    B200_LAUNCH(adaln_rows_kernel<true>, grid, 256, 0, st, x, cond, cond_width, alpha_col, beta_col, lns,
+                static_cast<__nv_bfloat16*>(y), rows, cols, 1e-5f);
   else
-    adaln_rows_kernel<false><<<grid, 256, 0, st>>>(x, cond, cond_width, alpha_col, beta_col, lns,
-                                                   static_cast<__nv_bfloat16*>(y), rows, cols, 1e-5f);
-  B200_AFTER_LAUNCH();
+    B200_LAUNCH(adaln_rows_kernel<false>, grid, 256, 0, st, x, cond, cond_width, alpha_col, beta_col, lns,
+                static_cast<__nv_bfloat16*>(y), rows, cols, 1e-5f);
   return B200_OK;
 }
 
@@ -1379,11 +1346,14 @@ int b200_gated_residual_fwd(void* x, const void* h, const float* cond, int cond_
   const int grid = grid_for(rows * (cols / 8), 256);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool xf = x_dtype == B200_DTYPE_F32, hf = h_dtype == B200_DTYPE_F32;
-  if (xf && hf) gated_residual_rows_kernel<true, true><<<grid, 256, 0, st>>>(x, h, cond, cond_width, gamma_col, rows, cols);
-  else if (xf) gated_residual_rows_kernel<true, false><<<grid, 256, 0, st>>>(x, h, cond, cond_width, gamma_col, rows, cols);
-  else if (hf) gated_residual_rows_kernel<false, true><<<grid, 256, 0, st>>>(x, h, cond, cond_width, gamma_col, rows, cols);
-  else gated_residual_rows_kernel<false, false><<<grid, 256, 0, st>>>(x, h, cond, cond_width, gamma_col, rows, cols);
-  B200_AFTER_LAUNCH();
+  if (xf && hf) B200_LAUNCH(gated_residual_rows_kernel<true, true>, grid, 256, 0, st, x, h, cond, cond_width, gamma_col,
+                            rows, cols);
+  else if (xf) B200_LAUNCH(gated_residual_rows_kernel<true, false>, grid, 256, 0, st, x, h, cond, cond_width, gamma_col,
+                           rows, cols);
+  else if (hf) B200_LAUNCH(gated_residual_rows_kernel<false, true>, grid, 256, 0, st, x, h, cond, cond_width, gamma_col,
+                           rows, cols);
+  else B200_LAUNCH(gated_residual_rows_kernel<false, false>, grid, 256, 0, st, x, h, cond, cond_width, gamma_col, rows,
+                   cols);
   return B200_OK;
 }
 
@@ -1394,9 +1364,8 @@ int b200_masked_softmax_rows(const void* logits, const uint8_t* mask, void* out,
   B200_CHECK_ARG(H > 0 && n > 0 && n_rows > 0 && pitch >= n && pitch % 8 == 0,
                  "need H, n_rows, n > 0 and a pitch >= n that is a multiple of 8");
   B200_CHECK_ARG(aligned(logits, 16) && aligned(out, 16), "logits/out must be 16-byte aligned");
-  masked_softmax_rows_kernel<<<grid_for((int64_t)H * n_rows, 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(logits), mask, static_cast<__nv_bfloat16*>(out), H, n_rows, n, pitch);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(masked_softmax_rows_kernel, grid_for((int64_t)H * n_rows, 8), 256, 0, static_cast<cudaStream_t>(stream),
+              static_cast<const __nv_bfloat16*>(logits), mask, static_cast<__nv_bfloat16*>(out), H, n_rows, n, pitch);
   return B200_OK;
 }
 
@@ -1405,9 +1374,9 @@ int b200_pwa_gate(const void* o, const void* g, void* og, int S, int n, int H, b
   B200_CHECK_ARG(o && g && og, "o/g/og is NULL");
   B200_CHECK_ARG(S > 0 && n > 0 && H > 0, "S, n, H must be positive");
   B200_CHECK_ARG(aligned(o, 16) && aligned(g, 16) && aligned(og, 16), "o/g/og must be 16-byte aligned");
-  pwa_gate_kernel<<<grid_for((int64_t)S * n * H * 4, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(g), static_cast<__nv_bfloat16*>(og), S, n, H);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(pwa_gate_kernel, grid_for((int64_t)S * n * H * 4, 256), 256, 0, static_cast<cudaStream_t>(stream),
+              static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(g), static_cast<__nv_bfloat16*>(og),
+              S, n, H);
   return B200_OK;
 }
 
@@ -1420,9 +1389,8 @@ int b200_split_rows(const void* x, void* y, const float* w, const float* b, int6
   B200_CHECK_ARG(order == 0 || order == 1, "order must be 0 (hi|hi|lo) or 1 (hi|lo|hi)");
   B200_CHECK_ARG(aligned(x, 32) && aligned(y, 16), "x must be 32-byte aligned, y 16-byte aligned");
   if (rows == 0) return B200_OK;
-  split_rows_kernel<<<grid_for(rows, 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const float*>(x), static_cast<__nv_bfloat16*>(y), w, b, rows, cols, eps, normalize, order);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(split_rows_kernel, grid_for(rows, 8), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const
+              float*>(x), static_cast<__nv_bfloat16*>(y), w, b, rows, cols, eps, normalize, order);
   return B200_OK;
 }
 
@@ -1435,9 +1403,8 @@ int b200_gate_rows_f32(const float* a, int64_t a_pitch, const float* b, int64_t 
   B200_CHECK_ARG(mode >= 0 && mode <= 2, "mode must be 0 (a * sigmoid(b)), 1 (silu(a) * b) or 2 (a)");
   B200_CHECK_ARG(aligned(a, 16) && aligned(b, 16) && aligned(out, 16), "a/b/out must be 16-byte aligned");
   if (rows == 0) return B200_OK;
-  gate_rows_f32_kernel<<<grid_for(rows * (cols / 4), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      a, a_pitch, b, b_pitch, rowmask, out, rows, cols, mode);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(gate_rows_f32_kernel, grid_for(rows * (cols / 4), 256), 256, 0, static_cast<cudaStream_t>(stream), a,
+              a_pitch, b, b_pitch, rowmask, out, rows, cols, mode);
   return B200_OK;
 }
 
@@ -1447,9 +1414,8 @@ int b200_softmax_bias_f32(float* s, const float* bias, const uint8_t* keymask, i
   B200_CHECK_ARG(s && keymask, "s/keymask is NULL");
   B200_CHECK_ARG(groups > 0 && n > 0 && H > 0 && bias_div > 0 && groups % ((int64_t)H * bias_div) == 0,
                  "groups must be a multiple of H * bias_div");
-  softmax_bias_f32_kernel<<<grid_for(groups * n, 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      s, bias, keymask, groups, n, H, bias_div, H * bias_div);
-  B200_AFTER_LAUNCH();
+  B200_LAUNCH(softmax_bias_f32_kernel, grid_for(groups * n, 8), 256, 0, static_cast<cudaStream_t>(stream), s, bias,
+              keymask, groups, n, H, bias_div, H * bias_div);
   return B200_OK;
 }
 

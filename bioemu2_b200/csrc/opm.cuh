@@ -73,6 +73,7 @@ opm_proj_kernel(const __grid_constant__ CUtensorMap tmW, OpmProjParams p) {
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   if (warp == 8) {
     // the whole warp waits on the barriers, one elected lane issues
@@ -199,6 +200,7 @@ opm_proj_kernel(const __grid_constant__ CUtensorMap tmW, OpmProjParams p) {
 
 // Number of MSA rows with at least one valid token -> 1 / max(count, 1).  One block.
 __global__ void opm_inv_row_count_kernel(const uint8_t* mask, int S, int N, float* inv_out) {
+  pdl_wait();
   __shared__ int count;
   if (threadIdx.x == 0) count = 0;
   __syncthreads();

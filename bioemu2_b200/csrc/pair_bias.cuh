@@ -63,6 +63,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmW, PairBiasParams p) {
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   if (warp == 12) {
     // The whole warp walks the tile loop and waits on the barriers; one elected lane issues the products and the

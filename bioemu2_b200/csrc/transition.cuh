@@ -102,6 +102,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
   // TMEM columns: D1[b] at b*128 (fc1 chunk 0..63, fc2 chunk 64..127); OUT[o] at 256 + o*128.
 
   int my_tiles = 0;

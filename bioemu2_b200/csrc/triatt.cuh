@@ -96,12 +96,14 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     prefetch_tmap(&tmVT);
     prefetch_tmap(&tmWB);
   }
-  if (threadIdx.x < 128) gb_s[threadIdx.x] = p.g_bias[threadIdx.x];
   if (warp == 12) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  if (threadIdx.x < 128) gb_s[threadIdx.x] = p.g_bias[threadIdx.x];
+  __syncthreads();
 
   if (warp == 12) {
     // The whole warp walks the tile loop and waits on the barriers; one elected lane issues the products and the

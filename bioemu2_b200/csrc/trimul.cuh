@@ -90,6 +90,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   if (warp >= 8) {
     // ------------------------------------------------------------------ producers
@@ -309,15 +310,17 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     prefetch_tmap(&tmT);
     prefetch_tmap(&tmO);
   }
-  if (threadIdx.x < 128) {
-    ln_s[threadIdx.x] = p.ln_out_w[threadIdx.x];
-    ln_s[128 + threadIdx.x] = p.ln_out_b[threadIdx.x];
-  }
   if (warp == 0) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  if (threadIdx.x < 128) {
+    ln_s[threadIdx.x] = p.ln_out_w[threadIdx.x];
+    ln_s[128 + threadIdx.x] = p.ln_out_b[threadIdx.x];
+  }
+  __syncthreads();
 
   if (warp >= 4 && warp < 8) {
     // ------------------------------------------------------------------ t transformers

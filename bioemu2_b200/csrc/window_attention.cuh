@@ -34,6 +34,7 @@ constexpr int kWindowMaxHeads = 16;
 template <bool F32>
 __global__ void __launch_bounds__(256)
 window_bias_kernel(WindowBiasParams p, int lpr) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int sub = lane / lpr, l = lane % lpr;
   const int rpw = 32 / lpr;
@@ -110,6 +111,7 @@ constexpr float kWindowMasked = -1e6f;  // the reference REPLACES masked logits 
 template <int DH>
 __global__ void __launch_bounds__(256)
 window_attention_kernel(WindowAttnParams p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const int c_s = p.heads * DH;
   __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(smem_raw);
