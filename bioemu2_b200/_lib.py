@@ -48,6 +48,20 @@ class TriAttWeights(Structure):
                 ("ln_b", c_void_p)]
 
 
+class TransitionWeights(Structure):
+    _fields_ = [("w13", c_void_p), ("w3", c_void_p), ("ln_w", c_void_p), ("ln_b", c_void_p)]
+
+
+class SwigluWeights(Structure):
+    _fields_ = [("w12", c_void_p), ("w3", c_void_p), ("ln_w", c_void_p), ("ln_b", c_void_p), ("hidden", c_int64)]
+
+
+class TrunkBlock(Structure):
+    _fields_ = [("tri_mul_out", TriMulWeights), ("tri_mul_in", TriMulWeights), ("tri_att_start", TriAttWeights),
+                ("tri_att_end", TriAttWeights), ("transition_z", TransitionWeights), ("attention", ApbWeights),
+                ("transition_s", SwigluWeights)]
+
+
 class AttentionCoreArgs(Structure):
     _fields_ = [
         ("qk", c_void_p), ("qk_width", c_int64), ("qk_batch_stride", c_int64), ("q_col0", c_int), ("k_col0", c_int),
@@ -123,6 +137,10 @@ SIGNATURES = {
                                           c_int, c_int, c_int, c_void_p]),
     "b200_pair_outer_sum": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "b200_add_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_void_p]),
+    "b200_trunk_workspace_bytes": (c_size_t, [POINTER(TrunkBlock), c_int, c_int, c_int]),
+    "b200_trunk_side_workspace_bytes": (c_size_t, [POINTER(TrunkBlock), c_int, c_int, c_int, c_int, c_int]),
+    "b200_trunk_fwd": (c_int, [POINTER(TrunkBlock), c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                               c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_size_t, c_void_p, c_void_p]),
     "b200_rows2_to_bf16": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int,
                                    c_void_p]),
 }

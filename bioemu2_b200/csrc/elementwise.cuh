@@ -201,6 +201,19 @@ add_rows_kernel(const float* x, const void* __restrict__ y, float* out, long lon
   }
 }
 
+// Pair mask of a padded batch: out[b, i, j] = tok[b, i] && tok[b, j], one byte per pair.
+__global__ void __launch_bounds__(256)
+pair_mask_kernel(const uint8_t* __restrict__ tok, uint8_t* __restrict__ out, int B, int N) {
+  pdl_wait();
+  const long long total = (long long)B * N * N;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+    const long long bi = t / N;
+    const int j = int(t - bi * N);
+    const long long b = bi / N;
+    out[t] = (tok[bi] != 0 && tok[b * N + j] != 0) ? 1 : 0;
+  }
+}
+
 // h[r, j] = silu(h12[r, j]) * h12[r, H + j]   (bf16 in, bf16 out; H multiple of 8)
 __global__ void __launch_bounds__(256)
 swiglu_rows_kernel(const __nv_bfloat16* __restrict__ h12, __nv_bfloat16* __restrict__ h, long long rows, int H) {

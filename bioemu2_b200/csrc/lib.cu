@@ -365,7 +365,8 @@ struct TriMulGeom {
 };
 
 static int launch_trimul_project(const void* z, const uint8_t* mask, __nv_bfloat16* a_buf, __nv_bfloat16* b_buf,
-                                 const b200_trimul_weights* w, const TriMulGeom& g, bool f32, cudaStream_t stream) {
+                                 const b200_trimul_weights* w, const TriMulGeom& g, bool f32, cudaStream_t stream,
+                                 long long z_copy_delta = 0) {
   CUtensorMap tmWin;
   const uint64_t dims[2] = {128, 512};
   const uint64_t str[1] = {256};
@@ -382,6 +383,7 @@ static int launch_trimul_project(const void* z, const uint8_t* mask, __nv_bfloat
   TriMulInParams pi;
   pi.z = z;
   pi.mask = mask;
+  pi.z_copy_delta = z_copy_delta;
   pi.ln_w = w->ln_in_w;
   pi.ln_b = w->ln_in_b;
   pi.a_out = a_buf;
@@ -397,10 +399,13 @@ static int launch_trimul_project(const void* z, const uint8_t* mask, __nv_bfloat
   pi.num_tiles = g.n_lines * (g.pos_pitch / 128);
   pi.eps = 1e-5f;
   const int grid = pi.num_tiles < sm_count() ? pi.num_tiles : sm_count();
-  if (f32)
-    B200_LAUNCH(trimul_in_kernel<true>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
-  else
-    B200_LAUNCH(trimul_in_kernel<false>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
+  if (z_copy_delta) {
+    if (f32) B200_LAUNCH(trimul_in_kernel<true, true>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
+    else B200_LAUNCH(trimul_in_kernel<false, true>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
+  } else {
+    if (f32) B200_LAUNCH(trimul_in_kernel<true, false>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
+    else B200_LAUNCH(trimul_in_kernel<false, false>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
+  }
   return 0;
 }
 
@@ -489,13 +494,16 @@ static int trimul_fwd_impl(const void* z, const uint8_t* mask, void* out, const 
   for (int bi = 0; bi < B; ++bi) {
     const uint8_t* zb = static_cast<const uint8_t*>(z) + size_t(bi) * N * N * kD * esz;
     uint8_t* ob = static_cast<uint8_t*>(out) + size_t(bi) * N * N * kD * esz;
-    if (int e = launch_trimul_project(zb, mask + size_t(bi) * N * N, a_buf, b_buf, w, gin, f32, stream)) return e;
+    // z + update into another tensor: the projection stage copies z there, the output stage then adds in place (reading
+    // the residual row by row in its epilogue took 84 us against 46 at N = 384)
+    const bool copy = add_residual && ob != zb;
+    if (int e = launch_trimul_project(zb, mask + size_t(bi) * N * N, a_buf, b_buf, w, gin, f32, stream, copy ? ob - zb : 0)) return e;
     {
       const int64_t plane_el = int64_t(Np) * Np;
       BmmLaunch a{a_buf, b_buf, t_buf, kD, Np, Np, Np, Np, Np, Np, plane_el, plane_el, plane_el};
       if (int e = launch_bmm(a, stream)) return e;
     }
-    if (int e = launch_trimul_output(zb, ob, t_buf, w, gout, add_residual != 0, f32, stream)) return e;
+    if (int e = launch_trimul_output(copy ? ob : zb, ob, t_buf, w, gout, add_residual != 0, f32, stream)) return e;
   }
   return B200_OK;
 }
@@ -863,7 +871,7 @@ size_t b200_apb_workspace_bytes(int B, int M, int N, int c_s, int H) {
 
 static int apb_run(const void* s, const void* z, const void* ext_bias, int64_t ext_bias_pitch, const uint8_t* mask,
                    void* out, const b200_apb_weights* w, int B, int M, int N, int c_s, int H, int s_dtype, int z_dtype,
-                   void* workspace, size_t workspace_bytes, b200_stream_t stream_) {
+                   bool add_residual, void* workspace, size_t workspace_bytes, b200_stream_t stream_) {
   if (int e = b200_check_device()) return e;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   B200_CHECK_ARG(s && (z || ext_bias) && mask && out && w, "s/z/mask/out/w is NULL");
@@ -899,8 +907,8 @@ static int apb_run(const void* s, const void* z, const void* ext_bias, int64_t e
     a.bias = w->b_qkg;
     if (int e = launch_bmm(a, stream)) return e;
   }
-  for (int b = 0; b < BM; ++b) {
-    BmmLaunch a{w->w_v, s_ln + size_t(b) * N * c_s, vT + size_t(b) * HD * pl.Nk, 1, HD, N, c_s, c_s, c_s, pl.Nk, 0, 0, 0};
+  {  // one launch for all batch items: they share the A operand
+    BmmLaunch a{w->w_v, s_ln, vT, BM, HD, N, c_s, c_s, c_s, pl.Nk, 0, int64_t(N) * c_s, int64_t(HD) * pl.Nk};
     if (int e = launch_bmm(a, stream)) return e;
   }
   // 3. pair bias, one pass over z per batch element (unless the caller supplies it)
@@ -951,6 +959,7 @@ static int apb_run(const void* s, const void* z, const void* ext_bias, int64_t e
   {
     BmmLaunch a{og, w->w_o, out, 1, int(rows), c_s, c_s, c_s, c_s, c_s, 0, 0, 0};
     a.out_f32 = s_dtype == B200_DTYPE_F32;
+    a.residual = add_residual ? s : nullptr;
     if (int e = launch_bmm(a, stream)) return e;
   }
   return B200_OK;
@@ -960,15 +969,16 @@ int b200_apb_fwd(const void* s, const void* z, const uint8_t* mask, void* out, c
                  int M, int N, int c_s, int H, int s_dtype, int z_dtype, void* workspace, size_t workspace_bytes,
                  b200_stream_t stream) {
   if (!z) return fail(B200_ERR_INVALID_ARGUMENT, "z is NULL");
-  return apb_run(s, z, nullptr, 0, mask, out, w, B, M, N, c_s, H, s_dtype, z_dtype, workspace, workspace_bytes, stream);
+  return apb_run(s, z, nullptr, 0, mask, out, w, B, M, N, c_s, H, s_dtype, z_dtype, false, workspace,
+                 workspace_bytes, stream);
 }
 
 int b200_apb_fwd_bias(const void* s, const void* bias, int64_t bias_pitch, const uint8_t* mask, void* out,
                       const b200_apb_weights* w, int B, int M, int N, int c_s, int H, int s_dtype, void* workspace,
                       size_t workspace_bytes, b200_stream_t stream) {
   if (!bias) return fail(B200_ERR_INVALID_ARGUMENT, "bias is NULL");
-  return apb_run(s, nullptr, bias, bias_pitch, mask, out, w, B, M, N, c_s, H, s_dtype, B200_DTYPE_F32, workspace,
-                 workspace_bytes, stream);
+  return apb_run(s, nullptr, bias, bias_pitch, mask, out, w, B, M, N, c_s, H, s_dtype, B200_DTYPE_F32, false,
+                 workspace, workspace_bytes, stream);
 }
 
 int b200_pair_bias_fwd(const void* z, const float* ln_w, const float* ln_b, const void* w_z, void* out, int n_rows,
@@ -1416,6 +1426,170 @@ int b200_softmax_bias_f32(float* s, const float* bias, const uint8_t* keymask, i
                  "groups must be a multiple of H * bias_div");
   B200_LAUNCH(softmax_bias_f32_kernel, grid_for(groups * n, 8), 256, 0, static_cast<cudaStream_t>(stream), s, bias,
               keymask, groups, n, H, bias_div, H * bias_div);
+  return B200_OK;
+}
+
+// ------------------------------------------------------------------------------------------------ trunk stack
+static size_t round_up_1k(size_t x) { return (x + 1023) / 1024 * 1024; }
+static bool has_triatt(const b200_trunk_block& w) { return w.tri_att_start.w_o != nullptr; }
+static bool has_single(const b200_trunk_block& w) { return w.attention.w_o != nullptr; }
+static size_t trunk_bias_bytes(int B, int N, int heads) {
+  return round_up_1k(size_t(B) * heads * N * ((N + 7) / 8 * 8) * 2);
+}
+static size_t trunk_scratch_bytes(const b200_trunk_block* blocks, int N) {
+  const size_t tm = b200_trimul_workspace_bytes(N), ta = has_triatt(blocks[0]) ? b200_triatt_workspace_bytes(N) : 0;
+  return round_up_1k(tm > ta ? tm : ta);
+}
+
+size_t b200_trunk_workspace_bytes(const b200_trunk_block* blocks, int B, int N, int heads) {
+  if (!blocks || B <= 0 || N <= 0) return 0;
+  return trunk_scratch_bytes(blocks, N) + (has_single(blocks[0]) ? 2 * trunk_bias_bytes(B, N, heads) : 0) +
+         round_up_1k(size_t(B) * N * N);
+}
+
+size_t b200_trunk_side_workspace_bytes(const b200_trunk_block* blocks, int n_blocks, int B, int N, int c_s, int heads) {
+  if (!blocks || n_blocks <= 0 || B <= 0 || N <= 0 || !has_single(blocks[0])) return 0;
+  size_t need = b200_apb_workspace_bytes(B, 1, N, c_s, heads);
+  const size_t rows = size_t(B) * N;
+  for (int i = 0; i < n_blocks; ++i) {
+    const size_t h = size_t(blocks[i].transition_s.hidden);
+    const size_t n = round_up_1k(rows * c_s * 2) + round_up_1k(rows * 2 * h * 2) + round_up_1k(rows * h * 2);
+    if (n > need) need = n;
+  }
+  return need;
+}
+
+// The events that order the two streams of a trunk call: two "bias ready", two "bias read", one for the joins.  Kept per
+// host thread and device -- an event may be recorded again as soon as the waits on it have been enqueued.
+struct TrunkEvents {
+  cudaEvent_t ev[5] = {};
+  int dev = -1;
+  void drop() {
+    for (cudaEvent_t& e : ev) {
+      if (e) cudaEventDestroy(e);
+      e = nullptr;
+    }
+  }
+  ~TrunkEvents() { drop(); }
+};
+
+static int trunk_events(cudaEvent_t** out) {
+  static thread_local TrunkEvents pool;
+  int dev = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  if (pool.dev != dev) {
+    pool.drop();
+    for (cudaEvent_t& e : pool.ev) B200_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    pool.dev = dev;
+  }
+  *out = pool.ev;
+  return 0;
+}
+
+// SwiGLU transition of any width in place on s[rows][c_s]: LayerNorm rows, [fc1 | fc2] product, SwiGLU, fc3 product that
+// adds into s.
+static int swiglu_transition_(void* s, const b200_swiglu_weights& w, int64_t rows, int c_s, bool f32, uint8_t* ws,
+                              cudaStream_t stream) {
+  const int hidden = int(w.hidden);
+  __nv_bfloat16* x = reinterpret_cast<__nv_bfloat16*>(ws);
+  __nv_bfloat16* h12 = reinterpret_cast<__nv_bfloat16*>(ws + round_up_1k(size_t(rows) * c_s * 2));
+  __nv_bfloat16* h = h12 + round_up_1k(size_t(rows) * 2 * hidden * 2) / 2;
+  if (int e = launch_rows_to_bf16(s, f32, x, w.ln_w, w.ln_b, rows, c_s, w.ln_w != nullptr, stream)) return e;
+  BmmLaunch a{x, w.w12, h12, 1, int(rows), 2 * hidden, c_s, c_s, c_s, 2 * hidden, 0, 0, 0};
+  if (int e = launch_bmm(a, stream)) return e;
+  B200_LAUNCH(swiglu_rows_kernel, grid_for(rows * (hidden / 8), 256), 256, 0, stream, h12, h, rows, hidden);
+  BmmLaunch b{h, w.w3, s, 1, int(rows), c_s, hidden, hidden, hidden, c_s, 0, 0, 0};
+  b.out_f32 = f32;
+  b.residual = s;
+  return launch_bmm(b, stream);
+}
+
+int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_in, void* z, void* s,
+                   const uint8_t* token_mask, const uint8_t* pair_mask, int B, int N, int c_s, int heads, int s_dtype,
+                   int z_dtype, void* workspace, size_t workspace_bytes, void* side_workspace, size_t side_bytes,
+                   b200_stream_t stream_, b200_stream_t side_stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(blocks && n_blocks > 0, "need at least one block");
+  B200_CHECK_ARG(z_in && z && (token_mask || pair_mask), "z_in/z/mask is NULL");
+  B200_CHECK_ARG(B > 0 && N > 0, "B=%d, N=%d must be positive", B, N);
+  B200_CHECK_ARG((s_dtype | 1) == 1 && (z_dtype | 1) == 1, "unknown dtype");
+  B200_CHECK_ARG(aligned(z, 32) && aligned(z_in, 32), "z must be 32-byte aligned");
+  const bool single = has_single(blocks[0]);
+  if (single) {
+    B200_CHECK_ARG(s && token_mask && aligned(s, 32), "the single track needs s (32-byte aligned) and token_mask");
+    B200_CHECK_ARG(c_s > 0 && c_s % 8 == 0 && c_s <= 1024 && heads > 0 && heads <= 16,
+                   "c_s=%d must be a multiple of 8 and <= 1024, heads=%d <= 16", c_s, heads);
+  }
+  for (int i = 0; i < n_blocks; ++i) {
+    const b200_trunk_block& w = blocks[i];
+    B200_CHECK_ARG(trimul_weights_ok(&w.tri_mul_out) && trimul_weights_ok(&w.tri_mul_in), "block %d: bad triangle weights", i);
+    B200_CHECK_ARG(has_triatt(w) == has_triatt(blocks[0]) && has_single(w) == single, "block %d: differs from block 0 in kind", i);
+    B200_CHECK_ARG(!has_triatt(w) || (triatt_weights_ok(&w.tri_att_start) && triatt_weights_ok(&w.tri_att_end)),
+                   "block %d: bad triangle attention weights", i);
+    B200_CHECK_ARG(!single || (w.transition_s.w12 && w.transition_s.w3 && w.transition_s.hidden > 0 && w.transition_s.hidden % 8 == 0),
+                   "block %d: bad single transition weights", i);
+  }
+  const size_t need = b200_trunk_workspace_bytes(blocks, B, N, heads);
+  const size_t side_need = b200_trunk_side_workspace_bytes(blocks, n_blocks, B, N, c_s, heads);
+  if (!workspace || workspace_bytes < need || !aligned(workspace, 1024) ||
+      (side_need && (!side_workspace || side_bytes < side_need || !aligned(side_workspace, 1024))))
+    return fail(B200_ERR_WORKSPACE, "workspaces must be 1024-byte aligned and hold %zu and %zu bytes (got %zu, %zu)", need,
+                side_need, workspace_bytes, side_bytes);
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  cudaStream_t side = side_stream ? static_cast<cudaStream_t>(side_stream) : stream;
+  const bool two = single && side != stream;
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  const size_t scratch = trunk_scratch_bytes(blocks, N), bias_bytes = single ? trunk_bias_bytes(B, N, heads) : 0;
+  __nv_bfloat16* bias[2] = {reinterpret_cast<__nv_bfloat16*>(ws + scratch),
+                            reinterpret_cast<__nv_bfloat16*>(ws + scratch + bias_bytes)};
+  cudaEvent_t* ev = nullptr;
+  if (two) {
+    if (int e = trunk_events(&ev)) return e;
+    B200_CUDA(cudaEventRecord(ev[4], stream));  // s, and all that was enqueued before this call
+    B200_CUDA(cudaStreamWaitEvent(side, ev[4], 0));
+  }
+  if (!pair_mask) {
+    uint8_t* pm = ws + scratch + 2 * bias_bytes;
+    B200_LAUNCH(pair_mask_kernel, grid_for(int64_t(B) * N * N, 1024), 256, 0, stream, token_mask, pm, B, N);
+    pair_mask = pm;
+  }
+  const bool zf32 = z_dtype == B200_DTYPE_F32, sf32 = s_dtype == B200_DTYPE_F32;
+  const size_t zsz = zf32 ? 4 : 2;
+  const int Nk = (N + 7) / 8 * 8;
+  for (int i = 0; i < n_blocks; ++i) {
+    const b200_trunk_block& w = blocks[i];
+    if (int e = trimul_fwd_impl(i == 0 ? z_in : z, pair_mask, z, &w.tri_mul_out, B, N, 0, 1, z_dtype, ws, scratch, stream)) return e;
+    if (int e = trimul_fwd_impl(z, pair_mask, z, &w.tri_mul_in, B, N, 1, 1, z_dtype, ws, scratch, stream)) return e;
+    if (has_triatt(w)) {
+      if (int e = b200_triatt_fwd(z, pair_mask, z, &w.tri_att_start, B, N, 0, 1, z_dtype, ws, scratch, stream)) return e;
+      if (int e = b200_triatt_fwd(z, pair_mask, z, &w.tri_att_end, B, N, 1, 1, z_dtype, ws, scratch, stream)) return e;
+    }
+    const b200_transition_weights& tz = w.transition_z;
+    if (int e = b200_transition_fwd(z, z, tz.w13, tz.w3, tz.ln_w, tz.ln_b, int64_t(B) * N * N, tz.ln_w != nullptr, 1, z_dtype, stream))
+      return e;
+    if (!single) continue;
+    const int k = i & 1;
+    if (two && i >= 2) B200_CUDA(cudaStreamWaitEvent(stream, ev[2 + k], 0));  // block i - 2 has read this bias buffer
+    for (int b = 0; b < B; ++b)
+      if (int e = launch_pair_bias(static_cast<const uint8_t*>(z) + size_t(b) * N * N * kD * zsz, zf32, w.attention.ln_z_w,
+                                   w.attention.ln_z_b, w.attention.w_z, bias[k] + size_t(b) * heads * N * Nk, N, N,
+                                   (long long)N * kD * zsz, (long long)kD * zsz, (long long)N * Nk, Nk, heads, stream))
+        return e;
+    if (two) {
+      B200_CUDA(cudaEventRecord(ev[k], stream));
+      B200_CUDA(cudaStreamWaitEvent(side, ev[k], 0));
+    }
+    if (int e = apb_run(s, nullptr, bias[k], Nk, token_mask, s, &w.attention, B, 1, N, c_s, heads, s_dtype, B200_DTYPE_F32,
+                        true, side_workspace, side_bytes, side))
+      return e;
+    if (two) B200_CUDA(cudaEventRecord(ev[2 + k], side));
+    if (int e = swiglu_transition_(s, w.transition_s, int64_t(B) * N, c_s, sf32, static_cast<uint8_t*>(side_workspace), side))
+      return e;
+  }
+  if (two) {
+    B200_CUDA(cudaEventRecord(ev[4], side));
+    B200_CUDA(cudaStreamWaitEvent(stream, ev[4], 0));
+  }
   return B200_OK;
 }
 

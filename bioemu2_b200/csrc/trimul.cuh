@@ -25,6 +25,7 @@ struct TriMulInParams {
   const uint8_t* mask;     // non-zero = valid
   const float* ln_w;
   const float* ln_b;
+  long long z_copy_delta;  // byte distance from z to a tensor that receives a copy of it (0: none)
   __nv_bfloat16* a_out;    // [128][lines_alloc][pos_pitch]
   __nv_bfloat16* b_out;
   int n_lines, n_pos;
@@ -52,7 +53,9 @@ constexpr int THREADS = 512;  // warps 0-3 epilogue of a, 4-7 epilogue of b (the
 // thread at 96 registers, which the LayerNorm producers spill at.  So there is no control warp: the first
 // thread of each epilogue group issues the two products of its own half (whose accumulators it has just
 // drained), and shared stage x is released when both have committed.
-template <bool F32>
+// COPY: the producers also store the raw rows at z_copy_delta from their source.  The first op of a stack that leaves its
+// input alone gets its working copy this way, for the write alone (N = 384: 26 us as a copy of its own before the stack).
+template <bool F32, bool COPY>
 __global__ void __launch_bounds__(512, 1)
 trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
                  const __grid_constant__ CUtensorMap tmB, TriMulInParams p) {
@@ -111,7 +114,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             const int pos = pos0 + r;
             return pos < p.n_pos ? base + pos * pos_stride : nullptr;
           },
-          gamma, beta, p.eps);
+          gamma, beta, p.eps, 1.0f, COPY ? p.z_copy_delta : 0);
       if (pt < 128) {
         const int pos = pos0 + pt;
         mreg = (pos < p.n_pos) ? p.mask[line * mline_stride + pos * mpos_stride] : 0;

@@ -7,6 +7,7 @@ modules do, before anything is launched.
 from __future__ import annotations
 
 import ctypes
+import threading
 
 import torch
 from torch import Tensor
@@ -14,7 +15,15 @@ from torch import Tensor
 from . import _lib
 from ._lib import lib
 
-_WORKSPACES: dict[tuple[int, int], Tensor] = {}
+class _Workspaces(threading.local):
+    """Scratch buffers of one host thread by (device, stream): kernels of two threads on one stream may interleave, so
+    threads do not share a buffer."""
+
+    def __init__(self) -> None:
+        self.buffers: dict[tuple[int, int], Tensor] = {}
+
+
+_WORKSPACES = _Workspaces()
 
 
 def _stream() -> int:
@@ -22,18 +31,19 @@ def _stream() -> int:
 
 
 def workspace(nbytes: int, device: torch.device) -> Tensor:
-    """Scratch buffer shared by all ops on (device, stream); grown on demand, 1024-byte aligned."""
+    """Scratch buffer shared by all ops of this thread on (device, stream); grown on demand, 1024-byte aligned."""
     key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
-    buf = _WORKSPACES.get(key)
+    buf = _WORKSPACES.buffers.get(key)
     if buf is None or buf.numel() < nbytes + 1024:
         buf = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
-        _WORKSPACES[key] = buf
+        _WORKSPACES.buffers[key] = buf
     off = (-buf.data_ptr()) % 1024
     return buf[off:off + nbytes]
 
 
 def release_workspaces() -> None:
-    _WORKSPACES.clear()
+    """Drops this thread's scratch buffers."""
+    _WORKSPACES.buffers.clear()
 
 
 def _zdtype(t: Tensor) -> int:
@@ -152,6 +162,7 @@ class TransitionPacked:
         self.w3 = fc3.to(bf).contiguous()
         self.norm_w = norm_w.detach().float().contiguous() if norm_w is not None else None
         self.norm_b = norm_b.detach().float().contiguous() if norm_b is not None else None
+        self.struct = _lib.TransitionWeights(self.w13.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b))
 
 
 def transition(x: Tensor, w: TransitionPacked, add_residual: bool = False, out: Tensor | None = None) -> Tensor:
@@ -529,7 +540,10 @@ class TransitionGenericPacked:
         bf = torch.bfloat16
         self.w12 = torch.cat([fc1.detach(), fc2.detach()], dim=0).to(bf).contiguous()
         self.w3 = fc3.detach().to(bf).contiguous()
-        self.norm_w, self.norm_b = norm_w, norm_b
+        self.norm_w = norm_w.detach().float().contiguous() if norm_w is not None else None
+        self.norm_b = norm_b.detach().float().contiguous() if norm_b is not None else None
+        self.struct = _lib.SwigluWeights(self.w12.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b),
+                                         fc1.shape[0])
         if fc1.shape[0] % 8 or fc1.shape[1] % 8 or fc3.shape[0] % 8 or fc1.shape[1] > 1024:
             raise ValueError("transition widths must be multiples of 8 and the input width at most 1024")
 
@@ -579,6 +593,49 @@ def attention_core(q: Tensor, k: Tensor, v: Tensor, bias: Tensor, key_mask: Tens
         N, H, Bt)
     _lib.check(lib.b200_attention_core_fwd(ctypes.byref(a), _stream()))
     return out.view(Bt, N, H, dh)
+
+
+# ----------------------------------------------------------------------------------- trunk stack
+class TrunkPacked:
+    """The weights of a stack of trunk blocks as the array ``b200_trunk_fwd`` takes; keeps the packed copies alive."""
+
+    def __init__(self, blocks) -> None:
+        """``blocks``: per block a dict of packed weights under the names of ``_lib.TrunkBlock``; absent parts are left out."""
+        self.keep = blocks
+        self.n = len(blocks)
+        self.array = (_lib.TrunkBlock * self.n)(*[_lib.TrunkBlock(**{k: v.struct for k, v in b.items()}) for b in blocks])
+
+
+def trunk_(z_in: Tensor, z: Tensor, s: Tensor | None, token_mask: Tensor | None, pair_mask: Tensor | None, w: TrunkPacked,
+           heads: int = 0, side: torch.cuda.Stream | None = None) -> None:
+    """Runs the stack: ``z_in[B,N,N,128]`` -> ``z`` (may be ``z_in``), ``s[B,N,c_s]`` in place (``None``: no single track).
+    ``pair_mask=None``: the outer product of ``token_mask``."""
+    _require_cuda(z_in, z)
+    B, N = z.shape[0], z.shape[1]
+    if tuple(z.shape) != (B, N, N, 128) or z_in.shape != z.shape or z_in.dtype != z.dtype:
+        raise ValueError(f"expected z[B,N,N,128], got {tuple(z_in.shape)} -> {tuple(z.shape)}")
+    if not z.is_contiguous() or not z_in.is_contiguous() or (s is not None and not s.is_contiguous()):
+        raise ValueError("the trunk updates contiguous tensors")
+    if token_mask is not None and tuple(token_mask.shape) != (B, N):
+        raise ValueError(f"token mask shape {tuple(token_mask.shape)} does not match z {tuple(z.shape)}")
+    if pair_mask is not None and tuple(pair_mask.shape) != (B, N, N):
+        raise ValueError(f"pair mask shape {tuple(pair_mask.shape)} does not match z {tuple(z.shape)}")
+    if s is not None and (s.ndim != 3 or s.shape[0] != B or s.shape[1] != N):
+        raise ValueError(f"s {tuple(s.shape)} does not match z {tuple(z.shape)}")
+    zd = _zdtype(z)
+    sd = _zdtype(s) if s is not None else 0
+    if z.numel() == 0:
+        return
+    c_s = s.shape[2] if s is not None else 0
+    tm = mask_u8(token_mask) if token_mask is not None else None
+    pm = mask_u8(pair_mask) if pair_mask is not None else None
+    nbytes = lib.b200_trunk_workspace_bytes(w.array, B, N, heads)
+    sbytes = lib.b200_trunk_side_workspace_bytes(w.array, w.n, B, N, c_s, heads)
+    # one buffer for both streams: the side stream has joined before the call returns to the current one
+    ws = workspace(nbytes + sbytes, z.device).data_ptr()
+    _lib.check(lib.b200_trunk_fwd(w.array, w.n, z_in.data_ptr(), z.data_ptr(), _ptr(s), _ptr(tm), _ptr(pm), B, N, c_s, heads,
+                                  sd, zd, ws, nbytes, ws + nbytes, sbytes, _stream(),
+                                  side.cuda_stream if side is not None else None))
 
 
 # ----------------------------------------------------------------------------------- staged triangle multiplication

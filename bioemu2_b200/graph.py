@@ -50,14 +50,10 @@ class GraphedTrunk:
 
     def _run(self) -> None:
         self.s_out.copy_(self.s_in)
-        self.z_out.copy_(self.z_in)
         if self.composite:
-            pm = (self.mask_in[:, :, None] & self.mask_in[:, None, :]).to(torch.uint8)
-            self.trunk.forward_(self.s_out, self.z_out, self.mask_in, pm)
+            self.trunk.forward_into(self.s_out, self.z_in, self.z_out, self.mask_in)
         else:
-            pm = self.mask_in.to(torch.uint8)
-            for layer in self.trunk.layers:
-                layer.forward_(self.z_out, pm)
+            self.trunk.forward_into(self.z_in, self.z_out, self.mask_in)
 
     def __call__(self, s: Tensor, z: Tensor, mask: Tensor | None = None) -> tuple[Tensor, Tensor]:
         """Same shapes and dtypes as at capture; ``mask=None`` keeps the captured mask.  Returns ``(s, z)`` in static

@@ -10,12 +10,12 @@ import torch
 import torch.nn as nn
 from torch import Tensor
 
-from . import _lib
+from . import _lib, precision
 from . import functional as F
 from .outer_product_mean import OuterProductMean
 from .pair_weighted_averaging import PairWeightedAveraging
 from .transition import Transition
-from .triangle_multiplication import TriangleMultiplication
+from .triangle_multiplication import PackedWeightsMixin, TriangleMultiplication
 
 
 class PairMixerLayer(nn.Module):
@@ -43,7 +43,7 @@ class PairMixerLayer(nn.Module):
         return z
 
 
-class PairMixerModule(nn.Module):
+class PairMixerModule(PackedWeightsMixin, nn.Module):
     def __init__(self, token_s: int, token_z: int, num_blocks: int, dropout: float = 0.25, trimul_variant=None,
                  trimul_tile_size: int | None = None, transition_chunk_size: int | None = None,
                  trimul_matmul_precision: str | None = None) -> None:
@@ -58,12 +58,26 @@ class PairMixerModule(nn.Module):
     def forward(self, s: Tensor, z: Tensor, pair_mask: Tensor) -> tuple[Tensor, Tensor]:
         if self.training:
             raise RuntimeError("bioemu2_b200 modules are inference-only: call .eval()")
-        z = z.clone()
-        mask8 = pair_mask.to(torch.uint8).contiguous()  # converted once for all layers
-        for layer in self.layers:
-            layer.forward_(z, mask8)
+        z = self.forward_into(z.contiguous(), torch.empty_like(z, memory_format=torch.contiguous_format), pair_mask)
         _lib.raise_if_device_wait()  # a kernel whose bounded wait ran out earlier in the stack invalidates the result
         return s, z
+
+    def _build_packed(self):
+        return F.TrunkPacked([{"tri_mul_out": m.tri_mul_out.packed(), "tri_mul_in": m.tri_mul_in.packed(),
+                               "transition_z": m.transition_z.packed()} for m in self.layers])
+
+    def forward_into(self, z_in: Tensor, z: Tensor, pair_mask: Tensor) -> Tensor:
+        """The block loop ``z_in`` -> ``z`` (contiguous; ``z`` may be ``z_in``) in one native call; returns ``z``."""
+        if len(self.layers) == 0 or precision.use_ieee(None, z) or any(
+                m.tri_mul_out.matmul_precision == "ieee" or m.tri_mul_in.matmul_precision == "ieee" for m in self.layers):
+            if z is not z_in:
+                z.copy_(z_in)
+            mask8 = F.mask_u8(pair_mask)
+            for layer in self.layers:
+                layer.forward_(z, mask8)
+            return z
+        F.trunk_(z_in, z, None, None, pair_mask, self.packed())
+        return z
 
     def graphed(self, s: Tensor, z: Tensor, pair_mask: Tensor):
         """The block loop captured in a CUDA graph for inputs of these shapes: ``g = trunk.graphed(s, z, pair_mask)``

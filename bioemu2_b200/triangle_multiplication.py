@@ -16,14 +16,48 @@ from . import functional as F
 from . import ieee, precision
 
 
+def _watch_list(module: nn.Module):
+    """Where a module tree keeps its parameters: (child dict, name, child) links and (parameter dict, name) slots."""
+    links, slots = [], []
+
+    def walk(m):
+        slots.extend((m._parameters, n) for n in m._parameters)
+        for n, c in m._modules.items():
+            links.append((m._modules, n, c))
+            if c is not None:
+                walk(c)
+
+    walk(module)
+    return links, slots
+
+
 class PackedWeightsMixin:
-    """Caches the bf16 kernel-layout copy of a module's parameters until one of them changes."""
+    """Caches the bf16 kernel-layout copy of a module's parameters until one of them changes.
+
+    The check runs on every forward, so it does not walk the module tree: it looks the parameters up through the
+    dictionaries that hold them (a replaced submodule or parameter is seen there) and compares storage address and
+    version counter -- addresses are unique over all devices."""
 
     _packed = None
     _packed_key = None
+    _watch = None
 
     def _pack_key(self):
-        return tuple((p.data_ptr(), p._version, str(p.device)) for p in self.parameters())
+        watch = self._watch
+        if watch is not None:
+            for d, n, c in watch[0]:
+                if d.get(n) is not c:
+                    watch = None
+                    break
+        if watch is None:
+            watch = self._watch = _watch_list(self)
+        key = []
+        for d, n in watch[1]:
+            p = d.get(n)
+            if p is not None:
+                key.append(p.data_ptr())
+                key.append(p._version)
+        return key
 
     def packed(self):
         key = self._pack_key()
@@ -38,7 +72,7 @@ class PackedWeightsMixin:
 
     def split_weights(self):
         """The (hi | lo | hi) split copies of the projection weights used by the fp32-accurate forms."""
-        key = tuple((p.data_ptr(), p._version, str(p.device)) for p in self.parameters())
+        key = self._pack_key()
         if self._split is None or key != self._split_key:
             with torch.no_grad():
                 self._split = self._build_split()

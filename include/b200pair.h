@@ -460,6 +460,55 @@ int b200_gate_rows_f32(const float* a, int64_t a_pitch, const float* b, int64_t 
 int b200_softmax_bias_f32(float* s, const float* bias, const uint8_t* keymask, int64_t groups, int n, int H, int bias_div,
                           b200_stream_t stream);
 
+/* ---------------------------------------------------------------------------------------------------
+ * A stack of trunk blocks in one call: PairMixerLayer (src/bioemu2/biomoa/modules/pairmixer.py:430-456) or the composite
+ * Pairformer block around it.  Per block, every step residual:
+ *   z: triangle multiplication outgoing, incoming [, triangle attention starting, ending], transition 128 -> 512 -> 128
+ *   s: [attention with pair bias from the block's final z, SwiGLU transition c_s -> hidden -> c_s]
+ * tri_att_start.w_o == NULL leaves the triangle attention out, attention.w_o == NULL (in block 0) the single track.
+ *
+ * z_in is read by the first block and may be z itself; otherwise it is left as it is and z needs no initial contents.
+ * s is updated in place.  pair_mask: uint8 [B][N][N], or NULL: token_mask[i] and token_mask[j].
+ * The single track of a block depends on the pair track only through the block's attention bias, so it runs on
+ * side_stream under the next block's pair track; both streams are joined before the call's last operation on `stream`.
+ * side_stream may be NULL (or equal to stream): one stream, same results.
+ *   b200_transition_weights  w13 bf16 [8][64 fc1 rows | 64 fc2 rows][128], w3 bf16 [128][512], LayerNorm fp32 [128]
+ *   b200_swiglu_weights      w12 bf16 [2*hidden][c_s] (fc1 rows, then fc2 rows), w3 bf16 [c_s][hidden], LayerNorm fp32 [c_s]
+ * Workspaces: 1024-byte aligned; the side one is for side_stream's kernels.
+ * ------------------------------------------------------------------------------------------------- */
+typedef struct {
+  const void* w13;
+  const void* w3;
+  const float* ln_w;
+  const float* ln_b;
+} b200_transition_weights;
+
+typedef struct {
+  const void* w12;
+  const void* w3;
+  const float* ln_w;
+  const float* ln_b;
+  int64_t hidden;
+} b200_swiglu_weights;
+
+typedef struct {
+  b200_trimul_weights tri_mul_out;
+  b200_trimul_weights tri_mul_in;
+  b200_triatt_weights tri_att_start;
+  b200_triatt_weights tri_att_end;
+  b200_transition_weights transition_z;
+  b200_apb_weights attention;
+  b200_swiglu_weights transition_s;
+} b200_trunk_block;
+
+size_t b200_trunk_workspace_bytes(const b200_trunk_block* blocks, int B, int N, int heads);
+size_t b200_trunk_side_workspace_bytes(const b200_trunk_block* blocks, int n_blocks, int B, int N, int c_s, int heads);
+
+int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_in, void* z, void* s,
+                   const uint8_t* token_mask, const uint8_t* pair_mask, int B, int N, int c_s, int heads, int s_dtype,
+                   int z_dtype, void* workspace, size_t workspace_bytes, void* side_workspace, size_t side_bytes,
+                   b200_stream_t stream, b200_stream_t side_stream);
+
 #ifdef __cplusplus
 }
 #endif
