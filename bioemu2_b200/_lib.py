@@ -6,7 +6,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int64, c_size_t, c_ulonglong, c_void_p
+from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_ulonglong, c_void_p
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 # BIOEMU2_B200_LIB points at an alternative build of the same library (profiling or experimental builds).
@@ -46,6 +46,14 @@ class ApbWeights(Structure):
 class TriAttWeights(Structure):
     _fields_ = [("w_qkgv", c_void_p), ("g_bias", c_void_p), ("w_b", c_void_p), ("w_o", c_void_p), ("ln_w", c_void_p),
                 ("ln_b", c_void_p)]
+
+
+class PackSegment(Structure):
+    _fields_ = [("src", c_void_p), ("dst_off", c_int64), ("groups", c_int32), ("group", c_int32), ("pitch", c_int32),
+                ("scale", c_float)]
+
+
+PACK_MAX = 24
 
 
 class TransitionWeights(Structure):
@@ -137,6 +145,7 @@ SIGNATURES = {
                                           c_int, c_int, c_int, c_void_p]),
     "b200_pair_outer_sum": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "b200_add_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_void_p]),
+    "b200_pack_bf16": (c_int, [POINTER(PackSegment), c_int, c_void_p, c_void_p]),
     "b200_trunk_workspace_bytes": (c_size_t, [POINTER(TrunkBlock), c_int, c_int, c_int]),
     "b200_trunk_side_workspace_bytes": (c_size_t, [POINTER(TrunkBlock), c_int, c_int, c_int, c_int, c_int]),
     "b200_trunk_fwd": (c_int, [POINTER(TrunkBlock), c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,

@@ -1,5 +1,6 @@
 // HBM-bound row kernels: 128-bit loads and stores, one warp per row, fp32 statistics.
 #pragma once
+#include "../../include/b200pair.h"
 #include "row_tile.cuh"
 
 namespace b200 {
@@ -198,6 +199,30 @@ add_rows_kernel(const float* x, const void* __restrict__ y, float* out, long lon
 #pragma unroll
     for (int e = 0; e < 8; ++e) fx[e] += fy[e];
     store8<true>(out + r * cols, v * 8, fx);
+  }
+}
+
+// Packed bf16 weights from fp32 parameters: blockIdx.y = segment, one thread per 8 destination elements.
+struct PackParams {
+  b200_pack_segment seg[B200_PACK_MAX];
+  __nv_bfloat16* dst;
+};
+__global__ void __launch_bounds__(256)
+pack_bf16_kernel(const __grid_constant__ PackParams p) {
+  pdl_wait();
+  const b200_pack_segment& s = p.seg[blockIdx.y];
+  const int total = s.groups * (s.pitch >> 3);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const int g = (t * 8) / s.pitch, r = t * 8 - g * s.pitch;
+    float x[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = 0.f;
+    if (s.src && r < s.group) {
+      load8<true>(s.src + (long long)g * s.group, r, x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] *= s.scale;
+    }
+    store8<false>(p.dst + s.dst_off, t * 8, x);
   }
 }
 

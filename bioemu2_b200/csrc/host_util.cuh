@@ -144,11 +144,11 @@ inline int set_smem_once(const void* kernel, uint32_t bytes) {
 // kernel before it in the stream have exited, so its launch latency and set-up (barriers, tensor-memory allocation,
 // descriptor prefetch) overlap the completion and memory flush of that kernel; see pdl_wait().
 template <class... Params, class... Args>
-inline int launch(void (*kernel)(Params...), int grid, int block, uint32_t smem, cudaStream_t stream, Args&&... args) {
+inline int launch(void (*kernel)(Params...), dim3 grid, int block, uint32_t smem, cudaStream_t stream, Args&&... args) {
   if (smem > 48 * 1024)
     if (int e = set_smem_once(reinterpret_cast<const void*>(kernel), smem)) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(grid));
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(unsigned(block));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

@@ -1429,6 +1429,28 @@ int b200_softmax_bias_f32(float* s, const float* bias, const uint8_t* keymask, i
   return B200_OK;
 }
 
+int b200_pack_bf16(const b200_pack_segment* segments, int n, void* dst, b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(segments && dst && n > 0 && n <= B200_PACK_MAX, "need 1..%d segments", B200_PACK_MAX);
+  B200_CHECK_ARG(aligned(dst, 16), "dst must be 16-byte aligned");
+  PackParams p;
+  p.dst = static_cast<__nv_bfloat16*>(dst);
+  int64_t most = 0;
+  for (int i = 0; i < n; ++i) {
+    const b200_pack_segment& s = segments[i];
+    B200_CHECK_ARG(s.groups >= 0 && s.group >= 0 && s.pitch > 0 && s.group <= s.pitch && s.group % 8 == 0 && s.pitch % 8 == 0 &&
+                       s.dst_off >= 0 && s.dst_off % 8 == 0 && int64_t(s.groups) * s.pitch < (int64_t(1) << 31),
+                   "segment %d: sizes and offsets must be multiples of 8", i);
+    B200_CHECK_ARG(aligned(s.src, 32), "segment %d: the source must be 32-byte aligned", i);
+    p.seg[i] = s;
+    if (int64_t(s.groups) * s.pitch > most) most = int64_t(s.groups) * s.pitch;
+  }
+  if (most == 0) return B200_OK;
+  B200_LAUNCH(pack_bf16_kernel, dim3(unsigned(grid_for(most / 8, 256)), unsigned(n)), 256, 0, static_cast<cudaStream_t>(stream), p);
+  g_launch_count.fetch_sub(1, std::memory_order_relaxed);  // preparation, not one of the kernels a forward counts
+  return B200_OK;
+}
+
 // ------------------------------------------------------------------------------------------------ trunk stack
 static size_t round_up_1k(size_t x) { return (x + 1023) / 1024 * 1024; }
 static bool has_triatt(const b200_trunk_block& w) { return w.tri_att_start.w_o != nullptr; }

@@ -27,7 +27,7 @@ _WORKSPACES = _Workspaces()
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # current_stream() builds an object per call
 
 
 def workspace(nbytes: int, device: torch.device) -> Tensor:
@@ -100,6 +100,39 @@ def bmm_nt(a: Tensor, b: Tensor, scale: float = 1.0) -> Tensor:
     return c
 
 
+class _Pack:
+    """Collects rows of fp32 parameters into one bf16 buffer in kernel layout, built by as few launches as possible.
+    ``add`` returns the element offset of what it added; ``build`` the buffer."""
+
+    def __init__(self) -> None:
+        self.parts, self.size = [], 0
+
+    def add(self, t: Tensor | None, scale: float = 1.0, groups: int = 1, pad_to: int = 0, count: int = 0) -> int:
+        """``t`` flattened; with ``groups`` every ``numel / groups`` elements are zero-padded to ``pad_to`` elements;
+        ``t=None``: ``count`` zeros."""
+        group = 0 if t is None else t.numel() // groups
+        pitch = pad_to or group or count
+        off = self.size
+        self.parts.append((t, off, groups, group, pitch, scale))
+        self.size += groups * pitch
+        return off
+
+    def build(self, device: torch.device) -> Tensor:
+        out = torch.empty(self.size, dtype=torch.bfloat16, device=device)
+        keep, segs = [], []
+        for t, off, groups, group, pitch, scale in self.parts:
+            if t is not None:
+                t = t.detach()
+                if t.dtype != torch.float32 or not t.is_contiguous() or t.data_ptr() % 32:
+                    t = t.to(torch.float32).contiguous().clone() if t.data_ptr() % 32 else t.to(torch.float32).contiguous()
+                keep.append(t)
+            segs.append(_lib.PackSegment(_ptr(t), off, groups, group, pitch, scale))
+        for i in range(0, len(segs), _lib.PACK_MAX):
+            part = segs[i:i + _lib.PACK_MAX]
+            _lib.check(lib.b200_pack_bf16((_lib.PackSegment * len(part))(*part), len(part), out.data_ptr(), _stream()))
+        return out
+
+
 class TriMulPacked:
     """Device copies of the triangle-multiplication weights in the layouts ``b200_trimul_fwd`` expects."""
 
@@ -107,9 +140,11 @@ class TriMulPacked:
         D = p_out.shape[0]
         if D != 128 or tuple(p_in.shape) != (256, 128):
             raise ValueError("the triangle-multiplication kernels are built for dim=128")
-        bf = torch.bfloat16
-        self.w_in = torch.cat([p_in[:D], g_in[:D], p_in[D:], g_in[D:]], dim=0).to(bf).contiguous()
-        self.w_out = torch.cat([p_out, g_out], dim=0).to(bf).contiguous()
+        pk = _Pack()
+        for t in (p_in[:D], g_in[:D], p_in[D:], g_in[D:], p_out, g_out):
+            pk.add(t)
+        buf = pk.build(p_out.device).view(-1, 128)
+        self.w_in, self.w_out = buf[:4 * D], buf[4 * D:]
         self.ln = [t.detach().float().contiguous() for t in (norm_in_w, norm_in_b, norm_out_w, norm_out_b)]
         self.struct = _lib.TriMulWeights(self.w_in.data_ptr(), self.w_out.data_ptr(), *[t.data_ptr() for t in self.ln])
 
@@ -152,14 +187,17 @@ class TransitionPacked:
         hidden = fc1.shape[0]
         if fc1.shape[1] != 128 or tuple(fc2.shape) != tuple(fc1.shape) or tuple(fc3.shape) != (128, hidden) or hidden > 512:
             raise ValueError("the fused pair-transition kernel is built for dim=128, hidden<=512")
-        if hidden < 512:
-            pad = torch.zeros(512 - hidden, 128, dtype=fc1.dtype, device=fc1.device)
-            fc1, fc2 = torch.cat([fc1.detach(), pad]), torch.cat([fc2.detach(), pad])
-            fc3 = torch.cat([fc3.detach(), pad.t()], dim=1)
-        bf = torch.bfloat16
-        w13 = torch.cat([fc1.reshape(8, 64, 128), fc2.reshape(8, 64, 128)], dim=1)  # [8][128][128]
-        self.w13 = w13.reshape(1024, 128).to(bf).contiguous()
-        self.w3 = fc3.to(bf).contiguous()
+        pk = _Pack()
+        for c in range(0, 512, 64):  # 8 chunks of [64 fc1 rows | 64 fc2 rows]
+            for fc in (fc1, fc2):
+                rows = fc[min(c, hidden):min(c + 64, hidden)]
+                if rows.shape[0]:
+                    pk.add(rows, pad_to=64 * 128)
+                else:
+                    pk.add(None, count=64 * 128)
+        pk.add(fc3, groups=128, pad_to=512)
+        buf = pk.build(fc3.device)
+        self.w13, self.w3 = buf[:1024 * 128].view(1024, 128), buf[1024 * 128:].view(128, 512)
         self.norm_w = norm_w.detach().float().contiguous() if norm_w is not None else None
         self.norm_b = norm_b.detach().float().contiguous() if norm_b is not None else None
         self.struct = _lib.TransitionWeights(self.w13.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b))
@@ -255,26 +293,26 @@ class ApbPacked:
             raise ValueError("pair-bias attention needs H <= 16 and a head dim that is a multiple of 8 and <= 64")
         DH = 32 if dh <= 32 else 64
         self.c_s, self.H = c_s, H
-        bf = torch.bfloat16
-        wq, wk, wv = proj_qkv.detach().float().chunk(3, dim=0)
         qscale = LOG2E / (dh ** 0.5)
-        self.w_qkg = torch.cat([_pad_heads(wq * qscale, H, dh, DH), _pad_heads(wk, H, dh, DH),
-                                proj_g.detach().float()], dim=0).to(bf).contiguous()
+        pk = _Pack()
+        for i, scale in enumerate((qscale, 1.0)):
+            pk.add(proj_qkv[i * c_s:(i + 1) * c_s], scale, groups=H, pad_to=DH * c_s)
+        pk.add(proj_g)
+        v0 = pk.add(proj_qkv[2 * c_s:], groups=H, pad_to=DH * c_s)
+        z0 = pk.add(proj_z, pad_to=16 * 128)
+        o0 = pk.add(proj_o)
+        buf = pk.build(proj_o.device)
+        self.w_qkg, self.w_v = buf[:v0].view(-1, c_s), buf[v0:z0].view(-1, c_s)
+        self.w_z, self.w_o = buf[z0:o0].view(16, 128), buf[o0:].view(c_s, c_s)
         b = torch.zeros(2 * H * DH + c_s, dtype=torch.float32, device=proj_qkv.device)
         b[: H * DH] = _pad_heads(proj_q_bias.detach().float() * qscale, H, dh, DH)
         self.b_qkg = b
-        self.w_v = _pad_heads(wv, H, dh, DH).to(bf).contiguous()
-        wz = torch.zeros(16, 128, dtype=torch.float32, device=proj_z.device)
-        wz[:H] = proj_z.detach().float()
-        self.w_z = wz.to(bf).contiguous()
         self.ln_z_w = norm_z_w.detach().float().contiguous()
         self.ln_z_b = norm_z_b.detach().float().contiguous() if norm_z_b is not None else None
         self.ln_s_w = norm_s_w.detach().float().contiguous() if norm_s_w is not None else None
         self.ln_s_b = norm_s_b.detach().float().contiguous() if norm_s_b is not None else None
-        self.w_o = proj_o.detach().to(bf).contiguous()
-        ptr = lambda t: t.data_ptr() if t is not None else None  # noqa: E731
-        self.struct = _lib.ApbWeights(ptr(self.w_qkg), ptr(self.b_qkg), ptr(self.w_v), ptr(self.w_z), ptr(self.ln_z_w),
-                                      ptr(self.ln_z_b), ptr(self.ln_s_w), ptr(self.ln_s_b), ptr(self.w_o))
+        self.struct = _lib.ApbWeights(_ptr(self.w_qkg), _ptr(self.b_qkg), _ptr(self.w_v), _ptr(self.w_z), _ptr(self.ln_z_w),
+                                      _ptr(self.ln_z_b), _ptr(self.ln_s_w), _ptr(self.ln_s_b), _ptr(self.w_o))
 
 
 def attention_pair_bias(s: Tensor, z: Tensor, mask: Tensor, w: ApbPacked, multiplicity: int = 1) -> Tensor:
@@ -306,14 +344,14 @@ class TriAttPacked:
     def __init__(self, ln_w, ln_b, wq, wk, wv, wb, wg, bg, wo):
         if tuple(wq.shape) != (128, 128) or tuple(wb.shape) != (4, 128) or tuple(wo.shape) != (128, 128):
             raise ValueError("triangle attention is built for dim=128, 4 heads of 32")
-        bf = torch.bfloat16
-        qscale = LOG2E / (32 ** 0.5)
-        self.w_qkgv = torch.cat([wq.detach().float() * qscale, wk.detach().float(), wg.detach().float(),
-                                 wv.detach().float()], dim=0).to(bf).contiguous()
-        wb16 = torch.zeros(16, 128, dtype=torch.float32, device=wb.device)
-        wb16[:4] = wb.detach().float()
-        self.w_b = wb16.to(bf).contiguous()
-        self.w_o = wo.detach().to(bf).contiguous()
+        pk = _Pack()
+        pk.add(wq, scale=LOG2E / (32 ** 0.5))
+        for t in (wk, wg, wv):
+            pk.add(t)
+        pk.add(wb, pad_to=16 * 128)
+        pk.add(wo)
+        buf = pk.build(wo.device).view(-1, 128)
+        self.w_qkgv, self.w_b, self.w_o = buf[:512], buf[512:528], buf[528:]
         self.f32 = [t.detach().float().contiguous() for t in (bg, ln_w, ln_b)]
         self.struct = _lib.TriAttWeights(self.w_qkgv.data_ptr(), self.f32[0].data_ptr(), self.w_b.data_ptr(),
                                          self.w_o.data_ptr(), self.f32[1].data_ptr(), self.f32[2].data_ptr())
@@ -537,15 +575,18 @@ class TransitionGenericPacked:
     """Weights of a SwiGLU transition of any width (multiples of 8): ``w12 = [fc1; fc2]``, ``w3``."""
 
     def __init__(self, norm_w, norm_b, fc1, fc2, fc3):
-        bf = torch.bfloat16
-        self.w12 = torch.cat([fc1.detach(), fc2.detach()], dim=0).to(bf).contiguous()
-        self.w3 = fc3.detach().to(bf).contiguous()
+        if fc1.shape[0] % 8 or fc1.shape[1] % 8 or fc3.shape[0] % 8 or fc1.shape[1] > 1024:
+            raise ValueError("transition widths must be multiples of 8 and the input width at most 1024")
+        pk = _Pack()
+        pk.add(fc1)
+        pk.add(fc2)
+        o3 = pk.add(fc3)
+        buf = pk.build(fc3.device)
+        self.w12, self.w3 = buf[:o3].view(-1, fc1.shape[1]), buf[o3:].view(fc3.shape)
         self.norm_w = norm_w.detach().float().contiguous() if norm_w is not None else None
         self.norm_b = norm_b.detach().float().contiguous() if norm_b is not None else None
         self.struct = _lib.SwigluWeights(self.w12.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b),
                                          fc1.shape[0])
-        if fc1.shape[0] % 8 or fc1.shape[1] % 8 or fc3.shape[0] % 8 or fc1.shape[1] > 1024:
-            raise ValueError("transition widths must be multiples of 8 and the input width at most 1024")
 
 
 def transition_generic(x: Tensor, w: TransitionGenericPacked, add_residual: bool = False,
@@ -604,6 +645,17 @@ class TrunkPacked:
         self.keep = blocks
         self.n = len(blocks)
         self.array = (_lib.TrunkBlock * self.n)(*[_lib.TrunkBlock(**{k: v.struct for k, v in b.items()}) for b in blocks])
+
+
+def trunk_blocks_(z_in: Tensor, z: Tensor, s: Tensor | None, token_mask: Tensor | None, pair_mask: Tensor | None, pack, n: int,
+                  heads: int = 0, side: torch.cuda.Stream | None = None) -> TrunkPacked:
+    """``trunk_`` for a stack whose weights are not packed yet: block ``i`` (``pack(i)``) is packed on the host while the GPU
+    runs the blocks before it.  Returns the packed stack for the next call."""
+    blocks = []
+    for i in range(n):
+        blocks.append(pack(i))
+        trunk_(z_in if i == 0 else z, z, s, token_mask, pair_mask, TrunkPacked(blocks[-1:]), heads, side)
+    return TrunkPacked(blocks)
 
 
 def trunk_(z_in: Tensor, z: Tensor, s: Tensor | None, token_mask: Tensor | None, pair_mask: Tensor | None, w: TrunkPacked,

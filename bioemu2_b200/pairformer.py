@@ -60,11 +60,12 @@ class PairformerModule(PackedWeightsMixin, nn.Module):
         self.num_blocks = num_blocks
         self.layers = nn.ModuleList([PairformerBlock(token_s, token_z, **block_kwargs) for _ in range(num_blocks)])
 
-    def _build_packed(self):
-        return F.TrunkPacked([{"tri_mul_out": m.tri_mul_out.packed(), "tri_mul_in": m.tri_mul_in.packed(),
-                               "tri_att_start": m.tri_att_start.packed(), "tri_att_end": m.tri_att_end.packed(),
-                               "transition_z": m.transition_z.packed(), "attention": m.attention.packed(),
-                               "transition_s": m.transition_s.packed()} for m in self.layers])
+    def _pack_block(self, i: int) -> dict:
+        m = self.layers[i]
+        return {"tri_mul_out": m.tri_mul_out.packed(), "tri_mul_in": m.tri_mul_in.packed(),
+                "tri_att_start": m.tri_att_start.packed(), "tri_att_end": m.tri_att_end.packed(),
+                "transition_z": m.transition_z.packed(), "attention": m.attention.packed(),
+                "transition_s": m.transition_s.packed()}
 
     def forward(self, s: Tensor, z: Tensor, token_mask: Tensor) -> tuple[Tensor, Tensor]:
         if self.training:
@@ -106,7 +107,17 @@ class PairformerModule(PackedWeightsMixin, nn.Module):
             if self._side is None or self._side.device != z.device:
                 self._side = torch.cuda.Stream(device=z.device)
             side = self._side
-        F.trunk_(z_in, z, s, token_mask, pair_mask_u8, self.packed(), self.layers[0].attention.num_heads, side)
+        heads = self.layers[0].attention.num_heads
+        done = False
+
+        def first_run():
+            nonlocal done
+            done = True
+            return F.trunk_blocks_(z_in, z, s, token_mask, pair_mask_u8, self._pack_block, len(self.layers), heads, side)
+
+        w = self.packed(first_run)
+        if not done:
+            F.trunk_(z_in, z, s, token_mask, pair_mask_u8, w, heads, side)
         return z
 
     _side = None

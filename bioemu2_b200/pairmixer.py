@@ -62,9 +62,10 @@ class PairMixerModule(PackedWeightsMixin, nn.Module):
         _lib.raise_if_device_wait()  # a kernel whose bounded wait ran out earlier in the stack invalidates the result
         return s, z
 
-    def _build_packed(self):
-        return F.TrunkPacked([{"tri_mul_out": m.tri_mul_out.packed(), "tri_mul_in": m.tri_mul_in.packed(),
-                               "transition_z": m.transition_z.packed()} for m in self.layers])
+    def _pack_block(self, i: int) -> dict:
+        m = self.layers[i]
+        return {"tri_mul_out": m.tri_mul_out.packed(), "tri_mul_in": m.tri_mul_in.packed(),
+                "transition_z": m.transition_z.packed()}
 
     def forward_into(self, z_in: Tensor, z: Tensor, pair_mask: Tensor) -> Tensor:
         """The block loop ``z_in`` -> ``z`` (contiguous; ``z`` may be ``z_in``) in one native call; returns ``z``."""
@@ -76,7 +77,16 @@ class PairMixerModule(PackedWeightsMixin, nn.Module):
             for layer in self.layers:
                 layer.forward_(z, mask8)
             return z
-        F.trunk_(z_in, z, None, None, pair_mask, self.packed())
+        done = False
+
+        def first_run():
+            nonlocal done
+            done = True
+            return F.trunk_blocks_(z_in, z, None, None, pair_mask, self._pack_block, len(self.layers))
+
+        w = self.packed(first_run)
+        if not done:
+            F.trunk_(z_in, z, None, None, pair_mask, w)
         return z
 
     def graphed(self, s: Tensor, z: Tensor, pair_mask: Tensor):

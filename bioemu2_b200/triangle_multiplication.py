@@ -59,11 +59,12 @@ class PackedWeightsMixin:
                 key.append(p._version)
         return key
 
-    def packed(self):
+    def packed(self, build=None):
+        """The packed copy; ``build`` replaces ``_build_packed`` when it has to be made anew."""
         key = self._pack_key()
         if self._packed is None or key != self._packed_key:
             with torch.no_grad():
-                self._packed = self._build_packed()
+                self._packed = self._build_packed() if build is None else build()
             self._packed_key = key
         return self._packed
 

@@ -65,7 +65,7 @@ int b200_device_status(int* status);
  * a collective, at the end of a forward). */
 int b200_peek_status(int* status);
 
-/* Number of kernels this library has launched since it was loaded (all threads, all devices). */
+/* Number of kernels this library has launched since it was loaded (all threads, all devices; weight packing not counted). */
 unsigned long long b200_launch_count(void);
 
 /* ---------------------------------------------------------------------------------------------------
@@ -459,6 +459,21 @@ int b200_gate_rows_f32(const float* a, int64_t a_pitch, const float* b, int64_t 
                        float* out, int64_t rows, int cols, int mode, b200_stream_t stream);
 int b200_softmax_bias_f32(float* s, const float* bias, const uint8_t* keymask, int64_t groups, int n, int H, int bias_div,
                           b200_stream_t stream);
+
+/* ---------------------------------------------------------------------------------------------------
+ * Builds bf16 kernel-layout weights from fp32 parameters in one launch: segment k writes groups * pitch elements at
+ * dst + dst_off, taking `group` source elements times scale per group (src contiguous) and zeros in the rest of the pitch
+ * (src == NULL: zeros only).  At most B200_PACK_MAX segments; counts and offsets are multiples of 8 elements.
+ * ------------------------------------------------------------------------------------------------- */
+#define B200_PACK_MAX 24
+typedef struct {
+  const float* src;
+  int64_t dst_off;
+  int32_t groups, group, pitch;
+  float scale;
+} b200_pack_segment;
+
+int b200_pack_bf16(const b200_pack_segment* segments, int n, void* dst, b200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------------
  * A stack of trunk blocks in one call: PairMixerLayer (src/bioemu2/biomoa/modules/pairmixer.py:430-456) or the composite
