@@ -54,6 +54,7 @@ struct FlashParams {
   int q_col0, k_col0, v_row0;
   int nqt, nkt;         // query tiles, key tiles (nkt <= FlashCfg::MAX_T)
   int nqg;              // query-tile groups per (b, h): ceil(nqt / G)
+  int npairs;           // flash_resident_kernel: passes per (bias group, head, query tile), ceil(bias_div / G)
   int total_work;
 };
 
@@ -126,7 +127,7 @@ flash_core_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   //   word t*8 + 4 + w  bit j <=> key t*128 + 32*w + j exists
   uint32_t* mask_bits = reinterpret_cast<uint32_t*>(smem + Cfg::MASK_OFF);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   constexpr int kLoaderWarp = 8 * G;
   constexpr int kMmaWarp = 8 * G + 1;     // issues for group 0; group 1 (if any) has its own issuing warp, 8 * G + 3

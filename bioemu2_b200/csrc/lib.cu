@@ -12,6 +12,7 @@
 #include "elementwise.cuh"
 #include "opm.cuh"
 #include "attention.cuh"
+#include "attention_resident.cuh"
 #include "pair_bias.cuh"
 #include "triatt.cuh"
 #include "window_attention.cuh"
@@ -158,32 +159,37 @@ struct FlashLaunch {
   FlashParams p;
 };
 
-template <int DH, int G>
-static int launch_flash_t(const FlashLaunch& a, cudaStream_t stream) {
-  using Cfg = FlashCfg<DH, G>;
-  const FlashParams& p0 = a.p;
-  CUtensorMap tmQ, tmV, tmB;
+// Tensor maps of the attention operands: Q / K tiles of DH columns, V^T tiles of v_rows rows, bias tiles.
+static int flash_maps(const FlashLaunch& a, int DH, int v_rows, CUtensorMap* tmQ, CUtensorMap* tmV, CUtensorMap* tmB) {
+  const FlashParams& p = a.p;
   {
-    const uint64_t dims[3] = {uint64_t(a.qk_width), uint64_t(p0.N), uint64_t(p0.Bt)};
+    const uint64_t dims[3] = {uint64_t(a.qk_width), uint64_t(p.N), uint64_t(p.Bt)};
     const uint64_t str[2] = {uint64_t(a.qk_width) * 2, uint64_t(a.qk_b_stride) * 2};
     const uint32_t box[3] = {uint32_t(DH), 128, 1};
-    if (int e = make_tmap_bf16(&tmQ, a.qk, 3, dims, str, box,
-                               DH == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B))
+    if (int e = make_tmap_bf16(tmQ, a.qk, 3, dims, str, box, DH == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B))
       return e;
   }
   {
-    const uint64_t dims[3] = {uint64_t(p0.N), uint64_t(p0.H) * DH, uint64_t(p0.Bt)};
-    const uint64_t str[2] = {uint64_t(a.v_pitch) * 2, uint64_t(a.v_pitch) * p0.H * DH * 2};
-    const uint32_t box[3] = {64, uint32_t(DH), 1};
-    if (int e = make_tmap_bf16(&tmV, a.vT, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+    const uint64_t dims[3] = {uint64_t(p.N), uint64_t(p.H) * DH, uint64_t(p.Bt)};
+    const uint64_t str[2] = {uint64_t(a.v_pitch) * 2, uint64_t(a.v_pitch) * p.H * DH * 2};
+    const uint32_t box[3] = {64, uint32_t(v_rows), 1};
+    if (int e = make_tmap_bf16(tmV, a.vT, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   {
-    const uint64_t dims[3] = {uint64_t(p0.N), uint64_t(p0.N), uint64_t(a.bias_groups) * p0.H};
-    const uint64_t str[2] = {uint64_t(a.bias_pitch) * 2, uint64_t(a.bias_pitch) * p0.N * 2};
+    const uint64_t dims[3] = {uint64_t(p.N), uint64_t(p.N), uint64_t(a.bias_groups) * p.H};
+    const uint64_t str[2] = {uint64_t(a.bias_pitch) * 2, uint64_t(a.bias_pitch) * p.N * 2};
     const uint32_t box[3] = {64, 128, 1};
-    if (int e = make_tmap_bf16(&tmB, a.bias, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+    if (int e = make_tmap_bf16(tmB, a.bias, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
-  FlashParams p = p0;
+  return 0;
+}
+
+template <int DH, int G>
+static int launch_flash_core(const FlashLaunch& a, cudaStream_t stream) {
+  using Cfg = FlashCfg<DH, G>;
+  CUtensorMap tmQ, tmV, tmB;
+  if (int e = flash_maps(a, DH, DH, &tmQ, &tmV, &tmB)) return e;
+  FlashParams p = a.p;
   p.nqt = (p.N + 127) / 128;
   p.nkt = (p.N + 127) / 128;
   if (p.nkt > Cfg::MAX_T)
@@ -195,8 +201,30 @@ static int launch_flash_t(const FlashLaunch& a, cudaStream_t stream) {
   return 0;
 }
 
+template <int DH, int VR, int G>
+static int launch_flash_resident(const FlashLaunch& a, cudaStream_t stream) {
+  using Cfg = FlashResidentCfg<DH, VR, G>;
+  CUtensorMap tmQ, tmV, tmB;
+  if (int e = flash_maps(a, DH, VR, &tmQ, &tmV, &tmB)) return e;
+  FlashParams p = a.p;
+  p.nqt = (p.N + 127) / 128;
+  p.nkt = (p.N + 127) / 128;
+  p.npairs = (p.bias_div + G - 1) / G;
+  p.total_work = (p.Bt + p.bias_div - 1) / p.bias_div * p.H * p.nqt * p.npairs;
+  const int grid = p.total_work < sm_count() ? p.total_work : sm_count();
+  B200_LAUNCH((flash_resident_kernel<DH, VR, G>), grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, tmQ, tmV, tmB, p);
+  return 0;
+}
+
+// Rows whose bias row block stays in shared memory go to flash_resident_kernel, longer ones to flash_core_kernel (why the
+// line lies there: attention_resident.cuh).  A head of 64 columns with more than 48 of them in use does not leave room for
+// two groups in tensor memory, nor, with the bias block, in shared memory.
 static int launch_flash(const FlashLaunch& a, int DH, cudaStream_t stream) {
-  return DH == 32 ? launch_flash_t<32, 2>(a, stream) : launch_flash_t<64, 1>(a, stream);
+  const int tiles = (a.p.N + 127) / 128;
+  if (DH == 32)
+    return tiles <= FlashResidentCfg<32, 32, 2>::NB ? launch_flash_resident<32, 32, 2>(a, stream) : launch_flash_core<32, 2>(a, stream);
+  if (a.p.dh_out <= 48 && tiles <= FlashResidentCfg<64, 48, 2>::NB) return launch_flash_resident<64, 48, 2>(a, stream);
+  return launch_flash_core<64, 1>(a, stream);
 }
 
 static int launch_pair_bias(const void* z, bool f32, const float* ln_w, const float* ln_b, const void* w_z,

@@ -53,7 +53,7 @@ opm_proj_kernel(const __grid_constant__ CUtensorMap tmW, OpmProjParams p) {
   uint64_t* acc_empty = acc_full + 2;  // [2] count 128
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int tiles_per_tok = (p.S + 127) >> 7;
 

@@ -43,7 +43,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmW, PairBiasParams p) {
   uint64_t* acc_full = x_empty + 2;
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int tiles_per_row = (p.n_pos + 127) >> 7;
 

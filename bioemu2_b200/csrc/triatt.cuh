@@ -55,16 +55,7 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   using namespace triatt_proj;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
-  if (smem_u32(smem) & 1023u) {  // the swizzled tiles need the alignment; there is no room to round up
-    if (threadIdx.x == 0 && atomicCAS(&g_dev_status, 0, kDevWaitTimeout | (99 << 8)) == 0) {
-      int* hp = g_host_status_ptr;
-      if (hp) {
-        *reinterpret_cast<volatile int*>(hp) = kDevWaitTimeout | (99 << 8);
-        __threadfence_system();
-      }
-    }
-    return;
-  }
+  if (smem_misaligned(smem)) return;  // the swizzled tiles need the alignment; there is no room to round up
   uint64_t* w_full = reinterpret_cast<uint64_t*>(smem + BAR_OFF);
   uint64_t* x_full = w_full + 1;     // [2] count 256
   uint64_t* x_empty = x_full + 2;    // [2] commit
@@ -76,7 +67,7 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const bool fuse_bias = p.tri_bias != nullptr;
   float* gb_s = reinterpret_cast<float*>(smem + GB_OFF);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int tiles_per_line = (p.n_pos + 127) >> 7;
 

@@ -71,7 +71,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   uint8_t* mask_s = smem + MASK_OFF;
   uint8_t* flag_s = smem + FLAG_OFF;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int tiles_per_line = p.pos_pitch >> 7;
 
@@ -293,7 +293,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   float* ln_s = reinterpret_cast<float*>(smem + LN_OFF);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int tiles_per_line = p.pos_pitch >> 7;
 

@@ -37,6 +37,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // 5.84 with the implicit one at kernel end; N = 384 PairMixer: 1.25 / 1.31 / 1.21 ms).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The warp's index in its block, as a value the compiler knows to be the same in all lanes: what is derived from it (roles,
+// descriptors, barrier addresses) then lives in uniform registers, which tcgen05.mma takes its operands from, instead of
+// being moved there lane by lane before every product.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
@@ -116,6 +121,21 @@ __device__ __noinline__ void mbar_wait_slow(uint64_t* bar, uint32_t parity, int 
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int site) {
   if (mbar_try_wait(bar, parity)) return;
   mbar_wait_slow(bar, parity, site);
+}
+
+// For kernels that fill the shared memory and cannot round their base up to the 1024 bytes of a swizzle atom: true, with
+// the status set, if the base is not aligned already.
+__device__ __forceinline__ bool smem_misaligned(const void* smem) {
+  if ((smem_u32(smem) & 1023u) == 0) return false;
+  const int code = kDevWaitTimeout | (99 << 8);
+  if (threadIdx.x == 0 && atomicCAS(&g_dev_status, 0, code) == 0) {
+    int* hp = g_host_status_ptr;
+    if (hp) {
+      *reinterpret_cast<volatile int*>(hp) = code;
+      __threadfence_system();
+    }
+  }
+  return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -297,6 +317,17 @@ __device__ __forceinline__ void tmem_st_32x16_f(uint32_t taddr, const float* v) 
       "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld_32x8_f(uint32_t taddr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x8_f(uint32_t taddr, const float* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
 // One fp32 column of 32 lanes (a per-row scalar kept in tensor memory).
 __device__ __forceinline__ float tmem_ld_32x1_f(uint32_t taddr) {
   float v;
@@ -315,6 +346,18 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&v
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
       ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
       "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+// 32 lanes x 32 32-bit columns from registers into TMEM.
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+      "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]),
+      "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]),
+      "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
 }
 // 32 lanes x 32 fp32 columns from registers into TMEM.

@@ -1,0 +1,33 @@
+"""The attention core at the edges of its two kernels: tile and row-block boundaries, an odd number of lines, and logits far
+outside the range in which a row's softmax reference stays put; against a plain fp32 softmax."""
+import pytest
+import torch
+
+from gpu_util import assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dh", [32, 48])
+@pytest.mark.parametrize("N,lines,scale", [(1, 1, 1.0), (7, 3, 1.0), (127, 2, 1.0), (128, 3, 40.0), (129, 5, 1.0), (256, 3, 1.0),
+                                           (257, 2, 40.0), (300, 3, 100.0), (512, 3, 1.0), (513, 2, 1.0)])
+def test_attention_core_edges(N, lines, scale, dh):
+    from bioemu2_b200 import _lib
+    from bioemu2_b200 import functional as F
+
+    g = torch.Generator().manual_seed(1000 + N)
+    H = 2
+    q, k, v = (torch.randn(lines, N, H, dh, generator=g).bfloat16() for _ in range(3))
+    bias = scale * torch.randn(1, H, N, N, generator=g)
+    if scale > 1:  # the maximum of a row grows from key tile to key tile
+        bias += scale * torch.arange(N)[None, None, None, :] / 64
+    mask = torch.rand(lines, N, generator=g) > 0.2
+    mask[-1] = False                      # a line without a valid key averages over all keys
+    bias_bf = (bias * F.LOG2E).bfloat16().float() / F.LOG2E   # the kernel takes the bias in bf16, base 2
+    qs = (q.float() * (F.LOG2E / dh ** 0.5)).bfloat16().float() / F.LOG2E
+    logits = torch.einsum("bqhd,bkhd->bhqk", qs, k.float()) + bias_bf
+    logits = torch.where(mask[:, None, None, :], logits, torch.full_like(logits, -1e6))
+    ref = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(logits.double(), -1), v.double())
+    out = F.attention_core(q.cuda(), k.cuda(), v.cuda(), bias.cuda(), mask.cuda(), bias_div=lines)
+    assert _lib.device_status() == 0
+    assert_close(f"attention_core_N{N}_dh{dh}", out, ref)
