@@ -57,7 +57,7 @@ PACK_MAX = 24
 
 
 class TransitionWeights(Structure):
-    _fields_ = [("w13", c_void_p), ("w3", c_void_p), ("ln_w", c_void_p), ("ln_b", c_void_p)]
+    _fields_ = [("w13", c_void_p), ("w3", c_void_p), ("ln_w", c_void_p), ("ln_b", c_void_p), ("hidden", c_int64)]
 
 
 class SwigluWeights(Structure):
@@ -106,6 +106,8 @@ SIGNATURES = {
                                        c_int, c_int, c_void_p]),
     "b200_transition_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int,
                                     c_int, c_int, c_void_p]),
+    "b200_transition_hidden_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int,
+                                           c_int, c_int, c_void_p]),
     "b200_opm_workspace_bytes": (c_size_t, [c_int, c_int]),
     "b200_opm_fwd": (c_int, [c_void_p, c_void_p, c_int, c_void_p, POINTER(OpmWeights), c_int, c_int, c_int, c_int,
                              c_int, c_void_p, c_size_t, c_void_p]),
@@ -145,6 +147,8 @@ SIGNATURES = {
                                           c_int, c_int, c_int, c_void_p]),
     "b200_pair_outer_sum": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "b200_add_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_void_p]),
+    "b200_ln_linear_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int,
+                                   c_void_p]),
     "b200_pack_bf16": (c_int, [POINTER(PackSegment), c_int, c_void_p, c_void_p]),
     "b200_trunk_workspace_bytes": (c_size_t, [POINTER(TrunkBlock), c_int, c_int, c_int]),
     "b200_trunk_side_workspace_bytes": (c_size_t, [POINTER(TrunkBlock), c_int, c_int, c_int, c_int, c_int]),

@@ -2,9 +2,9 @@
 (src/bioemu2/biomoa/modules/diffusion.py:464-534).
 
 ``z = Linear(LayerNorm(cat(z_trunk, token_rel_pos_feats)))`` followed by ``z = Transition(z) + z`` per transition.
-No pair talks to another pair: the module is three HBM-bound passes over the pair tensor.  The concatenation is never
-materialised (the LayerNorm kernel reads the two sources), the projection is one tcgen05 GEMM writing fp32, and every
-transition adds its residual in its final store.
+No pair talks to another pair: the module is three HBM-bound passes over the pair tensor.  At the model's widths (128 + 128
+-> 128) LayerNorm and projection are one kernel (``F.ln_linear``); otherwise the LayerNorm kernel reads the two sources
+without materialising the concatenation and a tcgen05 GEMM follows.  Every transition adds its residual in its final store.
 """
 from __future__ import annotations
 
@@ -53,8 +53,11 @@ class PairwiseConditioning(nn.Module):
         if token_rel_pos_feats.dtype != z_trunk.dtype:
             token_rel_pos_feats = token_rel_pos_feats.to(z_trunk.dtype)
         ln = self.dim_pairwise_init_proj[0]
-        zn = F.rows2_to_bf16(z_trunk, token_rel_pos_feats, ln.weight, ln.bias)
-        z = F.linear_bf16(zn, self._weight(), out_dtype=torch.float32)
+        if self.token_z == self.dim_token_rel_pos_feats == self.a_z == 128:
+            z = F.ln_linear(z_trunk, token_rel_pos_feats, ln.weight, ln.bias, self._weight())
+        else:
+            zn = F.rows2_to_bf16(z_trunk, token_rel_pos_feats, ln.weight, ln.bias)
+            z = F.linear_bf16(zn, self._weight(), out_dtype=torch.float32)
         for t in self.transitions:
             t.forward_residual_(z)
         return z

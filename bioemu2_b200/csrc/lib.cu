@@ -9,6 +9,7 @@
 #include "bmm_nt.cuh"
 #include "trimul.cuh"
 #include "transition.cuh"
+#include "ln_linear.cuh"
 #include "elementwise.cuh"
 #include "opm.cuh"
 #include "attention.cuh"
@@ -255,6 +256,27 @@ static int launch_pair_bias(const void* z, bool f32, const float* ln_w, const fl
     B200_LAUNCH(pair_bias_kernel<true>, grid, pair_bias::THREADS, pair_bias::SMEM_BYTES, stream, tmW, p);
   else
     B200_LAUNCH(pair_bias_kernel<false>, grid, pair_bias::THREADS, pair_bias::SMEM_BYTES, stream, tmW, p);
+  return 0;
+}
+
+template <bool F32, int SRC>
+static int launch_ln_linear(const LnLinearParams& p, const void* w, float* out, cudaStream_t stream) {
+  using Cfg = LnLinearCfg<SRC>;
+  CUtensorMap tmW, tmO;
+  {
+    const uint64_t dims[2] = {128 * SRC, 128};
+    const uint64_t str[1] = {256 * SRC};
+    const uint32_t box[2] = {64, 128};
+    if (int e = make_tmap_bf16(&tmW, w, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+  }
+  {
+    const uint64_t dims[2] = {128, uint64_t(p.rows)};
+    const uint64_t str[1] = {512};
+    const uint32_t box[2] = {32, 128};
+    if (int e = make_tmap(&tmO, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+  }
+  const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
+  B200_LAUNCH((ln_linear_kernel<F32, SRC>), grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, tmW, tmO, p);
   return 0;
 }
 
@@ -609,12 +631,12 @@ int b200_bmm_nt(const void* A, const void* B, void* C, int batch, int M, int N, 
   return launch_bmm(a, static_cast<cudaStream_t>(stream));
 }
 
-int b200_transition_fwd(const void* x, void* out, const void* w13, const void* w3, const float* ln_w,
-                        const float* ln_b, int64_t rows, int use_norm, int add_residual, int x_dtype,
-                        b200_stream_t stream_) {
+int b200_transition_hidden_fwd(const void* x, void* out, const void* w13, const void* w3, const float* ln_w, const float* ln_b,
+                               int64_t rows, int hidden, int use_norm, int add_residual, int x_dtype, b200_stream_t stream_) {
   if (int e = b200_check_device()) return e;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   B200_CHECK_ARG(x && out && w13 && w3, "x/out/w13/w3 is NULL");
+  B200_CHECK_ARG(hidden == 512 || hidden == 256, "hidden=%d must be 256 or 512", hidden);
   B200_CHECK_ARG(!use_norm || (ln_w && ln_b), "use_norm needs ln_w and ln_b");
   B200_CHECK_ARG(rows >= 0 && rows < (int64_t(1) << 31), "rows out of range");
   B200_CHECK_ARG(x_dtype == B200_DTYPE_BF16 || x_dtype == B200_DTYPE_F32, "unknown x_dtype %d", x_dtype);
@@ -623,25 +645,25 @@ int b200_transition_fwd(const void* x, void* out, const void* w13, const void* w
   if (rows == 0) return B200_OK;
   CUtensorMap tmW1, tmW3;
   {
-    const uint64_t dims[2] = {128, 1024};
+    const uint64_t dims[2] = {128, uint64_t(2 * hidden)};
     const uint64_t str[1] = {256};
     const uint32_t box[2] = {64, 128};
     if (int e = make_tmap_bf16(&tmW1, w13, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   {
-    const uint64_t dims[2] = {512, 128};
-    const uint64_t str[1] = {1024};
+    const uint64_t dims[2] = {uint64_t(hidden), 128};
+    const uint64_t str[1] = {uint64_t(hidden) * 2};
     const uint32_t box[2] = {64, 128};
     if (int e = make_tmap_bf16(&tmW3, w3, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
-  const bool tr_f32 = x_dtype == B200_DTYPE_F32;
+  const bool f32 = x_dtype == B200_DTYPE_F32;
   CUtensorMap tmO;  // output rows, [128 rows][64 B] boxes
   {
     const uint64_t dims[2] = {uint64_t(kD), uint64_t(rows)};
-    const uint64_t str[1] = {uint64_t(kD) * (tr_f32 ? 4 : 2)};
-    const uint32_t box[2] = {tr_f32 ? 16u : 32u, 128};
-    if (int e = make_tmap(&tmO, tr_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out, 2, dims, str,
-                          box, CU_TENSOR_MAP_SWIZZLE_64B))
+    const uint64_t str[1] = {uint64_t(kD) * (f32 ? 4 : 2)};
+    const uint32_t box[2] = {f32 ? 16u : 32u, 128};
+    if (int e = make_tmap(&tmO, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out, 2, dims, str, box,
+                          CU_TENSOR_MAP_SWIZZLE_64B))
       return e;
   }
   TransitionParams p;
@@ -655,11 +677,35 @@ int b200_transition_fwd(const void* x, void* out, const void* w13, const void* w
   p.add_residual = add_residual ? 1 : 0;
   p.eps = 1e-5f;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  if (x_dtype == B200_DTYPE_F32)
-    B200_LAUNCH(transition_kernel<true>, grid, transition::THREADS, transition::SMEM_BYTES, stream, tmW1, tmW3, tmO, p);
-  else
-    B200_LAUNCH(transition_kernel<false>, grid, transition::THREADS, transition::SMEM_BYTES, stream, tmW1, tmW3, tmO, p);
+  if (hidden == 512) {
+    if (f32) B200_LAUNCH((transition_kernel<true, 8>), grid, transition::THREADS, transition::SMEM_BYTES, stream, tmW1, tmW3, tmO, p);
+    else B200_LAUNCH((transition_kernel<false, 8>), grid, transition::THREADS, transition::SMEM_BYTES, stream, tmW1, tmW3, tmO, p);
+  } else {
+    if (f32) B200_LAUNCH((transition_kernel<true, 4>), grid, transition::THREADS, transition::SMEM_BYTES, stream, tmW1, tmW3, tmO, p);
+    else B200_LAUNCH((transition_kernel<false, 4>), grid, transition::THREADS, transition::SMEM_BYTES, stream, tmW1, tmW3, tmO, p);
+  }
   return B200_OK;
+}
+
+int b200_transition_fwd(const void* x, void* out, const void* w13, const void* w3, const float* ln_w, const float* ln_b,
+                        int64_t rows, int use_norm, int add_residual, int x_dtype, b200_stream_t stream) {
+  return b200_transition_hidden_fwd(x, out, w13, w3, ln_w, ln_b, rows, 512, use_norm, add_residual, x_dtype, stream);
+}
+
+int b200_ln_linear_fwd(const void* x1, const void* x2, const float* ln_w, const float* ln_b, const void* w,
+                       const float* residual, float* out, int64_t rows, int x_dtype, b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(x1 && w && out, "x1/w/out is NULL");
+  B200_CHECK_ARG(rows >= 0 && rows < (int64_t(1) << 31), "rows out of range");
+  B200_CHECK_ARG((x_dtype | 1) == 1, "unknown dtype");
+  B200_CHECK_ARG(aligned(x1, 32) && aligned(x2, 32) && aligned(w, 16) && aligned(out, 32) && aligned(residual, 32),
+                 "x1/x2/out/residual must be 32-byte aligned, w 16-byte aligned");
+  if (rows == 0) return B200_OK;
+  LnLinearParams p{x1, x2, ln_w, ln_b, residual, rows, int((rows + 127) / 128), 1e-5f};
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool f32 = x_dtype == B200_DTYPE_F32;
+  if (x2) return f32 ? launch_ln_linear<true, 2>(p, w, out, st) : launch_ln_linear<false, 2>(p, w, out, st);
+  return f32 ? launch_ln_linear<true, 1>(p, w, out, st) : launch_ln_linear<false, 1>(p, w, out, st);
 }
 
 // ------------------------------------------------------------------------------------------------ no-allocation variant
@@ -1615,7 +1661,8 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
       if (int e = b200_triatt_fwd(z, pair_mask, z, &w.tri_att_end, B, N, 1, 1, z_dtype, ws, scratch, stream)) return e;
     }
     const b200_transition_weights& tz = w.transition_z;
-    if (int e = b200_transition_fwd(z, z, tz.w13, tz.w3, tz.ln_w, tz.ln_b, int64_t(B) * N * N, tz.ln_w != nullptr, 1, z_dtype, stream))
+    if (int e = b200_transition_hidden_fwd(z, z, tz.w13, tz.w3, tz.ln_w, tz.ln_b, int64_t(B) * N * N, int(tz.hidden),
+                                           tz.ln_w != nullptr, 1, z_dtype, stream))
       return e;
     if (!single) continue;
     const int k = i & 1;

@@ -1,6 +1,6 @@
-// Pair transition: out = fc3( silu(fc1(h)) * fc2(h) ) [+ x],  h = LN(x) (or x), dim 128 -> hidden 512 -> 128.
+// Pair transition: out = fc3( silu(fc1(h)) * fc2(h) ) [+ x],  h = LN(x) (or x), dim 128 -> hidden 512 or 256 -> 128.
 //
-// One persistent CTA per SM walks tiles of 128 pair rows.  The hidden axis is processed in 8 chunks of
+// One persistent CTA per SM walks tiles of 128 pair rows.  The hidden axis is processed in chunks of
 // 64: GEMM1 writes [fc1 chunk | fc2 chunk] (128 x 128) to one of two TMEM buffers, a warpgroup turns it
 // into the bf16 SwiGLU product in shared memory (K-major operand), GEMM2 accumulates it against the
 // matching 64-wide slice of fc3 into the output accumulator (two of them, so the final store of a tile
@@ -38,7 +38,7 @@ struct TransitionParams {
 };
 
 namespace transition {
-constexpr int CHUNKS = 8;  // hidden 512 = 8 x 64
+// hidden = CHUNKS x 64 (a template parameter: 8 for the 4x transitions, 4 for the 2x ones of the pairwise conditioning)
 constexpr int WS = 3;      // weight chunk stages: the chunk loads come from L2 and need two chunk times to land
 constexpr uint32_t X_OFF = 0;                            // 32 KB (A of GEMM1)
 constexpr uint32_t W1_OFF = X_OFF + kOperandTile;        // WS stages x 32 KB ([fc1|fc2] chunk, 128 rows x 128 K)
@@ -50,7 +50,7 @@ constexpr uint32_t SMEM_BYTES = STAGE_OFF + 2 * 8192 + 1024;
 constexpr int THREADS = 640;
 }  // namespace transition
 
-template <bool F32>
+template <bool F32, int CHUNKS>
 __global__ void __launch_bounds__(640, 1)
 transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW3,
                   const __grid_constant__ CUtensorMap tmO, TransitionParams p) {
@@ -72,7 +72,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
   uint64_t* out_empty = bars + 24;    // [2] count 256
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -108,14 +108,14 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
   int my_tiles = 0;
   for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x) ++my_tiles;
   const int total_chunks = my_tiles * CHUNKS;
-  // A global chunk counter g = it*8 + c drives the rings: depth 2 (stage g&1, use g>>1) for the TMEM and H
+  // A global chunk counter g = it*CHUNKS + c drives the rings: depth 2 (stage g&1, use g>>1) for the TMEM and H
   // buffers, depth WS (stage g%WS, use g/WS) for the weight chunks.
 
   if (warp == 17) {
     // ------------------------------------------------------------------ [fc1|fc2] chunk loader (TMA)
     if (lane == 0) {
       for (int g = 0; g < total_chunks; ++g) {
-        const int c = g & 7, s = g % WS;
+        const int c = g % CHUNKS, s = g % WS;
         mbar_wait(&w1_empty[s], ((g / WS) & 1) ^ 1, 30);
         mbar_arrive_expect_tx(&w1_full[s], kOperandTile);
         tma_load_2d(smem + W1_OFF + s * kOperandTile, &tmW1, &w1_full[s], 0, c * 128);
@@ -126,7 +126,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
     // ------------------------------------------------------------------ fc3 slice loader (TMA)
     if (lane == 0) {
       for (int g = 0; g < total_chunks; ++g) {
-        const int c = g & 7, s = g % WS;
+        const int c = g % CHUNKS, s = g % WS;
         mbar_wait(&w3_empty[s], ((g / WS) & 1) ^ 1, 31);
         mbar_arrive_expect_tx(&w3_full[s], kOperandHalf);
         tma_load_2d(smem + W3_OFF + s * kOperandHalf, &tmW3, &w3_full[s], c * 64, 0);
@@ -139,7 +139,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
       const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_bf16(128, 128);
       for (int g = 0; g < total_chunks; ++g) {
-        const int c = g & 7, b = g & 1, it = g >> 3, ws = g % WS;
+        const int c = g % CHUNKS, b = g & 1, it = g / CHUNKS, ws = g % WS;
         if (c == 0) mbar_wait(x_full, it & 1, 35);
         mbar_wait(&w1_full[ws], (g / WS) & 1, 36);
         mbar_wait(&d1_empty[b], ((g >> 1) & 1) ^ 1, 37);
@@ -148,7 +148,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
           umma_k128(tmem_base + b * 128, smem_u32(smem + X_OFF), smem_u32(smem + W1_OFF + ws * kOperandTile), idesc, false);
           umma_commit(&w1_empty[ws]);
           umma_commit(&d1_full[b]);
-          if (c == 7) umma_commit(x_empty);
+          if (c == CHUNKS - 1) umma_commit(x_empty);
         }
         __syncwarp();
       }
@@ -159,10 +159,10 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
       const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_bf16(128, 128);
       for (int g = 0; g < total_chunks; ++g) {  // consumes H[g&1] and the fc3 slice of chunk g
-        const int c = g & 7, b = g & 1, o = (g >> 3) & 1, ws = g % WS;
+        const int c = g % CHUNKS, b = g & 1, o = (g / CHUNKS) & 1, ws = g % WS;
         mbar_wait(&h_full[b], (g >> 1) & 1, 32);
         mbar_wait(&w3_full[ws], (g / WS) & 1, 33);
-        if (c == 0) mbar_wait(&out_empty[o], (((g >> 3) >> 1) & 1) ^ 1, 34);
+        if (c == 0) mbar_wait(&out_empty[o], (((g / CHUNKS) >> 1) & 1) ^ 1, 34);
         tc_fence_after_sync();
         const uint32_t h_s = smem_u32(smem + H_OFF + b * kOperandHalf);
         const uint32_t w3_s = smem_u32(smem + W3_OFF + ws * kOperandHalf);
@@ -173,7 +173,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
             umma_bf16_ss2(tmem_base + 256 + o * 128, h_lo + 2 * k, kDescHiSw128, w3_lo + 2 * k, kDescHiSw128, idesc, (c | k) != 0);
           umma_commit(&h_empty[b]);
           umma_commit(&w3_empty[ws]);
-          if (c == 7) umma_commit(&out_full[o]);
+          if (c == CHUNKS - 1) umma_commit(&out_full[o]);
         }
         __syncwarp();
       }
@@ -312,10 +312,10 @@ transition_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constan
         fence_proxy_async_smem();
         mbar_arrive(&d1_empty[b]);
         mbar_arrive(&h_full[b]);
-        // one part of the previous tile's output (4 chunks per group and tile: every part finds its turn)
-        if (it > 0 && part < PARTS && (PARTS == 4 || (c >> 1) & 1)) {
-          drain_part(it - 1, tile - (int)gridDim.x, part);
-          ++part;
+        // the previous tile's output, spread over this tile's CHUNKS / 2 chunks of the group
+        if (it > 0) {
+          for (const int end = PARTS * ((c >> 1) + 1) / (CHUNKS / 2); part < end; ++part)
+            drain_part(it - 1, tile - (int)gridDim.x, part);
         }
       }
     }

@@ -179,28 +179,30 @@ def trimul(x: Tensor, mask: Tensor, w: TriMulPacked, incoming: bool, add_residua
 
 
 class TransitionPacked:
-    """Weights of a 128 -> 512 -> 128 SwiGLU transition in the layout ``b200_transition_fwd`` expects.  A narrower
-    hidden layer (the 128 -> 256 -> 128 transitions of the pairwise conditioning) is zero-padded to 512: the padded
-    units contribute ``silu(0) * 0 = 0`` exactly, and one fused pass still beats four un-fused ones."""
+    """Weights of a 128 -> hidden -> 128 SwiGLU transition in the layout ``b200_transition_hidden_fwd`` expects.  The kernel
+    takes 256 or 512 hidden units; other widths up to 512 are zero-padded to the next of these: the padded units contribute
+    ``silu(0) * 0 = 0`` exactly, and one fused pass still beats four un-fused ones."""
 
     def __init__(self, norm_w, norm_b, fc1, fc2, fc3):
         hidden = fc1.shape[0]
         if fc1.shape[1] != 128 or tuple(fc2.shape) != tuple(fc1.shape) or tuple(fc3.shape) != (128, hidden) or hidden > 512:
             raise ValueError("the fused pair-transition kernel is built for dim=128, hidden<=512")
+        width = self.hidden = 256 if hidden <= 256 else 512
         pk = _Pack()
-        for c in range(0, 512, 64):  # 8 chunks of [64 fc1 rows | 64 fc2 rows]
+        for c in range(0, width, 64):  # chunks of [64 fc1 rows | 64 fc2 rows]
             for fc in (fc1, fc2):
                 rows = fc[min(c, hidden):min(c + 64, hidden)]
                 if rows.shape[0]:
                     pk.add(rows, pad_to=64 * 128)
                 else:
                     pk.add(None, count=64 * 128)
-        pk.add(fc3, groups=128, pad_to=512)
+        pk.add(fc3, groups=128, pad_to=width)
         buf = pk.build(fc3.device)
-        self.w13, self.w3 = buf[:1024 * 128].view(1024, 128), buf[1024 * 128:].view(128, 512)
+        self.w13, self.w3 = buf[:2 * width * 128].view(-1, 128), buf[2 * width * 128:].view(128, width)
         self.norm_w = norm_w.detach().float().contiguous() if norm_w is not None else None
         self.norm_b = norm_b.detach().float().contiguous() if norm_b is not None else None
-        self.struct = _lib.TransitionWeights(self.w13.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b))
+        self.struct = _lib.TransitionWeights(self.w13.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b),
+                                             width)
 
 
 def transition(x: Tensor, w: TransitionPacked, add_residual: bool = False, out: Tensor | None = None) -> Tensor:
@@ -220,10 +222,9 @@ def transition(x: Tensor, w: TransitionPacked, add_residual: bool = False, out: 
     if rows == 0:
         return out
     use_norm = w.norm_w is not None
-    _lib.check(lib.b200_transition_fwd(x.data_ptr(), out.data_ptr(), w.w13.data_ptr(), w.w3.data_ptr(),
-                                       w.norm_w.data_ptr() if use_norm else None,
-                                       w.norm_b.data_ptr() if use_norm else None, rows, 1 if use_norm else 0,
-                                       1 if add_residual else 0, zd, _stream()))
+    _lib.check(lib.b200_transition_hidden_fwd(x.data_ptr(), out.data_ptr(), w.w13.data_ptr(), w.w3.data_ptr(),
+                                              _ptr(w.norm_w), _ptr(w.norm_b), rows, w.hidden, 1 if use_norm else 0,
+                                              1 if add_residual else 0, zd, _stream()))
     return out
 
 
@@ -446,6 +447,27 @@ def rows2_to_bf16(x1: Tensor, x2: Tensor, weight: Tensor | None = None, bias: Te
     _lib.check(lib.b200_rows2_to_bf16(x1.data_ptr(), c1, x2.data_ptr(), c2, y.data_ptr(), _ptr(w), _ptr(b),
                                       x1.numel() // c1, _zdtype(x1), 1 if normalize else 0, _stream()))
     return y
+
+
+def ln_linear(x1: Tensor, x2: Tensor | None, weight: Tensor | None, bias: Tensor | None, w_bf16: Tensor,
+              residual: Tensor | None = None) -> Tensor:
+    """``LayerNorm(cat(x1, x2)) @ w.T (+ residual)`` as fp32 for 128-channel sources and 128 outputs, one pass."""
+    _require_cuda(x1, w_bf16)
+    x1 = x1.contiguous()
+    x2 = x2.contiguous() if x2 is not None else None
+    if x1.shape[-1] != 128 or (x2 is not None and (x2.shape != x1.shape or x2.dtype != x1.dtype)) or \
+            tuple(w_bf16.shape) != (128, 128 if x2 is None else 256) or w_bf16.dtype != torch.bfloat16:
+        raise ValueError("ln_linear takes 128-channel sources and a bf16 weight [128, 128 * sources]")
+    out = torch.empty(x1.shape, dtype=torch.float32, device=x1.device)
+    if out.numel() == 0:
+        return out
+    if residual is not None and (residual.dtype != torch.float32 or residual.shape != out.shape or not residual.is_contiguous()):
+        raise ValueError("residual must match the output in shape and dtype and be contiguous")
+    w = weight.detach().float().contiguous() if weight is not None else None
+    b = bias.detach().float().contiguous() if bias is not None else None
+    _lib.check(lib.b200_ln_linear_fwd(x1.data_ptr(), _ptr(x2), _ptr(w), _ptr(b), w_bf16.data_ptr(), _ptr(residual),
+                                      out.data_ptr(), x1.numel() // 128, _zdtype(x1), _stream()))
+    return out
 
 
 def pair_outer_sum(a: Tensor, c: Tensor, extra: Tensor | None = None) -> Tensor:

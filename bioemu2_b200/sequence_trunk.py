@@ -191,7 +191,10 @@ class PairMixerSequenceEmbedder(nn.Module):
         return s_init, F.pair_outer_sum(a, c, extra)
 
     def _recycle(self, x: Tensor, x_init: Tensor, norm: nn.LayerNorm, name: str) -> Tensor:
-        """``x_init + recycle(norm(x))`` (pairmixer.py:282-283): LayerNorm pass, then a GEMM that adds ``x_init``."""
+        """``x_init + recycle(norm(x))`` (pairmixer.py:282-283): one kernel for the 128-channel pair tensor, a LayerNorm pass
+        and a GEMM that adds ``x_init`` for the single track."""
+        if x.shape[-1] == 128 and self._lin[name].linear.weight.shape == (128, 128):
+            return F.ln_linear(x, None, norm.weight, norm.bias, self._lin[name].weight(), residual=x_init)
         xn = F.rows_to_bf16(x, norm.weight, norm.bias)
         return F.linear_bf16(xn, self._lin[name].weight(), residual=x_init, out_dtype=torch.float32)
 

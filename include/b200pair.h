@@ -178,6 +178,9 @@ int b200_trimul_fwd_static(const void* z, const uint8_t* mask, void* out, const 
 int b200_transition_fwd(const void* x, void* out, const void* w13, const void* w3, const float* ln_w,
                         const float* ln_b, int64_t rows, int use_norm, int add_residual, int x_dtype,
                         b200_stream_t stream);
+/* The same with a hidden width of 256 or 512: w13 [hidden/64][64 fc1 rows | 64 fc2 rows][128], w3 [128][hidden]. */
+int b200_transition_hidden_fwd(const void* x, void* out, const void* w13, const void* w3, const float* ln_w, const float* ln_b,
+                               int64_t rows, int hidden, int use_norm, int add_residual, int x_dtype, b200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------------
  * Outer product mean, OuterProductMeanVanilla.forward (src/bioemu2/biomoa/ops/outer_product_mean.py:45-75)
@@ -461,6 +464,15 @@ int b200_softmax_bias_f32(float* s, const float* bias, const uint8_t* keymask, i
                           b200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------------
+ * out = W . LayerNorm(x1 | x2) [+ residual] in one pass: rows of 128 channels (x2 == NULL) or 128 + 128, W bf16
+ * [128][128 or 256], out and residual fp32 [rows][128] (out may be residual), ln_w / ln_b fp32 or NULL.  The input projection
+ * of PairwiseConditioning (src/bioemu2/biomoa/modules/diffusion.py:464-534) and the recycling update of the pair tensor
+ * (src/bioemu2/biomoa/modules/pairmixer.py:282-283).
+ * ------------------------------------------------------------------------------------------------- */
+int b200_ln_linear_fwd(const void* x1, const void* x2, const float* ln_w, const float* ln_b, const void* w,
+                       const float* residual, float* out, int64_t rows, int x_dtype, b200_stream_t stream);
+
+/* ---------------------------------------------------------------------------------------------------
  * Builds bf16 kernel-layout weights from fp32 parameters in one launch: segment k writes groups * pitch elements at
  * dst + dst_off, taking `group` source elements times scale per group (src contiguous) and zeros in the rest of the pitch
  * (src == NULL: zeros only).  At most B200_PACK_MAX segments; counts and offsets are multiples of 8 elements.
@@ -478,7 +490,7 @@ int b200_pack_bf16(const b200_pack_segment* segments, int n, void* dst, b200_str
 /* ---------------------------------------------------------------------------------------------------
  * A stack of trunk blocks in one call: PairMixerLayer (src/bioemu2/biomoa/modules/pairmixer.py:430-456) or the composite
  * Pairformer block around it.  Per block, every step residual:
- *   z: triangle multiplication outgoing, incoming [, triangle attention starting, ending], transition 128 -> 512 -> 128
+ *   z: triangle multiplication outgoing, incoming [, triangle attention starting, ending], transition 128 -> hidden -> 128
  *   s: [attention with pair bias from the block's final z, SwiGLU transition c_s -> hidden -> c_s]
  * tri_att_start.w_o == NULL leaves the triangle attention out, attention.w_o == NULL (in block 0) the single track.
  *
@@ -487,7 +499,8 @@ int b200_pack_bf16(const b200_pack_segment* segments, int n, void* dst, b200_str
  * The single track of a block depends on the pair track only through the block's attention bias, so it runs on
  * side_stream under the next block's pair track; both streams are joined before the call's last operation on `stream`.
  * side_stream may be NULL (or equal to stream): one stream, same results.
- *   b200_transition_weights  w13 bf16 [8][64 fc1 rows | 64 fc2 rows][128], w3 bf16 [128][512], LayerNorm fp32 [128]
+ *   b200_transition_weights  w13 bf16 [hidden/64][64 fc1 rows | 64 fc2 rows][128], w3 bf16 [128][hidden], LayerNorm fp32
+ *                            [128]; hidden 256 or 512
  *   b200_swiglu_weights      w12 bf16 [2*hidden][c_s] (fc1 rows, then fc2 rows), w3 bf16 [c_s][hidden], LayerNorm fp32 [c_s]
  * Workspaces: 1024-byte aligned; the side one is for side_stream's kernels.
  * ------------------------------------------------------------------------------------------------- */
@@ -496,6 +509,7 @@ typedef struct {
   const void* w3;
   const float* ln_w;
   const float* ln_b;
+  int64_t hidden;
 } b200_transition_weights;
 
 typedef struct {
