@@ -444,7 +444,8 @@ def run_window_attention_probe(args, dev, emit: bool = True) -> dict:
     mask = torch.ones(NW, W, dtype=torch.bool, device=dev)
     w = mod.packed()
     sn = F.rows_to_bf16(s, w.ln_s_w, w.ln_s_b)
-    qkv, gate = F.linear_bf16(sn, w.w_qkv, bias_f32=w.b_qkv), F.linear_bf16(sn, w.w_g)
+    qkv = F.linear_bf16(sn, w.w_qkvg[:3 * c_s], bias_f32=w.b_qkvg[:3 * c_s])
+    gate = F.linear_bf16(sn, w.w_qkvg[3 * c_s:])
     bias = torch.empty(1, NW, heads, W, Hk, dtype=torch.float32, device=dev)
     og = torch.empty(M * NW, W, c_s, dtype=torch.bfloat16, device=dev)
     m8 = mask.to(torch.uint8)

@@ -50,7 +50,7 @@ class TriAttWeights(Structure):
 
 class PackSegment(Structure):
     _fields_ = [("src", c_void_p), ("dst_off", c_int64), ("groups", c_int32), ("group", c_int32), ("pitch", c_int32),
-                ("scale", c_float)]
+                ("stride", c_int32), ("scale", c_float)]
 
 
 PACK_MAX = 24
@@ -68,6 +68,14 @@ class TrunkBlock(Structure):
     _fields_ = [("tri_mul_out", TriMulWeights), ("tri_mul_in", TriMulWeights), ("tri_att_start", TriAttWeights),
                 ("tri_att_end", TriAttWeights), ("transition_z", TransitionWeights), ("attention", ApbWeights),
                 ("transition_s", SwigluWeights)]
+
+
+class CondLayer(Structure):
+    _fields_ = [("B", c_int), ("M", c_int), ("N", c_int), ("dim", c_int), ("dim_cond", c_int), ("heads", c_int),
+                ("dim_pairwise", c_int), ("window_queries", c_int), ("window_keys", c_int), ("lns_scale", c_float),
+                ("ln_c_w", c_void_p), ("ln_c_b", c_void_p), ("w_cond", c_void_p), ("b_cond", c_void_p),
+                ("attention", ApbWeights), ("w_qkvg", c_void_p), ("b_qkvg", c_void_p), ("w_o", c_void_p), ("ln_z_w", c_void_p),
+                ("ln_z_b", c_void_p), ("w_z", c_void_p), ("transition_fused", TransitionWeights), ("transition", SwigluWeights)]
 
 
 class AttentionCoreArgs(Structure):
@@ -145,10 +153,18 @@ SIGNATURES = {
                                      c_int, c_void_p]),
     "b200_window_attention_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                           c_int, c_int, c_int, c_void_p]),
+    "b200_window_attention_pitched_fwd": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                                  c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "b200_pair_outer_sum": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "b200_add_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_void_p]),
     "b200_ln_linear_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int,
                                    c_void_p]),
+    "b200_swiglu_transition_workspace_bytes": (c_size_t, [c_int64, c_int, c_int64]),
+    "b200_swiglu_transition_fwd": (c_int, [c_void_p, c_void_p, POINTER(SwigluWeights), c_int64, c_int, c_int, c_int, c_int,
+                                           c_void_p, c_size_t, c_void_p]),
+    "b200_cond_layer_workspace_bytes": (c_size_t, [POINTER(CondLayer)]),
+    "b200_cond_layer_fwd": (c_int, [POINTER(CondLayer), c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
+                                    c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "b200_pack_bf16": (c_int, [POINTER(PackSegment), c_int, c_void_p, c_void_p]),
     "b200_trunk_workspace_bytes": (c_size_t, [POINTER(TrunkBlock), c_int, c_int, c_int]),
     "b200_trunk_side_workspace_bytes": (c_size_t, [POINTER(TrunkBlock), c_int, c_int, c_int, c_int, c_int]),

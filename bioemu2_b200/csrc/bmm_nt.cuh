@@ -35,6 +35,12 @@ struct BmmParams {
   // bf16 columns) and the C tensor map, 1 = stored, 2 = added into C (the residual is C itself, which the
   // epilogue then never reads).
   int tma_c;
+  // Bulk output only: the tile is multiplied element by element with fp32 mul[row * mul_pitch + column] (a per-token gate)
+  // before it is stored or added.
+  const float* mul;
+  int mul_pitch;
+  // Bulk bf16 output only: the columns are pairs of 64-column blocks (a | b), C gets silu(a) * b, half as many columns.
+  int swiglu;
   int a_shared;              // 1: every batch item multiplies the same A (the A tensor map has a single batch slice)
 };
 
@@ -162,6 +168,49 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       tc_fence_after_sync();
       const int row = tm * 128 + quarter * 32 + lane;
       const float scale = p.scale_ptr ? p.scale * p.scale_ptr[b] : p.scale;
+      if (p.swiglu) {
+        // 32 output columns at a time from the matching columns of both blocks; a staging tile is 64 output columns
+        const int r = quarter * 32 + lane;
+        const bool leader = threadIdx.x == 64;
+#pragma unroll
+        for (int c = 0; c < BN / 64; ++c) {
+          const int a_col = (c >> 1) * 128 + (c & 1) * 32;
+          uint32_t va[32], vb[32];
+          tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + a_col), va);
+          tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + a_col + 64), vb);
+          uint8_t* stage = smem + Cfg::OUT_OFFSET + ((it * (BN / 128) + (c >> 1)) & 1) * 16384;
+          if ((c & 1) == 0) {
+            if (leader) tma_store_wait_read1();  // the store that last used this staging tile has read it
+            named_bar_sync(1, 128);
+          }
+          tmem_ld_wait();
+          if (c + 1 == BN / 64) {
+            tc_fence_before_sync();
+            mbar_arrive(&acc_empty[acc]);
+          }
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            float x[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float a = __uint_as_float(va[g * 8 + e]);
+              x[e] = a * sigmoid_fast(a) * __uint_as_float(vb[g * 8 + e]);
+            }
+            *reinterpret_cast<uint4*>(stage + sw128_offset(r, (c & 1) * 4 + g)) =
+                make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+          }
+          if (c & 1) {
+            fence_proxy_async_smem();
+            named_bar_sync(1, 128);
+            const int col = tn * (BN / 2) + (c >> 1) * 64;
+            if (leader && col < p.n_valid / 2) {
+              tma_store_3d(&tmC, stage, col, tm * 128, b);
+              tma_store_commit();
+            }
+          }
+        }
+        continue;
+      }
       if (p.tma_c) {
         // 32 columns at a time into one of two swizzled staging tiles; warp 2's first lane sends each tile off.
         const int r = quarter * 32 + lane;
@@ -191,6 +240,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             mbar_arrive(&acc_empty[acc]);
           }
           const int col0 = tn * BN + c * 32;
+          const float* mrow = p.mul && row < p.m_valid ? p.mul + (long long)row * p.mul_pitch + col0 : nullptr;
           if (p.out_f32) {
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
@@ -203,6 +253,10 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
                 const float4 bv = *reinterpret_cast<const float4*>(p.bias + col0 + g * 4);
                 x.x += bv.x; x.y += bv.y; x.z += bv.z; x.w += bv.w;
               }
+              if (mrow && col0 + g * 4 < p.n_valid) {
+                const float4 mv = *reinterpret_cast<const float4*>(mrow + g * 4);
+                x.x *= mv.x; x.y *= mv.y; x.z *= mv.z; x.w *= mv.w;
+              }
               *reinterpret_cast<float4*>(stage + sw128_offset(r, g)) = x;
             }
           } else {
@@ -214,6 +268,10 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               if (p.bias && col0 + g * 8 < p.n_valid) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) x[e] += p.bias[col0 + g * 8 + e];
+              }
+              if (mrow && col0 + g * 8 < p.n_valid) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] *= mrow[g * 8 + e];
               }
               *reinterpret_cast<uint4*>(stage + sw128_offset(r, (c & 1) * 4 + g)) = make_uint4(
                   pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
@@ -234,6 +292,53 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         }
         continue;
       }
+      if (p.opm_ntok > 0) {
+        // A warp's 32 lanes x 32 columns are one pair's outer product, 2 KB in one piece: through one of the warp's four
+        // buffers and out as a bulk copy (16-byte stores of the lanes' 64-byte rows: 98 us against 49 for 256 x 256 pairs).
+        // The lanes of a quarter-warp write their four 16-byte units in rotated order, which keeps them on different banks.
+        const int i = tm * 4 + quarter;
+        uint8_t* buf = smem + Cfg::OUT_OFFSET + quarter * 8192;
+        uint32_t va[32], vb[32];
+        tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN), va);
+#pragma unroll
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t(&v)[32] = (c & 1) ? vb : va;
+          tmem_ld_wait();
+          if (c + 1 < BN / 32) {
+            tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + (c + 1) * 32), (c & 1) ? va : vb);
+          } else {
+            tc_fence_before_sync();
+            mbar_arrive(&acc_empty[acc]);
+          }
+          uint4 w[4];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            float x[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[g * 8 + e]) * scale;
+            w[g] = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+          }
+          const int j = (tn * BN >> 5) + c;
+          if (i * 32 < p.m_valid && j * 32 < p.n_valid) {
+            uint8_t* row = buf + (c & 3) * 2048 + lane * 64;
+            if (lane == 0) tma_store_wait_read3();  // the copy that last used this buffer has read it
+            __syncwarp();
+            const int rot = (lane >> 1) & 3;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              const int u = (g + rot) & 3;
+              *reinterpret_cast<uint4*>(row + u * 16) = u == 0 ? w[0] : u == 1 ? w[1] : u == 2 ? w[2] : w[3];
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              bulk_store(static_cast<__nv_bfloat16*>(p.C) + ((long long)i * p.opm_ntok + j) * 1024, buf + (c & 3) * 2048, 2048);
+              tma_store_commit();
+            }
+          }
+        }
+        continue;
+      }
       const size_t esz = p.out_f32 ? 4 : 2;
       uint8_t* cbase = static_cast<uint8_t*>(p.C) + (long long)b * p.c_batch_stride * esz;
       // 32 columns at a time; the next chunk's TMEM load and (when a residual is added) its residual row
@@ -242,7 +347,6 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
                                         : nullptr;
       auto chunk_off = [&](int c) -> long long {  // element offset of (row, first column of chunk c)
         const int col0 = tn * BN + c * 32;
-        if (p.opm_ntok > 0) return (((long long)(row >> 5) * p.opm_ntok + (col0 >> 5)) * 32 + (row & 31)) * 32;
         if (p.remap_n > 0) return ((long long)(row % p.remap_n) * p.remap_m + row / p.remap_n) * p.ldc + col0;
         return (long long)row * p.ldc + col0;
       };
@@ -302,7 +406,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     }
   }
 
-  if (p.tma_c && threadIdx.x == 64) tma_store_wait0();
+  if (warp >= 2 && (p.opm_ntok > 0 ? lane == 0 : p.tma_c && threadIdx.x == 64)) tma_store_wait0();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {

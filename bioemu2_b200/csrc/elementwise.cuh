@@ -222,7 +222,7 @@ pack_bf16_kernel(const __grid_constant__ PackParams p) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[e] *= s.scale;
     }
-    store8<false>(p.dst + s.dst_off, t * 8, x);
+    store8<false>(p.dst + s.dst_off + (long long)g * s.stride, r, x);
   }
 }
 
@@ -258,11 +258,12 @@ swiglu_rows_kernel(const __nv_bfloat16* __restrict__ h12, __nv_bfloat16* __restr
 }
 
 // y[r,:] = lns * (LN(x[r,:]) * (1 + alpha[r,:]) + beta[r,:]) with alpha/beta columns of a [rows][cw] fp32 tensor
-// (adaptive LayerNorm without learned affine); x fp32 or bf16, y bf16.  One warp per row, cols <= 1024.
+// (adaptive LayerNorm without learned affine); x fp32 or bf16, y bf16.  One warp per row, cols <= 1024.  x_copy: a tensor that
+// receives x unchanged, or nullptr.
 template <bool F32IN>
 __global__ void __launch_bounds__(256)
 adaln_rows_kernel(const void* __restrict__ x, const float* __restrict__ cond, int cw, int alpha_col, int beta_col,
-                  float lns, __nv_bfloat16* __restrict__ y, long long rows, int cols, float eps) {
+                  float lns, __nv_bfloat16* __restrict__ y, void* __restrict__ x_copy, long long rows, int cols, float eps) {
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int nvec = cols >> 3;
@@ -278,6 +279,7 @@ adaln_rows_kernel(const void* __restrict__ x, const float* __restrict__ cond, in
       const int vi = lane + i * 32;
       if (vi < nvec) {
         load8<F32IN>(xr, vi * 8, f[i]);
+        if (x_copy) store8<F32IN>(static_cast<uint8_t*>(x_copy) + r * cols * (long long)(F32IN ? 4 : 2), vi * 8, f[i]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) s += f[i][e];
       }
@@ -306,6 +308,52 @@ adaln_rows_kernel(const void* __restrict__ x, const float* __restrict__ cond, in
         for (int e = 0; e < 8; ++e) f[i][e] = lns * fmaf(f[i][e] * rstd, 1.0f + al[e], be[e]);
         store8<false>(y + r * cols, vi * 8, f[i]);
       }
+    }
+  }
+}
+
+// The same for rows of at most 128 columns, two rows per warp with 8 columns per lane, the conditioning in flight with x
+// (32768 x 128: one row per warp left half of the lanes idle and read alpha and beta after the statistics, 22 us).
+template <bool F32IN>
+__global__ void __launch_bounds__(256)
+adaln_rows_narrow_kernel(const void* __restrict__ x, const float* __restrict__ cond, int cw, int alpha_col, int beta_col,
+                         float lns, __nv_bfloat16* __restrict__ y, void* __restrict__ x_copy, long long rows, int cols, float eps) {
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int sub = lane >> 4, l = lane & 15;
+  const bool has = l < (cols >> 3);
+  const long long warp_global = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const long long warp_stride = (long long)gridDim.x * (blockDim.x >> 5);
+  const float inv = 1.0f / float(cols);
+  for (long long rb = warp_global * 2; rb < rows; rb += warp_stride * 2) {  // the shuffles are warp-wide
+    const long long r = rb + sub;
+    const bool act = has && r < rows;
+    float f[8], al[8], be[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = 0.f;
+    if (act) {
+      load8<F32IN>(static_cast<const uint8_t*>(x) + r * cols * (long long)(F32IN ? 4 : 2), l * 8, f);
+      load8<true>(cond + r * cw + alpha_col, l * 8, al);
+      load8<true>(cond + r * cw + beta_col, l * 8, be);
+      if (x_copy) store8<F32IN>(static_cast<uint8_t*>(x_copy) + r * cols * (long long)(F32IN ? 4 : 2), l * 8, f);
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s += f[e];
+    const float mean = group16_sum(s) * inv;
+    float ss = 0.f;
+    if (act) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        f[e] -= mean;
+        ss = fmaf(f[e], f[e], ss);
+      }
+    }
+    const float rstd = rsqrtf(group16_sum(ss) * inv + eps);
+    if (act) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = lns * fmaf(f[e] * rstd, 1.0f + al[e], be[e]);
+      store8<false>(y + r * cols, l * 8, f);
     }
   }
 }

@@ -22,9 +22,25 @@ namespace b200 {
 
 template <int DH>
 static int launch_window_attention(const WindowAttnParams& p, int BM, cudaStream_t st) {
+  // whole 16-query tiles, the 128 keys whose scores a warp holds in registers, and at most 16 warps: the mma.sync kernel
+  if (p.W % 16 == 0 && p.Hk == kWindowMmaKeys && p.heads * (p.W / 16) <= 16 && p.qkv_pitch % 8 == 0 && p.gate_pitch % 2 == 0) {
+    const uint32_t smem = uint32_t(2 * kWindowMmaKeys * (p.heads * DH * 2 + 16) + kWindowMmaKeys);
+    if (smem <= 227 * 1024) {
+      B200_LAUNCH(window_mma_kernel<DH>, BM * p.NW, p.heads * (p.W / 16) * 32, smem, st, p);
+      return B200_OK;
+    }
+  }
   const uint32_t smem = uint32_t(2u * p.Hk * p.heads * DH * 2u + p.Hk + 16);
   B200_LAUNCH(window_attention_kernel<DH>, BM * p.NW, p.heads * p.W, smem, st, p);
   return B200_OK;
+}
+
+static int grid_for(int64_t work_items, int per_block) {
+  int64_t blocks = (work_items + per_block - 1) / per_block;
+  const int64_t cap = int64_t(sm_count()) * 16;
+  if (blocks > cap) blocks = cap;
+  if (blocks < 1) blocks = 1;
+  return int(blocks);
 }
 
 struct BmmLaunch {
@@ -40,10 +56,34 @@ struct BmmLaunch {
   int opm_ntok = 0;
   const void* residual = nullptr;
   int remap_n = 0, remap_m = 0;
+  const float* mul = nullptr;  // bulk output: per-element fp32 factor, row pitch mul_pitch
+  int mul_pitch = 0;
+  bool swiglu = false;  // bulk bf16 output: N columns are 64-wide (a | b) block pairs, C has N / 2 columns of silu(a) * b
+};
+
+// Tile width by the estimated time of the busiest CTA.  A K block of 64 takes a 256-wide tile about 1.5 times as long as a
+// 128-wide one (48 against 32 KB through L2 for twice the product), the last tile's epilogue is exposed; in units of a
+// thousandth of a 128-wide block: 256 columns where they fill the waves, 128 where the narrow tile leaves fewer CTAs idle
+// (2816 x 768 columns for 2048 rows: 176 wide tiles in two waves, 24.0 us; 352 narrow ones, 20.9 us).
+static int bmm_tile_n(int M, int N, int K, int batch) {
+  const int64_t tm = (M + 127) / 128, kb = (K + 63) / 64, sms = sm_count();
+  auto cost = [&](int bn, int64_t per_block, int64_t tail) {
+    const int64_t tiles = tm * ((N + bn - 1) / bn) * batch;
+    return (tiles + sms - 1) / sms * (kb * per_block + 700) + tail;
+  };
+  return cost(256, 1500, 5000) <= cost(128, 1000, 2500) ? 256 : 128;
+}
+
+// Set while a thread enqueues products that run underneath another stream's kernels: there the SM time they take counts, not
+// how soon they end, so they take wide tiles (trunk N = 203: 1.24 ms, 1.31 with narrow ones).
+static thread_local bool t_background = false;
+struct BackgroundScope {
+  explicit BackgroundScope(bool on) { t_background = on; }
+  ~BackgroundScope() { t_background = false; }
 };
 
 static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
-  const int BN = (a.N % 256 == 0 || a.N > 1024) ? 256 : 128;
+  const int BN = t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.K, a.batch);
   CUtensorMap tmA, tmB;
   const bool a_shared = a.batch > 1 && a.sa == 0;  // one A for every batch item
   {
@@ -77,19 +117,22 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   p.remap_n = a.remap_n;
   p.remap_m = a.remap_m > 0 ? a.remap_m : a.remap_n;
   p.a_shared = a_shared ? 1 : 0;
-  // Bulk output through the C tensor map where the layout allows it: whole 128-byte column groups, the
+  p.mul = a.mul;
+  p.mul_pitch = a.mul_pitch;
+  p.swiglu = a.swiglu ? 1 : 0;
+  // Bulk output through the C tensor map where the layout allows it (the map clips the last column group): the
   // residual (if any) being C itself, and for the transposed pair store lines that are whole row tiles.
   p.tma_c = 0;
   CUtensorMap tmC = tmA;
   const int64_t c_batch = a.sc > 0 ? a.sc : a.ldc * int64_t(a.M);
   const int c_esz = a.out_f32 ? 4 : 2;
   const int c_cols = 128 / c_esz;  // columns of one staging tile
-  if (a.opm_ntok == 0 && a.N % c_cols == 0 && (a.ldc * c_esz) % 16 == 0 && (c_batch * c_esz) % 16 == 0 && aligned(a.C, 16) &&
+  if (a.opm_ntok == 0 && (a.ldc * c_esz) % 16 == 0 && (c_batch * c_esz) % 16 == 0 && aligned(a.C, 16) &&
       (a.residual == nullptr || a.residual == a.C) && (a.bias == nullptr || aligned(a.bias, 16)) &&
       (a.remap_n == 0 || (a.remap_n % 128 == 0 && a.batch == 1 && a.M == a.remap_n * p.remap_m))) {
     uint64_t dims[3], str[2];
     uint32_t box[3];
-    dims[0] = uint64_t(a.N);
+    dims[0] = uint64_t(a.swiglu ? a.N / 2 : a.N);
     box[0] = uint32_t(c_cols);
     if (a.remap_n > 0) {  // {column, line, pos}: pair (line, pos) lives in row pos * remap_m + line
       dims[1] = uint64_t(p.remap_m), dims[2] = uint64_t(a.remap_n);
@@ -105,6 +148,8 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
       return e;
     p.tma_c = a.residual ? 2 : 1;
   }
+  if ((a.mul || a.swiglu) && (!p.tma_c || (a.mul && (!aligned(a.mul, 16) || a.mul_pitch % 4 || a.N % 8))))
+    return fail(B200_ERR_INVALID_ARGUMENT, "a gated product needs bulk output and 16-byte aligned factors");
   const int total = p.tiles_m * p.tiles_n * a.batch;
   const int grid = total < sm_count() ? total : sm_count();
   if (BN == 256) {
@@ -144,6 +189,20 @@ static int launch_rows_to_bf16(const void* x, bool f32, __nv_bfloat16* y, const 
   else
     B200_LAUNCH(layernorm_rows_kernel<false>, int(blocks), warps * 32, 0, stream, x, y, w, b, rows, cols, 1e-5f,
                 normalize, silu, x2, cols1);
+  return 0;
+}
+
+static int launch_adaln(const void* x, bool f32, const float* cond, int cw, int alpha_col, int beta_col, float lns,
+                        __nv_bfloat16* y, void* x_copy, int64_t rows, int cols, cudaStream_t stream) {
+  if (cols <= 128) {
+    const int grid = grid_for(rows, 16);
+    if (f32) B200_LAUNCH(adaln_rows_narrow_kernel<true>, grid, 256, 0, stream, x, cond, cw, alpha_col, beta_col, lns, y, x_copy, rows, cols, 1e-5f);
+    else B200_LAUNCH(adaln_rows_narrow_kernel<false>, grid, 256, 0, stream, x, cond, cw, alpha_col, beta_col, lns, y, x_copy, rows, cols, 1e-5f);
+    return 0;
+  }
+  const int grid = grid_for(rows, 8);
+  if (f32) B200_LAUNCH(adaln_rows_kernel<true>, grid, 256, 0, stream, x, cond, cw, alpha_col, beta_col, lns, y, x_copy, rows, cols, 1e-5f);
+  else B200_LAUNCH(adaln_rows_kernel<false>, grid, 256, 0, stream, x, cond, cw, alpha_col, beta_col, lns, y, x_copy, rows, cols, 1e-5f);
   return 0;
 }
 
@@ -816,14 +875,15 @@ static int opm_run(const void* m, const uint8_t* mask, int mask_ndim, void* out,
     pp.Sp = Sp;
     pp.num_tiles = N * ((S + 127) / 128);
     pp.eps = 1e-5f;
-    const int grid = pp.num_tiles < sm_count() ? pp.num_tiles : sm_count();
+    pp.row_counters = reinterpret_cast<int*>(inv) + 1;
+    const int grid = pp.num_tiles < 2 * sm_count() ? pp.num_tiles : 2 * sm_count();
     if (m_dtype == B200_DTYPE_F32)
       B200_LAUNCH(opm_proj_kernel<true>, grid, opm_proj::THREADS, opm_proj::SMEM_BYTES, stream, tmW, pp);
     else
       B200_LAUNCH(opm_proj_kernel<false>, grid, opm_proj::THREADS, opm_proj::SMEM_BYTES, stream, tmW, pp);
     const float* scale_ptr = ext_scale;
     if (mask_ndim == 3 && !ext_scale) {
-      B200_LAUNCH(opm_inv_row_count_kernel, 1, 1024, 0, stream, pp.mask, S, N, inv);
+      B200_LAUNCH(opm_inv_row_count_kernel, grid_for(S, 8), 256, 0, stream, pp.mask, S, N, pp.row_counters, inv);
       scale_ptr = inv;
     }
     for (int i0 = 0; i0 < N; i0 += CI) {
@@ -943,9 +1003,18 @@ size_t b200_apb_workspace_bytes(int B, int M, int N, int c_s, int H) {
   return pl.total;
 }
 
+// Where the output projection goes instead of `out`: x += mul * (its result), x of its own dtype.
+struct ApbOutput {
+  void* x;
+  bool f32;
+  const float* mul;
+  int mul_pitch;
+};
+
 static int apb_run(const void* s, const void* z, const void* ext_bias, int64_t ext_bias_pitch, const uint8_t* mask,
                    void* out, const b200_apb_weights* w, int B, int M, int N, int c_s, int H, int s_dtype, int z_dtype,
-                   bool add_residual, void* workspace, size_t workspace_bytes, b200_stream_t stream_) {
+                   bool add_residual, void* workspace, size_t workspace_bytes, b200_stream_t stream_,
+                   const ApbOutput* into = nullptr) {
   if (int e = b200_check_device()) return e;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   B200_CHECK_ARG(s && (z || ext_bias) && mask && out && w, "s/z/mask/out/w is NULL");
@@ -971,10 +1040,13 @@ static int apb_run(const void* s, const void* z, const void* ext_bias, int64_t e
   const int64_t rows = int64_t(BM) * N;
   const int HD = H * pl.DH;
 
-  // 1. LayerNorm (or plain conversion) of the single track
-  if (int e = launch_rows_to_bf16(s, s_dtype == B200_DTYPE_F32, s_ln, w->ln_s_w, w->ln_s_b, rows, c_s,
-                                  w->ln_s_w != nullptr, stream))
+  // 1. LayerNorm (or plain conversion) of the single track; bf16 rows without a LayerNorm are used as they are
+  if (!w->ln_s_w && s_dtype == B200_DTYPE_BF16) {
+    s_ln = static_cast<__nv_bfloat16*>(const_cast<void*>(s));
+  } else if (int e = launch_rows_to_bf16(s, s_dtype == B200_DTYPE_F32, s_ln, w->ln_s_w, w->ln_s_b, rows, c_s,
+                                         w->ln_s_w != nullptr, stream)) {
     return e;
+  }
   // 2. q | k | g projection (heads padded to DH, q pre-scaled) and V^T per batch item
   {
     BmmLaunch a{s_ln, w->w_qkg, qkg, 1, int(rows), pl.W1, c_s, c_s, c_s, pl.W1, 0, 0, 0};
@@ -1034,6 +1106,13 @@ static int apb_run(const void* s, const void* z, const void* ext_bias, int64_t e
     BmmLaunch a{og, w->w_o, out, 1, int(rows), c_s, c_s, c_s, c_s, c_s, 0, 0, 0};
     a.out_f32 = s_dtype == B200_DTYPE_F32;
     a.residual = add_residual ? s : nullptr;
+    if (into) {
+      a.C = into->x;
+      a.residual = into->x;
+      a.out_f32 = into->f32;
+      a.mul = into->mul;
+      a.mul_pitch = into->mul_pitch;
+    }
     if (int e = launch_bmm(a, stream)) return e;
   }
   return B200_OK;
@@ -1268,13 +1347,6 @@ int b200_triatt_slab_fwd(const void* z, const uint8_t* mask, const void* bias, i
 }
 
 // ------------------------------------------------------------------------------------------------ single-track helpers
-static int grid_for(int64_t work_items, int per_block) {
-  int64_t blocks = (work_items + per_block - 1) / per_block;
-  const int64_t cap = int64_t(sm_count()) * 16;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  return int(blocks);
-}
 
 int b200_rows_to_bf16(const void* x, void* y, const float* w, const float* b, int64_t rows, int cols, int x_dtype,
                       int normalize, int silu, b200_stream_t stream) {
@@ -1312,6 +1384,12 @@ int b200_window_bias_fwd(const void* z, const float* ln_w, const float* ln_b, co
   B200_CHECK_ARG((z_dtype | 1) == 1, "unknown dtype");
   if (windows == 0) return B200_OK;
   WindowBiasParams p{z, ln_w, ln_b, w_z, bias, windows * W * Hk, W * Hk, c_z, heads, 1e-5f};
+  if (c_z == 16 && aligned(z, 32)) {
+    const int grid = grid_for(p.pairs, 256);
+    if (z_dtype == B200_DTYPE_F32) B200_LAUNCH(window_bias16_kernel<true>, grid, 256, 0, static_cast<cudaStream_t>(stream), p);
+    else B200_LAUNCH(window_bias16_kernel<false>, grid, 256, 0, static_cast<cudaStream_t>(stream), p);
+    return B200_OK;
+  }
   int lpr = 1;
   while (lpr * 4 < c_z) lpr *= 2;  // lanes per pair: four channels each
   const int grid = grid_for(p.pairs * lpr, 256);
@@ -1321,9 +1399,10 @@ int b200_window_bias_fwd(const void* z, const float* ln_w, const float* ln_b, co
   return B200_OK;
 }
 
-int b200_window_attention_fwd(const void* qkv, const void* gate, const float* bias, const uint8_t* mask, void* out, int B,
-                              int M, int NW, int W, int Hk, int heads, int head_dim, b200_stream_t stream) {
-  if (int e = b200_check_device()) return e;
+// qkv / gate rows of qkv_pitch / gate_pitch elements.
+static int window_attention_run(const void* qkv, int qkv_pitch, const void* gate, int gate_pitch, const float* bias,
+                                const uint8_t* mask, void* out, int B, int M, int NW, int W, int Hk, int heads, int head_dim,
+                                cudaStream_t st) {
   B200_CHECK_ARG(qkv && gate && bias && mask && out, "qkv/gate/bias/mask/out is NULL");
   B200_CHECK_ARG(B > 0 && M > 0 && NW > 0 && W > 0 && Hk >= W && Hk % 8 == 0 && (Hk - W) % 2 == 0,
                  "need B, M, NW, W > 0 and Hk >= W, a multiple of 8, with Hk - W even (W=%d, Hk=%d)", W, Hk);
@@ -1333,12 +1412,28 @@ int b200_window_attention_fwd(const void* qkv, const void* gate, const float* bi
   B200_CHECK_ARG((int64_t)B * M * NW < (int64_t(1) << 31), "too many windows");
   B200_CHECK_ARG(aligned(qkv, 16) && aligned(gate, 16) && aligned(out, 16) && aligned(bias, 16),
                  "qkv/gate/out/bias must be 16-byte aligned");
-  WindowAttnParams p{static_cast<const __nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(gate), bias, mask,
-                     static_cast<__nv_bfloat16*>(out), NW, W, Hk, heads, M, 1.0f / sqrtf(float(head_dim))};
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  WindowAttnParams p{static_cast<const __nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(gate), qkv_pitch, gate_pitch,
+                     bias, mask, static_cast<__nv_bfloat16*>(out), NW, W, Hk, heads, M, 1.0f / sqrtf(float(head_dim))};
   if (head_dim == 16) return launch_window_attention<16>(p, B * M, st);
   if (head_dim == 32) return launch_window_attention<32>(p, B * M, st);
   return launch_window_attention<64>(p, B * M, st);
+}
+
+int b200_window_attention_fwd(const void* qkv, const void* gate, const float* bias, const uint8_t* mask, void* out, int B,
+                              int M, int NW, int W, int Hk, int heads, int head_dim, b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  return window_attention_run(qkv, 3 * heads * head_dim, gate, heads * head_dim, bias, mask, out, B, M, NW, W, Hk, heads, head_dim,
+                              static_cast<cudaStream_t>(stream));
+}
+
+int b200_window_attention_pitched_fwd(const void* qkv, int qkv_pitch, const void* gate, int gate_pitch, const float* bias,
+                                      const uint8_t* mask, void* out, int B, int M, int NW, int W, int Hk, int heads,
+                                      int head_dim, b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(qkv_pitch >= 3 * heads * head_dim && gate_pitch >= heads * head_dim && qkv_pitch % 8 == 0 && gate_pitch % 8 == 0,
+                 "pitches must be multiples of 8 and hold a row");
+  return window_attention_run(qkv, qkv_pitch, gate, gate_pitch, bias, mask, out, B, M, NW, W, Hk, heads, head_dim,
+                              static_cast<cudaStream_t>(stream));
 }
 
 int b200_pair_outer_sum(const float* a, const float* c, const float* extra, float* z, int n_i, int n_j, int cols,
@@ -1407,15 +1502,8 @@ int b200_adaln_fwd(const void* x, const float* cond, int cond_width, int alpha_c
   B200_CHECK_ARG((x_dtype | 1) == 1, "unknown dtype");
   B200_CHECK_ARG(aligned(x, 32) && aligned(cond, 32) && aligned(y, 16), "x/cond must be 32-byte aligned, y 16-byte");
   if (rows == 0) return B200_OK;
-  const int grid = grid_for(rows, 8);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (x_dtype == B200_DTYPE_F32)
-    B200_LAUNCH(adaln_rows_kernel<true>, grid, 256, 0, st, x, cond, cond_width, alpha_col, beta_col, lns,
-                static_cast<__nv_bfloat16*>(y), rows, cols, 1e-5f);
-  else
-    B200_LAUNCH(adaln_rows_kernel<false>, grid, 256, 0, st, x, cond, cond_width, alpha_col, beta_col, lns,
-                static_cast<__nv_bfloat16*>(y), rows, cols, 1e-5f);
-  return B200_OK;
+  return launch_adaln(x, x_dtype == B200_DTYPE_F32, cond, cond_width, alpha_col, beta_col, lns, static_cast<__nv_bfloat16*>(y),
+                      nullptr, rows, cols, static_cast<cudaStream_t>(stream));
 }
 
 int b200_gated_residual_fwd(void* x, const void* h, const float* cond, int cond_width, int gamma_col, int64_t rows,
@@ -1513,6 +1601,7 @@ int b200_pack_bf16(const b200_pack_segment* segments, int n, void* dst, b200_str
   for (int i = 0; i < n; ++i) {
     const b200_pack_segment& s = segments[i];
     B200_CHECK_ARG(s.groups >= 0 && s.group >= 0 && s.pitch > 0 && s.group <= s.pitch && s.group % 8 == 0 && s.pitch % 8 == 0 &&
+                       s.stride >= s.pitch && s.stride % 8 == 0 &&
                        s.dst_off >= 0 && s.dst_off % 8 == 0 && int64_t(s.groups) * s.pitch < (int64_t(1) << 31),
                    "segment %d: sizes and offsets must be multiples of 8", i);
     B200_CHECK_ARG(aligned(s.src, 32), "segment %d: the source must be 32-byte aligned", i);
@@ -1527,6 +1616,10 @@ int b200_pack_bf16(const b200_pack_segment* segments, int n, void* dst, b200_str
 
 // ------------------------------------------------------------------------------------------------ trunk stack
 static size_t round_up_1k(size_t x) { return (x + 1023) / 1024 * 1024; }
+static size_t swiglu_workspace(int64_t rows, int cols, int64_t hidden) {
+  const size_t h12 = hidden % 64 ? round_up_1k(size_t(rows) * 2 * hidden * 2) : 0;
+  return round_up_1k(size_t(rows) * cols * 2) + h12 + round_up_1k(size_t(rows) * hidden * 2);
+}
 static bool has_triatt(const b200_trunk_block& w) { return w.tri_att_start.w_o != nullptr; }
 static bool has_single(const b200_trunk_block& w) { return w.attention.w_o != nullptr; }
 static size_t trunk_bias_bytes(int B, int N, int heads) {
@@ -1548,8 +1641,7 @@ size_t b200_trunk_side_workspace_bytes(const b200_trunk_block* blocks, int n_blo
   size_t need = b200_apb_workspace_bytes(B, 1, N, c_s, heads);
   const size_t rows = size_t(B) * N;
   for (int i = 0; i < n_blocks; ++i) {
-    const size_t h = size_t(blocks[i].transition_s.hidden);
-    const size_t n = round_up_1k(rows * c_s * 2) + round_up_1k(rows * 2 * h * 2) + round_up_1k(rows * h * 2);
+    const size_t n = swiglu_workspace(int64_t(rows), c_s, blocks[i].transition_s.hidden);
     if (n > need) need = n;
   }
   return need;
@@ -1582,22 +1674,169 @@ static int trunk_events(cudaEvent_t** out) {
   return 0;
 }
 
-// SwiGLU transition of any width in place on s[rows][c_s]: LayerNorm rows, [fc1 | fc2] product, SwiGLU, fc3 product that
-// adds into s.
-static int swiglu_transition_(void* s, const b200_swiglu_weights& w, int64_t rows, int c_s, bool f32, uint8_t* ws,
-                              cudaStream_t stream) {
+
+// SwiGLU transition of any width: [LayerNorm,] fc1 | fc2 product with the SwiGLU in its epilogue (hidden a multiple of 64;
+// otherwise a row kernel of its own), fc3 product.  x fp32 or bf16 [rows][cols], out [rows][out_cols]; residual: added into
+// out (== x's values); mul: gate of the fc3 product, as in BmmLaunch.
+static int swiglu_transition(const void* x, bool x_f32, void* out, bool out_f32, bool residual, const float* mul, int mul_pitch,
+                             const b200_swiglu_weights& w, int64_t rows, int cols, int out_cols, uint8_t* ws, cudaStream_t stream) {
   const int hidden = int(w.hidden);
-  __nv_bfloat16* x = reinterpret_cast<__nv_bfloat16*>(ws);
-  __nv_bfloat16* h12 = reinterpret_cast<__nv_bfloat16*>(ws + round_up_1k(size_t(rows) * c_s * 2));
-  __nv_bfloat16* h = h12 + round_up_1k(size_t(rows) * 2 * hidden * 2) / 2;
-  if (int e = launch_rows_to_bf16(s, f32, x, w.ln_w, w.ln_b, rows, c_s, w.ln_w != nullptr, stream)) return e;
-  BmmLaunch a{x, w.w12, h12, 1, int(rows), 2 * hidden, c_s, c_s, c_s, 2 * hidden, 0, 0, 0};
-  if (int e = launch_bmm(a, stream)) return e;
-  B200_LAUNCH(swiglu_rows_kernel, grid_for(rows * (hidden / 8), 256), 256, 0, stream, h12, h, rows, hidden);
-  BmmLaunch b{h, w.w3, s, 1, int(rows), c_s, hidden, hidden, hidden, c_s, 0, 0, 0};
-  b.out_f32 = f32;
-  b.residual = s;
+  const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
+  if (x_f32 || w.ln_w) {
+    __nv_bfloat16* xr = reinterpret_cast<__nv_bfloat16*>(ws);
+    if (int e = launch_rows_to_bf16(x, x_f32, xr, w.ln_w, w.ln_b, rows, cols, w.ln_w != nullptr, stream)) return e;
+    xb = xr;
+  }
+  ws += round_up_1k(size_t(rows) * cols * 2);
+  __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(ws);
+  if (hidden % 64 == 0) {
+    BmmLaunch a{xb, w.w12, h, 1, int(rows), 2 * hidden, cols, cols, cols, hidden, 0, 0, 0};
+    a.swiglu = true;
+    if (int e = launch_bmm(a, stream)) return e;
+  } else {
+    __nv_bfloat16* h12 = reinterpret_cast<__nv_bfloat16*>(ws + round_up_1k(size_t(rows) * hidden * 2));
+    BmmLaunch a{xb, w.w12, h12, 1, int(rows), 2 * hidden, cols, cols, cols, 2 * hidden, 0, 0, 0};
+    if (int e = launch_bmm(a, stream)) return e;
+    B200_LAUNCH(swiglu_rows_kernel, grid_for(rows * (hidden / 8), 256), 256, 0, stream, h12, h, rows, hidden);
+  }
+  BmmLaunch b{h, w.w3, out, 1, int(rows), out_cols, hidden, hidden, hidden, out_cols, 0, 0, 0};
+  b.out_f32 = out_f32;
+  b.residual = residual ? out : nullptr;
+  b.mul = mul;
+  b.mul_pitch = mul_pitch;
   return launch_bmm(b, stream);
+}
+
+size_t b200_swiglu_transition_workspace_bytes(int64_t rows, int cols, int64_t hidden) {
+  return rows > 0 && cols > 0 && hidden > 0 ? swiglu_workspace(rows, cols, hidden) : 0;
+}
+
+int b200_swiglu_transition_fwd(const void* x, void* out, const b200_swiglu_weights* w, int64_t rows, int cols, int out_cols,
+                               int add_residual, int x_dtype, void* workspace, size_t workspace_bytes, b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(x && out && w && w->w12 && w->w3, "x/out/weights is NULL");
+  B200_CHECK_ARG(rows >= 0 && rows < (int64_t(1) << 31), "rows out of range");
+  B200_CHECK_ARG(cols > 0 && cols % 8 == 0 && cols <= 1024 && out_cols > 0 && out_cols % 8 == 0 && w->hidden > 0 && w->hidden % 8 == 0,
+                 "widths must be multiples of 8 and the input width at most 1024");
+  B200_CHECK_ARG((x_dtype | 1) == 1, "unknown dtype");
+  B200_CHECK_ARG(!add_residual || x == out, "the residual form works in place");
+  B200_CHECK_ARG(aligned(x, 32) && aligned(out, 32), "x/out must be 32-byte aligned");
+  if (rows == 0) return B200_OK;
+  if (!workspace || workspace_bytes < swiglu_workspace(rows, cols, w->hidden) || !aligned(workspace, 1024))
+    return fail(B200_ERR_WORKSPACE, "workspace must be 1024-byte aligned and hold %zu bytes (got %zu)",
+                swiglu_workspace(rows, cols, w->hidden), workspace_bytes);
+  const bool f32 = x_dtype == B200_DTYPE_F32;
+  return swiglu_transition(x, f32, out, f32, add_residual != 0, nullptr, 0, *w, rows, cols, out_cols,
+                           static_cast<uint8_t*>(workspace), static_cast<cudaStream_t>(stream));
+}
+
+// ------------------------------------------------------------------------------------------------ conditioned block
+struct CondPlan {
+  size_t off_cn, off_cond, off_y, off_rest, total;
+};
+static void cond_plan(const b200_cond_layer* l, int64_t rows, CondPlan* pl) {
+  size_t o = 0;
+  pl->off_cn = o; o += round_up_1k(size_t(rows) * l->dim_cond * 2);
+  pl->off_cond = o; o += round_up_1k(size_t(rows) * 6 * l->dim * 4);
+  pl->off_y = o; o += round_up_1k(size_t(rows) * l->dim * 2);
+  pl->off_rest = o;
+  size_t attn;
+  if (l->window_queries) {
+    attn = round_up_1k(size_t(rows) * 4 * l->dim * 2) + round_up_1k(size_t(rows) * l->dim * 2) +
+           round_up_1k(size_t(l->B) * l->N * l->window_keys * l->heads * 4);
+  } else {
+    attn = b200_apb_workspace_bytes(l->B, l->M, l->N, l->dim, l->heads);
+  }
+  const size_t tr = l->transition_fused.w13 ? round_up_1k(size_t(rows) * l->dim * 2) : swiglu_workspace(rows, l->dim, l->transition.hidden);
+  pl->total = o + (attn > tr ? attn : tr);
+}
+
+size_t b200_cond_layer_workspace_bytes(const b200_cond_layer* l) {
+  if (!l || l->B <= 0 || l->M <= 0 || l->N <= 0 || l->dim <= 0) return 0;
+  CondPlan pl;
+  cond_plan(l, int64_t(l->B) * l->M * l->N, &pl);
+  return pl.total;
+}
+
+int b200_cond_layer_fwd(const b200_cond_layer* l, const void* x, const void* pairs, const void* bias, int64_t bias_pitch,
+                        const void* c, const uint8_t* mask, void* out, int x_dtype, int c_dtype, int pairs_dtype,
+                        void* workspace, size_t workspace_bytes, b200_stream_t stream_) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(l && x && c && mask && out && (pairs || bias), "an argument is NULL");
+  B200_CHECK_ARG(l->B > 0 && l->M > 0 && l->N > 0 && l->heads > 0, "B/M/N/heads must be positive");
+  B200_CHECK_ARG(l->dim > 0 && l->dim % 32 == 0 && l->dim <= 1024 && l->dim_cond > 0 && l->dim_cond % 8 == 0 && l->dim_cond <= 1024,
+                 "dim=%d must be a multiple of 32, dim_cond=%d of 8, both <= 1024", l->dim, l->dim_cond);
+  B200_CHECK_ARG((x_dtype | 1) == 1 && (c_dtype | 1) == 1 && (pairs_dtype | 1) == 1, "unknown dtype");
+  B200_CHECK_ARG(aligned(x, 32) && aligned(c, 32) && aligned(out, 32), "x/c/out must be 32-byte aligned");
+  B200_CHECK_ARG(l->w_cond && l->b_cond && (l->transition_fused.w13 || l->transition.w12), "a weight pointer is NULL");
+  const int64_t rows = int64_t(l->B) * l->M * l->N;
+  B200_CHECK_ARG(rows < (int64_t(1) << 31), "too many rows");
+  CondPlan pl;
+  cond_plan(l, rows, &pl);
+  if (!workspace || workspace_bytes < pl.total || !aligned(workspace, 1024))
+    return fail(B200_ERR_WORKSPACE, "workspace must be 1024-byte aligned and hold %zu bytes (got %zu)", pl.total, workspace_bytes);
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  __nv_bfloat16* cn = reinterpret_cast<__nv_bfloat16*>(ws + pl.off_cn);
+  float* cond = reinterpret_cast<float*>(ws + pl.off_cond);
+  __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(ws + pl.off_y);
+  uint8_t* rest = ws + pl.off_rest;
+  const int D = l->dim, CW = 6 * D;
+  const bool xf32 = x_dtype == B200_DTYPE_F32;
+  // alpha1 | beta1 | gamma1 | alpha2 | beta2 | gamma2 = Linear(silu(LayerNorm(c)))
+  if (int e = launch_rows_to_bf16(c, c_dtype == B200_DTYPE_F32, cn, l->ln_c_w, l->ln_c_b, rows, l->dim_cond, true, stream, true)) return e;
+  {
+    BmmLaunch a{cn, l->w_cond, cond, 1, int(rows), CW, l->dim_cond, l->dim_cond, l->dim_cond, CW, 0, 0, 0};
+    a.bias = l->b_cond;
+    a.out_f32 = 1;
+    if (int e = launch_bmm(a, stream)) return e;
+  }
+  auto adaln = [&](const void* in, int alpha, void* copy) -> int {
+    return launch_adaln(in, xf32, cond, CW, alpha * D, (alpha + 1) * D, l->lns_scale, y, copy, rows, D, stream);
+  };
+  auto gated_residual = [&](const __nv_bfloat16* h, int gamma) -> int {
+    const int grid = grid_for(rows * (D / 8), 256);
+    if (xf32) B200_LAUNCH((gated_residual_rows_kernel<true, false>), grid, 256, 0, stream, out, h, cond, CW, gamma * D, rows, D);
+    else B200_LAUNCH((gated_residual_rows_kernel<false, false>), grid, 256, 0, stream, out, h, cond, CW, gamma * D, rows, D);
+    return 0;
+  };
+  // out = x + gamma1 * attention(adaln(x)); x is copied on the way, the output projection adds into the copy
+  if (int e = adaln(x, 0, x == out ? nullptr : out)) return e;
+  if (l->window_queries) {
+    const int W = l->window_queries, Hk = l->window_keys, NW = l->N / W;
+    B200_CHECK_ARG(l->N % W == 0, "N=%d is not a multiple of the query window %d", l->N, W);
+    B200_CHECK_ARG(pairs && l->w_qkvg && l->b_qkvg && l->w_o && l->ln_z_w && l->w_z, "a window weight pointer is NULL");
+    B200_CHECK_ARG(D % l->heads == 0, "dim=%d is not a multiple of heads=%d", D, l->heads);
+    __nv_bfloat16* qkvg = reinterpret_cast<__nv_bfloat16*>(rest);
+    __nv_bfloat16* og = reinterpret_cast<__nv_bfloat16*>(rest + round_up_1k(size_t(rows) * 4 * D * 2));
+    float* wb = reinterpret_cast<float*>(rest + round_up_1k(size_t(rows) * 4 * D * 2) + round_up_1k(size_t(rows) * D * 2));
+    {
+      BmmLaunch a{y, l->w_qkvg, qkvg, 1, int(rows), 4 * D, D, D, D, 4 * D, 0, 0, 0};
+      a.bias = l->b_qkvg;
+      if (int e = launch_bmm(a, stream)) return e;
+    }
+    if (int e = b200_window_bias_fwd(pairs, l->ln_z_w, l->ln_z_b, l->w_z, wb, int64_t(l->B) * NW, W, Hk, l->dim_pairwise, l->heads, pairs_dtype, stream)) return e;
+    if (int e = window_attention_run(qkvg, 4 * D, qkvg + 3 * D, 4 * D, wb, mask, og, l->B, l->M, NW, W, Hk, l->heads, D / l->heads, stream)) return e;
+    // The gate as a row kernel of its own: in the epilogue of a product this short its scattered row reads are not hidden
+    // (32768 x 128 x 128: 26 us against 7 + 9).
+    BmmLaunch a{og, l->w_o, y, 1, int(rows), D, D, D, D, D, 0, 0, 0};
+    if (int e = launch_bmm(a, stream)) return e;
+    if (int e = gated_residual(y, 2)) return e;
+  } else {
+    const ApbOutput into{out, xf32, cond + 2 * D, CW};
+    if (int e = apb_run(y, pairs, bias, bias_pitch, mask, out, &l->attention, l->B, l->M, l->N, D, l->heads, B200_DTYPE_BF16, pairs_dtype,
+                        false, rest, workspace_bytes - pl.off_rest, stream, &into))
+      return e;
+  }
+  // out += gamma2 * transition(adaln(out))
+  if (int e = adaln(out, 3, nullptr)) return e;
+  if (l->transition_fused.w13) {
+    __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(rest);
+    const b200_transition_weights& tw = l->transition_fused;
+    if (int e = b200_transition_hidden_fwd(y, h, tw.w13, tw.w3, nullptr, nullptr, rows, int(tw.hidden), 0, 0, B200_DTYPE_BF16, stream)) return e;
+    return gated_residual(h, 5);
+  }
+  return swiglu_transition(y, false, out, xf32, true, cond + 5 * D, CW, l->transition, rows, D, D, rest, stream);
 }
 
 int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_in, void* z, void* s,
@@ -1676,11 +1915,13 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
       B200_CUDA(cudaEventRecord(ev[k], stream));
       B200_CUDA(cudaStreamWaitEvent(side, ev[k], 0));
     }
+    BackgroundScope background(two && N > 128);  // up to 128 tokens the pair track leaves SMs free
     if (int e = apb_run(s, nullptr, bias[k], Nk, token_mask, s, &w.attention, B, 1, N, c_s, heads, s_dtype, B200_DTYPE_F32,
                         true, side_workspace, side_bytes, side))
       return e;
     if (two) B200_CUDA(cudaEventRecord(ev[2 + k], side));
-    if (int e = swiglu_transition_(s, w.transition_s, int64_t(B) * N, c_s, sf32, static_cast<uint8_t*>(side_workspace), side))
+    if (int e = swiglu_transition(s, sf32, s, sf32, true, nullptr, 0, w.transition_s, int64_t(B) * N, c_s, c_s,
+                                  static_cast<uint8_t*>(side_workspace), side))
       return e;
   }
   if (two) {

@@ -4,9 +4,10 @@
 // store then lays each pair's 32x32 block out contiguously for the output projection.
 //
 // A tile is one token i and 128 consecutive MSA rows s.
-//   warps 0-3  epilogue (TMEM lane = s; mask; transposed bf16 stores)
+//   warps 0-3  epilogue (TMEM lane = s; mask; transposed bf16 stores); warp 0 also issues the products
 //   warps 4-7  producers (load rows, LayerNorm over 64 channels, write the A operand)
-//   warp  8    control (TMA of proj_ab, MMA issue)
+// What bounds it is the producers' chain load -> LayerNorm -> store, one 16 KB tile at a time: eight warps and 128 registers
+// let two CTAs share an SM (1024 x 384 rows: 51 us with one CTA of nine warps).
 #pragma once
 #include "row_tile.cuh"
 
@@ -20,6 +21,7 @@ struct OpmProjParams {
   const float* ln_b;
   __nv_bfloat16* aT;     // [N*32][Sp]
   __nv_bfloat16* bT;
+  int* row_counters;     // two ints this kernel sets to zero
   int S, N, Sp;
   int num_tiles;         // N * ceil(S/128)
   float eps;
@@ -30,7 +32,7 @@ constexpr uint32_t W_OFF = 0;                      // 64 rows x 128 B
 constexpr uint32_t X_OFF = 8192;                   // 2 stages x 16 KB
 constexpr uint32_t BAR_OFF = X_OFF + 2 * kOperandHalf;
 constexpr uint32_t SMEM_BYTES = BAR_OFF + 128 + 1024;
-constexpr int THREADS = 288;
+constexpr int THREADS = 256;
 }  // namespace opm_proj
 
 __device__ __forceinline__ float group8_sum(float x) {
@@ -41,7 +43,7 @@ __device__ __forceinline__ float group8_sum(float x) {
 }
 
 template <bool F32>
-__global__ void __launch_bounds__(288, 1)
+__global__ void __launch_bounds__(256, 2)
 opm_proj_kernel(const __grid_constant__ CUtensorMap tmW, OpmProjParams p) {
   using namespace opm_proj;
   extern __shared__ uint8_t smem_raw[];
@@ -68,42 +70,15 @@ opm_proj_kernel(const __grid_constant__ CUtensorMap tmW, OpmProjParams p) {
     fence_mbar_init();
     prefetch_tmap(&tmW);
   }
-  if (warp == 8) tmem_alloc(tmem_slot, 128);
+  if (warp == 0) tmem_alloc(tmem_slot, 128);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
+  if (blockIdx.x == 0 && threadIdx.x < 2) p.row_counters[threadIdx.x] = 0;
 
-  if (warp == 8) {
-    // the whole warp waits on the barriers, one elected lane issues
-    const bool leader = elect_one();
-    if (leader) {
-      mbar_arrive_expect_tx(w_full, 8192);
-      tma_load_2d(smem + W_OFF, &tmW, w_full, 0, 0);
-    }
-    __syncwarp();
-    mbar_wait(w_full, 0, 50);
-    constexpr uint32_t idesc = make_idesc_bf16(128, 64);
-    const uint32_t w_s = smem_u32(smem + W_OFF);
-    int it = 0;
-    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
-      const int s = it & 1;
-      mbar_wait(&x_full[s], (it >> 1) & 1, 51);
-      mbar_wait(&acc_empty[s], ((it >> 1) & 1) ^ 1, 52);
-      tc_fence_after_sync();
-      const uint32_t x_s = smem_u32(smem + X_OFF + s * kOperandHalf);
-      const uint32_t x_lo = desc_lo(x_s), w_lo = desc_lo(w_s);
-      if (leader) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_bf16_ss2(tmem_base + s * 64, x_lo + 2 * k, kDescHiSw128, w_lo + 2 * k, kDescHiSw128, idesc, k > 0);
-        umma_commit(&x_empty[s]);
-        umma_commit(&acc_full[s]);
-      }
-      __syncwarp();
-    }
-  } else if (warp >= 4) {
+  if (warp >= 4) {
     // producers: 8 threads per row (8 channels each), 16 rows per pass, 8 passes
     const int pt = threadIdx.x - 128;
     const int c8 = pt & 7;
@@ -163,9 +138,36 @@ opm_proj_kernel(const __grid_constant__ CUtensorMap tmW, OpmProjParams p) {
       if (next < p.num_tiles) load_tile(next);
     }
   } else {
-    // epilogue: lane = MSA row s of the tile
+    // epilogue: lane = MSA row s of the tile; warp 0 (all lanes wait, one issues) starts a tile's product first
+    const bool leader = warp == 0 && elect_one();
+    constexpr uint32_t idesc = make_idesc_bf16(128, 64);
+    const uint32_t w_lo = desc_lo(smem_u32(smem + W_OFF));
+    if (warp == 0) {
+      if (leader) {
+        mbar_arrive_expect_tx(w_full, 8192);
+        tma_load_2d(smem + W_OFF, &tmW, w_full, 0, 0);
+      }
+      __syncwarp();
+      mbar_wait(w_full, 0, 50);
+    }
+    auto issue = [&](int n) {  // product of this CTA's n-th tile
+      const int s = n & 1;
+      mbar_wait(&x_full[s], (n >> 1) & 1, 51);
+      mbar_wait(&acc_empty[s], ((n >> 1) & 1) ^ 1, 52);
+      tc_fence_after_sync();
+      const uint32_t x_lo = desc_lo(smem_u32(smem + X_OFF + s * kOperandHalf));
+      if (leader) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_bf16_ss2(tmem_base + s * 64, x_lo + 2 * k, kDescHiSw128, w_lo + 2 * k, kDescHiSw128, idesc, k > 0);
+        umma_commit(&x_empty[s]);
+        umma_commit(&acc_full[s]);
+      }
+      __syncwarp();
+    };
     int it = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      if (warp == 0) issue(it);
       const int tok = tile / tiles_per_tok;
       const int s = ((tile - tok * tiles_per_tok) << 7) + warp * 32 + lane;
       const int acc = it & 1;
@@ -192,28 +194,37 @@ opm_proj_kernel(const __grid_constant__ CUtensorMap tmW, OpmProjParams p) {
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 8) {
+  if (warp == 0) {
     __syncwarp();
     tmem_dealloc(tmem_base, 128);
   }
 }
 
-// Number of MSA rows with at least one valid token -> 1 / max(count, 1).  One block.
-__global__ void opm_inv_row_count_kernel(const uint8_t* mask, int S, int N, float* inv_out) {
+// Number of MSA rows with at least one valid token -> 1 / max(count, 1): a warp per row, the last block to finish writes the
+// result.  ctr: two counters, zero on entry (the projection kernel before it clears them).
+__global__ void __launch_bounds__(256)
+opm_inv_row_count_kernel(const uint8_t* __restrict__ mask, int S, int N, int* ctr, float* inv_out) {
   pdl_wait();
   __shared__ int count;
   if (threadIdx.x == 0) count = 0;
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   int local = 0;
-  for (int s = warp; s < S; s += nwarps) {
+  for (int s = blockIdx.x * 8 + (threadIdx.x >> 5); s < S; s += gridDim.x * 8) {
     bool any = false;
     for (int i = lane; i < N; i += 32) any |= mask[(long long)s * N + i] != 0;
     if (__any_sync(0xffffffffu, any)) ++local;
   }
   if (lane == 0 && local) atomicAdd(&count, local);
   __syncthreads();
-  if (threadIdx.x == 0) *inv_out = 1.0f / float(count > 0 ? count : 1);
+  if (threadIdx.x == 0) {
+    if (count) atomicAdd(&ctr[0], count);
+    __threadfence();
+    if (atomicAdd(&ctr[1], 1) == int(gridDim.x) - 1) {
+      const int total = atomicAdd(&ctr[0], 0);
+      *inv_out = 1.0f / float(total > 0 ? total : 1);
+    }
+  }
 }
 
 }  // namespace b200

@@ -1,14 +1,17 @@
 // Sliding-window attention with pair bias for the atom transformer: a query window of W atoms attends to the Hk keys
 // centred on it (context = (Hk - W) / 2 atoms on either side, zero rows beyond the ends of the sequence).
 //
-// The work is small and oddly shaped for the tensor cores (32 x 128 scores per window and head, head dim 32): for
-// ~4,000 atoms it is a fraction of a GFLOP per sample, while the pair features that feed the bias are tens of MB.
-// So the two kernels here are plain fp32 CUDA-core kernels and the arithmetic of the core - scores, softmax and the
-// weighted sum - is exact fp32, as in the reference's autocast-free block.
+// The work is small and oddly shaped (32 x 128 scores per window and head, head dim 32): for ~4,000 atoms it is a fraction of
+// a GFLOP per sample, while the pair features that feed the bias are tens of MB.
 //
-//   window_bias_kernel       bias[b][w][h][i][j] = proj_z(LayerNorm(z[b][w][i][j][:]))[h], c_z / 4 lanes per pair
-//   window_attention_kernel  one CTA per (sample, window): K and V rows of the window staged in shared memory as bf16,
-//                            one thread per (head, query), online softmax over the keys in chunks of 8
+//   window_bias16_kernel     bias[b][w][h][i][j] = proj_z(LayerNorm(z[b][w][i][j][:]))[h] for c_z = 16: one thread per pair
+//   window_bias_kernel       any c_z: c_z / 4 lanes per pair
+//   window_mma_kernel        windows of 16-query tiles and 128 keys: one CTA per (sample, window), a warp per head and 16
+//                            queries, scores and weighted sum by mma.sync (a tcgen05 tile of 128 rows would be three
+//                            quarters padding here).  fp32 softmax; the weights enter the second product as the sum of two
+//                            bf16 values, so they keep 16 bits
+//   window_attention_kernel  other shapes: fp32 CUDA cores, one thread per (head, query)
+// 4,096 atoms x 8 samples: window attention 115 us on CUDA cores (instruction-bound), bias 36 us (shuffles).
 #pragma once
 #include "elementwise.cuh"
 
@@ -96,9 +99,56 @@ window_bias_kernel(WindowBiasParams p, int lpr) {
   }
 }
 
+// c_z = 16: the 16 channels of a pair in one thread, no shuffles; a warp's stores are contiguous for every head.
+template <bool F32>
+__global__ void __launch_bounds__(256)
+window_bias16_kernel(WindowBiasParams p) {
+  pdl_wait();
+  __shared__ float ws[kWindowMaxHeads * 16 + 32];  // projection rows, LayerNorm weight, bias
+  for (int i = threadIdx.x; i < p.heads * 16; i += blockDim.x) ws[i] = p.w_z[i];
+  if (threadIdx.x < 16) {
+    ws[kWindowMaxHeads * 16 + threadIdx.x] = p.ln_w[threadIdx.x];
+    ws[kWindowMaxHeads * 16 + 16 + threadIdx.x] = p.ln_b ? p.ln_b[threadIdx.x] : 0.f;
+  }
+  __syncthreads();
+  const float* lnw = ws + kWindowMaxHeads * 16;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < p.pairs; t += (long long)gridDim.x * blockDim.x) {
+    float x[16];
+    const uint8_t* row = static_cast<const uint8_t*>(p.z) + t * 16 * (long long)zbytes<F32>();
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      float v[8];
+      load8<F32>(row, k * 8, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[k * 8 + e] = v[e];
+    }
+    float s = 0.f, ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) s += x[e];
+    const float mean = s * (1.0f / 16);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      x[e] -= mean;
+      ss = fmaf(x[e], x[e], ss);
+    }
+    const float rstd = rsqrtf(ss * (1.0f / 16) + p.eps);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) x[e] = fmaf(x[e] * rstd, lnw[e], lnw[16 + e]);
+    const long long win = t / p.window_pairs;
+    float* dst = p.bias + win * p.heads * p.window_pairs + (t - win * p.window_pairs);
+    for (int h = 0; h < p.heads; ++h) {
+      float acc = 0.f;
+#pragma unroll
+      for (int e = 0; e < 16; ++e) acc = fmaf(x[e], ws[h * 16 + e], acc);
+      dst[(long long)h * p.window_pairs] = acc;
+    }
+  }
+}
+
 struct WindowAttnParams {
-  const __nv_bfloat16* qkv;   // [BM][L][3 * c_s]: q (bias added) | k | v, L = NW * W atoms
-  const __nv_bfloat16* gate;  // [BM][L][c_s] gate logits
+  const __nv_bfloat16* qkv;   // [BM][L] rows of qkv_pitch: q (bias added) | k | v, L = NW * W atoms
+  const __nv_bfloat16* gate;  // [BM][L] rows of gate_pitch: gate logits
+  int qkv_pitch, gate_pitch;
   const float* bias;          // [B][NW][heads][W][Hk]
   const uint8_t* mask;        // [B][L], non-zero = valid atom
   __nv_bfloat16* out;         // [BM][L][c_s] = sigmoid(gate) * attention output
@@ -131,7 +181,7 @@ window_attention_kernel(WindowAttnParams p) {
     const int a = a0 + j;
     uint4 kk = make_uint4(0, 0, 0, 0), vv = make_uint4(0, 0, 0, 0);
     if (a >= 0 && a < L) {
-      const __nv_bfloat16* src = p.qkv + (item + a) * 3 * c_s + c_s + v * 8;
+      const __nv_bfloat16* src = p.qkv + (item + a) * p.qkv_pitch + c_s + v * 8;
       kk = *reinterpret_cast<const uint4*>(src);
       vv = *reinterpret_cast<const uint4*>(src + c_s);
     }
@@ -149,7 +199,7 @@ window_attention_kernel(WindowAttnParams p) {
   const long long atom = item + w * p.W + i;
   float q[DH], o[DH];
   {
-    const __nv_bfloat16* qs = p.qkv + atom * 3 * c_s + h * DH;
+    const __nv_bfloat16* qs = p.qkv + atom * p.qkv_pitch + h * DH;
 #pragma unroll
     for (int d = 0; d < DH; d += 8) {
       float x[8];
@@ -202,7 +252,7 @@ window_attention_kernel(WindowAttnParams p) {
     }
   }
   const float inv_l = 1.0f / l;
-  const __nv_bfloat16* gs = p.gate + atom * c_s + h * DH;
+  const __nv_bfloat16* gs = p.gate + atom * p.gate_pitch + h * DH;
   __nv_bfloat16* dst = p.out + atom * c_s + h * DH;
 #pragma unroll
   for (int d = 0; d < DH; d += 8) {
@@ -211,6 +261,175 @@ window_attention_kernel(WindowAttnParams p) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) y[e] = o[d + e] * inv_l / (1.0f + __expf(-g[e]));
     store8<false>(dst, d, y);
+  }
+}
+
+// ---- mma.sync m16n8k16 (bf16, fp32 accumulation) and its operand loads
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(smem))
+               : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(smem))
+               : "memory");
+}
+
+constexpr int kWindowMmaKeys = 128;
+
+// Shared memory: K and V rows of the window, pitch c_s * 2 + 16 bytes (eight consecutive rows of an 8 x 8 matrix fall on
+// different banks), then the keys' validity bytes.  Warp = (head, 16-query tile); blockDim = heads * W / 16 warps.
+template <int DH>
+__global__ void __launch_bounds__(512)
+window_mma_kernel(WindowAttnParams p) {
+  pdl_wait();
+  extern __shared__ uint8_t smem_raw[];
+  constexpr int HK = kWindowMmaKeys;
+  const int c_s = p.heads * DH;
+  const int pitch = c_s * 2 + 16;
+  uint8_t* Ks = smem_raw;
+  uint8_t* Vs = Ks + HK * pitch;
+  uint8_t* kvalid = Vs + HK * pitch;
+  const int f = blockIdx.x;
+  const int bm = f / p.NW, w = f - bm * p.NW, b = bm / p.M;
+  const int L = p.NW * p.W;
+  const int a0 = w * p.W - (HK - p.W) / 2;  // atom index of key 0 (may be negative)
+  const long long item = (long long)bm * L;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  const int vec_per_row = c_s >> 3;  // zero rows outside the sequence, as the zero-padded unfold gives
+  for (int idx = threadIdx.x; idx < HK * vec_per_row; idx += blockDim.x) {
+    const int j = idx / vec_per_row, v = idx - j * vec_per_row;
+    const int a = a0 + j;
+    const bool in = a >= 0 && a < L;
+    const __nv_bfloat16* src = p.qkv + (item + (in ? a : 0)) * p.qkv_pitch + c_s + v * 8;
+    const uint32_t n = in ? 16u : 0u;  // source bytes; the rest of the 16 is zero-filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(Ks + j * pitch + v * 16)), "l"(src), "r"(n) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(Vs + j * pitch + v * 16)), "l"(src + c_s), "r"(n) : "memory");
+  }
+  for (int j = threadIdx.x; j < HK; j += blockDim.x) {
+    const int a = a0 + j;
+    kvalid[j] = (a >= 0 && a < L && p.mask[(long long)b * L + a]) ? 1 : 0;
+  }
+  const int tiles = p.W >> 4;
+  const int h = warp / tiles, q0 = (warp - h * tiles) * 16;
+  const int gr = lane >> 2, gc = (lane & 3) * 2;  // this lane's accumulator rows gr, gr + 8 and columns gc, gc + 1
+  // Q fragments straight from global memory: rows gr / gr + 8, 16 dims per step
+  uint32_t qf[DH / 16][4];
+  {
+    const __nv_bfloat16* r0 = p.qkv + (item + w * p.W + q0 + gr) * p.qkv_pitch + h * DH + gc;
+    const __nv_bfloat16* r1 = r0 + 8ll * p.qkv_pitch;
+#pragma unroll
+    for (int k = 0; k < DH / 16; ++k) {
+      qf[k][0] = *reinterpret_cast<const uint32_t*>(r0 + k * 16);
+      qf[k][1] = *reinterpret_cast<const uint32_t*>(r1 + k * 16);
+      qf[k][2] = *reinterpret_cast<const uint32_t*>(r0 + k * 16 + 8);
+      qf[k][3] = *reinterpret_cast<const uint32_t*>(r1 + k * 16 + 8);
+    }
+  }
+  // The bias, divided by the score scale, is where the score accumulators start: its loads are in flight with K and V.
+  float s[HK / 8][4];
+  {
+    const float* brow = p.bias + ((((long long)b * p.NW + w) * p.heads + h) * p.W + q0 + gr) * HK + gc;
+    const float unscale = 1.0f / p.scale;
+#pragma unroll
+    for (int n = 0; n < HK / 8; ++n) {
+      const float2 b0 = *reinterpret_cast<const float2*>(brow + n * 8), b1 = *reinterpret_cast<const float2*>(brow + 8 * HK + n * 8);
+      s[n][0] = b0.x * unscale, s[n][1] = b0.y * unscale, s[n][2] = b1.x * unscale, s[n][3] = b1.y * unscale;
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+
+  // scores: 16 queries x 128 keys
+#pragma unroll
+  for (int k = 0; k < DH / 16; ++k) {
+#pragma unroll
+    for (int n = 0; n < HK / 8; n += 2) {  // two 8-key tiles x 16 dims per load
+      uint32_t kf[4];
+      ldmatrix_x4(kf, Ks + (n * 8 + (lane & 7) + ((lane >> 4) << 3)) * pitch + (h * DH + k * 16 + ((lane >> 3) & 1) * 8) * 2);
+      mma_bf16(s[n], qf[k], kf[0], kf[1]);
+      mma_bf16(s[n + 1], qf[k], kf[2], kf[3]);
+    }
+  }
+  float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+  for (int n = 0; n < HK / 8; ++n) {
+    const bool ok0 = kvalid[n * 8 + gc], ok1 = kvalid[n * 8 + gc + 1];
+    s[n][0] = ok0 ? s[n][0] * p.scale : kWindowMasked;
+    s[n][1] = ok1 ? s[n][1] * p.scale : kWindowMasked;
+    s[n][2] = ok0 ? s[n][2] * p.scale : kWindowMasked;
+    s[n][3] = ok1 ? s[n][3] * p.scale : kWindowMasked;
+    m0 = max3(m0, s[n][0], s[n][1]);
+    m1 = max3(m1, s[n][2], s[n][3]);
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+  float l0 = 0.f, l1 = 0.f;
+  float o[DH / 8][4];
+#pragma unroll
+  for (int d = 0; d < DH / 8; ++d)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[d][e] = 0.f;
+#pragma unroll
+  for (int k = 0; k < HK / 16; ++k) {  // 16 keys per step: the weights of two score tiles are the A operand
+    float e[8];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      e[u * 4 + 0] = __expf(s[2 * k + u][0] - m0);
+      e[u * 4 + 1] = __expf(s[2 * k + u][1] - m0);
+      e[u * 4 + 2] = __expf(s[2 * k + u][2] - m1);
+      e[u * 4 + 3] = __expf(s[2 * k + u][3] - m1);
+      l0 += e[u * 4 + 0] + e[u * 4 + 1];
+      l1 += e[u * 4 + 2] + e[u * 4 + 3];
+    }
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {  // register u: (row gr | gr + 8) of the first, then of the second tile
+      const float x0 = e[u * 2], x1 = e[u * 2 + 1];
+      hi[u] = pack_bf16x2(x0, x1);
+      lo[u] = pack_bf16x2(x0 - bf16lo(hi[u]), x1 - bf16hi(hi[u]));
+    }
+#pragma unroll
+    for (int d = 0; d < DH / 8; d += 2) {  // 16 keys x two 8-dim tiles per load
+      uint32_t vf[4];
+      ldmatrix_x4_trans(vf, Vs + (k * 16 + (lane & 15)) * pitch + (h * DH + d * 8 + (lane >> 4) * 8) * 2);
+      mma_bf16(o[d], hi, vf[0], vf[1]);
+      mma_bf16(o[d + 1], hi, vf[2], vf[3]);
+      mma_bf16(o[d], lo, vf[0], vf[1]);
+      mma_bf16(o[d + 1], lo, vf[2], vf[3]);
+    }
+  }
+#pragma unroll
+  for (int x = 1; x < 4; x <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, x);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, x);
+  }
+  const float i0 = 1.0f / l0, i1 = 1.0f / l1;
+  const long long atom = item + w * p.W + q0 + gr;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const __nv_bfloat16* gs = p.gate + (atom + half * 8) * p.gate_pitch + h * DH + gc;
+    __nv_bfloat16* dst = p.out + (atom + half * 8) * c_s + h * DH + gc;
+    const float inv = half ? i1 : i0;
+#pragma unroll
+    for (int d = 0; d < DH / 8; ++d) {
+      const uint32_t gv = *reinterpret_cast<const uint32_t*>(gs + d * 8);
+      const float y0 = o[d][half * 2] * inv / (1.0f + __expf(-bf16lo(gv)));
+      const float y1 = o[d][half * 2 + 1] * inv / (1.0f + __expf(-bf16hi(gv)));
+      *reinterpret_cast<uint32_t*>(dst + d * 8) = pack_bf16x2(y0, y1);
+    }
   }
 }
 

@@ -107,26 +107,35 @@ class _Pack:
     def __init__(self) -> None:
         self.parts, self.size = [], 0
 
+    def interleave(self, tensors, groups: int) -> int:
+        """The tensors' ``groups`` equal parts in turn: part 0 of each, part 1 of each, ..."""
+        off, n = self.size, len(tensors)
+        for k, t in enumerate(tensors):
+            group = t.numel() // groups
+            self.parts.append((t, off + k * group, groups, group, group, group * n, 1.0))
+        self.size += groups * group * n
+        return off
+
     def add(self, t: Tensor | None, scale: float = 1.0, groups: int = 1, pad_to: int = 0, count: int = 0) -> int:
         """``t`` flattened; with ``groups`` every ``numel / groups`` elements are zero-padded to ``pad_to`` elements;
         ``t=None``: ``count`` zeros."""
         group = 0 if t is None else t.numel() // groups
         pitch = pad_to or group or count
         off = self.size
-        self.parts.append((t, off, groups, group, pitch, scale))
+        self.parts.append((t, off, groups, group, pitch, pitch, scale))
         self.size += groups * pitch
         return off
 
     def build(self, device: torch.device) -> Tensor:
         out = torch.empty(self.size, dtype=torch.bfloat16, device=device)
         keep, segs = [], []
-        for t, off, groups, group, pitch, scale in self.parts:
+        for t, off, groups, group, pitch, stride, scale in self.parts:
             if t is not None:
                 t = t.detach()
                 if t.dtype != torch.float32 or not t.is_contiguous() or t.data_ptr() % 32:
                     t = t.to(torch.float32).contiguous().clone() if t.data_ptr() % 32 else t.to(torch.float32).contiguous()
                 keep.append(t)
-            segs.append(_lib.PackSegment(_ptr(t), off, groups, group, pitch, scale))
+            segs.append(_lib.PackSegment(_ptr(t), off, groups, group, pitch, stride, scale))
         for i in range(0, len(segs), _lib.PACK_MAX):
             part = segs[i:i + _lib.PACK_MAX]
             _lib.check(lib.b200_pack_bf16((_lib.PackSegment * len(part))(*part), len(part), out.data_ptr(), _stream()))
@@ -510,21 +519,23 @@ def add_rows(x: Tensor, y: Tensor, out: Tensor | None = None) -> Tensor:
 
 
 class WindowApbPacked:
-    """Weights of the sliding-window attention: ``proj_qkv`` with ``proj_q_bias`` folded into a GEMM bias on the q
-    columns, gate and output projections in bf16, the tiny pair-bias projection in fp32."""
+    """Weights of the sliding-window attention: one projection ``q | k | v | gate`` with ``proj_q_bias`` as its bias on the q
+    columns, the output projection in bf16, the tiny pair-bias projection in fp32."""
 
     def __init__(self, c_s, c_z, heads, proj_qkv, proj_q_bias, proj_g, norm_z_w, norm_z_b, proj_z, proj_o, norm_s_w, norm_s_b):
-        bf = torch.bfloat16
         dh = c_s // heads
         if dh not in (16, 32, 64) or heads > 16:
             raise ValueError(f"the sliding-window kernel serves head dims 16, 32, 64 and up to 16 heads, got {dh} x {heads}")
         self.c_s, self.c_z, self.H, self.dh = c_s, c_z, heads, dh
-        self.w_qkv = proj_qkv.detach().to(bf).contiguous()
-        b = torch.zeros(3 * c_s, dtype=torch.float32, device=proj_qkv.device)
+        pk = _Pack()
+        pk.add(proj_qkv)
+        pk.add(proj_g)
+        o = pk.add(proj_o)
+        buf = pk.build(proj_o.device)
+        self.w_qkvg, self.w_o = buf[:o].view(4 * c_s, c_s), buf[o:].view(c_s, c_s)
+        b = torch.zeros(4 * c_s, dtype=torch.float32, device=proj_qkv.device)
         b[:c_s] = proj_q_bias.detach().float()
-        self.b_qkv = b
-        self.w_g = proj_g.detach().to(bf).contiguous()
-        self.w_o = proj_o.detach().to(bf).contiguous()
+        self.b_qkvg = b
         self.w_z = proj_z.detach().float().contiguous()
         self.ln_z_w = norm_z_w.detach().float().contiguous()
         self.ln_z_b = norm_z_b.detach().float().contiguous() if norm_z_b is not None else None
@@ -543,18 +554,39 @@ def window_attention_pair_bias(s: Tensor, z: Tensor, mask: Tensor, w: WindowApbP
                          f"multiplicity {M}")
     if s.numel() == 0:
         return torch.empty_like(s)
-    sn = rows_to_bf16(s, w.ln_s_w, w.ln_s_b, normalize=w.ln_s_w is not None)
-    qkv = linear_bf16(sn, w.w_qkv, bias_f32=w.b_qkv)
-    gate = linear_bf16(sn, w.w_g)
+    sn = s if s.dtype == torch.bfloat16 and w.ln_s_w is None else rows_to_bf16(s, w.ln_s_w, w.ln_s_b, normalize=w.ln_s_w is not None)
+    qkvg = linear_bf16(sn, w.w_qkvg, bias_f32=w.b_qkvg)
     z = z.contiguous()
     bias = torch.empty(B, NW, w.H, W, Hk, dtype=torch.float32, device=s.device)
     _lib.check(lib.b200_window_bias_fwd(z.data_ptr(), w.ln_z_w.data_ptr(), _ptr(w.ln_z_b), w.w_z.data_ptr(), bias.data_ptr(),
                                         B * NW, W, Hk, c_z, w.H, _zdtype(z), _stream()))
     og = torch.empty(folded, W, c_s, dtype=torch.bfloat16, device=s.device)
     m8 = mask_u8(mask).contiguous()
-    _lib.check(lib.b200_window_attention_fwd(qkv.data_ptr(), gate.data_ptr(), bias.data_ptr(), m8.data_ptr(), og.data_ptr(),
-                                             B, M, NW, W, Hk, w.H, w.dh, _stream()))
+    _lib.check(lib.b200_window_attention_pitched_fwd(qkvg.data_ptr(), 4 * c_s, qkvg.data_ptr() + 6 * c_s, 4 * c_s,
+                                                     bias.data_ptr(), m8.data_ptr(), og.data_ptr(), B, M, NW, W, Hk, w.H, w.dh,
+                                                     _stream()))
     return linear_bf16(og, w.w_o, out_dtype=s.dtype)
+
+
+def cond_layer(layer: "_lib.CondLayer", x: Tensor, pairs: Tensor | None, bias: Tensor | None, c: Tensor, mask: Tensor,
+               out: Tensor | None = None) -> Tensor:
+    """A ``ConditionedTransformerLayer`` in one native call; ``layer`` carries sizes and weights, ``bias`` (bf16, base 2) replaces
+    the projection of ``pairs`` where it is given."""
+    _require_cuda(x, c, mask)
+    x, c = x.contiguous(), c.contiguous()
+    pairs = pairs.contiguous() if bias is None else None
+    m8 = mask_u8(mask)
+    if out is None:
+        out = torch.empty_like(x)
+    if out.numel() == 0:
+        return out
+    nbytes = lib.b200_cond_layer_workspace_bytes(ctypes.byref(layer))
+    ws = workspace(nbytes, x.device)
+    _lib.check(lib.b200_cond_layer_fwd(ctypes.byref(layer), x.data_ptr(), _ptr(pairs), _ptr(bias),
+                                       bias.shape[-1] if bias is not None else 0, c.data_ptr(), m8.data_ptr(), out.data_ptr(),
+                                       _zdtype(x), _zdtype(c), _zdtype(pairs) if pairs is not None else _lib.DTYPE_F32,
+                                       ws.data_ptr(), nbytes, _stream()))
+    return out
 
 
 def swiglu(h12: Tensor) -> Tensor:
@@ -594,35 +626,58 @@ def gated_residual_(x: Tensor, h: Tensor, cond: Tensor, gamma_col: int) -> Tenso
 
 
 class TransitionGenericPacked:
-    """Weights of a SwiGLU transition of any width (multiples of 8): ``w12 = [fc1; fc2]``, ``w3``."""
+    """Weights of a SwiGLU transition of any width (multiples of 8): ``w12`` (fc1 and fc2 rows, in alternating blocks of 64
+    when the hidden width allows, so that the product's epilogue holds both factors of a unit) and ``w3``."""
 
     def __init__(self, norm_w, norm_b, fc1, fc2, fc3):
         if fc1.shape[0] % 8 or fc1.shape[1] % 8 or fc3.shape[0] % 8 or fc1.shape[1] > 1024:
             raise ValueError("transition widths must be multiples of 8 and the input width at most 1024")
+        self.hidden, self.cols, self.out_cols = fc1.shape[0], fc1.shape[1], fc3.shape[0]
         pk = _Pack()
-        pk.add(fc1)
-        pk.add(fc2)
+        if self.hidden % 64 == 0:  # alternating blocks: block k of fc1 at 2k, of fc2 at 2k + 1
+            blocks = self.hidden // 64
+            pk.interleave((fc1, fc2), groups=blocks)
+        else:
+            pk.add(fc1)
+            pk.add(fc2)
         o3 = pk.add(fc3)
         buf = pk.build(fc3.device)
         self.w12, self.w3 = buf[:o3].view(-1, fc1.shape[1]), buf[o3:].view(fc3.shape)
         self.norm_w = norm_w.detach().float().contiguous() if norm_w is not None else None
         self.norm_b = norm_b.detach().float().contiguous() if norm_b is not None else None
         self.struct = _lib.SwigluWeights(self.w12.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b),
-                                         fc1.shape[0])
+                                         self.hidden)
 
 
 def transition_generic(x: Tensor, w: TransitionGenericPacked, add_residual: bool = False,
                        out: Tensor | None = None) -> Tensor:
-    """Un-fused transition for the single track: LayerNorm/convert, fc1|fc2 GEMM, SwiGLU, fc3 GEMM (+ residual)."""
+    """Transition of any width for the single track: LayerNorm/convert, fc1|fc2 GEMM with SwiGLU, fc3 GEMM (+ residual)."""
     _require_cuda(x)
-    x = x.contiguous()
-    xb = x if (x.dtype == torch.bfloat16 and w.norm_w is None) else rows_to_bf16(
-        x, w.norm_w, w.norm_b, normalize=w.norm_w is not None)
-    h = swiglu(linear_bf16(xb, w.w12))
-    same_width = w.w3.shape[0] == x.shape[-1]
-    if add_residual and not same_width:
+    xd = _zdtype(x)
+    if x.shape[-1] != w.cols:
+        raise ValueError(f"expected x[..., {w.cols}], got {tuple(x.shape)}")
+    if add_residual and w.out_cols != w.cols:
         raise ValueError("the residual needs out_dim == dim")
-    return linear_bf16(h, w.w3, residual=x if add_residual else None, out_dtype=x.dtype, out=out)
+    if not x.is_contiguous():
+        if out is x:
+            raise ValueError("in-place update needs a contiguous tensor")
+        x = x.contiguous()
+    shape = x.shape[:-1] + (w.out_cols,)
+    if out is None:
+        out = x.clone() if add_residual else torch.empty(shape, dtype=x.dtype, device=x.device)
+    elif out.dtype != x.dtype or out.shape != shape or not out.is_contiguous():
+        raise ValueError("out must match the result in shape and dtype and be contiguous")
+    elif add_residual and out is not x:
+        out.copy_(x)
+    rows = x.numel() // w.cols
+    if rows == 0:
+        return out
+    nbytes = lib.b200_swiglu_transition_workspace_bytes(rows, w.cols, w.hidden)
+    ws = workspace(nbytes, x.device)
+    _lib.check(lib.b200_swiglu_transition_fwd(out.data_ptr() if add_residual else x.data_ptr(), out.data_ptr(),
+                                              ctypes.byref(w.struct), rows, w.cols, w.out_cols, 1 if add_residual else 0, xd,
+                                              ws.data_ptr(), nbytes, _stream()))
+    return out
 
 
 def attention_core(q: Tensor, k: Tensor, v: Tensor, bias: Tensor, key_mask: Tensor, gate: Tensor | None = None,

@@ -16,6 +16,7 @@ import torch
 import torch.nn as nn
 from torch import Tensor
 
+from . import _lib
 from . import functional as F
 from .attention_pair_bias import AttentionPairBias, AttentionPairBiasSlidingWindow
 from .transition import Transition
@@ -75,6 +76,7 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
         super().__init__()
         self.lns_scale = lns_scale
         self.dim = dim
+        self._windowed = is_sliding_window
         self.cond = nn.Sequential(nn.LayerNorm(dim_cond), nn.SiLU(), nn.Linear(dim_cond, 6 * dim))
         if is_sliding_window:
             assert window_queries is not None and window_keys is not None, (
@@ -87,23 +89,71 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
                                             attn_pair_bias_tile_size=attn_pair_bias_tile_size)
         self.transition = Transition(dim=dim, hidden=transition_hidden, use_norm=False)
 
-    def _pack_key(self):
-        return tuple((p.data_ptr(), p._version, str(p.device)) for p in self.cond.parameters())
-
     def _build_packed(self):
-        return (self.cond[2].weight.detach().to(torch.bfloat16).contiguous(),
-                self.cond[2].bias.detach().float().contiguous())
+        """The conditioning projection in kernel layout, and the native layer's weights where the layer fits it."""
+        lin, ln = self.cond[2], self.cond[0]
+        pk = F._Pack()
+        pk.add(lin.weight)
+        w_cond = pk.build(lin.weight.device).view(lin.weight.shape)
+        b_cond = lin.bias.detach().float().contiguous()
+        ln_w, ln_b = (None if p is None else p.detach().float().contiguous() for p in (ln.weight, ln.bias))
+        attn = self.attention.attention_layer.pair_bias_attn if self._windowed else self.attention.pair_bias_attn
+        tr = self.transition
+        native = None
+        if self.dim % 32 == 0 and lin.in_features % 8 == 0 and lin.in_features <= 1024 and not tr.use_norm and not attn.initial_norm \
+                and ln.eps == 1e-5 and tr.fc3.out_features == self.dim and (self._windowed or attn.c_z == 128):
+            layer = _lib.CondLayer()
+            ap, tp = attn.packed(), tr.packed()
+            layer.dim, layer.dim_cond, layer.heads, layer.dim_pairwise = self.dim, lin.in_features, attn.num_heads, attn.c_z
+            layer.lns_scale = self.lns_scale
+            layer.ln_c_w, layer.ln_c_b, layer.w_cond, layer.b_cond = F._ptr(ln_w), F._ptr(ln_b), w_cond.data_ptr(), b_cond.data_ptr()
+            if self._windowed:
+                layer.window_queries, layer.window_keys = attn.window_queries, attn.window_keys
+                layer.w_qkvg, layer.b_qkvg, layer.w_o = ap.w_qkvg.data_ptr(), ap.b_qkvg.data_ptr(), ap.w_o.data_ptr()
+                layer.ln_z_w, layer.ln_z_b, layer.w_z = ap.ln_z_w.data_ptr(), F._ptr(ap.ln_z_b), ap.w_z.data_ptr()
+            else:
+                layer.attention = ap.struct
+            if tr._fused:
+                layer.transition_fused = tp.struct
+            else:
+                layer.transition = tp.struct
+            native = (layer, (ap, tp, ln_w, ln_b))
+        return w_cond, b_cond, native
 
     def forward(self, x: Tensor, pairs: Tensor, c: Tensor, mask: Tensor | None = None, multiplicity: int = 1) -> Tensor:
         if mask is None:  # full attention: pairs [B, T, T, .]; windowed: x [B*M, atoms, .]
             n = x.shape[1] if pairs.ndim == 5 else pairs.shape[1]
             mask = torch.ones(pairs.shape[0], n, dtype=torch.bool, device=x.device)
-        return self._forward(x, pairs, c, mask, multiplicity, self.attention)
+        native = self.packed()[2]
+        if native is None:
+            return self._forward(x, pairs, c, mask, multiplicity, self.attention)
+        layer, B = native[0], pairs.shape[0]
+        if x.ndim != 3 or x.shape[0] != B * multiplicity or x.shape[2] != self.dim or tuple(mask.shape) != (B, x.shape[1]) \
+                or c.shape[:2] != x.shape[:2] or c.shape[2] != layer.dim_cond:
+            raise ValueError(f"x {tuple(x.shape)}, c {tuple(c.shape)}, pairs {tuple(pairs.shape)}, mask {tuple(mask.shape)}, "
+                             f"multiplicity={multiplicity}")
+        bias, N = None, x.shape[1]
+        if self._windowed:
+            W, Hk = layer.window_queries, layer.window_keys
+            if N % W:
+                raise ValueError(f"the atom count {N} is not a multiple of the query window {W}")
+            if pairs.numel() != B * N * Hk * layer.dim_pairwise:
+                raise ValueError(f"pairs {tuple(pairs.shape)} do not hold {N // W} windows of {W} x {Hk}")
+        else:
+            if tuple(pairs.shape) != (B, N, N, 128):
+                raise ValueError(f"expected pairs[{B},{N},{N},128], got {tuple(pairs.shape)}")
+            attn = self.attention.pair_bias_attn
+            if attn._bias_cache is not None:
+                bias = attn._bias_cache[0].lookup(attn._bias_cache[1], pairs)
+        sized = _lib.CondLayer.from_buffer_copy(layer)  # the layer's own copy may be in use by another thread
+        sized.B, sized.M, sized.N = B, multiplicity, N
+        return F.cond_layer(sized, x, pairs, bias, c, mask)
 
     def _forward(self, x: Tensor, pairs: Tensor, c: Tensor, mask: Tensor, multiplicity: int, attention) -> Tensor:
-        """The block with the attention supplied by the caller (``attention(tokens, pairs, mask, multiplicity)``): the
-        serial layer passes its own, the context-parallel wrapper the sharded one; everything else is per token."""
-        w_cond, b_cond = self.packed()
+        """The block with the attention supplied by the caller (``attention(tokens, pairs, mask, multiplicity)``), for the
+        context-parallel wrapper's sharded attention and for widths the native layer does not take; everything else is per
+        token."""
+        w_cond, b_cond, _ = self.packed()
         D = self.dim
         cn = F.rows_to_bf16(c, self.cond[0].weight, self.cond[0].bias, normalize=True, silu=True)
         cond = F.linear_bf16(cn, w_cond, b_cond, out_dtype=torch.float32)  # [rows, 6*dim] fp32

@@ -422,6 +422,10 @@ int b200_window_bias_fwd(const void* z, const float* ln_w, const float* ln_b, co
                          int64_t windows, int W, int Hk, int c_z, int heads, int z_dtype, b200_stream_t stream);
 int b200_window_attention_fwd(const void* qkv, const void* gate, const float* bias, const uint8_t* mask, void* out, int B,
                               int M, int NW, int W, int Hk, int heads, int head_dim, b200_stream_t stream);
+/* The same with q | k | v and gate as columns of wider rows (pitches in elements, multiples of 8). */
+int b200_window_attention_pitched_fwd(const void* qkv, int qkv_pitch, const void* gate, int gate_pitch, const float* bias,
+                                      const uint8_t* mask, void* out, int B, int M, int NW, int W, int Hk, int heads,
+                                      int head_dim, b200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------------
  * Pair-weighted averaging, PairWeightedAveraging.forward (src/bioemu2/biomoa/ops/pair_weighted_averaging.py:121-153),
@@ -473,15 +477,15 @@ int b200_ln_linear_fwd(const void* x1, const void* x2, const float* ln_w, const 
                        const float* residual, float* out, int64_t rows, int x_dtype, b200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------------
- * Builds bf16 kernel-layout weights from fp32 parameters in one launch: segment k writes groups * pitch elements at
- * dst + dst_off, taking `group` source elements times scale per group (src contiguous) and zeros in the rest of the pitch
- * (src == NULL: zeros only).  At most B200_PACK_MAX segments; counts and offsets are multiples of 8 elements.
+ * Builds bf16 kernel-layout weights from fp32 parameters in one launch: segment k writes `groups` runs of `pitch` elements at
+ * dst + dst_off, `stride` elements apart, taking `group` source elements times scale per run (src contiguous) and zeros for
+ * the rest of it (src == NULL: zeros only).  At most B200_PACK_MAX segments; counts and offsets are multiples of 8 elements.
  * ------------------------------------------------------------------------------------------------- */
 #define B200_PACK_MAX 24
 typedef struct {
   const float* src;
   int64_t dst_off;
-  int32_t groups, group, pitch;
+  int32_t groups, group, pitch, stride;
   float scale;
 } b200_pack_segment;
 
@@ -501,7 +505,8 @@ int b200_pack_bf16(const b200_pack_segment* segments, int n, void* dst, b200_str
  * side_stream may be NULL (or equal to stream): one stream, same results.
  *   b200_transition_weights  w13 bf16 [hidden/64][64 fc1 rows | 64 fc2 rows][128], w3 bf16 [128][hidden], LayerNorm fp32
  *                            [128]; hidden 256 or 512
- *   b200_swiglu_weights      w12 bf16 [2*hidden][c_s] (fc1 rows, then fc2 rows), w3 bf16 [c_s][hidden], LayerNorm fp32 [c_s]
+ *   b200_swiglu_weights      w12 bf16 [2*hidden][c_s]: 64 fc1 rows, 64 fc2 rows, and so on, when hidden is a multiple of 64,
+ *                            else all fc1 rows, then all fc2 rows; w3 bf16 [c_s][hidden], LayerNorm fp32 [c_s]
  * Workspaces: 1024-byte aligned; the side one is for side_stream's kernels.
  * ------------------------------------------------------------------------------------------------- */
 typedef struct {
@@ -537,6 +542,46 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
                    const uint8_t* token_mask, const uint8_t* pair_mask, int B, int N, int c_s, int heads, int s_dtype,
                    int z_dtype, void* workspace, size_t workspace_bytes, void* side_workspace, size_t side_bytes,
                    b200_stream_t stream, b200_stream_t side_stream);
+
+/* SwiGLU transition of any width (multiples of 8) in one call: out = fc3(silu(fc1(h)) * fc2(h)) with h = LayerNorm(x), or x
+ * when ln_w is NULL; add_residual: out == x, in place.  out has x's dtype.  Workspace 1024-byte aligned. */
+size_t b200_swiglu_transition_workspace_bytes(int64_t rows, int cols, int64_t hidden);
+int b200_swiglu_transition_fwd(const void* x, void* out, const b200_swiglu_weights* w, int64_t rows, int cols, int out_cols,
+                               int add_residual, int x_dtype, void* workspace, size_t workspace_bytes, b200_stream_t stream);
+
+/* ---------------------------------------------------------------------------------------------------
+ * ConditionedTransformerLayer.forward (src/bioemu2/biomoa/modules/transformer.py:231-353) in one call:
+ *   alpha1, beta1, gamma1, alpha2, beta2, gamma2 = w_cond . silu(LayerNorm(c)) + b_cond
+ *   out  = x + gamma1 * attention(lns * ((1 + alpha1) * LN(x) + beta1))
+ *   out += gamma2 * transition(lns * ((1 + alpha2) * LN(out) + beta2))
+ * x, out: [B*M][N][dim], c: [B*M][N][dim_cond], mask uint8 [B][N].  out may be x.
+ * window_queries == 0: full attention (weights `attention`) with pairs [B][N][N][128], or, with pairs == NULL, the bias as
+ * for b200_apb_fwd_bias.  Otherwise sliding-window attention: N atoms, pairs [B][N/W][W][window_keys][dim_pairwise], w_qkvg
+ * bf16 [4*dim][dim] (q | k | v | gate), b_qkvg fp32 [4*dim], w_o bf16 [dim][dim], w_z fp32 [heads][dim_pairwise].
+ * transition_fused (dim 128, no LayerNorm) where its w13 is given, else `transition` (ln_w NULL).
+ * ------------------------------------------------------------------------------------------------- */
+typedef struct {
+  int B, M, N, dim, dim_cond, heads, dim_pairwise, window_queries, window_keys;
+  float lns_scale;
+  const float* ln_c_w;
+  const float* ln_c_b;
+  const void* w_cond;
+  const float* b_cond;
+  b200_apb_weights attention;
+  const void* w_qkvg;
+  const float* b_qkvg;
+  const void* w_o;
+  const float* ln_z_w;
+  const float* ln_z_b;
+  const float* w_z;
+  b200_transition_weights transition_fused;
+  b200_swiglu_weights transition;
+} b200_cond_layer;
+
+size_t b200_cond_layer_workspace_bytes(const b200_cond_layer* layer);
+int b200_cond_layer_fwd(const b200_cond_layer* layer, const void* x, const void* pairs, const void* bias, int64_t bias_pitch,
+                        const void* c, const uint8_t* mask, void* out, int x_dtype, int c_dtype, int pairs_dtype,
+                        void* workspace, size_t workspace_bytes, b200_stream_t stream);
 
 #ifdef __cplusplus
 }
