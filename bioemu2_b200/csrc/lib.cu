@@ -119,7 +119,6 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   p.a_shared = a_shared ? 1 : 0;
   p.mul = a.mul;
   p.mul_pitch = a.mul_pitch;
-  p.swiglu = a.swiglu ? 1 : 0;
   // Bulk output through the C tensor map where the layout allows it (the map clips the last column group): the
   // residual (if any) being C itself, and for the transposed pair store lines that are whole row tiles.
   p.tma_c = 0;
@@ -152,12 +151,22 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
     return fail(B200_ERR_INVALID_ARGUMENT, "a gated product needs bulk output and 16-byte aligned factors");
   const int total = p.tiles_m * p.tiles_n * a.batch;
   const int grid = total < sm_count() ? total : sm_count();
+  auto go = [&](auto kernel, uint32_t smem) -> int {
+    B200_LAUNCH(kernel, grid, 192, smem, stream, tmA, tmB, tmC, p);
+    return 0;
+  };
   if (BN == 256) {
-    B200_LAUNCH(bmm_nt_kernel<256>, grid, 192, BmmCfg<256>::SMEM_BYTES, stream, tmA, tmB, tmC, p);
-  } else {
-    B200_LAUNCH(bmm_nt_kernel<128>, grid, 192, BmmCfg<128>::SMEM_BYTES, stream, tmA, tmB, tmC, p);
+    constexpr uint32_t smem = BmmCfg<256>::SMEM_BYTES;
+    if (a.opm_ntok > 0) return go(bmm_nt_kernel<256, kEpiOuter>, smem);
+    if (a.swiglu) return go(bmm_nt_kernel<256, kEpiSwiglu>, smem);
+    if (a.mul) return go(bmm_nt_kernel<256, kEpiMul>, smem);
+    return p.tma_c ? go(bmm_nt_kernel<256, kEpiBulk>, smem) : go(bmm_nt_kernel<256, kEpiDirect>, smem);
   }
-  return 0;
+  constexpr uint32_t smem = BmmCfg<128>::SMEM_BYTES;
+  if (a.opm_ntok > 0) return go(bmm_nt_kernel<128, kEpiOuter>, smem);
+  if (a.swiglu) return go(bmm_nt_kernel<128, kEpiSwiglu>, smem);
+  if (a.mul) return go(bmm_nt_kernel<128, kEpiMul>, smem);
+  return p.tma_c ? go(bmm_nt_kernel<128, kEpiBulk>, smem) : go(bmm_nt_kernel<128, kEpiDirect>, smem);
 }
 
 static int launch_rows_to_bf16(const void* x, bool f32, __nv_bfloat16* y, const float* w, const float* b,
