@@ -145,6 +145,11 @@ SIGNATURES = {
     "b200_gate_rows_f32": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int, c_int,
                                    c_void_p]),
     "b200_softmax_bias_f32": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
+    "b200_accurate_trimul_workspace_bytes": (c_size_t, [c_int]),
+    "b200_accurate_trimul_fwd": (c_int, [c_void_p] * 10 + [c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "b200_accurate_transition_workspace_bytes": (c_size_t, [c_int64, c_int, c_int]),
+    "b200_accurate_transition_fwd": (c_int, [c_void_p] * 6 + [c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t,
+                                             c_void_p]),
     "b200_masked_softmax_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "b200_pwa_gate": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "b200_gated_residual_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int, c_int, c_int,

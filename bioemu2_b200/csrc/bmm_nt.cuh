@@ -8,6 +8,8 @@
 //   warp 1      MMA issuer     (tcgen05.mma 128 x BN x 16, two accumulator buffers in TMEM)
 //   warps 2..5  epilogue       (TMEM -> registers -> bf16 -> global)
 #pragma once
+#include <climits>
+
 #include "row_tile.cuh"
 
 namespace b200 {
@@ -39,6 +41,9 @@ struct BmmParams {
   // before it is stored or added.
   const float* mul;
   int mul_pitch;
+  // Split operands stored once as (hi | lo): a K block at or past the fold is loaded from that many blocks before, which
+  // makes the operand hi | hi | lo.  INT_MAX: none.
+  int a_fold, b_fold;
   int a_shared;              // 1: every batch item multiplies the same A (the A tensor map has a single batch slice)
 };
 
@@ -63,7 +68,8 @@ enum BmmEpilogue : int {
   kEpiBulk = 1,    // scale, bias; bulk stores through C's tensor map
   kEpiMul = 2,     // bulk, with the element-wise factor
   kEpiSwiglu = 3,  // bulk bf16: the columns are pairs of 64-column blocks (a | b), C gets silu(a) * b, half as many columns
-  kEpiOuter = 4,   // outer products of 32 x 32, one pair's 2 KB in one piece
+  kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b, with expf and exact division
+  kEpiOuter = 5,   // outer products of 32 x 32, one pair's 2 KB in one piece
 };
 
 template <int BN, int EPI>
@@ -118,8 +124,8 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           mbar_wait(&empty[stage], phase ^ 1, 1);
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           mbar_arrive_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-          tma_load_3d(sa, &tmA, &full[stage], kb * 64, tm * 128, p.a_shared ? 0 : b);
-          tma_load_3d(sa + Cfg::A_BYTES, &tmB, &full[stage], kb * 64, tn * BN, b);
+          tma_load_3d(sa, &tmA, &full[stage], (kb < p.a_fold ? kb : kb - p.a_fold) * 64, tm * 128, p.a_shared ? 0 : b);
+          tma_load_3d(sa + Cfg::A_BYTES, &tmB, &full[stage], (kb < p.b_fold ? kb : kb - p.b_fold) * 64, tn * BN, b);
           if (++stage == Cfg::STAGES) {
             stage = 0;
             phase ^= 1;
@@ -213,6 +219,53 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             const int col = tn * (BN / 2) + (c >> 1) * 64;
             if (leader && col < p.n_valid / 2) {
               tma_store_3d(&tmC, stage, col, tm * 128, b);
+              tma_store_commit();
+            }
+          }
+        }
+        continue;
+      }
+      if constexpr (EPI == kEpiSwigluSplit) {
+        // As above, with the hi and the lo part of 64 output columns in the two staging tiles.
+        const int r = quarter * 32 + lane;
+        const bool leader = threadIdx.x == 64;
+        uint8_t* stage = smem + Cfg::OUT_OFFSET;
+#pragma unroll
+        for (int c = 0; c < BN / 64; ++c) {
+          const int a_col = (c >> 1) * 128 + (c & 1) * 32;
+          uint32_t va[32], vb[32];
+          tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + a_col), va);
+          tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + a_col + 64), vb);
+          tmem_ld_wait();
+          if (c + 1 == BN / 64) {
+            tc_fence_before_sync();
+            mbar_arrive(&acc_empty[acc]);
+          }
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const float a = __uint_as_float(va[e]);
+            va[e] = __float_as_uint(a / (1.f + expf(-a)) * __uint_as_float(vb[e]));
+          }
+          if ((c & 1) == 0) {
+            if (leader) tma_store_wait_read0();  // the stores that last used the staging tiles have read them
+            named_bar_sync(1, 128);
+          }
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              split_pair(__uint_as_float(va[g * 8 + 2 * e]), __uint_as_float(va[g * 8 + 2 * e + 1]), hi[e], lo[e]);
+            *reinterpret_cast<uint4*>(stage + sw128_offset(r, (c & 1) * 4 + g)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(stage + 16384 + sw128_offset(r, (c & 1) * 4 + g)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+          if (c & 1) {
+            fence_proxy_async_smem();
+            named_bar_sync(1, 128);
+            const int col = tn * (BN / 2) + (c >> 1) * 64;
+            if (leader && col < p.n_valid / 2) {
+              tma_store_3d(&tmC, stage, col, tm * 128, b);
+              tma_store_3d(&tmC, stage + 16384, p.n_valid / 2 + col, tm * 128, b);
               tma_store_commit();
             }
           }

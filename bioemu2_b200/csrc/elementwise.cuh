@@ -463,8 +463,8 @@ pwa_gate_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __rest
 // With the three pieces laid side by side along K -- (hi | hi | lo) for one operand, (hi | lo | hi) for the other --
 // that sum is ONE ordinary K-major product of width 3K, so the GEMM kernel needs no change.
 //
-// y[r] = split([LayerNorm](x[r])) : x fp32 [rows][cols] -> bf16 [rows][3*cols].  order 0 = (hi | hi | lo), 1 = (hi | lo | hi).
-// One warp per row; LayerNorm (fp32, two-pass) only for cols <= 1024.
+// y[r] = split([LayerNorm](x[r])) : x fp32 [rows][cols] -> bf16 [rows][3*cols].  order 0 = (hi | hi | lo), 1 = (hi | lo | hi),
+// 2 = (hi | lo) in rows of 2*cols.  One warp per row; LayerNorm (fp32, two-pass) only for cols <= 1024.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, const float* __restrict__ w,
                   const float* __restrict__ b, long long rows, int cols, float eps, int normalize, int order) {
@@ -494,7 +494,7 @@ split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, co
       }
       rstd = rsqrtf(warp_sum(ss) / float(cols) + eps);
     }
-    __nv_bfloat16* yr = y + r * 3 * (long long)cols;
+    __nv_bfloat16* yr = y + r * (order == 2 ? 2 : 3) * (long long)cols;
     for (int v = lane; v < nvec; v += 32) {
       float f[8], hi[8], lo[8];
       load8<true>(xr, v * 8, f);
@@ -510,7 +510,7 @@ split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, co
       }
       store8<false>(yr, v * 8, hi);
       store8<false>(yr + cols, v * 8, order ? lo : hi);
-      store8<false>(yr + 2 * cols, v * 8, order ? hi : lo);
+      if (order != 2) store8<false>(yr + 2 * cols, v * 8, order ? hi : lo);
     }
   }
 }

@@ -11,6 +11,7 @@
 #include "transition.cuh"
 #include "ln_linear.cuh"
 #include "elementwise.cuh"
+#include "accurate.cuh"
 #include "opm.cuh"
 #include "attention.cuh"
 #include "attention_resident.cuh"
@@ -59,6 +60,8 @@ struct BmmLaunch {
   const float* mul = nullptr;  // bulk output: per-element fp32 factor, row pitch mul_pitch
   int mul_pitch = 0;
   bool swiglu = false;  // bulk bf16 output: N columns are 64-wide (a | b) block pairs, C has N / 2 columns of silu(a) * b
+  bool split = false;   // with swiglu: C has N columns, (hi | lo) of the fp32 values
+  int a_fold = 0, b_fold = 0;  // operand stored as (hi | lo), each part this many K blocks of 64, read as hi | hi | lo
 };
 
 // Tile width by the estimated time of the busiest CTA.  A K block of 64 takes a 256-wide tile about 1.5 times as long as a
@@ -87,13 +90,13 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   CUtensorMap tmA, tmB;
   const bool a_shared = a.batch > 1 && a.sa == 0;  // one A for every batch item
   {
-    const uint64_t dims[3] = {uint64_t(a.K), uint64_t(a.M), uint64_t(a_shared ? 1 : a.batch)};
+    const uint64_t dims[3] = {uint64_t(a.a_fold ? a.a_fold * 128 : a.K), uint64_t(a.M), uint64_t(a_shared ? 1 : a.batch)};
     const uint64_t str[2] = {uint64_t(a.lda) * 2, uint64_t(a.sa > 0 ? a.sa : a.lda * a.M) * 2};
     const uint32_t box[3] = {64, 128, 1};
     if (int e = make_tmap_bf16(&tmA, a.A, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   {
-    const uint64_t dims[3] = {uint64_t(a.K), uint64_t(a.N), uint64_t(a.batch)};
+    const uint64_t dims[3] = {uint64_t(a.b_fold ? a.b_fold * 128 : a.K), uint64_t(a.N), uint64_t(a.batch)};
     const uint64_t str[2] = {uint64_t(a.ldb) * 2, uint64_t(a.sb > 0 ? a.sb : a.ldb * a.N) * 2};
     const uint32_t box[3] = {64, uint32_t(BN), 1};
     if (int e = make_tmap_bf16(&tmB, a.B, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
@@ -117,6 +120,8 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   p.remap_n = a.remap_n;
   p.remap_m = a.remap_m > 0 ? a.remap_m : a.remap_n;
   p.a_shared = a_shared ? 1 : 0;
+  p.a_fold = a.a_fold ? a.a_fold : INT_MAX;
+  p.b_fold = a.b_fold ? a.b_fold : INT_MAX;
   p.mul = a.mul;
   p.mul_pitch = a.mul_pitch;
   // Bulk output through the C tensor map where the layout allows it (the map clips the last column group): the
@@ -131,7 +136,7 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
       (a.remap_n == 0 || (a.remap_n % 128 == 0 && a.batch == 1 && a.M == a.remap_n * p.remap_m))) {
     uint64_t dims[3], str[2];
     uint32_t box[3];
-    dims[0] = uint64_t(a.swiglu ? a.N / 2 : a.N);
+    dims[0] = uint64_t(a.swiglu && !a.split ? a.N / 2 : a.N);
     box[0] = uint32_t(c_cols);
     if (a.remap_n > 0) {  // {column, line, pos}: pair (line, pos) lives in row pos * remap_m + line
       dims[1] = uint64_t(p.remap_m), dims[2] = uint64_t(a.remap_n);
@@ -158,13 +163,13 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   if (BN == 256) {
     constexpr uint32_t smem = BmmCfg<256>::SMEM_BYTES;
     if (a.opm_ntok > 0) return go(bmm_nt_kernel<256, kEpiOuter>, smem);
-    if (a.swiglu) return go(bmm_nt_kernel<256, kEpiSwiglu>, smem);
+    if (a.swiglu) return a.split ? go(bmm_nt_kernel<256, kEpiSwigluSplit>, smem) : go(bmm_nt_kernel<256, kEpiSwiglu>, smem);
     if (a.mul) return go(bmm_nt_kernel<256, kEpiMul>, smem);
     return p.tma_c ? go(bmm_nt_kernel<256, kEpiBulk>, smem) : go(bmm_nt_kernel<256, kEpiDirect>, smem);
   }
   constexpr uint32_t smem = BmmCfg<128>::SMEM_BYTES;
   if (a.opm_ntok > 0) return go(bmm_nt_kernel<128, kEpiOuter>, smem);
-  if (a.swiglu) return go(bmm_nt_kernel<128, kEpiSwiglu>, smem);
+  if (a.swiglu) return a.split ? go(bmm_nt_kernel<128, kEpiSwigluSplit>, smem) : go(bmm_nt_kernel<128, kEpiSwiglu>, smem);
   if (a.mul) return go(bmm_nt_kernel<128, kEpiMul>, smem);
   return p.tma_c ? go(bmm_nt_kernel<128, kEpiBulk>, smem) : go(bmm_nt_kernel<128, kEpiDirect>, smem);
 }
@@ -1714,6 +1719,112 @@ static int swiglu_transition(const void* x, bool x_f32, void* out, bool out_f32,
   b.mul = mul;
   b.mul_pitch = mul_pitch;
   return launch_bmm(b, stream);
+}
+
+// Accurate triangle multiplication: hs | ts (hi | lo rows), a | b (three parts), and one fp32 region that holds the channel-
+// major projection, then t, the projected t and the gate logits, a quarter each.
+static size_t accurate_rows_bytes(int N) { return round_up_1k(size_t(N) * ((N + 7) / 8 * 8) * 256 * 2); }
+static size_t accurate_operand_bytes(int N) { return round_up_1k(size_t(128) * N * 3 * ((N + 7) / 8 * 8) * 2); }
+
+size_t b200_accurate_trimul_workspace_bytes(int N) {
+  if (N <= 0) return 0;
+  return accurate_rows_bytes(N) + 2 * accurate_operand_bytes(N) + 4 * accurate_rows_bytes(N);
+}
+
+int b200_accurate_trimul_fwd(const float* z, const uint8_t* mask, float* out, const void* w_in, const void* w_p_out,
+                             const void* w_g_out, const float* ln_in_w, const float* ln_in_b, const float* ln_out_w,
+                             const float* ln_out_b, int N, int incoming, int add_residual, void* workspace,
+                             size_t workspace_bytes, b200_stream_t stream_) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(z && mask && out && w_in && w_p_out && w_g_out && ln_in_w && ln_in_b && ln_out_w && ln_out_b,
+                 "an argument is NULL");
+  B200_CHECK_ARG(N > 0 && N <= 32768, "N=%d out of range", N);
+  B200_CHECK_ARG(aligned(z, 32) && aligned(out, 16) && aligned(w_in, 16) && aligned(w_p_out, 16) && aligned(w_g_out, 16),
+                 "z must be 32-byte aligned, out and the weights 16-byte aligned");
+  B200_CHECK_ARG(workspace && aligned(workspace, 1024) && workspace_bytes >= b200_accurate_trimul_workspace_bytes(N),
+                 "workspace missing, misaligned or too small");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  const int pitch = (N + 7) / 8 * 8;
+  const int64_t rows = int64_t(N) * pitch, pairs = int64_t(N) * N;
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  __nv_bfloat16* hs = reinterpret_cast<__nv_bfloat16*>(ws);
+  __nv_bfloat16* a = reinterpret_cast<__nv_bfloat16*>(ws + accurate_rows_bytes(N));
+  __nv_bfloat16* b = a + accurate_operand_bytes(N) / 2;
+  __nv_bfloat16* ts = a;  // after the contraction has read a
+  uint8_t* f = ws + accurate_rows_bytes(N) + 2 * accurate_operand_bytes(N);
+  float* pg = reinterpret_cast<float*>(f);
+  float* t = pg;
+  float* po = reinterpret_cast<float*>(f + accurate_rows_bytes(N));
+  float* go = reinterpret_cast<float*>(f + 2 * accurate_rows_bytes(N));
+  // incoming walks the pairs column by column: (line, pos) is pair (pos, line)
+  const long long ls = incoming ? 1 : N, ps = incoming ? N : 1;
+  B200_LAUNCH(ln_split128_kernel, grid_for(rows, 32), 256, 0, stream, z, hs, ln_in_w, ln_in_b, (long long)rows, N, pitch, ls,
+              ps, 1);
+  {
+    BmmLaunch m{w_in, hs, pg, 1, 512, int(rows), 384, 384, 256, rows, 0, 0, 0};
+    m.out_f32 = 1;
+    m.b_fold = 2;
+    if (int e = launch_bmm(m, stream)) return e;
+  }
+  B200_LAUNCH(gate_split_kernel, dim3(unsigned((rows / 8 + 255) / 256), 32), 256, 0, stream, pg, mask, a, b, N, N, pitch, ls, ps);
+  {
+    const int64_t k3 = 3 * int64_t(pitch);
+    BmmLaunch m{a, b, t, 128, N, N, int(k3), k3, k3, pitch, N * k3, N * k3, int64_t(N) * pitch};
+    m.out_f32 = 1;
+    if (int e = launch_bmm(m, stream)) return e;
+  }
+  B200_LAUNCH(ln_split_channels_kernel, dim3((N + 31) / 32, N), 256, 0, stream, t, ts, ln_out_w, ln_out_b, N, N, pitch);
+  {
+    BmmLaunch m{ts, w_p_out, po, 1, int(pairs), 128, 384, 256, 384, 128, 0, 0, 0};
+    m.out_f32 = 1;
+    m.a_fold = 2;
+    if (int e = launch_bmm(m, stream)) return e;
+    m.A = hs, m.B = w_g_out, m.C = go, m.M = int(rows);
+    if (int e = launch_bmm(m, stream)) return e;
+  }
+  B200_LAUNCH(gate_pairs_kernel, grid_for(pairs * 32, 256), 256, 0, stream, po, go, add_residual ? z : nullptr, out, N, pitch,
+              incoming);
+  return B200_OK;
+}
+
+size_t b200_accurate_transition_workspace_bytes(int64_t rows, int cols, int hidden) {
+  if (rows <= 0 || cols <= 0 || hidden <= 0) return 0;
+  return round_up_1k(size_t(rows) * cols * 4) + size_t(rows) * hidden * 4;
+}
+
+int b200_accurate_transition_fwd(const float* x, float* out, const void* w12, const void* w3, const float* ln_w,
+                                 const float* ln_b, int64_t rows, int cols, int hidden, int out_cols, int normalize,
+                                 int add_residual, void* workspace, size_t workspace_bytes, b200_stream_t stream_) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(x && out && w12 && w3, "x/out/w12/w3 is NULL");
+  B200_CHECK_ARG(rows >= 0 && rows < (int64_t(1) << 31), "rows out of range");
+  B200_CHECK_ARG(cols > 0 && cols <= 1024 && cols % 64 == 0 && hidden > 0 && hidden % 64 == 0 && out_cols > 0 && out_cols % 8 == 0,
+                 "cols=%d and hidden=%d must be multiples of 64 (cols <= 1024), out_cols=%d of 8", cols, hidden, out_cols);
+  B200_CHECK_ARG(!add_residual || out_cols == cols, "a residual needs out_cols == cols");
+  B200_CHECK_ARG(aligned(x, 32) && aligned(out, 16) && aligned(w12, 16) && aligned(w3, 16),
+                 "x must be 32-byte aligned, out and the weights 16-byte aligned");
+  if (rows == 0) return B200_OK;
+  B200_CHECK_ARG(workspace && aligned(workspace, 1024) &&
+                     workspace_bytes >= b200_accurate_transition_workspace_bytes(rows, cols, hidden),
+                 "workspace missing, misaligned or too small");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  __nv_bfloat16* xs = static_cast<__nv_bfloat16*>(workspace);
+  __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(static_cast<uint8_t*>(workspace) + round_up_1k(size_t(rows) * cols * 4));
+  if (cols == 128) {  // rows that fit a warp's registers, four at a time
+    B200_LAUNCH(ln_split128_kernel, grid_for(rows, 32), 256, 0, stream, x, xs, ln_w, ln_b, (long long)rows, int(rows),
+                int(rows), 0ll, 1ll, normalize);
+  } else {
+    B200_LAUNCH(split_rows_kernel, grid_for(rows, 8), 256, 0, stream, x, xs, ln_w, ln_b, rows, cols, 1e-5f, normalize, 2);
+  }
+  BmmLaunch m{xs, w12, h, 1, int(rows), 2 * hidden, 3 * cols, 2 * cols, 3 * cols, 2 * hidden, 0, 0, 0};
+  m.swiglu = m.split = true;
+  m.a_fold = cols / 64;
+  if (int e = launch_bmm(m, stream)) return e;
+  BmmLaunch o{h, w3, out, 1, int(rows), out_cols, 3 * hidden, 2 * hidden, 3 * hidden, out_cols, 0, 0, 0};
+  o.out_f32 = 1;
+  o.a_fold = hidden / 64;
+  o.residual = add_residual ? x : nullptr;
+  return launch_bmm(o, stream);
 }
 
 size_t b200_swiglu_transition_workspace_bytes(int64_t rows, int cols, int64_t hidden) {

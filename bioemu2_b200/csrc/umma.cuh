@@ -521,4 +521,13 @@ __device__ __forceinline__ float bf16hi(uint32_t u) { return __uint_as_float(u &
 
 
 
+// hi = bf16(v), lo = bf16(v - hi) of two neighbours.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const float2 f = __bfloat1622float2(h);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
+  hi = reinterpret_cast<const uint32_t&>(h);
+  lo = reinterpret_cast<const uint32_t&>(l);
+}
+
 }  // namespace b200

@@ -6,9 +6,8 @@ denoiser, biomoa/models/score_model.py:355) and offers ``matmul_precision="ieee"
 (triangle_multiplication.py:119-136).  Here an fp32 value travels as ``hi = bf16(x)``, ``lo = bf16(x - hi)``; one operand
 is laid out along K as ``(hi | hi | lo)``, the other as ``(hi | lo | hi)``, and the ordinary tcgen05 GEMM of width 3K
 accumulates ``hi.hi + hi.lo + lo.hi`` in fp32 (relative error of a product ~2^-16).  LayerNorm, gates, SwiGLU and the
-softmax run in fp32 with exact exponentials.  The compositions below are un-fused -- every intermediate goes through
-HBM and the layout changes between pair-major and channel-major tensors are plain tensor permutes -- because this mode
-exists for the 1e-4 accuracy contract, not for speed; the bf16 path is the fast one.
+softmax run in fp32 with exact exponentials.  Triangle multiplication and the transition are one native call each; the
+attention and the outer product mean are un-fused compositions with plain tensor permutes between their products.
 """
 from __future__ import annotations
 
@@ -23,7 +22,7 @@ from ._lib import lib
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return F._stream()
 
 
 def split(x: Tensor, order: int, ln_w: Tensor | None = None, ln_b: Tensor | None = None, normalize: bool = False,
@@ -79,40 +78,81 @@ class SplitWeights:
         for k, v in weights.items():
             setattr(self, k, split(v.detach(), 1))
 
+    def norms(self, **norms) -> "SplitWeights":
+        """fp32 weight and bias of LayerNorms (``None``: none), kept as ``<name>_w`` and ``<name>_b``."""
+        for k, n in norms.items():
+            for s, p in (("_w", getattr(n, "weight", None)), ("_b", getattr(n, "bias", None))):
+                setattr(self, k + s, None if p is None else p.detach().float().contiguous())
+        return self
+
+
+def transition_weights(norm, fc1, fc2, fc3) -> SplitWeights:
+    """fc1 | fc2, or their 64-row blocks in turn where the native transition takes the widths (whole K blocks of 64)."""
+    hidden, dim = fc1.weight.shape
+    native = hidden % 64 == 0 and dim % 64 == 0
+    if native:
+        w12 = torch.stack([fc1.weight.view(hidden // 64, 64, dim), fc2.weight.view(hidden // 64, 64, dim)], dim=1)
+    else:
+        w12 = torch.cat([fc1.weight, fc2.weight], dim=0)
+    ws = SplitWeights(w12=w12.reshape(2 * hidden, dim), w3=fc3.weight).norms(norm=norm)
+    ws.native = native
+    return ws
+
+
+def _workspace(nbytes: int, device: torch.device) -> tuple[Tensor, int]:
+    """A buffer for one call and its first 1024-byte aligned address: these workspaces are several times the pair tensor, so
+    they go back to torch's allocator instead of staying with the thread."""
+    buf = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
+    return buf, (buf.data_ptr() + 1023) // 1024 * 1024
+
 
 # ------------------------------------------------------------------------------------------------------ the ops
-def transition(x: Tensor, norm, fc1, fc2, fc3, ws: SplitWeights, add_residual: bool = False) -> Tensor:
+def transition(x: Tensor, norm, fc1, fc2, fc3, ws: SplitWeights, add_residual: bool = False,
+               out: Tensor | None = None) -> Tensor:
+    """``out`` (fp32, contiguous): where the result goes; it may be ``x``."""
     shape = x.shape
     x2 = x.float().contiguous().view(-1, shape[-1])
+    hidden, out_cols = ws.w3.shape[1] // 3, ws.w3.shape[0]
+    rows, cols = x2.shape
+    if out is not None and not (out.is_contiguous() and out.dtype == torch.float32):
+        return out.copy_(transition(x, norm, fc1, fc2, fc3, ws, add_residual))
+    if getattr(ws, "native", False):
+        if out is None:
+            out = torch.empty(shape[:-1] + (out_cols,), dtype=torch.float32, device=x.device)
+        nbytes = lib.b200_accurate_transition_workspace_bytes(rows, cols, hidden)
+        buf, work = _workspace(nbytes, x.device)
+        _lib.check(lib.b200_accurate_transition_fwd(
+            x2.data_ptr(), out.data_ptr(), ws.w12.data_ptr(), ws.w3.data_ptr(), F._ptr(ws.norm_w), F._ptr(ws.norm_b), rows,
+            cols, hidden, out_cols, 0 if norm is None else 1, 1 if add_residual else 0, work, nbytes, _stream()))
+        return out
     xs = split(x2, 0, norm.weight if norm is not None else None, norm.bias if norm is not None else None,
                normalize=norm is not None)
     h12 = linear32(xs, ws.w12)
-    hidden = h12.shape[-1] // 2
     h = gate(h12[:, :hidden], h12[:, hidden:], 1)
-    out = linear32(split(h, 0), ws.w3, residual=x2 if add_residual else None)
-    return out.view(shape[:-1] + (out.shape[-1],))
+    y = linear32(split(h, 0), ws.w3, residual=x2 if add_residual else None).view(shape[:-1] + (out_cols,))
+    return y if out is None else out.copy_(y)
 
 
-def triangle_multiplication(x: Tensor, mask: Tensor, mod, ws: SplitWeights) -> Tensor:
+def triangle_multiplication(x: Tensor, mask: Tensor, mod, ws: SplitWeights, add_residual: bool = False,
+                            out: Tensor | None = None) -> Tensor:
+    """``out`` (fp32, contiguous): where the result goes; it may be ``x``."""
     B, N, _, D = x.shape
-    outs = []
-    Nk = (N + 7) // 8 * 8
+    if out is not None and not (out.is_contiguous() and out.dtype == torch.float32):
+        return out.copy_(triangle_multiplication(x, mask, mod, ws, add_residual))
+    if not hasattr(ws, "norm_in_w"):
+        ws.norms(norm_in=mod.norm_in, norm_out=mod.norm_out)
+    x, m8 = x.float().contiguous(), F.mask_u8(mask)
+    if out is None:
+        out = torch.empty_like(x)
+    nbytes = lib.b200_accurate_trimul_workspace_bytes(N)
+    buf, work = _workspace(nbytes, x.device)
     for b in range(B):
-        xb = x[b].float().contiguous().view(N * N, D)
-        hs = split(xb, 0, mod.norm_in.weight, mod.norm_in.bias, normalize=True)
-        pg = linear32(hs, ws.w_in)                                     # [P, 4D]: p_in | g_in
-        ab = gate(pg[:, :2 * D], pg[:, 2 * D:], 0, rowmask=mask[b]).view(N, N, 2 * D)
-        perm = (2, 1, 0) if mod.mode == "incoming" else (2, 0, 1)       # -> [d][i or j][k]
-        a_t = torch.zeros(D, Nk, Nk, dtype=torch.float32, device=x.device)
-        b_t = torch.zeros(D, Nk, Nk, dtype=torch.float32, device=x.device)
-        a_t[:, :N, :N] = ab[:, :, :D].permute(*perm)
-        b_t[:, :N, :N] = ab[:, :, D:].permute(*perm)
-        t = torch.empty(D, Nk, Nk, dtype=torch.float32, device=x.device)
-        F.bmm_nt_into(split(a_t, 0), split(b_t, 1), t)                 # t[d][i][j] = sum_k a.b, fp32
-        tp = t[:, :N, :N].permute(1, 2, 0).contiguous().view(N * N, D)
-        ts = split(tp, 0, mod.norm_out.weight, mod.norm_out.bias, normalize=True)
-        outs.append(gate(linear32(ts, ws.w_p_out), linear32(hs, ws.w_g_out), 0).view(N, N, D))
-    return torch.stack(outs)
+        _lib.check(lib.b200_accurate_trimul_fwd(
+            x[b].data_ptr(), m8[b].data_ptr(), out[b].data_ptr(), ws.w_in.data_ptr(), ws.w_p_out.data_ptr(),
+            ws.w_g_out.data_ptr(), ws.norm_in_w.data_ptr(), ws.norm_in_b.data_ptr(), ws.norm_out_w.data_ptr(),
+            ws.norm_out_b.data_ptr(), N, 1 if mod.mode == "incoming" else 0, 1 if add_residual else 0, work, nbytes,
+            _stream()))
+    return out
 
 
 def outer_product_mean(m: Tensor, mask: Tensor, mod, ws: SplitWeights) -> Tensor:

@@ -38,13 +38,11 @@ class Transition(PackedWeightsMixin, nn.Module):
                    self.fc1.weight, self.fc2.weight, self.fc3.weight)
 
     def _build_split(self):
-        import torch
+        return ieee.transition_weights(self.norm if self.use_norm else None, self.fc1, self.fc2, self.fc3)
 
-        return ieee.SplitWeights(w12=torch.cat([self.fc1.weight, self.fc2.weight], dim=0), w3=self.fc3.weight)
-
-    def _ieee(self, x: Tensor, add_residual: bool) -> Tensor:
+    def _ieee(self, x: Tensor, add_residual: bool, out: Tensor | None = None) -> Tensor:
         return ieee.transition(x, self.norm if self.use_norm else None, self.fc1, self.fc2, self.fc3, self.split_weights(),
-                               add_residual)
+                               add_residual, out)
 
     def forward(self, x: Tensor) -> Tensor:
         if precision.use_ieee(None, x):
@@ -56,7 +54,7 @@ class Transition(PackedWeightsMixin, nn.Module):
     def forward_residual_(self, x: Tensor) -> Tensor:
         """``x += forward(x)`` in place, fused into the kernel's final store; returns ``x``."""
         if precision.use_ieee(None, x):
-            return x.copy_(self._ieee(x, True))
+            return self._ieee(x, True, x)
         if self._fused:
             return F.transition(x, self.packed(), add_residual=True, out=x)
         return F.transition_generic(x, self.packed(), add_residual=True, out=x)

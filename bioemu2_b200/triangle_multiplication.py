@@ -111,7 +111,8 @@ class TriangleMultiplication(PackedWeightsMixin, nn.Module):
 
     def _build_split(self):
         return ieee.SplitWeights(w_in=torch.cat([self.p_in.weight, self.g_in.weight], dim=0),
-                                 w_p_out=self.p_out.weight, w_g_out=self.g_out.weight)
+                                 w_p_out=self.p_out.weight, w_g_out=self.g_out.weight
+                                 ).norms(norm_in=self.norm_in, norm_out=self.norm_out)
 
     def forward(self, x: Tensor, mask: Tensor) -> Tensor:
         """``x[B,N,N,dim]``, ``mask[B,N,N]`` -> update ``[B,N,N,dim]`` (no residual, like the reference)."""
@@ -122,7 +123,7 @@ class TriangleMultiplication(PackedWeightsMixin, nn.Module):
     def forward_residual_(self, x: Tensor, mask: Tensor) -> Tensor:
         """``x += forward(x, mask)`` in place with the add fused into the output kernel; returns ``x``."""
         if precision.use_ieee(self.matmul_precision, x):
-            return x.add_(ieee.triangle_multiplication(x, mask, self, self.split_weights()))
+            return ieee.triangle_multiplication(x, mask, self, self.split_weights(), add_residual=True, out=x)
         return F.trimul(x, mask, self.packed(), incoming=self.mode == "incoming", add_residual=True, out=x)
 
 

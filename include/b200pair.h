@@ -467,6 +467,21 @@ int b200_gate_rows_f32(const float* a, int64_t a_pitch, const float* b, int64_t 
 int b200_softmax_bias_f32(float* s, const float* bias, const uint8_t* keymask, int64_t groups, int n, int H, int bias_div,
                           b200_stream_t stream);
 
+/* Triangle multiplication in the accurate form, one batch item: z fp32 [N][N][128], mask [N][N], out may be z.  w_in = split
+ * (order 1) of p_in | g_in [512][384], w_p_out and w_g_out [128][384].  Workspace 1024-byte aligned. */
+size_t b200_accurate_trimul_workspace_bytes(int N);
+int b200_accurate_trimul_fwd(const float* z, const uint8_t* mask, float* out, const void* w_in, const void* w_p_out,
+                             const void* w_g_out, const float* ln_in_w, const float* ln_in_b, const float* ln_out_w,
+                             const float* ln_out_b, int N, int incoming, int add_residual, void* workspace,
+                             size_t workspace_bytes, b200_stream_t stream);
+
+/* SwiGLU transition in the accurate form: out = [x +] fc3(silu(fc1(h)) * fc2(h)), h = LayerNorm(x) or x; out may be x.  cols
+ * and hidden multiples of 64; w12 = split (order 1) of the 64-row blocks of fc1 and fc2 in turn, w3 = split of fc3. */
+size_t b200_accurate_transition_workspace_bytes(int64_t rows, int cols, int hidden);
+int b200_accurate_transition_fwd(const float* x, float* out, const void* w12, const void* w3, const float* ln_w,
+                                 const float* ln_b, int64_t rows, int cols, int hidden, int out_cols, int normalize,
+                                 int add_residual, void* workspace, size_t workspace_bytes, b200_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------------------
  * out = W . LayerNorm(x1 | x2) [+ residual] in one pass: rows of 128 channels (x2 == NULL) or 128 + 128, W bf16
  * [128][128 or 256], out and residual fp32 [rows][128] (out may be residual), ln_w / ln_b fp32 or NULL.  The input projection
