@@ -188,6 +188,119 @@ struct RowTile {
   }
 };
 
+// The same share of a tile as a stream: the rows are loaded, normalised and written in G groups, and a group's loads for
+// the next tile go out as soon as it has been written, so that (G - 1) / G of a tile's rows are always on their way while
+// the rest is being normalised.  (RowTile, which keeps a normalised tile in registers, has nothing on its way during its
+// arithmetic: it took trimul_in_kernel's producers 9,500 clocks a tile.)
+// A thread has rows first + i * step, i < G * R, as far as they are below 128.
+template <bool F32, int G, int R>
+struct RowStream {
+  static constexpr int W = F32 ? 8 : 4;
+  uint32_t raw[G * R][W];  // as loaded: converting here would wait for the load
+  uint4 v[R];
+  int c16, first, step;
+
+  template <class RowPtr>
+  __device__ __forceinline__ void load(int g, RowPtr row_ptr) {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const void* src = row_ptr(first + (g * R + q) * step);
+      uint32_t(&w)[W] = raw[g * R + q];
+      if (src) {
+        const uint32_t* a = static_cast<const uint32_t*>(src) + c16 * W;
+        if constexpr (F32) {
+          asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                       : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                       : "l"(a)
+                       : "memory");
+        } else {
+          asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                       : "l"(a)
+                       : "memory");
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < W; ++i) w[i] = 0;
+      }
+    }
+  }
+
+  // The raw rows of a group, stored at their address + delta bytes.
+  template <class RowPtr>
+  __device__ __forceinline__ void copy(int g, RowPtr row_ptr, long long delta) const {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const void* src = row_ptr(first + (g * R + q) * step);
+      const uint32_t(&w)[W] = raw[g * R + q];
+      if (src) {
+        uint4* a = reinterpret_cast<uint4*>(const_cast<uint8_t*>(static_cast<const uint8_t*>(src)) + delta + c16 * W * 4);
+#pragma unroll
+        for (int i = 0; i < W / 4; ++i) a[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+      }
+    }
+  }
+
+  // LayerNorm of a group's rows into v: one pass, in lock step (see RowTile).
+  __device__ __forceinline__ void normalize(int g, const float (&gamma)[8], const float (&beta)[8], float eps) {
+    float x[R][8], s1[R], s2[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      float* xr = x[q];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t w = raw[g * R + q][F32 ? i : i >> 1];
+        xr[i] = F32 ? __uint_as_float(w) : (i & 1) ? bf16hi(w) : bf16lo(w);
+      }
+      float a0 = xr[0], a1 = xr[1], b0, b1;
+      add_f32x2(a0, a1, xr[2], xr[3]);
+      add_f32x2(a0, a1, xr[4], xr[5]);
+      add_f32x2(a0, a1, xr[6], xr[7]);
+      mul_f32x2(b0 = xr[0], b1 = xr[1], xr[0], xr[1]);
+      fma_f32x2(b0, b1, xr[2], xr[3], xr[2], xr[3], b0, b1);
+      fma_f32x2(b0, b1, xr[4], xr[5], xr[4], xr[5], b0, b1);
+      fma_f32x2(b0, b1, xr[6], xr[7], xr[6], xr[7], b0, b1);
+      s1[q] = a0 + a1;
+      s2[q] = b0 + b1;
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const float o1 = __shfl_xor_sync(0xffffffffu, s1[q], off);
+        const float o2 = __shfl_xor_sync(0xffffffffu, s2[q], off);
+        add_f32x2(s1[q], s2[q], o1, o2);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      float* xr = x[q];
+      const float mean = s1[q] * (1.0f / kD);
+      const float var = fmaxf(fmaf(-mean, mean, s2[q] * (1.0f / kD)), 0.f);
+      const float rstd = rsqrtf(var + eps);
+      const float nmr = -mean * rstd;
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        float g0 = gamma[i], g1 = gamma[i + 1], b0, b1;
+        fma_f32x2(b0, b1, g0, g1, nmr, nmr, beta[i], beta[i + 1]);  // beta - mean * rstd * gamma
+        mul_f32x2(g0, g1, rstd, rstd);                              // rstd * gamma
+        fma_f32x2(xr[i], xr[i + 1], xr[i], xr[i + 1], g0, g1, b0, b1);
+      }
+      v[q] = make_uint4(pack_bf16x2(xr[0], xr[1]), pack_bf16x2(xr[2], xr[3]), pack_bf16x2(xr[4], xr[5]), pack_bf16x2(xr[6], xr[7]));
+    }
+  }
+
+  // v into the operand tile at dst.
+  __device__ __forceinline__ void store(int g, uint8_t* dst) const {
+    uint8_t* half = dst + (c16 >> 3) * kOperandHalf;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int r = first + (g * R + q) * step;
+      if (r < 128) *reinterpret_cast<uint4*>(half + sw128_offset(r, c16 & 7)) = v[q];
+    }
+  }
+};
+
 // scale multiplies the LayerNorm output; a power of two keeps the result a bit-exact multiple.
 __device__ __forceinline__ void load_gamma_beta(const float* w, const float* b, int pt, float (&gamma)[8],
                                                 float (&beta)[8], float scale = 1.0f) {

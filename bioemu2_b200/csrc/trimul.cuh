@@ -44,15 +44,16 @@ constexpr uint32_t BAR_OFF = MASK_OFF + 4 * 128;
 constexpr uint32_t FLAG_OFF = BAR_OFF + 96;          // 4 stages x 4 "every pair of this quarter valid" bytes
 constexpr uint32_t STAGE_OFF = MASK_OFF + 1024;      // per epilogue group a 16 KB tile [128 channels][64 pairs]
 constexpr uint32_t SMEM_BYTES = STAGE_OFF + 2 * kOperandHalf + 1024;
-constexpr int THREADS = 512;  // warps 0-3 epilogue of a, 4-7 epilogue of b (their first threads issue the MMAs), 8-15 producers
+constexpr int THREADS = 512;  // warps 0-3 epilogue of pairs 0-63, 4-7 of pairs 64-127, 8-15 producers (8 issues the MMAs)
 }  // namespace trimul_in
 
 // The LayerNorm output is halved (exactly) before the projections, so the accumulators hold p/2 and g/2
 // and the gate is p * sigmoid(g) = p/2 + p/2 * tanh(g/2): one MUFU and one FMA per element.
 // 512 threads, not 544: a 17th warp would round the register allocation up to 640 threads and cap every
-// thread at 96 registers, which the LayerNorm producers spill at.  So there is no control warp: the first
-// thread of each epilogue group issues the two products of its own half (whose accumulators it has just
-// drained), and shared stage x is released when both have committed.
+// thread at 96 registers, which the LayerNorm producers spill at.  So there is no control warp: one of the producers issues.
+// p and g of one half (a or b) are 256 TMEM columns, so the two halves of a tile double-buffer each other: both epilogue
+// groups drain a half together, 64 pairs each, while the other half's products run (with a group per half, whose products
+// had to wait for its own drain, a tile was a chain of products, drain and store: 78.5 us at N = 512).
 // COPY: the producers also store the raw rows at z_copy_delta from their source.  The first op of a stack that leaves its
 // input alone gets its working copy this way, for the write alone (N = 384: 26 us as a copy of its own before the stack).
 template <bool F32, bool COPY>
@@ -79,9 +80,9 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     mbar_init(w_full, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&x_full[i], 256);
-      mbar_init(&x_empty[i], 2);
+      mbar_init(&x_empty[i], 1);
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], 128);
+      mbar_init(&acc_empty[i], 256);
     }
     fence_mbar_init();
     prefetch_tmap(&tmW);
@@ -102,31 +103,43 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     load_gamma_beta(p.ln_w, p.ln_b, pt, gamma, beta, 0.5f);
     const long long pos_stride = p.z_pos_stride, line_stride = p.z_line_stride;
     const long long mpos_stride = p.m_pos_stride, mline_stride = p.m_line_stride;
-    RowTile<256> regs;
+    // Warps 9-15 have nine pairs of rows each, warp 8 the last pair: it is the issuer (all its lanes wait on the barriers and
+    // one elected lane issues -- a converged warp issues a tcgen05.mma several times faster than a lone thread of a diverged
+    // one).  The tensor pipe takes only a few products ahead, so the issuing warp stands still for most of their time: as
+    // one of the epilogue's warps it held up its whole group.
+    const bool issuer = warp == 8;
+    constexpr int G = 3;
+    RowStream<F32, G, 3> rows;
+    rows.c16 = lane & 15;
+    rows.first = (issuer ? 126 : (warp - 9) * 2) + (lane >> 4);
+    rows.step = 14;
+    const int groups = issuer ? 1 : G;
     uint8_t mreg = 0;
-    auto load_tile = [&](int tile) {
+    auto row_ptr = [&](int tile) {
       const int line = tile / tiles_per_line;
       const int pos0 = (tile - line * tiles_per_line) << 7;
-      const uint8_t* base = static_cast<const uint8_t*>(p.z) + line * line_stride;
-      regs.template load<F32, true, 8>(
-          pt,
-          [&](int r) -> const void* {
-            const int pos = pos0 + r;
-            return pos < p.n_pos ? base + pos * pos_stride : nullptr;
-          },
-          gamma, beta, p.eps, 1.0f, COPY ? p.z_copy_delta : 0);
-      if (pt < 128) {
-        const int pos = pos0 + pt;
-        mreg = (pos < p.n_pos) ? p.mask[line * mline_stride + pos * mpos_stride] : 0;
-      }
+      const uint8_t* base = static_cast<const uint8_t*>(p.z) + line * line_stride + pos0 * pos_stride;
+      const int left = p.n_pos - pos0 < 128 ? p.n_pos - pos0 : 128;
+      return [=](int r) -> const void* { return r < left ? base + r * pos_stride : nullptr; };
     };
-    int it = 0;
-    int tile = blockIdx.x;
-    if (tile < p.num_tiles) load_tile(tile);
-    for (; tile < p.num_tiles; tile += gridDim.x, ++it) {
+    auto load_mask = [&](int tile) {
+      const int line = tile / tiles_per_line;
+      const int pos = ((tile - line * tiles_per_line) << 7) + pt;
+      if (pt < 128) mreg = (pos < p.n_pos) ? p.mask[line * mline_stride + pos * mpos_stride] : 0;
+    };
+    // Tile number `it` into its operand stage, and the loads of the block's next tile on their way.
+    auto produce = [&](int tile, int it) {
       const int s = it & 1;
-      mbar_wait(&x_empty[s], ((it >> 1) & 1) ^ 1, 13);
-      regs.store_operand(pt, smem + X_OFF + s * kOperandTile);
+      const int next = tile + gridDim.x;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        if (g >= groups) break;
+        if (COPY) rows.copy(g, row_ptr(tile), p.z_copy_delta);
+        rows.normalize(g, gamma, beta, p.eps);
+        if (g == 0) mbar_wait(&x_empty[s], ((it >> 1) & 1) ^ 1, 13);
+        rows.store(g, smem + X_OFF + s * kOperandTile);
+        if (next < p.num_tiles) rows.load(g, row_ptr(next));
+      }
       if (pt < 128) {
         mask_s[(it & 3) * 128 + pt] = mreg;
         const bool quarter_valid = __all_sync(0xffffffffu, mreg != 0);
@@ -134,102 +147,111 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
       fence_proxy_async_smem();
       mbar_arrive(&x_full[s]);
-      const int next = tile + gridDim.x;
-      if (next < p.num_tiles) load_tile(next);
+      if (next < p.num_tiles) load_mask(next);
+    };
+    int tile = blockIdx.x;
+    if (tile < p.num_tiles) {
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (g < groups) rows.load(g, row_ptr(tile));
+      load_mask(tile);
     }
-  } else {
-    // ------------------------------------------------------------------ epilogue
-    // Group 0 (warps 0-3) gates and stores the a half, group 1 (warps 4-7) the b half, concurrently.  Lane =
-    // channel, columns = pairs; 16 columns at a time with the next chunk's TMEM loads in flight.  The gated
-    // values go to the group's swizzled [128 channels][64 pairs] staging tile and leave by TMA store (a row
-    // per channel of the channel-major plane).
-    const int half = warp >> 2;
-    const int d = (warp & 3) * 32 + lane;  // channel inside the half == TMEM lane
-    uint8_t* stage = smem + STAGE_OFF + half * kOperandHalf;
-    const CUtensorMap* tmOut = half ? &tmB : &tmA;
-    const uint32_t p_addr = tmem_addr(tmem_base, (warp & 3) * 32, (half * 2) * 128);
-    const uint32_t g_addr = p_addr + 128;
-    // The first WARP of the group issues the group's products: all its lanes wait on the barriers and one elected
-    // lane issues (a converged warp issues a tcgen05.mma several times faster than a lone thread of a diverged one).
-    const bool issue_warp = (warp & 3) == 0;
-    const bool leader = issue_warp && elect_one();
-    constexpr uint32_t idesc = make_idesc_bf16(128, 128);
-    const uint32_t w_s = smem_u32(smem + W_OFF);
-    if (issue_warp) {
-      if (half == 0 && leader) {
+    if (!issuer) {
+      for (int it = 0; tile < p.num_tiles; tile += gridDim.x, ++it) produce(tile, it);
+    } else if (tile < p.num_tiles) {
+      const bool leader = elect_one();
+      constexpr uint32_t idesc = make_idesc_bf16(128, 128);
+      const uint32_t w_s = smem_u32(smem + W_OFF);
+      if (leader) {
         mbar_arrive_expect_tx(w_full, 4 * kOperandTile);
         for (int mt = 0; mt < 4; ++mt)
           for (int h = 0; h < 2; ++h)
             tma_load_2d(smem + W_OFF + mt * kOperandTile + h * kOperandHalf, &tmW, w_full, h * 64, mt * 128);
       }
       __syncwarp();
+      produce(tile, 0);
       mbar_wait(w_full, 0, 10);
+      for (int it = 0; tile < p.num_tiles; tile += gridDim.x, ++it) {
+        const int s = it & 1;
+        const uint32_t x_s = smem_u32(smem + X_OFF + s * kOperandTile);
+        mbar_wait(&x_full[s], (it >> 1) & 1, 11);
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {  // p and g products of one half
+          mbar_wait(&acc_empty[half], (it & 1) ^ 1, 12);  // both groups have drained this half of the previous tile
+          tc_fence_after_sync();
+          if (leader) {
+            umma_k128(tmem_base + (half * 2) * 128, w_s + (half * 2) * kOperandTile, x_s, idesc, false);
+            umma_k128(tmem_base + (half * 2 + 1) * 128, w_s + (half * 2 + 1) * kOperandTile, x_s, idesc, false);
+            umma_commit(&acc_full[half]);
+            if (half == 1) umma_commit(&x_empty[s]);
+          }
+          __syncwarp();
+          // with products in the pipe, this warp's own rows of the next tile
+          if (half == 0 && tile + int(gridDim.x) < p.num_tiles) produce(tile + gridDim.x, it + 1);
+        }
+      }
     }
+  } else {
+    // ------------------------------------------------------------------ epilogue
+    // Lane = channel, columns = pairs; 16 columns at a time with the next chunk's TMEM loads in flight.  The gated
+    // values go to the group's swizzled [128 channels][64 pairs] staging tile and leave by TMA store (a row
+    // per channel of the channel-major plane).
+    const int grp = warp >> 2;
+    const int d = (warp & 3) * 32 + lane;  // channel inside the half == TMEM lane
+    uint8_t* stage = smem + STAGE_OFF + grp * kOperandHalf;
+    const uint32_t acc_addr = tmem_addr(tmem_base, (warp & 3) * 32, grp * 64);
     int it = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
       const int line = tile / tiles_per_line;
-      const int pos0 = (tile - line * tiles_per_line) << 7;
-      const uint32_t* msk = reinterpret_cast<const uint32_t*>(mask_s + (it & 3) * 128);
-      if (issue_warp) {  // this half's products for the tile: p and g projections against operand stage it & 1
-        const int s = it & 1;
-        mbar_wait(&x_full[s], (it >> 1) & 1, 11);
-        mbar_wait(&acc_empty[half], (it & 1) ^ 1, 12);  // the whole group has drained the previous tile
+      const int pos0 = ((tile - line * tiles_per_line) << 7) + grp * 64;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        mbar_wait(&acc_full[half], it & 1, 14);
         tc_fence_after_sync();
-        const uint32_t x_s = smem_u32(smem + X_OFF + s * kOperandTile);
-        if (leader) {
-          umma_k128(tmem_base + (half * 2) * 128, w_s + (half * 2) * kOperandTile, x_s, idesc, false);
-          umma_k128(tmem_base + (half * 2 + 1) * 128, w_s + (half * 2 + 1) * kOperandTile, x_s, idesc, false);
-          umma_commit(&acc_full[half]);
-          umma_commit(&x_empty[s]);
-        }
-      }
-      __syncwarp();
-      mbar_wait(&acc_full[half], it & 1, 14);
-      tc_fence_after_sync();
-      // every pair of the tile unmasked?  (tiles away from the padding are, and then no select is needed)
-      const bool all_valid = *reinterpret_cast<const uint32_t*>(flag_s + (it & 3) * 4) == 0x01010101u;
-      uint32_t pa[16], ga[16], pb[16], gb[16];
-      tmem_ld_32x16(p_addr, pa);
-      tmem_ld_32x16(g_addr, ga);
+        const uint32_t* msk = reinterpret_cast<const uint32_t*>(mask_s + (it & 3) * 128 + grp * 64);
+        // every pair of the tile unmasked?  (tiles away from the padding are, and then no select is needed)
+        const bool all_valid = *reinterpret_cast<const uint32_t*>(flag_s + (it & 3) * 4) == 0x01010101u;
+        const uint32_t p_addr = acc_addr + half * 256, g_addr = p_addr + 128;
+        uint32_t pa[16], ga[16], pb[16], gb[16];
+        tmem_ld_32x16(p_addr, pa);
+        tmem_ld_32x16(g_addr, ga);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint32_t(&pv)[16] = (c & 1) ? pb : pa;
-        uint32_t(&gv)[16] = (c & 1) ? gb : ga;
-        tmem_ld_wait();
-        if (c < 7) {
-          tmem_ld_32x16(p_addr + (c + 1) * 16, (c & 1) ? pa : pb);
-          tmem_ld_32x16(g_addr + (c + 1) * 16, (c & 1) ? ga : gb);
-        } else {
-          tc_fence_before_sync();
-          mbar_arrive(&acc_empty[half]);
-        }
-        uint32_t packed[8];
+        for (int c = 0; c < 4; ++c) {
+          uint32_t(&pv)[16] = (c & 1) ? pb : pa;
+          uint32_t(&gv)[16] = (c & 1) ? gb : ga;
+          tmem_ld_wait();
+          if (c < 3) {
+            tmem_ld_32x16(p_addr + (c + 1) * 16, (c & 1) ? pa : pb);
+            tmem_ld_32x16(g_addr + (c + 1) * 16, (c & 1) ? ga : gb);
+          } else {
+            tc_fence_before_sync();
+            mbar_arrive(&acc_empty[half]);
+          }
+          uint32_t packed[8];
 #pragma unroll
-        for (int j = 0; j < 16; j += 2) {
-          const float h0 = __uint_as_float(pv[j]), h1 = __uint_as_float(pv[j + 1]);
-          float v0 = fmaf(h0, tanh_approx(__uint_as_float(gv[j])), h0);
-          float v1 = fmaf(h1, tanh_approx(__uint_as_float(gv[j + 1])), h1);
-          if (!all_valid) {
-            const uint32_t m4 = msk[(c * 16 + j) >> 2];
-            v0 = ((m4 >> ((j & 3) * 8)) & 0xff) ? v0 : 0.f;
-            v1 = ((m4 >> (((j + 1) & 3) * 8)) & 0xff) ? v1 : 0.f;
+          for (int j = 0; j < 16; j += 2) {
+            const float h0 = __uint_as_float(pv[j]), h1 = __uint_as_float(pv[j + 1]);
+            float v0 = fmaf(h0, tanh_approx(__uint_as_float(gv[j])), h0);
+            float v1 = fmaf(h1, tanh_approx(__uint_as_float(gv[j + 1])), h1);
+            if (!all_valid) {
+              const uint32_t m4 = msk[(c * 16 + j) >> 2];
+              v0 = ((m4 >> ((j & 3) * 8)) & 0xff) ? v0 : 0.f;
+              v1 = ((m4 >> (((j + 1) & 3) * 8)) & 0xff) ? v1 : 0.f;
+            }
+            packed[j >> 1] = pack_bf16x2(v0, v1);
           }
-          packed[j >> 1] = pack_bf16x2(v0, v1);
-        }
-        if ((c & 3) == 0) {  // the previous store has finished reading the staging tile (its wait hides behind the
-          if (d == 0) tma_store_wait_read0();  // chunk's arithmetic above)
-          named_bar_sync(1 + half, 128);
-        }
-        *reinterpret_cast<uint4*>(stage + sw128_offset(d, (c & 3) * 2)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        *reinterpret_cast<uint4*>(stage + sw128_offset(d, (c & 3) * 2 + 1)) =
-            make_uint4(packed[4], packed[5], packed[6], packed[7]);
-        if ((c & 3) == 3) {
-          fence_proxy_async_smem();
-          named_bar_sync(1 + half, 128);
-          if (d == 0) {
-            tma_store_3d(tmOut, stage, pos0 + (c >> 2) * 64, line, 0);
-            tma_store_commit();
+          if (c == 0) {  // the previous store has finished reading the staging tile (its wait hides behind the
+            if (d == 0) tma_store_wait_read0();  // chunk's arithmetic above)
+            named_bar_sync(1 + grp, 128);
           }
+          *reinterpret_cast<uint4*>(stage + sw128_offset(d, c * 2)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+          *reinterpret_cast<uint4*>(stage + sw128_offset(d, c * 2 + 1)) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+        }
+        fence_proxy_async_smem();
+        named_bar_sync(1 + grp, 128);
+        if (d == 0) {
+          tma_store_3d(half ? &tmB : &tmA, stage, pos0, line, 0);
+          tma_store_commit();
         }
       }
     }
