@@ -37,28 +37,10 @@ struct BmmParams {
   // bf16 columns) and the C tensor map, 1 = stored, 2 = added into C (the residual is C itself, which the
   // epilogue then never reads).
   int tma_c;
-  // kEpiMul: the tile is multiplied element by element with fp32 mul[row * mul_pitch + column] (a per-token gate)
-  // before it is stored or added.
-  const float* mul;
-  int mul_pitch;
   // Split operands stored once as (hi | lo): a K block at or past the fold is loaded from that many blocks before, which
   // makes the operand hi | hi | lo.  INT_MAX: none.
   int a_fold, b_fold;
   int a_shared;              // 1: every batch item multiplies the same A (the A tensor map has a single batch slice)
-};
-
-template <int BN>
-struct BmmCfg {
-  static constexpr int BM = 128;
-  static constexpr int BK = 64;
-  static constexpr int STAGES = (BN == 256) ? 4 : 6;
-  static constexpr uint32_t A_BYTES = BM * BK * 2;
-  static constexpr uint32_t B_BYTES = BN * BK * 2;
-  static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr uint32_t BAR_OFFSET = STAGES * STAGE_BYTES;
-  static constexpr uint32_t OUT_OFFSET = BAR_OFFSET + 1024;        // two [128 rows][128 B] tiles for bulk output
-  static constexpr uint32_t SMEM_BYTES = OUT_OFFSET + 2 * 16384 + 1024;  // + alignment slack
-  static constexpr int THREADS = 192;
 };
 
 // The epilogues are separate instantiations: with all of them in one kernel the plain one, which triangle multiplication's
@@ -66,24 +48,46 @@ struct BmmCfg {
 enum BmmEpilogue : int {
   kEpiDirect = 0,  // scale, bias, residual; stores by the threads themselves
   kEpiBulk = 1,    // scale, bias; bulk stores through C's tensor map
-  kEpiMul = 2,     // bulk, with the element-wise factor
+  // Bulk, the tile multiplied element by element with fp32 factors (a per-token gate) before it is stored or added.  They
+  // come by TMA during the product's K loop (read by the lanes from their rows: 16 against 9 us without the gate for
+  // 2048 x 768 x 768, 23 against 13 for K = 3072).
+  kEpiMul = 2,
   kEpiSwiglu = 3,  // bulk bf16: the columns are pairs of 64-column blocks (a | b), C gets silu(a) * b, half as many columns
   kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b, with expf and exact division
   kEpiOuter = 5,   // outer products of 32 x 32, one pair's 2 KB in one piece
 };
 
 template <int BN, int EPI>
+struct BmmCfg {
+  static constexpr int BM = 128;
+  static constexpr int BK = 64;
+  static constexpr int STAGES = EPI == kEpiMul || BN == 256 ? 4 : 6;
+  static constexpr uint32_t A_BYTES = BM * BK * 2;
+  static constexpr uint32_t B_BYTES = BN * BK * 2;
+  static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr uint32_t MUL_OFFSET = STAGES * STAGE_BYTES;     // kEpiMul: the factors' [128 rows][32 columns] tiles
+  static constexpr uint32_t MUL_BYTES = EPI == kEpiMul ? BN * 128 * 4 : 0;
+  static constexpr uint32_t BAR_OFFSET = MUL_OFFSET + MUL_BYTES;
+  static constexpr uint32_t BIAS_OFFSET = BAR_OFFSET + 1024;       // the tile's BN bias values
+  static constexpr uint32_t OUT_OFFSET = BAR_OFFSET + 2048;        // two [128 rows][128 B] tiles for bulk output
+  static constexpr uint32_t SMEM_BYTES = OUT_OFFSET + 2 * 16384 + 1024;  // + alignment slack
+  static constexpr int THREADS = 192;
+};
+
+template <int BN, int EPI>
 __global__ void __launch_bounds__(192, 1)
 bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-              const __grid_constant__ CUtensorMap tmC, BmmParams p) {
-  using Cfg = BmmCfg<BN>;
+              const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmM, BmmParams p) {
+  using Cfg = BmmCfg<BN, EPI>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFFSET);
   uint64_t* empty = full + Cfg::STAGES;
   uint64_t* acc_full = empty + Cfg::STAGES;
   uint64_t* acc_empty = acc_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* mul_full = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mul_full + 1);
+  float* bias_s = reinterpret_cast<float*>(smem + Cfg::BIAS_OFFSET);
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
@@ -99,10 +103,12 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], 128);
     }
+    mbar_init(mul_full, 1);
     fence_mbar_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
     if (EPI != kEpiDirect && EPI != kEpiOuter) prefetch_tmap(&tmC);
+    if (EPI == kEpiMul) prefetch_tmap(&tmM);
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
@@ -172,12 +178,32 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   } else {
     const int quarter = warp & 3;  // TMEM lanes this warp may read: 32*quarter .. +31
     int it = 0;
+    auto load_factors = [&](int tile) {
+      const int rem = tile % tiles_per_batch;
+      const int tm = rem / p.tiles_n, tn = rem - tm * p.tiles_n;
+      mbar_arrive_expect_tx(mul_full, Cfg::MUL_BYTES);
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c)
+        tma_load_2d(smem + Cfg::MUL_OFFSET + c * 16384, &tmM, mul_full, tn * BN + c * 32, tm * 128);
+    };
+    if (EPI == kEpiMul && threadIdx.x == 64 && int(blockIdx.x) < total_tiles) load_factors(blockIdx.x);
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
       const int b = tile / tiles_per_batch;
       const int rem = tile - b * tiles_per_batch;
       const int tm = rem / p.tiles_n;
       const int tn = rem - tm * p.tiles_n;
       const int acc = it & 1;
+      if ((EPI == kEpiBulk || EPI == kEpiMul) && p.bias) {
+        // Read by every lane from shared memory (by every lane from global memory: 25 against 17 us without a bias for
+        // 2048 x 4608 x 768).  The previous tile's values have been read before its last barrier; the first barrier
+        // of this one makes the new ones visible.
+#pragma unroll
+        for (int i = 0; i < BN; i += 128) {
+          const int col = tn * BN + i + quarter * 32 + lane;
+          bias_s[i + quarter * 32 + lane] = col < p.n_valid ? p.bias[col] : 0.f;
+        }
+      }
+      if (EPI == kEpiMul) mbar_wait(mul_full, it & 1, 5);
       mbar_wait(&acc_full[acc], (it >> 1) & 1, 4);
       tc_fence_after_sync();
       const int row = tm * 128 + quarter * 32 + lane;
@@ -300,8 +326,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             tc_fence_before_sync();
             mbar_arrive(&acc_empty[acc]);
           }
-          const int col0 = tn * BN + c * 32;
-          const float* mrow = EPI == kEpiMul && row < p.m_valid ? p.mul + (long long)row * p.mul_pitch + col0 : nullptr;
+          const uint8_t* factors = smem + Cfg::MUL_OFFSET + c * 16384;
           if (p.out_f32) {
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
@@ -310,12 +335,12 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               x.y = __uint_as_float(v[g * 4 + 1]) * scale;
               x.z = __uint_as_float(v[g * 4 + 2]) * scale;
               x.w = __uint_as_float(v[g * 4 + 3]) * scale;
-              if (p.bias && col0 + g * 4 < p.n_valid) {  // n_valid % 8 == 0: a group of four is inside or outside
-                const float4 bv = *reinterpret_cast<const float4*>(p.bias + col0 + g * 4);
+              if (p.bias) {
+                const float4 bv = *reinterpret_cast<const float4*>(bias_s + c * 32 + g * 4);
                 x.x += bv.x; x.y += bv.y; x.z += bv.z; x.w += bv.w;
               }
-              if (EPI == kEpiMul && mrow && col0 + g * 4 < p.n_valid) {
-                const float4 mv = *reinterpret_cast<const float4*>(mrow + g * 4);
+              if (EPI == kEpiMul) {
+                const float4 mv = *reinterpret_cast<const float4*>(factors + sw128_offset(r, g));
                 x.x *= mv.x; x.y *= mv.y; x.z *= mv.z; x.w *= mv.w;
               }
               *reinterpret_cast<float4*>(stage + sw128_offset(r, g)) = x;
@@ -326,13 +351,17 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               float x[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[g * 8 + e]) * scale;
-              if (p.bias && col0 + g * 8 < p.n_valid) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) x[e] += p.bias[col0 + g * 8 + e];
+              if (p.bias) {
+                const float4 b0 = *reinterpret_cast<const float4*>(bias_s + c * 32 + g * 8);
+                const float4 b1 = *reinterpret_cast<const float4*>(bias_s + c * 32 + g * 8 + 4);
+                x[0] += b0.x; x[1] += b0.y; x[2] += b0.z; x[3] += b0.w;
+                x[4] += b1.x; x[5] += b1.y; x[6] += b1.z; x[7] += b1.w;
               }
-              if (EPI == kEpiMul && mrow && col0 + g * 8 < p.n_valid) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) x[e] *= mrow[g * 8 + e];
+              if (EPI == kEpiMul) {
+                const float4 m0 = *reinterpret_cast<const float4*>(factors + sw128_offset(r, g * 2));
+                const float4 m1 = *reinterpret_cast<const float4*>(factors + sw128_offset(r, g * 2 + 1));
+                x[0] *= m0.x; x[1] *= m0.y; x[2] *= m0.z; x[3] *= m0.w;
+                x[4] *= m1.x; x[5] *= m1.y; x[6] *= m1.z; x[7] *= m1.w;
               }
               *reinterpret_cast<uint4*>(stage + sw128_offset(r, (c & 1) * 4 + g)) = make_uint4(
                   pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
@@ -351,6 +380,8 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             }
           }
         }
+        // every thread has read its factors before the last barrier above
+        if (EPI == kEpiMul && leader && tile + int(gridDim.x) < total_tiles) load_factors(tile + gridDim.x);
         continue;
       }
       if constexpr (EPI == kEpiOuter) {

@@ -2,6 +2,7 @@
 // construction and kernel launches.  The kernels live in the .cuh files beside this one and are
 // compiled into this single translation unit.
 #include <cstdarg>
+#include <type_traits>
 
 #include "host_util.cuh"
 #include "umma.cuh"
@@ -86,7 +87,7 @@ struct BackgroundScope {
 };
 
 static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
-  const int BN = t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.K, a.batch);
+  const int BN = a.mul ? 128 : t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.K, a.batch);
   CUtensorMap tmA, tmB;
   const bool a_shared = a.batch > 1 && a.sa == 0;  // one A for every batch item
   {
@@ -122,8 +123,6 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   p.a_shared = a_shared ? 1 : 0;
   p.a_fold = a.a_fold ? a.a_fold : INT_MAX;
   p.b_fold = a.b_fold ? a.b_fold : INT_MAX;
-  p.mul = a.mul;
-  p.mul_pitch = a.mul_pitch;
   // Bulk output through the C tensor map where the layout allows it (the map clips the last column group): the
   // residual (if any) being C itself, and for the transposed pair store lines that are whole row tiles.
   p.tma_c = 0;
@@ -152,26 +151,29 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
       return e;
     p.tma_c = a.residual ? 2 : 1;
   }
-  if ((a.mul || a.swiglu) && (!p.tma_c || (a.mul && (!aligned(a.mul, 16) || a.mul_pitch % 4 || a.N % 8))))
+  if ((a.mul || a.swiglu) && (!p.tma_c || (a.mul && (!aligned(a.mul, 16) || a.mul_pitch % 4 || a.batch != 1))))
     return fail(B200_ERR_INVALID_ARGUMENT, "a gated product needs bulk output and 16-byte aligned factors");
+  CUtensorMap tmM = tmC;
+  if (a.mul) {
+    const uint64_t dims[2] = {uint64_t(a.N), uint64_t(a.M)};
+    const uint64_t str[1] = {uint64_t(a.mul_pitch) * 4};
+    const uint32_t box[2] = {32, 128};
+    if (int e = make_tmap(&tmM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.mul, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+  }
   const int total = p.tiles_m * p.tiles_n * a.batch;
   const int grid = total < sm_count() ? total : sm_count();
-  auto go = [&](auto kernel, uint32_t smem) -> int {
-    B200_LAUNCH(kernel, grid, 192, smem, stream, tmA, tmB, tmC, p);
+  auto go = [&](auto bn, auto epi) -> int {
+    B200_LAUNCH((bmm_nt_kernel<bn.value, epi.value>), grid, 192, (BmmCfg<bn.value, epi.value>::SMEM_BYTES), stream, tmA, tmB, tmC,
+                tmM, p);
     return 0;
   };
-  if (BN == 256) {
-    constexpr uint32_t smem = BmmCfg<256>::SMEM_BYTES;
-    if (a.opm_ntok > 0) return go(bmm_nt_kernel<256, kEpiOuter>, smem);
-    if (a.swiglu) return a.split ? go(bmm_nt_kernel<256, kEpiSwigluSplit>, smem) : go(bmm_nt_kernel<256, kEpiSwiglu>, smem);
-    if (a.mul) return go(bmm_nt_kernel<256, kEpiMul>, smem);
-    return p.tma_c ? go(bmm_nt_kernel<256, kEpiBulk>, smem) : go(bmm_nt_kernel<256, kEpiDirect>, smem);
-  }
-  constexpr uint32_t smem = BmmCfg<128>::SMEM_BYTES;
-  if (a.opm_ntok > 0) return go(bmm_nt_kernel<128, kEpiOuter>, smem);
-  if (a.swiglu) return a.split ? go(bmm_nt_kernel<128, kEpiSwigluSplit>, smem) : go(bmm_nt_kernel<128, kEpiSwiglu>, smem);
-  if (a.mul) return go(bmm_nt_kernel<128, kEpiMul>, smem);
-  return p.tma_c ? go(bmm_nt_kernel<128, kEpiBulk>, smem) : go(bmm_nt_kernel<128, kEpiDirect>, smem);
+  auto pick = [&](auto bn) -> int {
+    if (a.opm_ntok > 0) return go(bn, std::integral_constant<int, kEpiOuter>());
+    if (a.swiglu) return a.split ? go(bn, std::integral_constant<int, kEpiSwigluSplit>()) : go(bn, std::integral_constant<int, kEpiSwiglu>());
+    return p.tma_c ? go(bn, std::integral_constant<int, kEpiBulk>()) : go(bn, std::integral_constant<int, kEpiDirect>());
+  };
+  if (a.mul) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiMul>());
+  return BN == 256 ? pick(std::integral_constant<int, 256>()) : pick(std::integral_constant<int, 128>());
 }
 
 static int launch_rows_to_bf16(const void* x, bool f32, __nv_bfloat16* y, const float* w, const float* b,
@@ -1937,11 +1939,12 @@ int b200_cond_layer_fwd(const b200_cond_layer* l, const void* x, const void* pai
     }
     if (int e = b200_window_bias_fwd(pairs, l->ln_z_w, l->ln_z_b, l->w_z, wb, int64_t(l->B) * NW, W, Hk, l->dim_pairwise, l->heads, pairs_dtype, stream)) return e;
     if (int e = window_attention_run(qkvg, 4 * D, qkvg + 3 * D, 4 * D, wb, mask, og, l->B, l->M, NW, W, Hk, l->heads, D / l->heads, stream)) return e;
-    // The gate as a row kernel of its own: in the epilogue of a product this short its scattered row reads are not hidden
-    // (32768 x 128 x 128: 26 us against 7 + 9).
-    BmmLaunch a{og, l->w_o, y, 1, int(rows), D, D, D, D, D, 0, 0, 0};
+    BmmLaunch a{og, l->w_o, out, 1, int(rows), D, D, D, D, D, 0, 0, 0};
+    a.residual = out;
+    a.out_f32 = xf32;
+    a.mul = cond + 2 * D;
+    a.mul_pitch = CW;
     if (int e = launch_bmm(a, stream)) return e;
-    if (int e = gated_residual(y, 2)) return e;
   } else {
     const ApbOutput into{out, xf32, cond + 2 * D, CW};
     if (int e = apb_run(y, pairs, bias, bias_pitch, mask, out, &l->attention, l->B, l->M, l->N, D, l->heads, B200_DTYPE_BF16, pairs_dtype,
