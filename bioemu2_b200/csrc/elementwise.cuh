@@ -272,13 +272,22 @@ adaln_rows_kernel(const void* __restrict__ x, const float* __restrict__ cond, in
   const float inv = 1.0f / float(cols);
   for (long long r = warp_global; r < rows; r += warp_stride) {
     const uint8_t* xr = static_cast<const uint8_t*>(x) + r * cols * (long long)(F32IN ? 4 : 2);
-    float f[4][8];
+    const float* cr = cond + r * cw;
+    float f[4][8], al[4][8], be[4][8];  // all of the row's loads go out together
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int vi = lane + i * 32;
       if (vi < nvec) {
         load8<F32IN>(xr, vi * 8, f[i]);
+        load8<true>(cr + alpha_col, vi * 8, al[i]);
+        load8<true>(cr + beta_col, vi * 8, be[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int vi = lane + i * 32;
+      if (vi < nvec) {
         if (x_copy) store8<F32IN>(static_cast<uint8_t*>(x_copy) + r * cols * (long long)(F32IN ? 4 : 2), vi * 8, f[i]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) s += f[i][e];
@@ -296,16 +305,12 @@ adaln_rows_kernel(const void* __restrict__ x, const float* __restrict__ cond, in
         }
       }
     const float rstd = rsqrtf(warp_sum(ss) * inv + eps);
-    const float* cr = cond + r * cw;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int vi = lane + i * 32;
       if (vi < nvec) {
-        float al[8], be[8];
-        load8<true>(cr + alpha_col, vi * 8, al);
-        load8<true>(cr + beta_col, vi * 8, be);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[i][e] = lns * fmaf(f[i][e] * rstd, 1.0f + al[e], be[e]);
+        for (int e = 0; e < 8; ++e) f[i][e] = lns * fmaf(f[i][e] * rstd, 1.0f + al[i][e], be[i][e]);
         store8<false>(y + r * cols, vi * 8, f[i]);
       }
     }

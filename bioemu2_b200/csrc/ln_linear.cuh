@@ -5,7 +5,7 @@
 // memory twice (two sources, N = 384: 97 + 23 us for 226 MB that have to move, 35 us).  Here the LayerNorm writes the product's
 // operand in shared memory.  A tile is 128 rows; W stays resident.
 //   warps 0-3   epilogue: accumulator (+ residual) -> swizzled staging tiles -> TMA store
-//   warps 4-11  producers: 16 threads per row, two rows in flight per thread beside the two being normalised
+//   warps 4-11  producers: 16 threads per row, two (one source: four) rows in flight per thread beside those being normalised
 //   warp  12    control: TMA of W, MMA issue
 #pragma once
 #include "row_tile.cuh"
@@ -105,11 +105,12 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         gamma[k][i] = p.ln_w ? p.ln_w[k * 128 + c0 + i] : 1.0f;
         beta[k][i] = p.ln_b ? p.ln_b[k * 128 + c0 + i] : 0.0f;
       }
-    float xa[2][SRC][8], xb[2][SRC][8];
-    auto load = [&](int tile, int q, float (&x)[2][SRC][8]) {  // rows q*32 + rbase and + 16 of the tile
+    constexpr int U = SRC == 1 ? 4 : 2;  // rows of a thread's group: half of its rows, as far as they fit its registers
+    float xa[U][SRC][8], xb[U][SRC][8];
+    auto load = [&](int tile, int q, float (&x)[U][SRC][8]) {  // rows (q*U + u)*16 + rbase of the tile
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const long long row = (long long)tile * 128 + q * 32 + u * 16 + rbase;
+      for (int u = 0; u < U; ++u) {
+        const long long row = (long long)tile * 128 + (q * U + u) * 16 + rbase;
 #pragma unroll
         for (int k = 0; k < SRC; ++k) {
           if (row < p.rows && tile < p.num_tiles) {
@@ -121,9 +122,9 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
       }
     };
-    auto emit = [&](uint8_t* dst, int q, float (&x)[2][SRC][8]) {
+    auto emit = [&](uint8_t* dst, int q, float (&x)[U][SRC][8]) {
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < U; ++u) {
         float sm = 0.f;
 #pragma unroll
         for (int k = 0; k < SRC; ++k)
@@ -139,7 +140,7 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             ss = fmaf(x[u][k][i], x[u][k][i], ss);
           }
         const float rstd = rsqrtf(group16_sum(ss) * (1.0f / (128 * SRC)) + p.eps);
-        const int r = q * 32 + u * 16 + rbase;
+        const int r = (q * U + u) * 16 + rbase;
 #pragma unroll
         for (int k = 0; k < SRC; ++k) {
           float y[8];
@@ -157,13 +158,14 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       uint8_t* dst = smem + Cfg::X_OFF + s * SRC * kOperandTile;
       load(tile, 1, xb);
       mbar_wait(&x_empty[s], ((it >> 1) & 1) ^ 1, 103);
-      emit(dst, 0, xa);
-      load(tile, 2, xa);
-      emit(dst, 1, xb);
-      load(tile, 3, xb);
-      emit(dst, 2, xa);
-      load(tile + gridDim.x, 0, xa);
-      emit(dst, 3, xb);
+#pragma unroll
+      for (int q = 0; q < 8 / U; q += 2) {
+        emit(dst, q, xa);
+        if (q + 2 < 8 / U) load(tile, q + 2, xa);
+        else load(tile + gridDim.x, 0, xa);
+        emit(dst, q + 1, xb);
+        if (q + 3 < 8 / U) load(tile, q + 3, xb);
+      }
       fence_proxy_async_smem();
       mbar_arrive(&x_full[s]);
     }
@@ -172,11 +174,23 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     const int r = warp * 32 + lane;
     const bool leader = threadIdx.x == 0;
     int it = 0;
+    float res[4][8];  // the next 32 channels of the residual, loaded a chunk ahead
+    auto load_res = [&](int tile, int c) {
+      const long long row = (long long)tile * 128 + r;
+      const bool there = p.residual && row < p.rows && tile < p.num_tiles;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        if (there) {
+          ld_global_v8(p.residual + row * 128 + c * 32 + g * 8, res[g]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) res[g][e] = 0.f;
+        }
+      }
+    };
+    load_res(blockIdx.x, 0);
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
       const int acc = it & 1;
-      const long long row = (long long)tile * 128 + r;
-      const bool res = p.residual && row < p.rows;
-      const float* rrow = p.residual + row * 128;
       mbar_wait(&acc_full[acc], (it >> 1) & 1, 104);
       tc_fence_after_sync();
       uint32_t va[32], vb[32];
@@ -197,17 +211,13 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           float x[8];
-          if (res) {
-            ld_global_v8(rrow + c * 32 + g * 8, x);
-          } else {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x[e] = 0.f;
-          }
-#pragma unroll
-          for (int e = 0; e < 8; ++e) x[e] += __uint_as_float(v[g * 8 + e]);
+          for (int e = 0; e < 8; ++e) x[e] = res[g][e] + __uint_as_float(v[g * 8 + e]);
           *reinterpret_cast<float4*>(stage + sw128_offset(r, g * 2)) = make_float4(x[0], x[1], x[2], x[3]);
           *reinterpret_cast<float4*>(stage + sw128_offset(r, g * 2 + 1)) = make_float4(x[4], x[5], x[6], x[7]);
         }
+        if (c < 3) load_res(tile, c + 1);
+        else load_res(tile + gridDim.x, 0);
         fence_proxy_async_smem();
         named_bar_sync(1, 128);
         if (leader) {

@@ -100,27 +100,34 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmW, PairBiasParams p) {
     const int pt = threadIdx.x - 128;
     float gamma[8], beta[8];
     load_gamma_beta(p.ln_w, p.ln_b, pt, gamma, beta);
-    RowTile<256> regs;
     const long long pos_stride = p.z_pos_stride, line_stride = p.z_line_stride;
-    auto load_tile = [&](int tile) {
+    constexpr int G = 2;
+    RowStream<F32, G, 4> rows;
+    rows.place(pt);
+    auto row_ptr = [&](int tile) {
       const int i = tile / tiles_per_row;
-      const int j0 = (tile - i * tiles_per_row) << 7;
-      const uint8_t* base = static_cast<const uint8_t*>(p.z) + i * line_stride;
-      regs.template load<F32, true>(
-          pt, [&](int r) -> const void* { return (j0 + r) < p.n_pos ? base + (j0 + r) * pos_stride : nullptr; },
-          gamma, beta, p.eps);
+      const int pos0 = (tile - i * tiles_per_row) << 7;
+      const uint8_t* base = static_cast<const uint8_t*>(p.z) + i * line_stride + pos0 * pos_stride;
+      const int left = p.n_pos - pos0 < 128 ? p.n_pos - pos0 : 128;
+      return [=](int r) -> const void* { return r < left ? base + r * pos_stride : nullptr; };
     };
     int it = 0;
     int tile = blockIdx.x;
-    if (tile < p.num_tiles) load_tile(tile);
+    if (tile < p.num_tiles) {
+#pragma unroll
+      for (int g = 0; g < G; ++g) rows.load(g, row_ptr(tile));
+    }
     for (; tile < p.num_tiles; tile += gridDim.x, ++it) {
-      const int s = it & 1;
-      mbar_wait(&x_empty[s], ((it >> 1) & 1) ^ 1, 83);
-      regs.store_operand(pt, smem + X_OFF + s * kOperandTile);
-      fence_proxy_async_smem();
-      mbar_arrive(&x_full[s]);
       const int next = tile + gridDim.x;
-      if (next < p.num_tiles) load_tile(next);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        rows.normalize(g, gamma, beta, p.eps);
+        if (g == 0) mbar_wait(&x_empty[it & 1], ((it >> 1) & 1) ^ 1, 83);
+        rows.store(g, smem + X_OFF + (it & 1) * kOperandTile);
+        if (next < p.num_tiles) rows.load(g, row_ptr(next));
+      }
+      fence_proxy_async_smem();
+      mbar_arrive(&x_full[it & 1]);
     }
   } else {
     int it = 0;

@@ -200,6 +200,9 @@ struct RowStream {
   uint4 v[R];
   int c16, first, step;
 
+  // Thread pt of 256: the rows are dealt out sixteen at a time.
+  __device__ __forceinline__ void place(int pt) { c16 = pt & 15, first = pt >> 4, step = 16; }
+
   template <class RowPtr>
   __device__ __forceinline__ void load(int g, RowPtr row_ptr) {
 #pragma unroll

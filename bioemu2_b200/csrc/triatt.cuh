@@ -158,30 +158,33 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     float gamma[8], beta[8];
     load_gamma_beta(p.ln_w, p.ln_b, pt, gamma, beta);
     const long long pos_stride = p.z_pos_stride, line_stride = p.z_line_stride;
-    RowTile<256> regs;
-    auto load_tile = [&](int tile) {
+    constexpr int G = 2;
+    RowStream<F32, G, 4> rows;
+    rows.place(pt);
+    auto row_ptr = [&](int tile) {
       const int line = tile / tiles_per_line;
       const int pos0 = (tile - line * tiles_per_line) << 7;
-      const uint8_t* base = static_cast<const uint8_t*>(p.z) + line * line_stride;
-      regs.template load<F32, true>(
-          pt,
-          [&](int r) -> const void* {
-            const int pos = pos0 + r;
-            return pos < p.n_pos ? base + pos * pos_stride : nullptr;
-          },
-          gamma, beta, p.eps);
+      const uint8_t* base = static_cast<const uint8_t*>(p.z) + line * line_stride + pos0 * pos_stride;
+      const int left = p.n_pos - pos0 < 128 ? p.n_pos - pos0 : 128;
+      return [=](int r) -> const void* { return r < left ? base + r * pos_stride : nullptr; };
     };
     int it = 0;
     int tile = blockIdx.x;
-    if (tile < p.num_tiles) load_tile(tile);
+    if (tile < p.num_tiles) {
+#pragma unroll
+      for (int g = 0; g < G; ++g) rows.load(g, row_ptr(tile));
+    }
     for (; tile < p.num_tiles; tile += gridDim.x, ++it) {
-      const int s = it & 1;
-      mbar_wait(&x_empty[s], ((it >> 1) & 1) ^ 1, 94);
-      regs.store_operand(pt, smem + X_OFF + s * kOperandTile);
-      fence_proxy_async_smem();
-      mbar_arrive(&x_full[s]);
       const int next = tile + gridDim.x;
-      if (next < p.num_tiles) load_tile(next);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        rows.normalize(g, gamma, beta, p.eps);
+        if (g == 0) mbar_wait(&x_empty[it & 1], ((it >> 1) & 1) ^ 1, 94);
+        rows.store(g, smem + X_OFF + (it & 1) * kOperandTile);
+        if (next < p.num_tiles) rows.load(g, row_ptr(next));
+      }
+      fence_proxy_async_smem();
+      mbar_arrive(&x_full[it & 1]);
     }
   } else {
     const int r = warp * 32 + lane;  // TMEM lane: pair of the tile for q/k/g, channel for V^T
