@@ -61,7 +61,7 @@ template <int BN, int EPI>
 struct BmmCfg {
   static constexpr int BM = 128;
   static constexpr int BK = 64;
-  static constexpr int STAGES = EPI == kEpiMul || BN == 256 ? 4 : 6;
+  static constexpr int STAGES = EPI == kEpiSwigluSplit ? 3 : EPI == kEpiMul || BN == 256 ? 4 : 6;
   static constexpr uint32_t A_BYTES = BM * BK * 2;
   static constexpr uint32_t B_BYTES = BN * BK * 2;
   static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
@@ -69,13 +69,17 @@ struct BmmCfg {
   static constexpr uint32_t MUL_BYTES = EPI == kEpiMul ? BN * 128 * 4 : 0;
   static constexpr uint32_t BAR_OFFSET = MUL_OFFSET + MUL_BYTES;
   static constexpr uint32_t BIAS_OFFSET = BAR_OFFSET + 1024;       // the tile's BN bias values
-  static constexpr uint32_t OUT_OFFSET = BAR_OFFSET + 2048;        // two [128 rows][128 B] tiles for bulk output
-  static constexpr uint32_t SMEM_BYTES = OUT_OFFSET + 2 * 16384 + 1024;  // + alignment slack
-  static constexpr int THREADS = 192;
+  static constexpr uint32_t OUT_OFFSET = BAR_OFFSET + 2048;        // [128 rows][128 B] tiles for bulk output
+  static constexpr int OUT_TILES = EPI == kEpiSwigluSplit ? 4 : 2;
+  static constexpr uint32_t SMEM_BYTES = OUT_OFFSET + OUT_TILES * 16384 + 1024;  // + alignment slack
+  // The split SwiGLU's expf and division keep four warps busy for longer than the product (40000 x 1024 x 384: 105 us): it
+  // has eight, each group of four with one of the tile's two 64-column groups.
+  static constexpr int EPI_THREADS = EPI == kEpiSwigluSplit ? 256 : 128;
+  static constexpr int THREADS = 64 + EPI_THREADS;
 };
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(BmmCfg<BN, EPI>::THREADS, 1)
 bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
               const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmM, BmmParams p) {
   using Cfg = BmmCfg<BN, EPI>;
@@ -101,7 +105,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 128);
+      mbar_init(&acc_empty[a], Cfg::EPI_THREADS);
     }
     mbar_init(mul_full, 1);
     fence_mbar_init();
@@ -252,18 +256,20 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         continue;
       }
       if constexpr (EPI == kEpiSwigluSplit) {
-        // As above, with the hi and the lo part of 64 output columns in the two staging tiles.
+        // The hi and the lo part of the group's 64 output columns in a staging tile each.
+        static_assert(BN == 256 || EPI != kEpiSwigluSplit, "a column group per warp group");
         const int r = quarter * 32 + lane;
-        const bool leader = threadIdx.x == 64;
-        uint8_t* stage = smem + Cfg::OUT_OFFSET;
+        const int half = (warp - 2) >> 2;
+        const bool leader = (threadIdx.x & 127) == 64;
+        uint8_t* stage = smem + Cfg::OUT_OFFSET + half * 32768;
 #pragma unroll
-        for (int c = 0; c < BN / 64; ++c) {
-          const int a_col = (c >> 1) * 128 + (c & 1) * 32;
+        for (int c = 0; c < 2; ++c) {
+          const int a_col = half * 128 + c * 32;
           uint32_t va[32], vb[32];
           tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + a_col), va);
           tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + a_col + 64), vb);
           tmem_ld_wait();
-          if (c + 1 == BN / 64) {
+          if (c == 1) {
             tc_fence_before_sync();
             mbar_arrive(&acc_empty[acc]);
           }
@@ -272,9 +278,9 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             const float a = __uint_as_float(va[e]);
             va[e] = __float_as_uint(a / (1.f + expf(-a)) * __uint_as_float(vb[e]));
           }
-          if ((c & 1) == 0) {
+          if (c == 0) {
             if (leader) tma_store_wait_read0();  // the stores that last used the staging tiles have read them
-            named_bar_sync(1, 128);
+            named_bar_sync(1 + half, 128);
           }
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
@@ -282,13 +288,13 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               split_pair(__uint_as_float(va[g * 8 + 2 * e]), __uint_as_float(va[g * 8 + 2 * e + 1]), hi[e], lo[e]);
-            *reinterpret_cast<uint4*>(stage + sw128_offset(r, (c & 1) * 4 + g)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(stage + 16384 + sw128_offset(r, (c & 1) * 4 + g)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            *reinterpret_cast<uint4*>(stage + sw128_offset(r, c * 4 + g)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(stage + 16384 + sw128_offset(r, c * 4 + g)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
-          if (c & 1) {
+          if (c == 1) {
             fence_proxy_async_smem();
-            named_bar_sync(1, 128);
-            const int col = tn * (BN / 2) + (c >> 1) * 64;
+            named_bar_sync(1 + half, 128);
+            const int col = tn * (BN / 2) + half * 64;
             if (leader && col < p.n_valid / 2) {
               tma_store_3d(&tmC, stage, col, tm * 128, b);
               tma_store_3d(&tmC, stage + 16384, p.n_valid / 2 + col, tm * 128, b);
@@ -500,7 +506,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     }
   }
 
-  if (warp >= 2 && (EPI == kEpiOuter ? lane == 0 : EPI != kEpiDirect && threadIdx.x == 64)) tma_store_wait0();
+  if (warp >= 2 && (EPI == kEpiOuter ? lane == 0 : EPI != kEpiDirect && (threadIdx.x & 127) == 64)) tma_store_wait0();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {

@@ -87,7 +87,7 @@ struct BackgroundScope {
 };
 
 static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
-  const int BN = a.mul ? 128 : t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.K, a.batch);
+  const int BN = a.mul ? 128 : a.split ? 256 : t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.K, a.batch);
   CUtensorMap tmA, tmB;
   const bool a_shared = a.batch > 1 && a.sa == 0;  // one A for every batch item
   {
@@ -163,15 +163,16 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   const int total = p.tiles_m * p.tiles_n * a.batch;
   const int grid = total < sm_count() ? total : sm_count();
   auto go = [&](auto bn, auto epi) -> int {
-    B200_LAUNCH((bmm_nt_kernel<bn.value, epi.value>), grid, 192, (BmmCfg<bn.value, epi.value>::SMEM_BYTES), stream, tmA, tmB, tmC,
+    B200_LAUNCH((bmm_nt_kernel<bn.value, epi.value>), grid, (BmmCfg<bn.value, epi.value>::THREADS), (BmmCfg<bn.value, epi.value>::SMEM_BYTES), stream, tmA, tmB, tmC,
                 tmM, p);
     return 0;
   };
   auto pick = [&](auto bn) -> int {
     if (a.opm_ntok > 0) return go(bn, std::integral_constant<int, kEpiOuter>());
-    if (a.swiglu) return a.split ? go(bn, std::integral_constant<int, kEpiSwigluSplit>()) : go(bn, std::integral_constant<int, kEpiSwiglu>());
+    if (a.swiglu) return go(bn, std::integral_constant<int, kEpiSwiglu>());
     return p.tma_c ? go(bn, std::integral_constant<int, kEpiBulk>()) : go(bn, std::integral_constant<int, kEpiDirect>());
   };
+  if (a.split) return go(std::integral_constant<int, 256>(), std::integral_constant<int, kEpiSwigluSplit>());
   if (a.mul) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiMul>());
   return BN == 256 ? pick(std::integral_constant<int, 256>()) : pick(std::integral_constant<int, 128>());
 }
