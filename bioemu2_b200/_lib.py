@@ -119,6 +119,8 @@ SIGNATURES = {
     "b200_opm_workspace_bytes": (c_size_t, [c_int, c_int]),
     "b200_opm_fwd": (c_int, [c_void_p, c_void_p, c_int, c_void_p, POINTER(OpmWeights), c_int, c_int, c_int, c_int,
                              c_int, c_void_p, c_size_t, c_void_p]),
+    "b200_opm_add_fwd": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, POINTER(OpmWeights), c_int, c_int, c_int,
+                                 c_int, c_void_p, c_size_t, c_void_p]),
     "b200_attention_core_fwd": (c_int, [POINTER(AttentionCoreArgs), c_void_p]),
     "b200_opm_cols_fwd": (c_int, [c_void_p, c_void_p, c_void_p, POINTER(OpmWeights), c_int, c_int, c_int, c_int, c_void_p,
                                   c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
@@ -151,6 +153,7 @@ SIGNATURES = {
     "b200_accurate_transition_fwd": (c_int, [c_void_p] * 6 + [c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t,
                                              c_void_p]),
     "b200_masked_softmax_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
+    "b200_pwa_values": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "b200_pwa_gate": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "b200_gated_residual_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int, c_int, c_int,
                                         c_void_p]),

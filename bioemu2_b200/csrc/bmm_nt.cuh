@@ -35,7 +35,7 @@ struct BmmParams {
   int remap_n, remap_m;
   // Bulk output: the scaled (+ bias) tile leaves through 16 KB staging tiles ([128 rows][128 B]: 32 fp32 or 64
   // bf16 columns) and the C tensor map, 1 = stored, 2 = added into C (the residual is C itself, which the
-  // epilogue then never reads).
+  // epilogue then never reads), 3 = stored with the rows as groups of 32, {column, row in group, group, batch}.
   int tma_c;
   // Split operands stored once as (hi | lo): a K block at or past the fold is loaded from that many blocks before, which
   // makes the operand hi | hi | lo.  INT_MAX: none.
@@ -52,21 +52,25 @@ enum BmmEpilogue : int {
   // come by TMA during the product's K loop (read by the lanes from their rows: 16 against 9 us without the gate for
   // 2048 x 768 x 768, 23 against 13 for K = 3072).
   kEpiMul = 2,
+  kEpiAdd = 6,     // the same with fp32 addends: a residual that is not C itself
   kEpiSwiglu = 3,  // bulk bf16: the columns are pairs of 64-column blocks (a | b), C gets silu(a) * b, half as many columns
   kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b, with expf and exact division
   kEpiOuter = 5,   // outer products of 32 x 32, one pair's 2 KB in one piece
 };
 
+template <int EPI>
+inline constexpr bool kTileOperand = EPI == kEpiMul || EPI == kEpiAdd;
+
 template <int BN, int EPI>
 struct BmmCfg {
   static constexpr int BM = 128;
   static constexpr int BK = 64;
-  static constexpr int STAGES = EPI == kEpiSwigluSplit ? 3 : EPI == kEpiMul || BN == 256 ? 4 : 6;
+  static constexpr int STAGES = EPI == kEpiSwigluSplit ? 3 : kTileOperand<EPI> || BN == 256 ? 4 : 6;
   static constexpr uint32_t A_BYTES = BM * BK * 2;
   static constexpr uint32_t B_BYTES = BN * BK * 2;
   static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr uint32_t MUL_OFFSET = STAGES * STAGE_BYTES;     // kEpiMul: the factors' [128 rows][32 columns] tiles
-  static constexpr uint32_t MUL_BYTES = EPI == kEpiMul ? BN * 128 * 4 : 0;
+  static constexpr uint32_t MUL_OFFSET = STAGES * STAGE_BYTES;     // the factors' or addends' [128 rows][32 columns] tiles
+  static constexpr uint32_t MUL_BYTES = kTileOperand<EPI> ? BN * 128 * 4 : 0;
   static constexpr uint32_t BAR_OFFSET = MUL_OFFSET + MUL_BYTES;
   static constexpr uint32_t BIAS_OFFSET = BAR_OFFSET + 1024;       // the tile's BN bias values
   static constexpr uint32_t OUT_OFFSET = BAR_OFFSET + 2048;        // [128 rows][128 B] tiles for bulk output
@@ -112,7 +116,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
     if (EPI != kEpiDirect && EPI != kEpiOuter) prefetch_tmap(&tmC);
-    if (EPI == kEpiMul) prefetch_tmap(&tmM);
+    if (kTileOperand<EPI>) prefetch_tmap(&tmM);
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
@@ -190,14 +194,14 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       for (int c = 0; c < BN / 32; ++c)
         tma_load_2d(smem + Cfg::MUL_OFFSET + c * 16384, &tmM, mul_full, tn * BN + c * 32, tm * 128);
     };
-    if (EPI == kEpiMul && threadIdx.x == 64 && int(blockIdx.x) < total_tiles) load_factors(blockIdx.x);
+    if (kTileOperand<EPI> && threadIdx.x == 64 && int(blockIdx.x) < total_tiles) load_factors(blockIdx.x);
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
       const int b = tile / tiles_per_batch;
       const int rem = tile - b * tiles_per_batch;
       const int tm = rem / p.tiles_n;
       const int tn = rem - tm * p.tiles_n;
       const int acc = it & 1;
-      if ((EPI == kEpiBulk || EPI == kEpiMul) && p.bias) {
+      if ((EPI == kEpiBulk || kTileOperand<EPI>) && p.bias) {
         // Read by every lane from shared memory (by every lane from global memory: 25 against 17 us without a bias for
         // 2048 x 4608 x 768).  The previous tile's values have been read before its last barrier; the first barrier
         // of this one makes the new ones visible.
@@ -207,7 +211,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           bias_s[i + quarter * 32 + lane] = col < p.n_valid ? p.bias[col] : 0.f;
         }
       }
-      if (EPI == kEpiMul) mbar_wait(mul_full, it & 1, 5);
+      if (kTileOperand<EPI>) mbar_wait(mul_full, it & 1, 5);
       mbar_wait(&acc_full[acc], (it >> 1) & 1, 4);
       tc_fence_after_sync();
       const int row = tm * 128 + quarter * 32 + lane;
@@ -304,7 +308,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         }
         continue;
       }
-      if constexpr (EPI == kEpiMul || EPI == kEpiBulk) {
+      if constexpr (EPI == kEpiBulk || kTileOperand<EPI>) {
         // 32 columns at a time into one of two swizzled staging tiles; warp 2's first lane sends each tile off.
         const int r = quarter * 32 + lane;
         const bool leader = threadIdx.x == 64;
@@ -349,6 +353,10 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
                 const float4 mv = *reinterpret_cast<const float4*>(factors + sw128_offset(r, g));
                 x.x *= mv.x; x.y *= mv.y; x.z *= mv.z; x.w *= mv.w;
               }
+              if (EPI == kEpiAdd) {
+                const float4 av = *reinterpret_cast<const float4*>(factors + sw128_offset(r, g));
+                x.x += av.x; x.y += av.y; x.z += av.z; x.w += av.w;
+              }
               *reinterpret_cast<float4*>(stage + sw128_offset(r, g)) = x;
             }
           } else {
@@ -380,14 +388,16 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             if (leader && tcol0 < p.n_valid) {
               if (p.tma_c == 2)
                 tma_reduce_add_3d(&tmC, stage, tcol0, c1, c2);
+              else if (p.tma_c == 3)
+                tma_store_4d(&tmC, stage, tcol0, 0, tm * 4, b);
               else
                 tma_store_3d(&tmC, stage, tcol0, c1, c2);
               tma_store_commit();
             }
           }
         }
-        // every thread has read its factors before the last barrier above
-        if (EPI == kEpiMul && leader && tile + int(gridDim.x) < total_tiles) load_factors(tile + gridDim.x);
+        // every thread has read its part before the last barrier above
+        if (kTileOperand<EPI> && leader && tile + int(gridDim.x) < total_tiles) load_factors(tile + gridDim.x);
         continue;
       }
       if constexpr (EPI == kEpiOuter) {

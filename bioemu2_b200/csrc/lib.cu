@@ -61,6 +61,9 @@ struct BmmLaunch {
   const float* mul = nullptr;  // bulk output: per-element fp32 factor, row pitch mul_pitch
   int mul_pitch = 0;
   bool swiglu = false;  // bulk bf16 output: N columns are 64-wide (a | b) block pairs, C has N / 2 columns of silu(a) * b
+  int row_groups = 0;          // bulk bf16 output, M = 32 * row_groups: group g of batch item b is C + g * group_stride + b * sc
+  int64_t group_stride = 0;
+  int b_rows = 0;              // rows of B that exist, if fewer than N (the rest count as zeros)
   bool split = false;   // with swiglu: C has N columns, (hi | lo) of the fp32 values
   int a_fold = 0, b_fold = 0;  // operand stored as (hi | lo), each part this many K blocks of 64, read as hi | hi | lo
 };
@@ -87,7 +90,17 @@ struct BackgroundScope {
 };
 
 static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
-  const int BN = a.mul ? 128 : a.split ? 256 : t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.K, a.batch);
+  const int64_t c_batch = a.sc > 0 ? a.sc : a.ldc * int64_t(a.M);
+  const int c_esz = a.out_f32 ? 4 : 2;
+  // Bulk output through the C tensor map where the layout allows it (the map clips the last column group): the
+  // residual (if any) being C itself, and for the transposed pair store lines that are whole row tiles.
+  const bool bulk_c = a.opm_ntok == 0 && (a.ldc * c_esz) % 16 == 0 && (c_batch * c_esz) % 16 == 0 && aligned(a.C, 16) &&
+                      (a.remap_n == 0 || (a.remap_n % 128 == 0 && a.batch == 1 && a.M == a.remap_n * (a.remap_m > 0 ? a.remap_m : a.remap_n)));
+  // An fp32 residual elsewhere comes by TMA tiles, as a gate's factors do (read by the lanes from their rows: 11 us against 7
+  // for 65536 x 128 x 128).
+  const bool add = bulk_c && a.residual && a.residual != a.C && a.out_f32 && a.batch == 1 && a.remap_n == 0 && !a.mul &&
+                   !a.swiglu && aligned(a.residual, 16);
+  const int BN = a.mul || add ? 128 : a.split ? 256 : t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.K, a.batch);
   CUtensorMap tmA, tmB;
   const bool a_shared = a.batch > 1 && a.sa == 0;  // one A for every batch item
   {
@@ -97,8 +110,8 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
     if (int e = make_tmap_bf16(&tmA, a.A, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   {
-    const uint64_t dims[3] = {uint64_t(a.b_fold ? a.b_fold * 128 : a.K), uint64_t(a.N), uint64_t(a.batch)};
-    const uint64_t str[2] = {uint64_t(a.ldb) * 2, uint64_t(a.sb > 0 ? a.sb : a.ldb * a.N) * 2};
+    const uint64_t dims[3] = {uint64_t(a.b_fold ? a.b_fold * 128 : a.K), uint64_t(a.b_rows ? a.b_rows : a.N), uint64_t(a.batch)};
+    const uint64_t str[2] = {uint64_t(a.ldb) * 2, uint64_t(a.sb > 0 ? a.sb : a.ldb * (a.b_rows ? a.b_rows : a.N)) * 2};
     const uint32_t box[3] = {64, uint32_t(BN), 1};
     if (int e = make_tmap_bf16(&tmB, a.B, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
@@ -123,16 +136,18 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   p.a_shared = a_shared ? 1 : 0;
   p.a_fold = a.a_fold ? a.a_fold : INT_MAX;
   p.b_fold = a.b_fold ? a.b_fold : INT_MAX;
-  // Bulk output through the C tensor map where the layout allows it (the map clips the last column group): the
-  // residual (if any) being C itself, and for the transposed pair store lines that are whole row tiles.
   p.tma_c = 0;
   CUtensorMap tmC = tmA;
-  const int64_t c_batch = a.sc > 0 ? a.sc : a.ldc * int64_t(a.M);
-  const int c_esz = a.out_f32 ? 4 : 2;
   const int c_cols = 128 / c_esz;  // columns of one staging tile
-  if (a.opm_ntok == 0 && (a.ldc * c_esz) % 16 == 0 && (c_batch * c_esz) % 16 == 0 && aligned(a.C, 16) &&
-      (a.residual == nullptr || a.residual == a.C) && (a.bias == nullptr || aligned(a.bias, 16)) &&
-      (a.remap_n == 0 || (a.remap_n % 128 == 0 && a.batch == 1 && a.M == a.remap_n * p.remap_m))) {
+  if (a.row_groups > 0) {
+    if (!bulk_c || a.out_f32 || a.residual || a.M != 32 * a.row_groups || a.group_stride % 8)
+      return fail(B200_ERR_INVALID_ARGUMENT, "grouped rows need aligned bf16 bulk output");
+    const uint64_t dims[4] = {uint64_t(a.N), 32, uint64_t(a.row_groups), uint64_t(a.batch)};
+    const uint64_t str[3] = {uint64_t(a.ldc) * 2, uint64_t(a.group_stride) * 2, uint64_t(a.sc) * 2};
+    const uint32_t box[4] = {64, 32, 4, 1};
+    if (int e = make_tmap_bf16(&tmC, a.C, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+    p.tma_c = 3;
+  } else if (bulk_c && (add || a.residual == nullptr || a.residual == a.C) && (a.bias == nullptr || aligned(a.bias, 16))) {
     uint64_t dims[3], str[2];
     uint32_t box[3];
     dims[0] = uint64_t(a.swiglu && !a.split ? a.N / 2 : a.N);
@@ -149,16 +164,16 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
     if (int e = make_tmap(&tmC, a.out_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.C, 3, dims,
                           str, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return e;
-    p.tma_c = a.residual ? 2 : 1;
+    p.tma_c = a.residual && !add ? 2 : 1;
   }
   if ((a.mul || a.swiglu) && (!p.tma_c || (a.mul && (!aligned(a.mul, 16) || a.mul_pitch % 4 || a.batch != 1))))
     return fail(B200_ERR_INVALID_ARGUMENT, "a gated product needs bulk output and 16-byte aligned factors");
   CUtensorMap tmM = tmC;
-  if (a.mul) {
+  if (a.mul || add) {
     const uint64_t dims[2] = {uint64_t(a.N), uint64_t(a.M)};
-    const uint64_t str[1] = {uint64_t(a.mul_pitch) * 4};
+    const uint64_t str[1] = {uint64_t(add ? a.ldc : a.mul_pitch) * 4};
     const uint32_t box[2] = {32, 128};
-    if (int e = make_tmap(&tmM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.mul, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+    if (int e = make_tmap(&tmM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, add ? a.residual : a.mul, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   const int total = p.tiles_m * p.tiles_n * a.batch;
   const int grid = total < sm_count() ? total : sm_count();
@@ -173,6 +188,7 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
     return p.tma_c ? go(bn, std::integral_constant<int, kEpiBulk>()) : go(bn, std::integral_constant<int, kEpiDirect>());
   };
   if (a.split) return go(std::integral_constant<int, 256>(), std::integral_constant<int, kEpiSwigluSplit>());
+  if (add && p.tma_c) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiAdd>());
   if (a.mul) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiMul>());
   return BN == 256 ? pick(std::integral_constant<int, 256>()) : pick(std::integral_constant<int, 128>());
 }
@@ -845,7 +861,7 @@ size_t b200_opm_workspace_bytes(int S, int N) {
 // is added (exactly one of the partial results that are later summed should carry it).
 static int opm_run(const void* m, const uint8_t* mask, int mask_ndim, void* out, const b200_opm_weights* w, int B,
                    int S, int N, int j0, int nj, const float* ext_scale, bool add_bias, int m_dtype, int out_dtype,
-                   void* workspace, size_t workspace_bytes, b200_stream_t stream_) {
+                   void* workspace, size_t workspace_bytes, b200_stream_t stream_, const float* residual = nullptr) {
   if (int e = b200_check_device()) return e;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   B200_CHECK_ARG(m && mask && out && w, "m/mask/out/w is NULL");
@@ -916,6 +932,7 @@ static int opm_run(const void* m, const uint8_t* mask, int mask_ndim, void* out,
         BmmLaunch a{outer, w->w_o, dst, 1, ci * nj, 128, 1024, 1024, 1024, 128, 0, 0, 0};
         a.bias = add_bias ? w->bias_o : nullptr;
         a.out_f32 = out_dtype == B200_DTYPE_F32;
+        if (residual) a.residual = residual + (size_t(bi) * N * nj + size_t(i0) * nj) * 128;
         if (int e = launch_bmm(a, stream)) return e;
       }
     }
@@ -928,6 +945,14 @@ int b200_opm_fwd(const void* m, const uint8_t* mask, int mask_ndim, void* out, c
                  b200_stream_t stream) {
   return opm_run(m, mask, mask_ndim, out, w, B, S, N, 0, N, nullptr, true, m_dtype, out_dtype, workspace, workspace_bytes,
                  stream);
+}
+
+int b200_opm_add_fwd(const void* m, const uint8_t* mask, int mask_ndim, const float* residual, float* out,
+                     const b200_opm_weights* w, int B, int S, int N, int m_dtype, void* workspace, size_t workspace_bytes,
+                     b200_stream_t stream) {
+  B200_CHECK_ARG(residual && residual != out && aligned(residual, 16), "residual must be 16-byte aligned and not the output");
+  return opm_run(m, mask, mask_ndim, out, w, B, S, N, 0, N, nullptr, true, m_dtype, B200_DTYPE_F32, workspace, workspace_bytes,
+                 stream, residual);
 }
 
 int b200_opm_cols_fwd(const void* m, const uint8_t* mask, void* out, const b200_opm_weights* w, int S, int N, int j0,
@@ -1556,6 +1581,21 @@ int b200_masked_softmax_rows(const void* logits, const uint8_t* mask, void* out,
   B200_LAUNCH(masked_softmax_rows_kernel, grid_for((int64_t)H * n_rows, 8), 256, 0, static_cast<cudaStream_t>(stream),
               static_cast<const __nv_bfloat16*>(logits), mask, static_cast<__nv_bfloat16*>(out), H, n_rows, n, pitch);
   return B200_OK;
+}
+
+int b200_pwa_values(const void* w_m, const void* mn, void* vT, int S, int n, int c_m, int H, int pitch, b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(w_m && mn && vT, "w_m/mn/vT is NULL");
+  B200_CHECK_ARG(S > 0 && n > 0 && H > 0 && c_m > 0 && c_m % 8 == 0, "S, n, H must be positive, c_m=%d a multiple of 8", c_m);
+  B200_CHECK_ARG(pitch >= n && pitch % 8 == 0, "pitch=%d must be a multiple of 8 and >= n", pitch);
+  B200_CHECK_ARG(aligned(w_m, 16) && aligned(mn, 16) && aligned(vT, 16), "w_m/mn/vT must be 16-byte aligned");
+  // v_h^T[s] = W_m[h] . mn[s]^T of every head and MSA row in one launch: one A for all S batch items, 32 rows of C a head.
+  // (A launch per head: 8 x 6.3 us for 128 rows of 256 tokens.)
+  BmmLaunch a{w_m, mn, vT, S, 32 * H, pitch, c_m, c_m, c_m, pitch, 0, int64_t(n) * c_m, int64_t(32) * pitch};
+  a.b_rows = n;
+  a.row_groups = H;
+  a.group_stride = int64_t(S) * 32 * pitch;
+  return launch_bmm(a, static_cast<cudaStream_t>(stream));
 }
 
 int b200_pwa_gate(const void* o, const void* g, void* og, int S, int n, int H, b200_stream_t stream) {

@@ -251,8 +251,9 @@ class OpmPacked:
                                       self.f32[1].data_ptr(), self.f32[2].data_ptr())
 
 
-def outer_product_mean(m: Tensor, mask: Tensor, w: OpmPacked) -> Tensor:
-    """``m[B,S,N,64]`` (fp32 or bf16), ``mask[B,S,N]`` or ``[B,N]`` -> ``[B,N,N,128]`` in ``m.dtype``."""
+def outer_product_mean(m: Tensor, mask: Tensor, w: OpmPacked, residual: Tensor | None = None) -> Tensor:
+    """``m[B,S,N,64]`` (fp32 or bf16), ``mask[B,S,N]`` or ``[B,N]`` -> ``[B,N,N,128]`` in ``m.dtype``; ``residual`` (fp32
+    like ``m``, contiguous) is added."""
     _require_cuda(m, mask)
     if m.ndim != 4 or m.shape[-1] != 64:
         raise ValueError(f"expected m[B,S,N,64], got {tuple(m.shape)}")
@@ -268,13 +269,21 @@ def outer_product_mean(m: Tensor, mask: Tensor, w: OpmPacked) -> Tensor:
     zd = _zdtype(m)
     m = m.contiguous()
     out = torch.empty(B, N, N, 128, dtype=m.dtype, device=m.device)
+    if residual is not None and (residual.dtype != torch.float32 or m.dtype != torch.float32 or residual.shape != out.shape
+                                 or not residual.is_contiguous()):
+        raise ValueError("residual must be contiguous float32 [B,N,N,128], and m float32")
     if out.numel() == 0:
         return out
     if S == 0:  # no MSA rows: the mean of nothing is zero, so every pair gets proj_o's bias
-        return out.copy_(w.f32[2].to(out.dtype).expand_as(out))
+        out.copy_(w.f32[2].to(out.dtype).expand_as(out))
+        return out if residual is None else out.add_(residual)
     m8 = mask_u8(mask)
     nbytes = lib.b200_opm_workspace_bytes(S, N)
     ws = workspace(nbytes, m.device)
+    if residual is not None:
+        _lib.check(lib.b200_opm_add_fwd(m.data_ptr(), m8.data_ptr(), mask.ndim, residual.data_ptr(), out.data_ptr(),
+                                        ctypes.byref(w.struct), B, S, N, zd, ws.data_ptr(), nbytes, _stream()))
+        return out
     _lib.check(lib.b200_opm_fwd(m.data_ptr(), m8.data_ptr(), mask.ndim, out.data_ptr(), ctypes.byref(w.struct), B, S, N,
                                 zd, zd, ws.data_ptr(), nbytes, _stream()))
     return out
@@ -921,7 +930,7 @@ def pair_weighted_averaging(m: Tensor, z: Tensor, mask: Tensor, w: PwaPacked, ad
 
     Per batch item: ``norm_m`` and the gate / value projections of the MSA rows, the per-head weights
     ``softmax_j(proj_z(norm_z(z))[i,j,h])`` with masked pairs at -1e6, the per-head product ``w_h . v_h^T`` on the tensor
-    cores (``v_h^T`` is written transposed by its projection GEMM, so both operands are K-major), gating, ``proj_o``.
+    cores (the values' projection writes ``v_h^T``, so both operands are K-major), gating, ``proj_o``.
     """
     _require_cuda(m, z, mask)
     if m.ndim != 4 or z.ndim != 4 or tuple(z.shape[1:]) != (m.shape[2], m.shape[2], 128) or z.shape[0] != m.shape[0]:
@@ -960,13 +969,9 @@ def pwa_apply(mn_all: Tensor, mn_own: Tensor, logits: Tensor, mask8: Tensor, w: 
     bf = torch.bfloat16
     if tuple(logits.shape) != (H, n_i, Nk) or tuple(mask8.shape) != (n_i, N) or tuple(out.shape) != (S, n_i, c_m):
         raise ValueError(f"inconsistent shapes: logits {tuple(logits.shape)}, mask {tuple(mask8.shape)}, out {tuple(out.shape)}")
-    mn_p = mn_all
-    if N != Nk:   # the token axis is the GEMM's column count, which the kernel wants in multiples of 8
-        mn_p = torch.zeros(S, Nk, c_m, dtype=bf, device=mn_all.device)
-        mn_p[:, :N] = mn_all
     vT = torch.empty(H, S * 32, Nk, dtype=bf, device=mn_all.device)                                # [h][(s, d)][j]
-    for h in range(H):   # v_h^T[s] = W_m[h] . mn[s]^T : one A for all S batch items
-        bmm_nt_into(w.w_m[h * 32:(h + 1) * 32].unsqueeze(0).expand(S, 32, c_m), mn_p, vT[h].view(S, 32, Nk))
+    mn_all = mn_all.contiguous()
+    _lib.check(lib.b200_pwa_values(w.w_m.data_ptr(), mn_all.data_ptr(), vT.data_ptr(), S, N, c_m, H, Nk, _stream()))
     wts = torch.empty_like(logits)
     _lib.check(lib.b200_masked_softmax_rows(logits.data_ptr(), mask8.contiguous().data_ptr(), wts.data_ptr(), H, n_i, N, Nk,
                                             _stream()))

@@ -9,6 +9,7 @@ products pair-contiguously, and ``proj_o`` is a second GEMM over them.
 """
 from __future__ import annotations
 
+import torch
 import torch.nn as nn
 from torch import Tensor
 
@@ -46,6 +47,13 @@ class OuterProductMean(PackedWeightsMixin, nn.Module):
         if precision.use_ieee(self.matmul_precision, m):
             return ieee.outer_product_mean(m, mask, self, self.split_weights())
         return F.outer_product_mean(m, mask, self.packed())
+
+    def forward_add(self, m: Tensor, mask: Tensor, z: Tensor) -> Tensor:
+        """``z + forward(m, mask)`` as a new tensor of z's dtype."""
+        if z.dtype != torch.float32 or m.dtype != torch.float32 or precision.use_ieee(self.matmul_precision, m):
+            upd = self.forward(m, mask)
+            return F.add_rows(z.contiguous(), upd) if z.dtype == torch.float32 else z + upd.to(z.dtype)
+        return F.outer_product_mean(m, mask, self.packed(), residual=z.contiguous())
 
 
 OuterProductMeanVanilla = OuterProductMean

@@ -78,10 +78,12 @@ class PairMixerMSAModule(nn.Module):
         self._s_proj, self._msa_proj = _PaddedLinear(self.s_proj), _PaddedLinear(self.msa_proj)
 
     def forward(self, s: Tensor | None, z: Tensor, emb: Tensor, msa: Tensor, msa_mask: Tensor, has_deletion: Tensor,
-                deletion_value: Tensor, msa_paired: Tensor, token_pad_mask: Tensor) -> tuple[Tensor | None, Tensor]:
+                deletion_value: Tensor, msa_paired: Tensor, token_pad_mask: Tensor,
+                embedded: Tensor | None = None) -> tuple[Tensor | None, Tensor]:
+        """``embedded``: what ``embed_msa`` returns for these features, where a caller has it already."""
         if self.training:
             raise RuntimeError("bioemu2_b200 modules are inference-only: call .eval()")
-        m = self.embed_msa(emb, msa, has_deletion, deletion_value, msa_paired)
+        m = embedded if embedded is not None else self.embed_msa(emb, msa, has_deletion, deletion_value, msa_paired)
         tok = token_pad_mask.bool()
         token_mask = tok.unsqueeze(-1) & tok.unsqueeze(-2)
         for layer in self.layers:
@@ -190,9 +192,13 @@ class PairMixerSequenceEmbedder(nn.Module):
             extra = extra.expand(a.shape[0], a.shape[1], c.shape[1], a.shape[2])
         return s_init, F.pair_outer_sum(a, c, extra)
 
-    def _recycle(self, x: Tensor, x_init: Tensor, norm: nn.LayerNorm, name: str) -> Tensor:
+    def _recycle(self, x: Tensor | None, x_init: Tensor, norm: nn.LayerNorm, name: str) -> Tensor:
         """``x_init + recycle(norm(x))`` (pairmixer.py:282-283): one kernel for the 128-channel pair tensor, a LayerNorm pass
-        and a GEMM that adds ``x_init`` for the single track."""
+        and a GEMM that adds ``x_init`` for the single track.  ``None``: the zeros of the first step, whose norm is the
+        LayerNorm's bias in every row."""
+        if x is None:
+            row = norm.bias.detach().to(torch.bfloat16).view(1, -1)
+            return F.add_rows(x_init, F.linear_bf16(row, self._lin[name].weight(), out_dtype=torch.float32).view(-1))
         if x.shape[-1] == 128 and self._lin[name].linear.weight.shape == (128, 128):
             return F.ln_linear(x, None, norm.weight, norm.bias, self._lin[name].weight(), residual=x_init)
         xn = F.rows_to_bf16(x, norm.weight, norm.bias)
@@ -214,11 +220,14 @@ class PairMixerSequenceEmbedder(nn.Module):
             return s_init, F.add_rows(z_init, self.uncond_transition(zn))
         mask = feats["token_pad_mask"].bool()
         pair_mask = mask.unsqueeze(-1) & mask.unsqueeze(-2)
-        s, z = torch.zeros_like(s_init), torch.zeros_like(z_init)
+        # The MSA embedding is the same in every recycling step (the blocks leave their input alone).
+        m = self.msa_module.embed_msa(s_inputs, feats["msa"], feats["has_deletion"], feats["deletion_value"],
+                                      feats["msa_paired"])
+        s = z = None
         for _ in range(num_steps_recycle + 1):
             s = self._recycle(s, s_init, self.s_norm, "s_recycle")
             z = self._recycle(z, z_init, self.z_norm, "z_recycle")
             _, z = self.msa_module(None, z, s_inputs, feats["msa"], feats["msa_mask"], feats["has_deletion"],
-                                   feats["deletion_value"], feats["msa_paired"], feats["token_pad_mask"])
+                                   feats["deletion_value"], feats["msa_paired"], feats["token_pad_mask"], embedded=m)
             s, z = self.pairmixer_module(s, z, pair_mask=pair_mask)
         return s, z

@@ -211,6 +211,11 @@ int b200_opm_fwd(const void* m, const uint8_t* mask, int mask_ndim, void* out, c
                  int S, int N, int m_dtype, int out_dtype, void* workspace, size_t workspace_bytes,
                  b200_stream_t stream);
 
+/* The same as fp32 with residual [B][N][N][128] (fp32, not out) added. */
+int b200_opm_add_fwd(const void* m, const uint8_t* mask, int mask_ndim, const float* residual, float* out,
+                     const b200_opm_weights* w, int B, int S, int N, int m_dtype, void* workspace, size_t workspace_bytes,
+                     b200_stream_t stream);
+
 /* Partial form for callers that shard the MSA depth and the pair columns (DistributedOuterProductMean,
  * src/bioemu2/context_parallel/ops/outer_product_mean.py:116-262): m[S][N][64] holds only this caller's MSA rows,
  * the output is out[N][nj][128] for token columns j0 .. j0+nj-1, scaled by the device scalar *scale (1 / global
@@ -430,8 +435,10 @@ int b200_window_attention_pitched_fwd(const void* qkv, int qkv_pitch, const void
 /* ---------------------------------------------------------------------------------------------------
  * Pair-weighted averaging, PairWeightedAveraging.forward (src/bioemu2/biomoa/ops/pair_weighted_averaging.py:121-153),
  * is assembled from b200_rows_to_bf16 (norm_m), b200_linear_bf16 (proj_g, proj_o), b200_pair_bias_fwd (proj_z(norm_z(z))),
- * b200_bmm_nt (proj_m written transposed per head; the weighted average itself) and the two kernels below.
+ * b200_bmm_nt (the weighted average itself) and the kernels below.
  *
+ * b200_pwa_values           vT[h][(s, d)][j] = (W_m[h] . mn[s]^T)[d][j]: the values of every head, transposed; w_m bf16
+ *                           [H*32][c_m], mn bf16 [S][n][c_m], vT bf16 [H][S*32][pitch] with zeros in columns n .. pitch-1.
  * b200_masked_softmax_rows  w[h][i][j] = softmax_j(mask[i][j] ? logits[h][i][j] : -1e6) (:141-142); logits bf16 in base-2
  *                           units [H][n_rows][pitch] as b200_pair_bias_fwd writes them, mask one byte per pair
  *                           [n_rows][n], w bf16 [H][n_rows][pitch] with zeros in columns n .. pitch-1.  n_rows == n
@@ -439,6 +446,7 @@ int b200_window_attention_pitched_fwd(const void* qkv, int qkv_pitch, const void
  * b200_pwa_gate             og[(s,i)][h*32+d] = sigmoid(g[(s,i)][h*32+d]) * o[h][i][s*32+d] (:145-151): gating and the
  *                           re-layout from per-head products to MSA rows; heads of 32 channels.
  * ------------------------------------------------------------------------------------------------- */
+int b200_pwa_values(const void* w_m, const void* mn, void* vT, int S, int n, int c_m, int H, int pitch, b200_stream_t stream);
 int b200_masked_softmax_rows(const void* logits, const uint8_t* mask, void* out, int H, int n_rows, int n, int pitch,
                              b200_stream_t stream);
 int b200_pwa_gate(const void* o, const void* g, void* og, int S, int n, int H, b200_stream_t stream);
