@@ -55,9 +55,14 @@ enum BmmEpilogue : int {
   kEpiAdd = 6,     // the same with fp32 addends: a residual that is not C itself
   kEpiSwiglu = 3,  // bulk bf16: the columns are pairs of 64-column blocks (a | b), C gets silu(a) * b, half as many columns
   kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b, with expf and exact division
+  // kEpiBulk with eight epilogue warps, each group of four draining half of the tile's columns: a short product's tile is
+  // its epilogue (K = 128: 2 K blocks of 64 against 128 columns of TMEM reads, staging and stores a lane).
+  kEpiBulkWide = 7,
   kEpiOuter = 5,   // outer products of 32 x 32, one pair's 2 KB in one piece
 };
 
+template <int EPI>
+inline constexpr bool kBulk = EPI == kEpiBulk || EPI == kEpiBulkWide;
 template <int EPI>
 inline constexpr bool kTileOperand = EPI == kEpiMul || EPI == kEpiAdd;
 
@@ -65,7 +70,7 @@ template <int BN, int EPI>
 struct BmmCfg {
   static constexpr int BM = 128;
   static constexpr int BK = 64;
-  static constexpr int STAGES = EPI == kEpiSwigluSplit ? 3 : kTileOperand<EPI> || BN == 256 ? 4 : 6;
+  static constexpr int STAGES = EPI == kEpiSwigluSplit || (EPI == kEpiBulkWide && BN == 256) ? 3 : EPI == kEpiBulkWide ? 5 : kTileOperand<EPI> || BN == 256 ? 4 : 6;
   static constexpr uint32_t A_BYTES = BM * BK * 2;
   static constexpr uint32_t B_BYTES = BN * BK * 2;
   static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
@@ -74,11 +79,12 @@ struct BmmCfg {
   static constexpr uint32_t BAR_OFFSET = MUL_OFFSET + MUL_BYTES;
   static constexpr uint32_t BIAS_OFFSET = BAR_OFFSET + 1024;       // the tile's BN bias values
   static constexpr uint32_t OUT_OFFSET = BAR_OFFSET + 2048;        // [128 rows][128 B] tiles for bulk output
-  static constexpr int OUT_TILES = EPI == kEpiSwigluSplit ? 4 : 2;
+  static constexpr int OUT_TILES = EPI == kEpiSwigluSplit || EPI == kEpiBulkWide ? 4 : 2;
   static constexpr uint32_t SMEM_BYTES = OUT_OFFSET + OUT_TILES * 16384 + 1024;  // + alignment slack
   // The split SwiGLU's expf and division keep four warps busy for longer than the product (40000 x 1024 x 384: 105 us): it
   // has eight, each group of four with one of the tile's two 64-column groups.
-  static constexpr int EPI_THREADS = EPI == kEpiSwigluSplit ? 256 : 128;
+  static constexpr int EPI_THREADS = EPI == kEpiSwigluSplit || EPI == kEpiBulkWide ? 256 : 128;
+  static constexpr int GROUPS = EPI_THREADS / 128;
   static constexpr int THREADS = 64 + EPI_THREADS;
 };
 
@@ -201,14 +207,16 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int tm = rem / p.tiles_n;
       const int tn = rem - tm * p.tiles_n;
       const int acc = it & 1;
-      if ((EPI == kEpiBulk || kTileOperand<EPI>) && p.bias) {
+      const int grp = Cfg::GROUPS == 1 ? 0 : (warp - 2) >> 2;
+      constexpr int GCOLS = BN / Cfg::GROUPS;            // columns a group drains
+      if ((kBulk<EPI> || kTileOperand<EPI>) && p.bias) {
         // Read by every lane from shared memory (by every lane from global memory: 25 against 17 us without a bias for
         // 2048 x 4608 x 768).  The previous tile's values have been read before its last barrier; the first barrier
         // of this one makes the new ones visible.
 #pragma unroll
-        for (int i = 0; i < BN; i += 128) {
-          const int col = tn * BN + i + quarter * 32 + lane;
-          bias_s[i + quarter * 32 + lane] = col < p.n_valid ? p.bias[col] : 0.f;
+        for (int i = 0; i < GCOLS; i += 128) {
+          const int k = grp * GCOLS + i + quarter * 32 + lane, col = tn * BN + k;
+          if (GCOLS >= 128 || quarter * 32 < GCOLS) bias_s[k] = col < p.n_valid ? p.bias[col] : 0.f;
         }
       }
       if (kTileOperand<EPI>) mbar_wait(mul_full, it & 1, 5);
@@ -251,9 +259,9 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             fence_proxy_async_smem();
             named_bar_sync(1, 128);
             const int col = tn * (BN / 2) + (c >> 1) * 64;
-            if (leader && col < p.n_valid / 2) {
-              tma_store_3d(&tmC, stage, col, tm * 128, b);
-              tma_store_commit();
+            if (leader) {
+              if (col < p.n_valid / 2) tma_store_3d(&tmC, stage, col, tm * 128, b);
+              tma_store_commit();  // an empty group too: the waits count groups
             }
           }
         }
@@ -263,12 +271,11 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         // The hi and the lo part of the group's 64 output columns in a staging tile each.
         static_assert(BN == 256 || EPI != kEpiSwigluSplit, "a column group per warp group");
         const int r = quarter * 32 + lane;
-        const int half = (warp - 2) >> 2;
         const bool leader = (threadIdx.x & 127) == 64;
-        uint8_t* stage = smem + Cfg::OUT_OFFSET + half * 32768;
+        uint8_t* stage = smem + Cfg::OUT_OFFSET + grp * 32768;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          const int a_col = half * 128 + c * 32;
+          const int a_col = grp * 128 + c * 32;
           uint32_t va[32], vb[32];
           tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + a_col), va);
           tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + a_col + 64), vb);
@@ -284,7 +291,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           }
           if (c == 0) {
             if (leader) tma_store_wait_read0();  // the stores that last used the staging tiles have read them
-            named_bar_sync(1 + half, 128);
+            named_bar_sync(1 + grp, 128);
           }
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
@@ -297,8 +304,8 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           }
           if (c == 1) {
             fence_proxy_async_smem();
-            named_bar_sync(1 + half, 128);
-            const int col = tn * (BN / 2) + half * 64;
+            named_bar_sync(1 + grp, 128);
+            const int col = tn * (BN / 2) + grp * 64;
             if (leader && col < p.n_valid / 2) {
               tma_store_3d(&tmC, stage, col, tm * 128, b);
               tma_store_3d(&tmC, stage + 16384, p.n_valid / 2 + col, tm * 128, b);
@@ -308,10 +315,10 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         }
         continue;
       }
-      if constexpr (EPI == kEpiBulk || kTileOperand<EPI>) {
+      if constexpr (kBulk<EPI> || kTileOperand<EPI>) {
         // 32 columns at a time into one of two swizzled staging tiles; warp 2's first lane sends each tile off.
         const int r = quarter * 32 + lane;
-        const bool leader = threadIdx.x == 64;
+        const bool leader = (threadIdx.x & 127) == 64;
         int c1 = tm * 128, c2 = b;  // tensor map {column, row, batch}, or {column, line, pos} when remapped
         if (p.remap_n > 0) {
           c1 = (tm * 128) / p.remap_n;
@@ -319,19 +326,22 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         }
         const int cps = p.out_f32 ? 1 : 2;  // 32-column chunks per staging tile
         uint32_t va[32], vb[32];
-        tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN), va);
+        constexpr int CHUNKS = GCOLS / 32;
+        const uint32_t t_addr = tmem_addr(tmem_base, quarter * 32, acc * BN + grp * GCOLS);
+        uint8_t* stages = smem + Cfg::OUT_OFFSET + grp * 32768;
+        tmem_ld_32x32(t_addr, va);
 #pragma unroll
-        for (int c = 0; c < BN / 32; ++c) {
+        for (int c = 0; c < CHUNKS; ++c) {
           uint32_t(&v)[32] = (c & 1) ? vb : va;
           const int st = p.out_f32 ? c : (c >> 1);  // staging tile number within the output tile
-          uint8_t* stage = smem + Cfg::OUT_OFFSET + (st & 1) * 16384;
+          uint8_t* stage = stages + ((it * (CHUNKS / cps) + st) & 1) * 16384;
           if (p.out_f32 || (c & 1) == 0) {
             if (leader) tma_store_wait_read1();  // the store that last used this staging tile has read it
-            named_bar_sync(1, 128);
+            named_bar_sync(1 + grp, 128);
           }
           tmem_ld_wait();
-          if (c + 1 < BN / 32) {
-            tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + (c + 1) * 32), (c & 1) ? va : vb);
+          if (c + 1 < CHUNKS) {
+            tmem_ld_32x32(t_addr + (c + 1) * 32, (c & 1) ? va : vb);
           } else {
             tc_fence_before_sync();
             mbar_arrive(&acc_empty[acc]);
@@ -346,7 +356,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               x.z = __uint_as_float(v[g * 4 + 2]) * scale;
               x.w = __uint_as_float(v[g * 4 + 3]) * scale;
               if (p.bias) {
-                const float4 bv = *reinterpret_cast<const float4*>(bias_s + c * 32 + g * 4);
+                const float4 bv = *reinterpret_cast<const float4*>(bias_s + grp * GCOLS + c * 32 + g * 4);
                 x.x += bv.x; x.y += bv.y; x.z += bv.z; x.w += bv.w;
               }
               if (EPI == kEpiMul) {
@@ -366,8 +376,8 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
 #pragma unroll
               for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[g * 8 + e]) * scale;
               if (p.bias) {
-                const float4 b0 = *reinterpret_cast<const float4*>(bias_s + c * 32 + g * 8);
-                const float4 b1 = *reinterpret_cast<const float4*>(bias_s + c * 32 + g * 8 + 4);
+                const float4 b0 = *reinterpret_cast<const float4*>(bias_s + grp * GCOLS + c * 32 + g * 8);
+                const float4 b1 = *reinterpret_cast<const float4*>(bias_s + grp * GCOLS + c * 32 + g * 8 + 4);
                 x[0] += b0.x; x[1] += b0.y; x[2] += b0.z; x[3] += b0.w;
                 x[4] += b1.x; x[5] += b1.y; x[6] += b1.z; x[7] += b1.w;
               }
@@ -382,17 +392,18 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             }
           }
           if (p.out_f32 || (c & 1) == 1) {
-            const int tcol0 = tn * BN + st * 32 * cps;
+            const int tcol0 = tn * BN + grp * GCOLS + st * 32 * cps;
             fence_proxy_async_smem();
-            named_bar_sync(1, 128);
-            if (leader && tcol0 < p.n_valid) {
-              if (p.tma_c == 2)
+            named_bar_sync(1 + grp, 128);
+            if (leader) {
+              if (tcol0 >= p.n_valid) {
+              } else if (p.tma_c == 2)
                 tma_reduce_add_3d(&tmC, stage, tcol0, c1, c2);
               else if (p.tma_c == 3)
                 tma_store_4d(&tmC, stage, tcol0, 0, tm * 4, b);
               else
                 tma_store_3d(&tmC, stage, tcol0, c1, c2);
-              tma_store_commit();
+              tma_store_commit();  // an empty group too: the waits count groups
             }
           }
         }
@@ -439,11 +450,10 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             }
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) {
+            if (lane == 0)
               bulk_store(static_cast<__nv_bfloat16*>(p.C) + ((long long)i * p.opm_ntok + j) * 1024, buf + (c & 3) * 2048, 2048);
-              tma_store_commit();
-            }
           }
+          if (lane == 0) tma_store_commit();  // an empty group too: the waits count groups
         }
         continue;
       }

@@ -185,7 +185,11 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   auto pick = [&](auto bn) -> int {
     if (a.opm_ntok > 0) return go(bn, std::integral_constant<int, kEpiOuter>());
     if (a.swiglu) return go(bn, std::integral_constant<int, kEpiSwiglu>());
-    return p.tma_c ? go(bn, std::integral_constant<int, kEpiBulk>()) : go(bn, std::integral_constant<int, kEpiDirect>());
+    if (!p.tma_c) return go(bn, std::integral_constant<int, kEpiDirect>());
+    // Up to four K blocks the epilogue is the longer part of a tile; beyond, its warps are covered and the K stages that
+    // the second pair of staging tiles takes the place of count (us, four warps against eight: 32768 x 768 x 128 29.1 / 21.7,
+    // 128 x 256^3 10.0 / 8.5, 128 x 384^3 21.5 / 23.9, 512 x 40000 x 384 26.5 / 30.1).
+    return p.k_blocks <= 4 ? go(bn, std::integral_constant<int, kEpiBulkWide>()) : go(bn, std::integral_constant<int, kEpiBulk>());
   };
   if (a.split) return go(std::integral_constant<int, 256>(), std::integral_constant<int, kEpiSwigluSplit>());
   if (add && p.tma_c) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiAdd>());

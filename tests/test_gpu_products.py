@@ -159,3 +159,16 @@ def test_packed_weights_layout():
     assert not buf[o2:o3].any()
     assert torch.equal(buf[o3:o4].view(2, 2, 32), torch.stack([c.to(BF16).view(2, 32), d.to(BF16).view(2, 32)], 1))
     assert torch.equal(buf[o4:o4 + 240], a.to(BF16).view(-1))
+
+
+@pytest.mark.parametrize("n", [8, 128, 200, 264])
+@pytest.mark.parametrize("k", [64, 256, 264])
+@pytest.mark.parametrize("dtype", [F32, BF16])
+def test_batched_products_on_both_sides_of_the_epilogue_rule(n, k, dtype):
+    """Four K blocks and fewer drain with eight warps; enough tiles that every CTA reuses its staging tiles."""
+    from bioemu2_b200 import functional as F
+
+    g = _gen(n, k)
+    a, b = (torch.randn(300, r, k, generator=g).to(BF16).cuda() for r in (130, n))
+    out = torch.empty(300, 130, n, dtype=dtype, device="cuda")
+    _close(F.bmm_nt_into(a, b, out), torch.einsum("bik,bjk->bij", a.float(), b.float()))
