@@ -2,8 +2,8 @@
 //
 // An fp32 value travels as hi = bf16(x), lo = bf16(x - hi).  A product of split operands is three ordinary products
 // (hi.hi + hi.lo + lo.hi) laid end to end along K: one operand reads hi | hi | lo, the other hi | lo | hi.  Activations whose
-// hi part is whole K blocks of 64 are stored once as (hi | lo) and read twice by the product's loads; the operands of the
-// triangle contraction, whose K is the token count, are stored three wide.  All arithmetic here is fp32 with expf and exact
+// hi part is whole K blocks of 64 are stored once as (hi | lo) and the operands of the triangle contraction, whose K is the
+// token count, as hi and lo planes; the product's loads read hi twice.  All arithmetic here is fp32 with expf and exact
 // division.  Every kernel is bound by memory: each reads its input once, 16 bytes a lane, and writes its output once.
 #pragma once
 #include "elementwise.cuh"
@@ -63,45 +63,6 @@ ln_split128_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, c
       *reinterpret_cast<uint2*>(yr) = hi;
       *reinterpret_cast<uint2*>(yr + 128) = lo;
     }
-  }
-}
-
-// Gated operands of the triangle contraction from the channel-major projection pg fp32 [512][n_lines * pitch] (p of a, p of b,
-// g of a, g of b): a[d][line][hi | hi | lo], b[d][line][hi | lo | hi], each part `pitch` wide, masked pairs and padding zero.
-// The projection writes channel-major, so nothing is transposed here (gate, two permutes, two zero fills and two splits of
-// the row-major form: 95 us at 200 tokens).  A thread keeps the mask of its eight pairs over eight channels.
-__global__ void __launch_bounds__(256)
-gate_split_kernel(const float* __restrict__ pg, const uint8_t* __restrict__ mask, __nv_bfloat16* __restrict__ a,
-                  __nv_bfloat16* __restrict__ b, int n_lines, int n_pos, int pitch, long long line_stride,
-                  long long pos_stride) {
-  constexpr int CH = 8;
-  pdl_wait();
-  const int per_line = pitch >> 3;
-  const long long octet = (long long)blockIdx.x * blockDim.x + threadIdx.x, pairs = (long long)n_lines * pitch;
-  if (octet * 8 >= pairs) return;
-  const int line = int(octet / per_line), pos = int(octet - (long long)line * per_line) * 8;
-  uint32_t keep = 0;
-#pragma unroll
-  for (int e = 0; e < 8; ++e)
-    if (pos + e < n_pos && mask[line * line_stride + (pos + e) * pos_stride]) keep |= 1u << e;
-  const int c0 = blockIdx.y * CH;  // of 256: a's channels, then b's
-  const bool is_b = c0 >= 128;
-  __nv_bfloat16* dst = (is_b ? b : a) + ((long long)(c0 & 127) * n_lines + line) * 3 * pitch + pos;
-  const float* src = pg + c0 * pairs + octet * 8;
-#pragma unroll 2
-  for (int c = 0; c < CH; ++c, src += pairs, dst += 3ll * n_lines * pitch) {
-    float p[8], g[8];
-    load8<true>(src, 0, p);
-    load8<true>(src + 256 * pairs, 0, g);
-    uint32_t hi[4], lo[4];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) p[e] = (keep >> e) & 1 ? p[e] / (1.f + expf(-g[e])) : 0.f;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) split_pair(p[2 * e], p[2 * e + 1], hi[e], lo[e]);
-    const uint4 h = make_uint4(hi[0], hi[1], hi[2], hi[3]), l = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    *reinterpret_cast<uint4*>(dst) = h;
-    *reinterpret_cast<uint4*>(dst + pitch) = is_b ? l : h;
-    *reinterpret_cast<uint4*>(dst + 2 * pitch) = is_b ? h : l;
   }
 }
 

@@ -40,6 +40,14 @@ struct BmmParams {
   // Split operands stored once as (hi | lo): a K block at or past the fold is loaded from that many blocks before, which
   // makes the operand hi | hi | lo.  INT_MAX: none.
   int a_fold, b_fold;
+  // Operands stored as hi and lo planes part_batch batch slices apart, each part_blocks K blocks wide: A is read hi, hi, lo,
+  // B hi, lo, hi.  0: none.
+  int part_blocks, part_batch;
+  // kEpiGateSplit: row r of A is pair (line, pos) = (r / mask_pitch, r % mask_pitch), kept where pos < mask_n and
+  // mask[line * mask_line + pos * mask_pos] != 0.
+  const uint8_t* mask;
+  int mask_pitch, mask_n;
+  long long mask_line, mask_pos;
   int a_shared;              // 1: every batch item multiplies the same A (the A tensor map has a single batch slice)
 };
 
@@ -58,9 +66,16 @@ enum BmmEpilogue : int {
   // kEpiBulk with eight epilogue warps, each group of four draining half of the tile's columns: a short product's tile is
   // its epilogue (K = 128: 2 K blocks of 64 against 128 columns of TMEM reads, staging and stores a lane).
   kEpiBulkWide = 7,
+  // Gated operands of the accurate triangle contraction, from split operands: the weights' 256 rows are p and g of 128
+  // channels and take the M side, so a lane is a channel and its columns are consecutive pairs -- the order in which the
+  // contraction reads them.  C gets hi and lo of p * sigmoid(g) (expf, exact division; masked pairs zero) as rows part *
+  // 128 + channel of column tile tn.  (Projection to fp32 and a gate kernel over it: 26 + 33 us for 40000 pairs.)
+  kEpiGateSplit = 8,
   kEpiOuter = 5,   // outer products of 32 x 32, one pair's 2 KB in one piece
 };
 
+template <int EPI>
+inline constexpr bool kTwoGroups = EPI == kEpiSwigluSplit || EPI == kEpiBulkWide || EPI == kEpiGateSplit;
 template <int EPI>
 inline constexpr bool kBulk = EPI == kEpiBulk || EPI == kEpiBulkWide;
 template <int EPI>
@@ -70,7 +85,7 @@ template <int BN, int EPI>
 struct BmmCfg {
   static constexpr int BM = 128;
   static constexpr int BK = 64;
-  static constexpr int STAGES = EPI == kEpiSwigluSplit || (EPI == kEpiBulkWide && BN == 256) ? 3 : EPI == kEpiBulkWide ? 5 : kTileOperand<EPI> || BN == 256 ? 4 : 6;
+  static constexpr int STAGES = kTwoGroups<EPI> ? (BN == 256 ? 3 : 5) : kTileOperand<EPI> || BN == 256 ? 4 : 6;
   static constexpr uint32_t A_BYTES = BM * BK * 2;
   static constexpr uint32_t B_BYTES = BN * BK * 2;
   static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
@@ -79,11 +94,11 @@ struct BmmCfg {
   static constexpr uint32_t BAR_OFFSET = MUL_OFFSET + MUL_BYTES;
   static constexpr uint32_t BIAS_OFFSET = BAR_OFFSET + 1024;       // the tile's BN bias values
   static constexpr uint32_t OUT_OFFSET = BAR_OFFSET + 2048;        // [128 rows][128 B] tiles for bulk output
-  static constexpr int OUT_TILES = EPI == kEpiSwigluSplit || EPI == kEpiBulkWide ? 4 : 2;
+  static constexpr int OUT_TILES = kTwoGroups<EPI> ? 4 : 2;
   static constexpr uint32_t SMEM_BYTES = OUT_OFFSET + OUT_TILES * 16384 + 1024;  // + alignment slack
   // The split SwiGLU's expf and division keep four warps busy for longer than the product (40000 x 1024 x 384: 105 us): it
   // has eight, each group of four with one of the tile's two 64-column groups.
-  static constexpr int EPI_THREADS = EPI == kEpiSwigluSplit || EPI == kEpiBulkWide ? 256 : 128;
+  static constexpr int EPI_THREADS = kTwoGroups<EPI> ? 256 : 128;
   static constexpr int GROUPS = EPI_THREADS / 128;
   static constexpr int THREADS = 64 + EPI_THREADS;
 };
@@ -144,8 +159,16 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           mbar_wait(&empty[stage], phase ^ 1, 1);
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           mbar_arrive_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-          tma_load_3d(sa, &tmA, &full[stage], (kb < p.a_fold ? kb : kb - p.a_fold) * 64, tm * 128, p.a_shared ? 0 : b);
-          tma_load_3d(sa + Cfg::A_BYTES, &tmB, &full[stage], (kb < p.b_fold ? kb : kb - p.b_fold) * 64, tn * BN, b);
+          int ka = kb < p.a_fold ? kb : kb - p.a_fold, kbb = kb < p.b_fold ? kb : kb - p.b_fold;
+          int ab = p.a_shared ? 0 : b, bb = b;
+          if (p.part_blocks > 0) {
+            const int part = kb / p.part_blocks;
+            ka = kbb = kb - part * p.part_blocks;
+            if (part == 2) ab += p.part_batch;
+            if (part == 1) bb += p.part_batch;
+          }
+          tma_load_3d(sa, &tmA, &full[stage], ka * 64, tm * 128, ab);
+          tma_load_3d(sa + Cfg::A_BYTES, &tmB, &full[stage], kbb * 64, tn * BN, bb);
           if (++stage == Cfg::STAGES) {
             stage = 0;
             phase ^= 1;
@@ -158,7 +181,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     // the commits (a converged warp issues a tcgen05.mma several times faster than a lone thread of a diverged one).
     {
       const bool leader = elect_one();
-      constexpr uint32_t idesc = make_idesc_bf16(128, BN);
+      constexpr uint32_t idesc = make_idesc_bf16(128, EPI == kEpiGateSplit ? 128 : BN);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -175,8 +198,14 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           const uint32_t a_lo = desc_lo(sa), b_lo = desc_lo(sb);
           if (leader) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_bf16_ss2(d_tmem, a_lo + 2 * k, kDescHiSw128, b_lo + 2 * k, kDescHiSw128, idesc, (kb | k) != 0);
+            for (int k = 0; k < 4; ++k) {
+              if constexpr (EPI == kEpiGateSplit) {
+                umma_bf16_ss2(d_tmem, b_lo + 2 * k, kDescHiSw128, a_lo + 2 * k, kDescHiSw128, idesc, (kb | k) != 0);
+                umma_bf16_ss2(d_tmem + 128, b_lo + 1024 + 2 * k, kDescHiSw128, a_lo + 2 * k, kDescHiSw128, idesc, (kb | k) != 0);
+              } else {
+                umma_bf16_ss2(d_tmem, a_lo + 2 * k, kDescHiSw128, b_lo + 2 * k, kDescHiSw128, idesc, (kb | k) != 0);
+              }
+            }
             umma_commit(&empty[stage]);
           }
           __syncwarp();
@@ -217,6 +246,16 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         for (int i = 0; i < GCOLS; i += 128) {
           const int k = grp * GCOLS + i + quarter * 32 + lane, col = tn * BN + k;
           if (GCOLS >= 128 || quarter * 32 < GCOLS) bias_s[k] = col < p.n_valid ? p.bias[col] : 0.f;
+        }
+      }
+      uint32_t keep[2];  // kEpiGateSplit: bit j = column j of the group's first / second 32 is kept
+      if constexpr (EPI == kEpiGateSplit) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int pair = tm * 128 + grp * 64 + c * 32 + lane;
+          const int line = pair / p.mask_pitch, pos = pair - line * p.mask_pitch;
+          const bool k = pair < p.m_valid && pos < p.mask_n && p.mask[line * p.mask_line + pos * p.mask_pos] != 0;
+          keep[c] = __ballot_sync(0xffffffffu, k);
         }
       }
       if (kTileOperand<EPI>) mbar_wait(mul_full, it & 1, 5);
@@ -312,6 +351,48 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               tma_store_commit();
             }
           }
+        }
+        continue;
+      }
+      if constexpr (EPI == kEpiGateSplit) {
+        static_assert(BN == 256 || EPI != kEpiGateSplit, "p and g of 128 channels");
+        const int r = quarter * 32 + lane;  // channel
+        const bool leader = (threadIdx.x & 127) == 64;
+        uint8_t* stage = smem + Cfg::OUT_OFFSET + grp * 32768;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t va[32], vb[32];
+          tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + grp * 64 + c * 32), va);
+          tmem_ld_32x32(tmem_addr(tmem_base, quarter * 32, acc * BN + 128 + grp * 64 + c * 32), vb);
+          tmem_ld_wait();
+          if (c == 1) {
+            tc_fence_before_sync();
+            mbar_arrive(&acc_empty[acc]);
+          }
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            va[e] = (keep[c] >> e) & 1 ? __float_as_uint(__uint_as_float(va[e]) / (1.f + expf(-__uint_as_float(vb[e])))) : 0u;
+          if (c == 0) {
+            if (leader) tma_store_wait_read0();  // the stores that last used the staging tiles have read them
+            named_bar_sync(1 + grp, 128);
+          }
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              split_pair(__uint_as_float(va[g * 8 + 2 * e]), __uint_as_float(va[g * 8 + 2 * e + 1]), hi[e], lo[e]);
+            *reinterpret_cast<uint4*>(stage + sw128_offset(r, c * 4 + g)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(stage + 16384 + sw128_offset(r, c * 4 + g)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+        }
+        fence_proxy_async_smem();
+        named_bar_sync(1 + grp, 128);
+        const int pair0 = tm * 128 + grp * 64;
+        if (leader && pair0 < p.m_valid) {
+          tma_store_3d(&tmC, stage, pair0, 0, tn);
+          tma_store_3d(&tmC, stage + 16384, pair0, 128, tn);
+          tma_store_commit();
         }
         continue;
       }

@@ -65,6 +65,10 @@ struct BmmLaunch {
   int64_t group_stride = 0;
   int b_rows = 0;              // rows of B that exist, if fewer than N (the rest count as zeros)
   bool split = false;   // with swiglu: C has N columns, (hi | lo) of the fp32 values
+  bool parts = false;   // A and B are hi and lo planes, `batch` slices each, K is one part's width
+  const uint8_t* gate_mask = nullptr;  // gated split operands (kEpiGateSplit): C [N / 256][2 * 128][M], M contiguous
+  int mask_pitch = 0, mask_n = 0;
+  int64_t mask_line = 0, mask_pos = 0;
   int a_fold = 0, b_fold = 0;  // operand stored as (hi | lo), each part this many K blocks of 64, read as hi | hi | lo
 };
 
@@ -100,17 +104,17 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   // for 65536 x 128 x 128).
   const bool add = bulk_c && a.residual && a.residual != a.C && a.out_f32 && a.batch == 1 && a.remap_n == 0 && !a.mul &&
                    !a.swiglu && aligned(a.residual, 16);
-  const int BN = a.mul || add ? 128 : a.split ? 256 : t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.K, a.batch);
+  const int BN = a.mul || add ? 128 : a.split || a.gate_mask ? 256 : t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.parts ? 3 * a.K : a.K, a.batch);
   CUtensorMap tmA, tmB;
   const bool a_shared = a.batch > 1 && a.sa == 0;  // one A for every batch item
   {
-    const uint64_t dims[3] = {uint64_t(a.a_fold ? a.a_fold * 128 : a.K), uint64_t(a.M), uint64_t(a_shared ? 1 : a.batch)};
+    const uint64_t dims[3] = {uint64_t(a.a_fold ? a.a_fold * 128 : a.K), uint64_t(a.M), uint64_t(a_shared ? 1 : a.parts ? 2 * a.batch : a.batch)};
     const uint64_t str[2] = {uint64_t(a.lda) * 2, uint64_t(a.sa > 0 ? a.sa : a.lda * a.M) * 2};
     const uint32_t box[3] = {64, 128, 1};
     if (int e = make_tmap_bf16(&tmA, a.A, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   {
-    const uint64_t dims[3] = {uint64_t(a.b_fold ? a.b_fold * 128 : a.K), uint64_t(a.b_rows ? a.b_rows : a.N), uint64_t(a.batch)};
+    const uint64_t dims[3] = {uint64_t(a.b_fold ? a.b_fold * 128 : a.K), uint64_t(a.b_rows ? a.b_rows : a.N), uint64_t(a.parts ? 2 * a.batch : a.batch)};
     const uint64_t str[2] = {uint64_t(a.ldb) * 2, uint64_t(a.sb > 0 ? a.sb : a.ldb * (a.b_rows ? a.b_rows : a.N)) * 2};
     const uint32_t box[3] = {64, uint32_t(BN), 1};
     if (int e = make_tmap_bf16(&tmB, a.B, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
@@ -124,7 +128,14 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   p.tiles_m = (a.M + 127) / 128;
   p.tiles_n = (a.N + BN - 1) / BN;
   p.batch = a.batch;
-  p.k_blocks = (a.K + 63) / 64;
+  p.k_blocks = (a.K + 63) / 64 * (a.parts ? 3 : 1);
+  p.part_blocks = a.parts ? (a.K + 63) / 64 : 0;
+  p.part_batch = a.batch;
+  p.mask = a.gate_mask;
+  p.mask_pitch = a.mask_pitch;
+  p.mask_n = a.mask_n;
+  p.mask_line = a.mask_line;
+  p.mask_pos = a.mask_pos;
   p.scale = a.scale;
   p.scale_ptr = a.scale_ptr;
   p.bias = a.bias;
@@ -139,7 +150,13 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   p.tma_c = 0;
   CUtensorMap tmC = tmA;
   const int c_cols = 128 / c_esz;  // columns of one staging tile
-  if (a.row_groups > 0) {
+  if (a.gate_mask) {
+    const uint64_t dims[3] = {uint64_t(a.M), 256, uint64_t(a.N / 256)};
+    const uint64_t str[2] = {uint64_t(a.M) * 2, uint64_t(a.sc) * 2};
+    const uint32_t box[3] = {64, 128, 1};
+    if (int e = make_tmap_bf16(&tmC, a.C, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+    p.tma_c = 1;
+  } else if (a.row_groups > 0) {
     if (!bulk_c || a.out_f32 || a.residual || a.M != 32 * a.row_groups || a.group_stride % 8)
       return fail(B200_ERR_INVALID_ARGUMENT, "grouped rows need aligned bf16 bulk output");
     const uint64_t dims[4] = {uint64_t(a.N), 32, uint64_t(a.row_groups), uint64_t(a.batch)};
@@ -191,6 +208,7 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
     // 128 x 256^3 10.0 / 8.5, 128 x 384^3 21.5 / 23.9, 512 x 40000 x 384 26.5 / 30.1).
     return p.k_blocks <= 4 ? go(bn, std::integral_constant<int, kEpiBulkWide>()) : go(bn, std::integral_constant<int, kEpiBulk>());
   };
+  if (a.gate_mask) return go(std::integral_constant<int, 256>(), std::integral_constant<int, kEpiGateSplit>());
   if (a.split) return go(std::integral_constant<int, 256>(), std::integral_constant<int, kEpiSwigluSplit>());
   if (add && p.tma_c) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiAdd>());
   if (a.mul) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiMul>());
@@ -1768,14 +1786,13 @@ static int swiglu_transition(const void* x, bool x_f32, void* out, bool out_f32,
   return launch_bmm(b, stream);
 }
 
-// Accurate triangle multiplication: hs | ts (hi | lo rows), a | b (three parts), and one fp32 region that holds the channel-
-// major projection, then t, the projected t and the gate logits, a quarter each.
+// Accurate triangle multiplication: hs (hi | lo rows), the operands a and b (hi and lo planes; later ts), and in fp32 t, the
+// projected t and the gate logits.
 static size_t accurate_rows_bytes(int N) { return round_up_1k(size_t(N) * ((N + 7) / 8 * 8) * 256 * 2); }
-static size_t accurate_operand_bytes(int N) { return round_up_1k(size_t(128) * N * 3 * ((N + 7) / 8 * 8) * 2); }
 
 size_t b200_accurate_trimul_workspace_bytes(int N) {
   if (N <= 0) return 0;
-  return accurate_rows_bytes(N) + 2 * accurate_operand_bytes(N) + 4 * accurate_rows_bytes(N);
+  return 6 * accurate_rows_bytes(N);
 }
 
 int b200_accurate_trimul_fwd(const float* z, const uint8_t* mask, float* out, const void* w_in, const void* w_p_out,
@@ -1795,29 +1812,31 @@ int b200_accurate_trimul_fwd(const float* z, const uint8_t* mask, float* out, co
   const int64_t rows = int64_t(N) * pitch, pairs = int64_t(N) * N;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   __nv_bfloat16* hs = reinterpret_cast<__nv_bfloat16*>(ws);
-  __nv_bfloat16* a = reinterpret_cast<__nv_bfloat16*>(ws + accurate_rows_bytes(N));
-  __nv_bfloat16* b = a + accurate_operand_bytes(N) / 2;
+  const size_t part = accurate_rows_bytes(N);
+  __nv_bfloat16* a = reinterpret_cast<__nv_bfloat16*>(ws + part);
+  __nv_bfloat16* b = a + part / 2;
   __nv_bfloat16* ts = a;  // after the contraction has read a
-  uint8_t* f = ws + accurate_rows_bytes(N) + 2 * accurate_operand_bytes(N);
-  float* pg = reinterpret_cast<float*>(f);
-  float* t = pg;
-  float* po = reinterpret_cast<float*>(f + accurate_rows_bytes(N));
-  float* go = reinterpret_cast<float*>(f + 2 * accurate_rows_bytes(N));
+  float* t = reinterpret_cast<float*>(ws + 3 * part);
+  float* po = reinterpret_cast<float*>(ws + 4 * part);
+  float* go = reinterpret_cast<float*>(ws + 5 * part);
   // incoming walks the pairs column by column: (line, pos) is pair (pos, line)
   const long long ls = incoming ? 1 : N, ps = incoming ? N : 1;
   B200_LAUNCH(ln_split128_kernel, grid_for(rows, 32), 256, 0, stream, z, hs, ln_in_w, ln_in_b, (long long)rows, N, pitch, ls,
               ps, 1);
   {
-    BmmLaunch m{w_in, hs, pg, 1, 512, int(rows), 384, 384, 256, rows, 0, 0, 0};
-    m.out_f32 = 1;
-    m.b_fold = 2;
+    BmmLaunch m{hs, w_in, a, 1, int(rows), 512, 384, 256, 384, rows, 0, 0, int64_t(part / 2)};
+    m.a_fold = 2;
+    m.gate_mask = mask;
+    m.mask_pitch = pitch;
+    m.mask_n = N;
+    m.mask_line = ls;
+    m.mask_pos = ps;
     if (int e = launch_bmm(m, stream)) return e;
   }
-  B200_LAUNCH(gate_split_kernel, dim3(unsigned((rows / 8 + 255) / 256), 32), 256, 0, stream, pg, mask, a, b, N, N, pitch, ls, ps);
   {
-    const int64_t k3 = 3 * int64_t(pitch);
-    BmmLaunch m{a, b, t, 128, N, N, int(k3), k3, k3, pitch, N * k3, N * k3, int64_t(N) * pitch};
+    BmmLaunch m{a, b, t, 128, N, N, pitch, pitch, pitch, pitch, int64_t(N) * pitch, int64_t(N) * pitch, int64_t(N) * pitch};
     m.out_f32 = 1;
+    m.parts = true;
     if (int e = launch_bmm(m, stream)) return e;
   }
   B200_LAUNCH(ln_split_channels_kernel, dim3((N + 31) / 32, N), 256, 0, stream, t, ts, ln_out_w, ln_out_b, N, N, pitch);

@@ -32,8 +32,13 @@ class PairMixerLayer(nn.Module):
     def forward(self, s: Tensor, z: Tensor, pair_mask: Tensor) -> tuple[Tensor, Tensor]:
         if self.training:
             raise RuntimeError("bioemu2_b200 modules are inference-only: call .eval()")
-        z = z.clone()  # the reference returns a new tensor; the three updates then run in place on the copy
-        return s, self.forward_(z, pair_mask)
+        # the reference returns a new tensor: the first update writes it, or the three run in place on a copy
+        if precision.use_ieee(self.tri_mul_out.matmul_precision, z):
+            z = self.tri_mul_out.forward_residual(z, pair_mask)
+            self.tri_mul_in.forward_residual_(z, pair_mask)
+            self.transition_z.forward_residual_(z)
+            return s, z
+        return s, self.forward_(z.clone(), pair_mask)
 
     def forward_(self, z: Tensor, pair_mask: Tensor) -> Tensor:
         """In-place form used by the trunk loop: updates and returns ``z``."""

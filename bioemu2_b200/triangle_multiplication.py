@@ -110,7 +110,8 @@ class TriangleMultiplication(PackedWeightsMixin, nn.Module):
                               self.norm_out.weight, self.norm_out.bias, self.p_out.weight, self.g_out.weight)
 
     def _build_split(self):
-        return ieee.SplitWeights(w_in=torch.cat([self.p_in.weight, self.g_in.weight], dim=0),
+        p, g = self.p_in.weight, self.g_in.weight
+        return ieee.SplitWeights(w_in=torch.cat([p[:128], g[:128], p[128:], g[128:]], dim=0),  # p and g of a, then of b
                                  w_p_out=self.p_out.weight, w_g_out=self.g_out.weight
                                  ).norms(norm_in=self.norm_in, norm_out=self.norm_out)
 
@@ -119,6 +120,12 @@ class TriangleMultiplication(PackedWeightsMixin, nn.Module):
         if precision.use_ieee(self.matmul_precision, x):
             return ieee.triangle_multiplication(x, mask, self, self.split_weights())
         return F.trimul(x, mask, self.packed(), incoming=self.mode == "incoming")
+
+    def forward_residual(self, x: Tensor, mask: Tensor) -> Tensor:
+        """``x + forward(x, mask)`` as a new tensor."""
+        if precision.use_ieee(self.matmul_precision, x):
+            return ieee.triangle_multiplication(x, mask, self, self.split_weights(), add_residual=True)
+        return self.forward_residual_(x.clone(), mask)
 
     def forward_residual_(self, x: Tensor, mask: Tensor) -> Tensor:
         """``x += forward(x, mask)`` in place with the add fused into the output kernel; returns ``x``."""

@@ -476,7 +476,7 @@ int b200_softmax_bias_f32(float* s, const float* bias, const uint8_t* keymask, i
                           b200_stream_t stream);
 
 /* Triangle multiplication in the accurate form, one batch item: z fp32 [N][N][128], mask [N][N], out may be z.  w_in = split
- * (order 1) of p_in | g_in [512][384], w_p_out and w_g_out [128][384].  Workspace 1024-byte aligned. */
+ * (order 1) of the 128-row halves of p_in and g_in in turn [512][384], w_p_out and w_g_out [128][384].  Workspace 1024-byte aligned. */
 size_t b200_accurate_trimul_workspace_bytes(int N);
 int b200_accurate_trimul_fwd(const float* z, const uint8_t* mask, float* out, const void* w_in, const void* w_p_out,
                              const void* w_g_out, const float* ln_in_w, const float* ln_in_b, const float* ln_out_w,
