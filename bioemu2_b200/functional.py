@@ -31,14 +31,15 @@ def _stream() -> int:
 
 
 def workspace(nbytes: int, device: torch.device) -> Tensor:
-    """Scratch buffer shared by all ops of this thread on (device, stream); grown on demand, 1024-byte aligned."""
+    """Scratch buffer of at least ``nbytes`` shared by all ops of this thread on (device, stream); grown on demand,
+    1024-byte aligned (kept as the aligned view: cutting it on every call cost as much as half a launch)."""
     key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
     buf = _WORKSPACES.buffers.get(key)
-    if buf is None or buf.numel() < nbytes + 1024:
+    if buf is None or buf.numel() < nbytes:
         buf = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
-        _WORKSPACES.buffers[key] = buf
-    off = (-buf.data_ptr()) % 1024
-    return buf[off:off + nbytes]
+        off = (-buf.data_ptr()) % 1024
+        buf = _WORKSPACES.buffers[key] = buf[off:off + nbytes]
+    return buf
 
 
 def release_workspaces() -> None:
@@ -164,7 +165,7 @@ def trimul(x: Tensor, mask: Tensor, w: TriMulPacked, incoming: bool, add_residua
     _require_cuda(x, mask)
     if x.ndim != 4 or x.shape[1] != x.shape[2] or x.shape[3] != 128:
         raise ValueError(f"expected x[B,N,N,128], got {tuple(x.shape)}")
-    if tuple(mask.shape) != tuple(x.shape[:3]):
+    if mask.shape != x.shape[:3]:
         raise ValueError(f"mask shape {tuple(mask.shape)} does not match x {tuple(x.shape)}")
     zd = _zdtype(x)
     if not x.is_contiguous():
@@ -382,7 +383,7 @@ def triangle_attention(x: Tensor, mask: Tensor, w: TriAttPacked, ending: bool, a
     _require_cuda(x, mask)
     if x.ndim != 4 or x.shape[1] != x.shape[2] or x.shape[3] != 128:
         raise ValueError(f"expected x[B,N,N,128], got {tuple(x.shape)}")
-    if tuple(mask.shape) != tuple(x.shape[:3]):
+    if mask.shape != x.shape[:3]:
         raise ValueError(f"mask shape {tuple(mask.shape)} does not match x {tuple(x.shape)}")
     zd = _zdtype(x)
     if not x.is_contiguous():
