@@ -70,10 +70,9 @@ struct RowTile {
   // row_ptr(r) -> address of channel 0 of tile row r (elements of the z stream), or nullptr if absent.
   // LS: rows normalised in lock step by the one-pass packed form (8 where the kernel has registers to spare);
   // LS = 1 selects the register-tight two-pass form.
-  // copy_delta != 0: the raw rows are also stored at their address + copy_delta bytes (a copy of the tensor for free).
   template <bool F32, bool NORM, int LS = 8, class RowPtr>
   __device__ __forceinline__ void load(int pt, RowPtr row_ptr, const float (&gamma)[8], const float (&beta)[8],
-                                       float eps, float raw_scale = 1.0f, long long copy_delta = 0) {
+                                       float eps, float raw_scale = 1.0f) {
     const int c0 = (pt & 15) * 8;
     const int rbase = pt >> 4;
 #pragma unroll
@@ -87,13 +86,6 @@ struct RowTile {
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) x[q][i] = 0.f;
-        }
-      }
-      if (copy_delta != 0) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const void* src = row_ptr((q0 + q) * RSTEP + rbase);
-          if (src) store8<F32>(const_cast<uint8_t*>(static_cast<const uint8_t*>(src)) + copy_delta, c0, x[q]);
         }
       }
       if (NORM && LS == 1) {
