@@ -111,8 +111,11 @@ def transition(x: Tensor, norm, fc1, fc2, fc3, ws: SplitWeights, add_residual: b
                out: Tensor | None = None) -> Tensor:
     """``out`` (fp32, contiguous): where the result goes; it may be ``x``."""
     shape = x.shape
-    x2 = x.float().contiguous().view(-1, shape[-1])
     hidden, out_cols = ws.w3.shape[1] // 3, ws.w3.shape[0]
+    if shape[-1] != ws.w12.shape[1] // 3:
+        raise ValueError(f"expected x[..., {ws.w12.shape[1] // 3}], got {tuple(shape)}")
+    F._require_cuda(x)
+    x2 = x.float().contiguous().view(-1, shape[-1])
     rows, cols = x2.shape
     if out is not None and not (out.is_contiguous() and out.dtype == torch.float32):
         return out.copy_(transition(x, norm, fc1, fc2, fc3, ws, add_residual))
@@ -136,7 +139,12 @@ def transition(x: Tensor, norm, fc1, fc2, fc3, ws: SplitWeights, add_residual: b
 def triangle_multiplication(x: Tensor, mask: Tensor, mod, ws: SplitWeights, add_residual: bool = False,
                             out: Tensor | None = None) -> Tensor:
     """``out`` (fp32, contiguous): where the result goes; it may be ``x``."""
-    B, N, _, D = x.shape
+    if x.ndim != 4 or x.shape[1] != x.shape[2] or x.shape[3] != 128:
+        raise ValueError(f"expected x[B,N,N,128], got {tuple(x.shape)}")
+    if mask.shape != x.shape[:3]:
+        raise ValueError(f"mask shape {tuple(mask.shape)} does not match x {tuple(x.shape)}")
+    F._require_cuda(x, mask)
+    B, N = x.shape[:2]
     if out is not None and not (out.is_contiguous() and out.dtype == torch.float32):
         return out.copy_(triangle_multiplication(x, mask, mod, ws, add_residual))
     if not hasattr(ws, "norm_in_w"):

@@ -1,0 +1,31 @@
+"""Arguments that a call cannot serve are refused on the host, before a kernel is given their addresses (no GPU needed)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from bioemu2_b200 import ieee
+
+
+@pytest.mark.parametrize("shape,mask,exc", [
+    ((1, 20, 12, 128), (1, 20, 12), ValueError),      # not square
+    ((1, 12, 12, 64), (1, 12, 12), ValueError),       # another width
+    ((12, 12, 128), (12, 12), ValueError),
+    ((2, 12, 12, 128), (1, 12, 12), ValueError),
+    ((1, 12, 12, 128), (1, 12, 11), ValueError),
+    ((1, 12, 12, 128), (1, 12, 12), RuntimeError),    # on the host
+])
+@pytest.mark.parametrize("add_residual", [False, True])
+def test_accurate_triangle_multiplication(shape, mask, exc, add_residual):
+    x = torch.zeros(shape)
+    with pytest.raises(exc, match="CUDA tensors" if exc is RuntimeError else "expected x|mask shape"):
+        ieee.triangle_multiplication(x, torch.ones(mask, dtype=torch.bool), SimpleNamespace(mode="outgoing"), SimpleNamespace(),
+                                     add_residual, out=x if add_residual else None)
+
+
+@pytest.mark.parametrize("native", [False, True])
+@pytest.mark.parametrize("width,exc", [(192, ValueError), (64, ValueError), (128, RuntimeError)])
+def test_accurate_transition(width, exc, native):
+    ws = SimpleNamespace(w12=torch.empty(512, 3 * 128), w3=torch.empty(128, 3 * 256), norm_w=None, norm_b=None, native=native)
+    with pytest.raises(exc, match="CUDA tensors" if exc is RuntimeError else "expected x"):
+        ieee.transition(torch.zeros(5, width), None, None, None, None, ws)
