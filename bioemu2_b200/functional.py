@@ -132,6 +132,7 @@ class _Pack:
         keep, segs = [], []
         for t, off, groups, group, pitch, stride, scale in self.parts:
             if t is not None:
+                _require_cuda(t)
                 t = t.detach()
                 if t.dtype != torch.float32 or not t.is_contiguous() or t.data_ptr() % 32:
                     t = t.to(torch.float32).contiguous().clone() if t.data_ptr() % 32 else t.to(torch.float32).contiguous()
@@ -268,6 +269,8 @@ def outer_product_mean(m: Tensor, mask: Tensor, w: OpmPacked, residual: Tensor |
     else:
         raise ValueError("mask must be [B,S,N] or [B,N]")
     zd = _zdtype(m)
+    if residual is not None:
+        _require_cuda(residual)
     m = m.contiguous()
     out = torch.empty(B, N, N, 128, dtype=m.dtype, device=m.device)
     if residual is not None and (residual.dtype != torch.float32 or m.dtype != torch.float32 or residual.shape != out.shape
@@ -471,7 +474,7 @@ def rows2_to_bf16(x1: Tensor, x2: Tensor, weight: Tensor | None = None, bias: Te
 def ln_linear(x1: Tensor, x2: Tensor | None, weight: Tensor | None, bias: Tensor | None, w_bf16: Tensor,
               residual: Tensor | None = None) -> Tensor:
     """``LayerNorm(cat(x1, x2)) @ w.T (+ residual)`` as fp32 for 128-channel sources and 128 outputs, one pass."""
-    _require_cuda(x1, w_bf16)
+    _require_cuda(*(t for t in (x1, x2, w_bf16, residual) if t is not None))
     x1 = x1.contiguous()
     x2 = x2.contiguous() if x2 is not None else None
     if x1.shape[-1] != 128 or (x2 is not None and (x2.shape != x1.shape or x2.dtype != x1.dtype)) or \
@@ -582,7 +585,7 @@ def cond_layer(layer: "_lib.CondLayer", x: Tensor, pairs: Tensor | None, bias: T
                out: Tensor | None = None) -> Tensor:
     """A ``ConditionedTransformerLayer`` in one native call; ``layer`` carries sizes and weights, ``bias`` (bf16, base 2) replaces
     the projection of ``pairs`` where it is given."""
-    _require_cuda(x, c, mask)
+    _require_cuda(x, pairs if bias is None else bias, c, mask)
     x, c = x.contiguous(), c.contiguous()
     pairs = pairs.contiguous() if bias is None else None
     m8 = mask_u8(mask)
@@ -749,7 +752,7 @@ def trunk_(z_in: Tensor, z: Tensor, s: Tensor | None, token_mask: Tensor | None,
            heads: int = 0, side: torch.cuda.Stream | None = None) -> None:
     """Runs the stack: ``z_in[B,N,N,128]`` -> ``z`` (may be ``z_in``), ``s[B,N,c_s]`` in place (``None``: no single track).
     ``pair_mask=None``: the outer product of ``token_mask``."""
-    _require_cuda(z_in, z)
+    _require_cuda(*(t for t in (z_in, z, s, token_mask, pair_mask) if t is not None))
     B, N = z.shape[0], z.shape[1]
     if tuple(z.shape) != (B, N, N, 128) or z_in.shape != z.shape or z_in.dtype != z.dtype:
         raise ValueError(f"expected z[B,N,N,128], got {tuple(z_in.shape)} -> {tuple(z.shape)}")

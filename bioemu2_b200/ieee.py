@@ -29,6 +29,7 @@ def split(x: Tensor, order: int, ln_w: Tensor | None = None, ln_b: Tensor | None
           eps: float = 1e-5) -> Tensor:
     """``x[..., C]`` fp32 -> bf16 ``[..., 3C]``: (hi | hi | lo) for ``order`` 0, (hi | lo | hi) for 1, after an optional
     fp32 LayerNorm over the last axis."""
+    F._require_cuda(x)
     if x.dtype != torch.float32:
         x = x.float()
     x = x.contiguous()

@@ -4,6 +4,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
+from bioemu2_b200 import functional as F
 from bioemu2_b200 import ieee
 
 
@@ -29,3 +30,25 @@ def test_accurate_transition(width, exc, native):
     ws = SimpleNamespace(w12=torch.empty(512, 3 * 128), w3=torch.empty(128, 3 * 256), norm_w=None, norm_b=None, native=native)
     with pytest.raises(exc, match="CUDA tensors" if exc is RuntimeError else "expected x"):
         ieee.transition(torch.zeros(5, width), None, None, None, None, ws)
+
+
+class _OnDevice(torch.Tensor):
+    """A tensor that says it is on the GPU."""
+
+    is_cuda = property(lambda self: True)
+
+
+@pytest.mark.parametrize("call", [
+    lambda d, h: F.ln_linear(d(4, 128), h(4, 128), None, None, d(128, 256).bfloat16()),
+    lambda d, h: F.ln_linear(d(4, 128), None, None, None, d(128, 128).bfloat16(), residual=h(4, 128)),
+    lambda d, h: F.outer_product_mean(d(1, 3, 4, 64), d(1, 3, 4), None, residual=h(1, 4, 4, 128)),
+    lambda d, h: F.trunk_(d(1, 4, 4, 128), d(1, 4, 4, 128), None, None, h(1, 4, 4), None),
+    lambda d, h: F.trunk_(d(1, 4, 4, 128), d(1, 4, 4, 128), d(1, 4, 64), h(1, 4), None, None),
+    lambda d, h: F.trunk_(d(1, 4, 4, 128), d(1, 4, 4, 128), h(1, 4, 64), d(1, 4), None, None),
+    lambda d, h: F.cond_layer(None, d(1, 4, 64), h(1, 4, 4, 128), None, d(1, 4, 64), d(1, 4)),
+    lambda d, h: F.TransitionGenericPacked(None, None, d(64, 64), d(64, 64), h(64, 64)),
+    lambda d, h: ieee.split(h(4, 64), 0),
+], ids=["second_source", "residual", "opm_residual", "pair_mask", "token_mask", "single", "pairs", "weights", "split"])
+def test_one_tensor_on_the_host(call):
+    with pytest.raises(RuntimeError, match="CUDA tensors"):
+        call(lambda *s: torch.zeros(s).as_subclass(_OnDevice), lambda *s: torch.zeros(s))
