@@ -734,6 +734,9 @@ class TrunkPacked:
         """``blocks``: per block a dict of packed weights under the names of ``_lib.TrunkBlock``; absent parts are left out."""
         self.keep = blocks
         self.n = len(blocks)
+        # width and heads of the single track, one value over all blocks
+        self.single = {(b["attention"].c_s, b["attention"].H) for b in blocks if "attention" in b} | {
+            (b["transition_s"].cols, b["attention"].H) for b in blocks if "transition_s" in b}
         self.array = (_lib.TrunkBlock * self.n)(*[_lib.TrunkBlock(**{k: v.struct for k, v in b.items()}) for b in blocks])
 
 
@@ -764,6 +767,8 @@ def trunk_(z_in: Tensor, z: Tensor, s: Tensor | None, token_mask: Tensor | None,
         raise ValueError(f"pair mask shape {tuple(pair_mask.shape)} does not match z {tuple(z.shape)}")
     if s is not None and (s.ndim != 3 or s.shape[0] != B or s.shape[1] != N):
         raise ValueError(f"s {tuple(s.shape)} does not match z {tuple(z.shape)}")
+    if s is not None and w.single != {(s.shape[2], heads)}:
+        raise ValueError(f"s {tuple(s.shape)} and {heads} heads do not match the blocks' widths and heads {sorted(w.single)}")
     zd = _zdtype(z)
     sd = _zdtype(s) if s is not None else 0
     if z.numel() == 0:

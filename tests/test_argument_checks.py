@@ -4,6 +4,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
+from bioemu2_b200 import _lib
 from bioemu2_b200 import functional as F
 from bioemu2_b200 import ieee
 
@@ -52,3 +53,24 @@ class _OnDevice(torch.Tensor):
 def test_one_tensor_on_the_host(call):
     with pytest.raises(RuntimeError, match="CUDA tensors"):
         call(lambda *s: torch.zeros(s).as_subclass(_OnDevice), lambda *s: torch.zeros(s))
+
+
+@pytest.mark.parametrize("width,heads", [(768, 16), (192, 16), (384, 8)])
+def test_trunk_single_track_of_another_width(width, heads):
+    w = F.TrunkPacked([])
+    w.single = {(384, 16)}
+    z = torch.zeros(1, 4, 4, 128).as_subclass(_OnDevice)
+    s, mask = torch.zeros(1, 4, width).as_subclass(_OnDevice), torch.ones(1, 4).as_subclass(_OnDevice)
+    with pytest.raises(ValueError, match="do not match the blocks"):
+        F.trunk_(z, z, s, mask, None, w, heads)
+
+
+def test_trunk_single_track_widths_come_from_every_block():
+    def block(c_s, cols, heads):
+        return {"attention": SimpleNamespace(c_s=c_s, H=heads, struct=_lib.ApbWeights()),
+                "transition_s": SimpleNamespace(cols=cols, struct=_lib.SwigluWeights())}
+
+    assert F.TrunkPacked([block(384, 384, 16)] * 2).single == {(384, 16)}
+    assert F.TrunkPacked([{}]).single == set()
+    assert len(F.TrunkPacked([block(384, 384, 16), block(384, 384, 8)]).single) == 2
+    assert len(F.TrunkPacked([block(384, 768, 16)]).single) == 2
