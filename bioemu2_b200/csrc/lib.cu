@@ -1906,7 +1906,9 @@ int b200_swiglu_transition_fwd(const void* x, void* out, const b200_swiglu_weigh
                  "widths must be multiples of 8 and the input width at most 1024");
   B200_CHECK_ARG((x_dtype | 1) == 1, "unknown dtype");
   B200_CHECK_ARG(!add_residual || x == out, "the residual form works in place");
-  B200_CHECK_ARG(aligned(x, 32) && aligned(out, 32), "x/out must be 32-byte aligned");
+  // bf16 rows without a LayerNorm are the product's operand as they are, others are read 32 bytes at a time
+  B200_CHECK_ARG(aligned(x, x_dtype == B200_DTYPE_BF16 && !w->ln_w ? 16 : 32) && aligned(out, 32),
+                 "out must be 32-byte aligned, x 32-byte (16 for bf16 without a LayerNorm)");
   if (rows == 0) return B200_OK;
   if (!workspace || workspace_bytes < swiglu_workspace(rows, cols, w->hidden) || !aligned(workspace, 1024))
     return fail(B200_ERR_WORKSPACE, "workspace must be 1024-byte aligned and hold %zu bytes (got %zu)",

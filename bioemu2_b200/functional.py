@@ -70,6 +70,12 @@ def _require_cuda(*tensors: Tensor) -> None:
             raise RuntimeError("bioemu2_b200 runs on CUDA tensors only (there is no CPU path)")
 
 
+def aligned(t: Tensor) -> Tensor:
+    """``t``, or a contiguous copy if it does not start on the 32 bytes that the kernels load at once (a view into a larger
+    buffer may not)."""
+    return t if t.data_ptr() % 32 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 def layernorm(x: Tensor, weight: Tensor | None, bias: Tensor | None, eps: float = 1e-5) -> Tensor:
     _require_cuda(x)
     if x.dtype != torch.bfloat16:
@@ -586,7 +592,7 @@ def cond_layer(layer: "_lib.CondLayer", x: Tensor, pairs: Tensor | None, bias: T
     """A ``ConditionedTransformerLayer`` in one native call; ``layer`` carries sizes and weights, ``bias`` (bf16, base 2) replaces
     the projection of ``pairs`` where it is given."""
     _require_cuda(x, pairs if bias is None else bias, c, mask)
-    x, c = x.contiguous(), c.contiguous()
+    x, c = aligned(x.contiguous()), c.contiguous()
     pairs = pairs.contiguous() if bias is None else None
     m8 = mask_u8(mask)
     if out is None:

@@ -71,7 +71,7 @@ class PairformerModule(PackedWeightsMixin, nn.Module):
         if self.training:
             raise RuntimeError("bioemu2_b200 modules are inference-only: call .eval()")
         s = s.clone(memory_format=torch.contiguous_format)
-        z = self.forward_into(s, z.contiguous(), torch.empty_like(z, memory_format=torch.contiguous_format), token_mask)
+        z = self.forward_into(s, F.aligned(z.contiguous()), torch.empty_like(z, memory_format=torch.contiguous_format), token_mask)
         _lib.raise_if_device_wait()  # a kernel whose bounded wait ran out earlier in the stack invalidates the result
         return s, z
 

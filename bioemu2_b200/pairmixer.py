@@ -34,7 +34,7 @@ class PairMixerLayer(nn.Module):
             raise RuntimeError("bioemu2_b200 modules are inference-only: call .eval()")
         # the reference returns a new tensor: the first update writes it, or the three run in place on a copy
         if precision.use_ieee(self.tri_mul_out.matmul_precision, z):
-            z = self.tri_mul_out.forward_residual(z, pair_mask)
+            z = self.tri_mul_out.forward_residual(F.aligned(z), pair_mask)
             self.tri_mul_in.forward_residual_(z, pair_mask)
             self.transition_z.forward_residual_(z)
             return s, z
@@ -63,7 +63,7 @@ class PairMixerModule(PackedWeightsMixin, nn.Module):
     def forward(self, s: Tensor, z: Tensor, pair_mask: Tensor) -> tuple[Tensor, Tensor]:
         if self.training:
             raise RuntimeError("bioemu2_b200 modules are inference-only: call .eval()")
-        z = self.forward_into(z.contiguous(), torch.empty_like(z, memory_format=torch.contiguous_format), pair_mask)
+        z = self.forward_into(F.aligned(z.contiguous()), torch.empty_like(z, memory_format=torch.contiguous_format), pair_mask)
         _lib.raise_if_device_wait()  # a kernel whose bounded wait ran out earlier in the stack invalidates the result
         return s, z
 
