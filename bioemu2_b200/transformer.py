@@ -128,8 +128,10 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
         if native is None:
             return self._forward(x, pairs, c, mask, multiplicity, self.attention)
         layer, B = native[0], pairs.shape[0]
+        if self._windowed and x.ndim == 3 and mask.numel() == B * x.shape[1]:
+            mask = mask.reshape(B, x.shape[1])  # it may come by query windows
         if x.ndim != 3 or x.shape[0] != B * multiplicity or x.shape[2] != self.dim or tuple(mask.shape) != (B, x.shape[1]) \
-                or c.shape[:2] != x.shape[:2] or c.shape[2] != layer.dim_cond:
+                or c.shape[-1] != layer.dim_cond or c.numel() != x.shape[0] * x.shape[1] * c.shape[-1]:
             raise ValueError(f"x {tuple(x.shape)}, c {tuple(c.shape)}, pairs {tuple(pairs.shape)}, mask {tuple(mask.shape)}, "
                              f"multiplicity={multiplicity}")
         bias, N = None, x.shape[1]

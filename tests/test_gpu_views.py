@@ -42,3 +42,28 @@ def test_offset_views(kind):
         assert w is v is None or torch.equal(w, v)
     for k, v in zip(kept, views):
         assert k is v is None or torch.equal(k, v)  # the inputs stay as they were
+
+
+@pytest.mark.parametrize("windowed", [False, True])
+def test_conditioned_layer_takes_conditioning_by_rows_and_masks_by_windows(windowed):
+    import bioemu2_b200 as b
+
+    g = torch.Generator(device="cuda").manual_seed(6)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    kw = dict(is_sliding_window=True, window_queries=32, window_keys=128) if windowed else {}
+    with torch.device("cuda"):
+        m = b.ConditionedTransformerLayer(128, 16 if windowed else 128, 128, 4, 256, **kw).eval()
+    x, c = randn(2, 64, 128), randn(2, 64, 128)
+    pairs = randn(1, 2, 32, 128, 16) if windowed else randn(1, 64, 64, 128)
+    mask = torch.rand(1, 64, device="cuda", generator=g) > 0.1
+    with torch.no_grad():
+        want = m(x, pairs, c, mask, 2)
+        assert torch.equal(m(x, pairs, c.view(128, 128), mask, 2), want)
+        for shape in ((2, 32), (1, 2, 32)):
+            if windowed:
+                assert torch.equal(m(x, pairs, c, mask.view(shape), 2), want)
+            else:
+                with pytest.raises(ValueError):
+                    m(x, pairs, c, mask.view(shape), 2)
+        with pytest.raises(ValueError):
+            m(x, pairs, c[:1], mask, 2)
