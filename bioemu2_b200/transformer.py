@@ -105,7 +105,6 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
             layer = _lib.CondLayer()
             ap, tp = attn.packed(), tr.packed()
             layer.dim, layer.dim_cond, layer.heads, layer.dim_pairwise = self.dim, lin.in_features, attn.num_heads, attn.c_z
-            layer.lns_scale = self.lns_scale
             layer.ln_c_w, layer.ln_c_b, layer.w_cond, layer.b_cond = F._ptr(ln_w), F._ptr(ln_b), w_cond.data_ptr(), b_cond.data_ptr()
             if self._windowed:
                 layer.window_queries, layer.window_keys = attn.window_queries, attn.window_keys
@@ -148,7 +147,7 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
             if attn._bias_cache is not None:
                 bias = attn._bias_cache[0].lookup(attn._bias_cache[1], pairs)
         sized = _lib.CondLayer.from_buffer_copy(layer)  # the layer's own copy may be in use by another thread
-        sized.B, sized.M, sized.N = B, multiplicity, N
+        sized.B, sized.M, sized.N, sized.lns_scale = B, multiplicity, N, self.lns_scale
         return F.cond_layer(sized, x, pairs, bias, c, mask)
 
     def _forward(self, x: Tensor, pairs: Tensor, c: Tensor, mask: Tensor, multiplicity: int, attention) -> Tensor:
