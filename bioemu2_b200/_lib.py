@@ -200,15 +200,17 @@ def last_error() -> str:
 
 
 class DeviceWaitError(RuntimeError):
-    """A kernel gave up one of its bounded waits: its results, and those of the kernels queued behind it, are invalid."""
+    """A kernel gave up one of its bounded waits, or could not run: its results, and those of the kernels queued behind it,
+    are invalid."""
 
 
 def decode_status(word: int) -> str:
-    """Readable form of the device status word: low byte = kind (1: a bounded wait ran out), bits 8.. = wait site."""
+    """Readable form of the device status word: low byte = kind (1: a bounded wait ran out, 2: shared memory that does not
+    start where the kernel needs it), bits 8.. = site."""
     if word == 0:
         return "ok"
-    kind = {1: "bounded wait ran out"}.get(word & 0xFF, f"unknown kind {word & 0xFF}")
-    return f"{kind} at wait site {word >> 8} (status {word:#x})"
+    kind = {1: "bounded wait ran out at wait", 2: "shared memory misaligned at"}.get(word & 0xFF, f"unknown kind {word & 0xFF} at")
+    return f"{kind} site {word >> 8} (status {word:#x})"
 
 
 def check(status: int) -> None:

@@ -421,7 +421,7 @@ static int check_arch(int* dev_out) {
 }
 
 // Host-visible copy of the device status word, one per device ordinal: 64 bytes of pinned, mapped host memory
-// that a kernel writes when one of its bounded waits runs out.  Set up by the first ordinary call on a device.
+// that a kernel writes when one of its bounded waits runs out (or it cannot run at all).  Set up by the first ordinary call on a device.
 static int* g_host_status[64] = {nullptr};
 
 static int ensure_host_status(int dev) {
@@ -447,9 +447,9 @@ int b200_check_device(void) {
   const int st = *reinterpret_cast<volatile int*>(g_host_status[dev]);
   if (st != 0)
     return fail(B200_ERR_DEVICE_WAIT,
-                "an earlier kernel on device %d gave up a bounded wait (status %#x, wait site %d): its results and "
+                "an earlier kernel on device %d %s (status %#x, site %d): its results and "
                 "those of the kernels after it are invalid; b200_device_status() reads and clears the status",
-                dev, st, st >> 8);
+                dev, (st & 0xff) == kDevMisaligned ? "found its shared memory misaligned" : "gave up a bounded wait", st, st >> 8);
   return B200_OK;
 }
 

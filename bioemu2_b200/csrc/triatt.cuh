@@ -55,7 +55,10 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   using namespace triatt_proj;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
-  if (smem_misaligned(smem)) return;  // the swizzled tiles need the alignment; there is no room to round up
+  if (smem_misaligned(smem, 97)) {  // the swizzled tiles need the alignment; there is no room to round up
+    pdl_wait();
+    return;
+  }
   uint64_t* w_full = reinterpret_cast<uint64_t*>(smem + BAR_OFF);
   uint64_t* x_full = w_full + 1;     // [2] count 256
   uint64_t* x_empty = x_full + 2;    // [2] commit

@@ -22,7 +22,8 @@ __device__ int* g_host_status_ptr = nullptr;
 
 enum DevStatus : int {
   kDevOk = 0,
-  kDevWaitTimeout = 1,  // low byte; the site id of the wait is stored in bits 8..
+  kDevWaitTimeout = 1,   // low byte; the site id of the wait is stored in bits 8..
+  kDevMisaligned = 2,    // a kernel's shared memory did not start where its swizzled tiles need it; bits 8..: the kernel's site
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -124,10 +125,10 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int si
 }
 
 // For kernels that fill the shared memory and cannot round their base up to the 1024 bytes of a swizzle atom: true, with
-// the status set, if the base is not aligned already.
-__device__ __forceinline__ bool smem_misaligned(const void* smem) {
+// the status set, if the base is not aligned already.  The kernel then returns, after pdl_wait() like any other.
+__device__ __forceinline__ bool smem_misaligned(const void* smem, int site) {
   if ((smem_u32(smem) & 1023u) == 0) return false;
-  const int code = kDevWaitTimeout | (99 << 8);
+  const int code = kDevMisaligned | (site << 8);
   if (threadIdx.x == 0 && atomicCAS(&g_dev_status, 0, code) == 0) {
     int* hp = g_host_status_ptr;
     if (hp) {

@@ -57,7 +57,8 @@ const char* b200_last_error(void);
 int b200_check_device(void);
 
 /* Synchronises the device, then reads and clears the device status word into *status (host pointer).
- * 0 = every kernel wait completed; otherwise low byte 1 = a bounded wait ran out, bits 8.. = its site. */
+ * 0 = every kernel wait completed; otherwise low byte 1 = a bounded wait ran out, 2 = a kernel's shared memory did not start
+ * on the boundary it needs; bits 8.. = the site. */
 int b200_device_status(int* status);
 
 /* The same word as far as kernels that have FINISHED wrote it, read from host memory: no synchronisation, no

@@ -42,6 +42,22 @@ def test_status_word_decoding():
     assert "unknown kind 9" in L.decode_status(9 | (3 << 8))
 
 
+def test_every_kind_the_kernels_report_has_a_text_and_sites_of_its_own():
+    """The kinds of csrc/umma.cuh are told apart by decode_status, and a kernel that cannot run reports no wait's site."""
+    import os
+    import re
+
+    csrc = os.path.join(L.HERE, "csrc")
+    text = "".join(open(os.path.join(csrc, f)).read() for f in sorted(os.listdir(csrc)))
+    kinds = {int(k) for k in re.findall(r"\bkDev\w+ = (\d+),", text)} - {0}
+    assert kinds == {1, 2}
+    words = [L.decode_status(k | (97 << 8)) for k in sorted(kinds)]
+    assert len(set(words)) == 2 and not any("unknown" in w for w in words) and "wait" not in words[1]
+    waits = set(re.findall(r"\bmbar_wait\([^;]*, (\d+)\);", text))
+    others = set(re.findall(r"\bsmem_misaligned\(\w+, (\d+)\)", text))
+    assert waits and others and not waits & others
+
+
 def test_header_and_binding_agree_on_every_symbol():
     """Every function include/b200pair.h declares is bound, with the declared number of arguments, and exported."""
     import os
