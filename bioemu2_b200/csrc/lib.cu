@@ -1753,6 +1753,24 @@ static int trunk_events(cudaEvent_t** out) {
   return 0;
 }
 
+// Makes `stream` wait for what has been enqueued on `side`, at the latest when the scope ends: a call that fails on its way
+// must not leave kernels on the side stream that still read the workspace its next call will write, nor a fork open in a
+// stream that is being captured.
+struct SideJoin {
+  cudaStream_t side, stream;
+  cudaEvent_t ev;  // null: nothing to join
+  int join() {
+    if (!ev) return B200_OK;
+    const cudaEvent_t e = ev;
+    ev = nullptr;
+    B200_CUDA(cudaEventRecord(e, side));
+    B200_CUDA(cudaStreamWaitEvent(stream, e, 0));
+    return B200_OK;
+  }
+  ~SideJoin() {  // a failed call: its own error stays the one that is reported
+    if (ev && cudaEventRecord(ev, side) == cudaSuccess) (void)cudaStreamWaitEvent(stream, ev, 0);
+  }
+};
 
 // SwiGLU transition of any width: [LayerNorm,] fc1 | fc2 product with the SwiGLU in its epilogue (hidden a multiple of 64;
 // otherwise a row kernel of its own), fc3 product.  x fp32 or bf16 [rows][cols], out [rows][out_cols]; residual: added into
@@ -2072,6 +2090,7 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
     B200_CUDA(cudaEventRecord(ev[4], stream));  // s, and all that was enqueued before this call
     B200_CUDA(cudaStreamWaitEvent(side, ev[4], 0));
   }
+  SideJoin forked{side, stream, two ? ev[4] : nullptr};
   if (!pair_mask) {
     uint8_t* pm = ws + scratch + 2 * bias_bytes;
     B200_LAUNCH(pair_mask_kernel, grid_for(int64_t(B) * N * N, 1024), 256, 0, stream, token_mask, pm, B, N);
@@ -2113,11 +2132,7 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
                                   static_cast<uint8_t*>(side_workspace), side))
       return e;
   }
-  if (two) {
-    B200_CUDA(cudaEventRecord(ev[4], side));
-    B200_CUDA(cudaStreamWaitEvent(stream, ev[4], 0));
-  }
-  return B200_OK;
+  return forked.join();
 }
 
 }  // extern "C"
