@@ -42,6 +42,13 @@ class PackedWeightsMixin:
     _packed_key = None
     _watch = None
 
+    def __getstate__(self):
+        """Copies and pickles of a module go without what is derived from its parameters (device addresses among it)."""
+        kept = dict(self.__dict__)
+        for name in ("_packed", "_packed_key", "_watch", "_split", "_split_key", "_side"):
+            kept.pop(name, None)
+        return kept
+
     def _pack_key(self):
         watch = self._watch
         if watch is not None:

@@ -1,4 +1,9 @@
 """What a module keeps between calls, and what it does not (no GPU needed)."""
+import copy
+import pickle
+from types import SimpleNamespace
+
+import pytest
 import torch
 
 from bioemu2_b200 import _lib
@@ -17,3 +22,21 @@ def test_conditioned_layer_reads_its_scale_on_every_call(monkeypatch):
     assert m(*args) == 0.5
     m.lns_scale = 0.25
     assert m(*args) == 0.25
+
+
+@pytest.mark.parametrize("make", [lambda b: b.Transition(128, 512), lambda b: b.PairwiseConditioning(128, 128),
+                                  lambda b: b.PairMixerModule(384, 128, 1)])
+def test_a_module_that_has_packed_its_weights_can_be_copied(make):
+    import bioemu2_b200 as b
+
+    m = make(b)
+    for child in m.modules():
+        if hasattr(child, "packed"):
+            child._pack_key()
+            child._packed, child._split = (SimpleNamespace(struct=_lib.TransitionWeights(1, 2, 3, 4, 512)) for _ in range(2))
+    for other in (copy.deepcopy(m), pickle.loads(pickle.dumps(m))):
+        assert [k for k, _ in other.named_parameters()] == [k for k, _ in m.named_parameters()]
+        for child, kept in zip(other.modules(), m.modules()):
+            if hasattr(child, "packed"):
+                assert child._packed is None and child._split is None and kept._packed is not None
+                assert child._pack_key() != kept._pack_key()
