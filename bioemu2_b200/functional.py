@@ -139,9 +139,8 @@ class _Pack:
         for t, off, groups, group, pitch, stride, scale in self.parts:
             if t is not None:
                 _require_cuda(t)
-                t = t.detach()
                 if t.dtype != torch.float32 or not t.is_contiguous() or t.data_ptr() % 32:
-                    t = t.to(torch.float32).contiguous().clone() if t.data_ptr() % 32 else t.to(torch.float32).contiguous()
+                    t = aligned(t.detach().to(torch.float32).contiguous())
                 keep.append(t)
             segs.append(_lib.PackSegment(_ptr(t), off, groups, group, pitch, stride, scale))
         for i in range(0, len(segs), _lib.PACK_MAX):
@@ -206,13 +205,16 @@ class TransitionPacked:
             raise ValueError("the fused pair-transition kernel is built for dim=128, hidden<=512")
         width = self.hidden = 256 if hidden <= 256 else 512
         pk = _Pack()
-        for c in range(0, width, 64):  # chunks of [64 fc1 rows | 64 fc2 rows]
-            for fc in (fc1, fc2):
-                rows = fc[min(c, hidden):min(c + 64, hidden)]
-                if rows.shape[0]:
-                    pk.add(rows, pad_to=64 * 128)
-                else:
-                    pk.add(None, count=64 * 128)
+        if hidden == width:  # chunks of [64 fc1 rows | 64 fc2 rows]
+            pk.interleave((fc1, fc2), groups=width // 64)
+        else:
+            for c in range(0, width, 64):
+                for fc in (fc1, fc2):
+                    rows = fc[min(c, hidden):min(c + 64, hidden)]
+                    if rows.shape[0]:
+                        pk.add(rows, pad_to=64 * 128)
+                    else:
+                        pk.add(None, count=64 * 128)
         pk.add(fc3, groups=128, pad_to=width)
         buf = pk.build(fc3.device)
         self.w13, self.w3 = buf[:2 * width * 128].view(-1, 128), buf[2 * width * 128:].view(128, width)
@@ -750,6 +752,7 @@ def trunk_blocks_(z_in: Tensor, z: Tensor, s: Tensor | None, token_mask: Tensor 
                   heads: int = 0, side: torch.cuda.Stream | None = None) -> TrunkPacked:
     """``trunk_`` for a stack whose weights are not packed yet: block ``i`` (``pack(i)``) is packed on the host while the GPU
     runs the blocks before it.  Returns the packed stack for the next call."""
+    token_mask, pair_mask = (None if m is None else mask_u8(m) for m in (token_mask, pair_mask))
     blocks = []
     for i in range(n):
         blocks.append(pack(i))

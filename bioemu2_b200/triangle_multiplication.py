@@ -18,16 +18,14 @@ from . import ieee, precision
 
 def _watch_list(module: nn.Module):
     """Where a module tree keeps its parameters: (child dict, name, child) links and (parameter dict, name) slots."""
-    links, slots = [], []
-
-    def walk(m):
-        slots.extend((m._parameters, n) for n in m._parameters)
-        for n, c in m._modules.items():
-            links.append((m._modules, n, c))
-            if c is not None:
-                walk(c)
-
-    walk(module)
+    links, slots, todo = [], [], [module]
+    for m in todo:  # grows under way
+        d = m._parameters
+        slots += [(d, n) for n in d]
+        d = m._modules
+        if d:
+            links += [(d, n, c) for n, c in d.items()]
+            todo += [c for c in d.values() if c is not None]
     return links, slots
 
 
@@ -57,7 +55,7 @@ class PackedWeightsMixin:
                     watch = None
                     break
         if watch is None:
-            watch = self._watch = _watch_list(self)
+            watch = self.__dict__["_watch"] = _watch_list(self)  # (a module's own setattr looks for parameters first)
         key = []
         for d, n in watch[1]:
             p = d.get(n)
@@ -71,8 +69,8 @@ class PackedWeightsMixin:
         key = self._pack_key()
         if self._packed is None or key != self._packed_key:
             with torch.no_grad():
-                self._packed = self._build_packed() if build is None else build()
-            self._packed_key = key
+                self.__dict__["_packed"] = self._build_packed() if build is None else build()
+            self.__dict__["_packed_key"] = key
         return self._packed
 
     _split = None

@@ -40,3 +40,28 @@ def test_a_module_that_has_packed_its_weights_can_be_copied(make):
             if hasattr(child, "packed"):
                 assert child._packed is None and child._split is None and kept._packed is not None
                 assert child._pack_key() != kept._pack_key()
+
+
+@pytest.mark.parametrize("hidden", [256, 512, 200, 64, 448])
+def test_fused_transition_weights(monkeypatch, hidden):
+    """Alternating blocks of 64 rows of fc1 and fc2, padded with zeros to the kernel's width; whole widths are few segments, for
+    packing them is most of what a first pass on new weights costs the host."""
+    parts = []
+
+    def build(pk, device):
+        out = torch.zeros(pk.size)
+        for t, off, groups, group, pitch, stride, scale in pk.parts:
+            parts.append(t)
+            for k in range(groups if t is not None else 0):
+                out[off + k * stride:off + k * stride + group] = scale * t.reshape(-1)[k * group:(k + 1) * group]
+        return out
+
+    monkeypatch.setattr(F._Pack, "build", build)
+    fc1, fc2, fc3 = torch.randn(hidden, 128), torch.randn(hidden, 128), torch.randn(128, hidden)
+    w = F.TransitionPacked(None, None, fc1, fc2, fc3)
+    width = 256 if hidden <= 256 else 512
+    wide = torch.zeros(2, width, 128)
+    wide[0, :hidden], wide[1, :hidden] = fc1, fc2
+    assert torch.equal(w.w13.view(width // 64, 2, 64, 128), wide.view(2, width // 64, 64, 128).transpose(0, 1))
+    assert torch.equal(w.w3[:, :hidden], fc3) and not w.w3[:, hidden:].any()
+    assert len(parts) == 3 or hidden != width
