@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import threading
+import weakref
 
 import torch
 from torch import Tensor
@@ -15,12 +16,21 @@ from torch import Tensor
 from . import _lib
 from ._lib import lib
 
+class _Buffers(dict):
+    """The scratch buffers of one host thread by (device, stream)."""
+
+
 class _Workspaces(threading.local):
-    """Scratch buffers of one host thread by (device, stream): kernels of two threads on one stream may interleave, so
-    threads do not share a buffer."""
+    """Kernels of two threads on one stream may interleave, so threads do not share a buffer; every thread's buffers are
+    listed for as long as the thread lives, so that any thread can give them all back."""
+
+    lock = threading.Lock()
+    of_all_threads: "weakref.WeakValueDictionary[int, _Buffers]" = weakref.WeakValueDictionary()
 
     def __init__(self) -> None:
-        self.buffers: dict[tuple[int, int], Tensor] = {}
+        self.buffers = _Buffers()
+        with self.lock:
+            self.of_all_threads[id(self.buffers)] = self.buffers
 
 
 _WORKSPACES = _Workspaces()
@@ -43,8 +53,12 @@ def workspace(nbytes: int, device: torch.device) -> Tensor:
 
 
 def release_workspaces() -> None:
-    """Drops this thread's scratch buffers."""
-    _WORKSPACES.buffers.clear()
+    """Drops the scratch buffers of all threads.  A call that is under way keeps its own until it returns; what its kernels
+    still have to do then comes before any later use of the memory, which goes back to the stream it was taken on."""
+    with _WORKSPACES.lock:
+        held = list(_WORKSPACES.of_all_threads.values())
+    for buffers in held:
+        buffers.clear()
 
 
 def _zdtype(t: Tensor) -> int:
@@ -788,7 +802,8 @@ def trunk_(z_in: Tensor, z: Tensor, s: Tensor | None, token_mask: Tensor | None,
     nbytes = lib.b200_trunk_workspace_bytes(w.array, B, N, heads)
     sbytes = lib.b200_trunk_side_workspace_bytes(w.array, w.n, B, N, c_s, heads)
     # one buffer for both streams: the side stream has joined before the call returns to the current one
-    ws = workspace(nbytes + sbytes, z.device).data_ptr()
+    buf = workspace(nbytes + sbytes, z.device)
+    ws = buf.data_ptr()
     _lib.check(lib.b200_trunk_fwd(w.array, w.n, z_in.data_ptr(), z.data_ptr(), _ptr(s), _ptr(tm), _ptr(pm), B, N, c_s, heads,
                                   sd, zd, ws, nbytes, ws + nbytes, sbytes, _stream(),
                                   side.cuda_stream if side is not None else None))

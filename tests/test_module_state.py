@@ -1,6 +1,8 @@
 """What a module keeps between calls, and what it does not (no GPU needed)."""
 import copy
+import gc
 import pickle
+import threading
 from types import SimpleNamespace
 
 import pytest
@@ -65,3 +67,29 @@ def test_fused_transition_weights(monkeypatch, hidden):
     assert torch.equal(w.w13.view(width // 64, 2, 64, 128), wide.view(2, width // 64, 64, 128).transpose(0, 1))
     assert torch.equal(w.w3[:, :hidden], fc3) and not w.w3[:, hidden:].any()
     assert len(parts) == 3 or hidden != width
+
+
+def test_workspaces_of_threads_are_apart_and_go_back_together(monkeypatch):
+    monkeypatch.setattr(F, "_stream", lambda: 7)
+    cpu, seen, go, done = torch.device("cpu", 0), {}, threading.Event(), threading.Event()
+
+    def work():
+        seen["first"] = F.workspace(4096, cpu)
+        done.set()
+        go.wait(30)
+        seen["again"] = F.workspace(100, cpu)
+
+    mine = F.workspace(4096, cpu)
+    thread = threading.Thread(target=work)
+    thread.start()
+    assert done.wait(30)
+    assert seen["first"].data_ptr() != mine.data_ptr() and seen["first"].data_ptr() % 1024 == 0
+    assert F.workspace(100, cpu) is mine
+    F.release_workspaces()
+    go.set()
+    thread.join()
+    assert seen["again"] is not seen["first"] and F.workspace(100, cpu) is not mine
+    del seen["again"]
+    gc.collect()
+    assert all(b is F._WORKSPACES.buffers for b in F._WORKSPACES.of_all_threads.values())  # the thread's went with it
+    F.release_workspaces()
