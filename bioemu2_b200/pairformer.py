@@ -20,8 +20,11 @@ from . import _lib, precision
 from . import functional as F
 from .attention_pair_bias import AttentionPairBias
 from .transition import Transition
-from .triangle_attention import TriangleAttention
-from .triangle_multiplication import PackedWeightsMixin, TriangleMultiplication
+from .triangle_attention import TriangleAttention, TriangleAttentionEndingNode, TriangleAttentionStartingNode
+from .triangle_multiplication import PackedWeightsMixin, TriangleMultiplication, native_trimul
+
+
+_OWN_TRIATT = (TriangleAttention, TriangleAttentionStartingNode, TriangleAttentionEndingNode)
 
 
 class PairformerBlock(nn.Module):
@@ -60,6 +63,18 @@ class PairformerModule(PackedWeightsMixin, nn.Module):
         self.num_blocks = num_blocks
         self.layers = nn.ModuleList([PairformerBlock(token_s, token_z, **block_kwargs) for _ in range(num_blocks)])
 
+    @staticmethod
+    def _native(m) -> bool:
+        """Whether the native call covers a block: one with a module or a path of its own runs by itself."""
+        if type(m) is not PairformerBlock:
+            return False
+        op = m._modules  # (looked up on every pass, and a module's own getattr is ten times a dict's)
+        start, end, tz, attention, ts = (op[k] for k in ("tri_att_start", "tri_att_end", "transition_z", "attention", "transition_s"))
+        return native_trimul(op["tri_mul_out"], "outgoing") and native_trimul(op["tri_mul_in"], "incoming") \
+            and type(start) in _OWN_TRIATT and not start.ending and type(end) in _OWN_TRIATT and end.ending \
+            and type(tz) is Transition and tz._fused and type(attention) is AttentionPairBias and attention._bias_cache is None \
+            and type(ts) is Transition and not ts._fused
+
     def _pack_block(self, i: int) -> dict:
         m = self.layers[i]
         return {"tri_mul_out": m.tri_mul_out.packed(), "tri_mul_in": m.tri_mul_in.packed(),
@@ -91,10 +106,8 @@ class PairformerModule(PackedWeightsMixin, nn.Module):
         track of the NEXT block; the streams join at the end of the stack.  Both forms launch the same kernels on the same
         data and give identical results.
         """
-        native = len(self.layers) > 0 and not precision.use_ieee(None, s, z) and all(
-            m.attention._bias_cache is None and not m.transition_s._fused and m.tri_mul_out.matmul_precision != "ieee"
-            and m.tri_mul_in.matmul_precision != "ieee" for m in self.layers)
-        if not native:  # a layer with a path of its own (accurate mode, adopted bias cache, 128-wide single track)
+        native = len(self.layers) > 0 and not precision.use_ieee(None, s, z) and all(self._native(m) for m in self.layers)
+        if not native:  # a layer with a module or a path of its own (accurate mode, adopted bias cache, 128-wide single track)
             if z is not z_in:
                 z.copy_(z_in)
             if pair_mask_u8 is None:

@@ -15,7 +15,7 @@ from . import functional as F
 from .outer_product_mean import OuterProductMean
 from .pair_weighted_averaging import PairWeightedAveraging
 from .transition import Transition
-from .triangle_multiplication import PackedWeightsMixin, TriangleMultiplication
+from .triangle_multiplication import PackedWeightsMixin, TriangleMultiplication, native_trimul, plain
 
 
 class PairMixerLayer(nn.Module):
@@ -33,7 +33,7 @@ class PairMixerLayer(nn.Module):
         if self.training:
             raise RuntimeError("bioemu2_b200 modules are inference-only: call .eval()")
         # the reference returns a new tensor: the first update writes it, or the three run in place on a copy
-        if precision.use_ieee(self.tri_mul_out.matmul_precision, z):
+        if type(self.tri_mul_out) is TriangleMultiplication and precision.use_ieee(self.tri_mul_out.matmul_precision, z):
             z = self.tri_mul_out.forward_residual(F.aligned(z), pair_mask)
             self.tri_mul_in.forward_residual_(z, pair_mask)
             self.transition_z.forward_residual_(z)
@@ -67,6 +67,15 @@ class PairMixerModule(PackedWeightsMixin, nn.Module):
         _lib.raise_if_device_wait()  # a kernel whose bounded wait ran out earlier in the stack invalidates the result
         return s, z
 
+    @staticmethod
+    def _native(m) -> bool:
+        """Whether the native call covers a layer: one with a module or a path of its own runs by itself."""
+        if type(m) is not PairMixerLayer:
+            return False
+        op = m._modules  # (looked up on every pass, and a module's own getattr is ten times a dict's)
+        return native_trimul(op["tri_mul_out"], "outgoing") and native_trimul(op["tri_mul_in"], "incoming") \
+            and type(op["transition_z"]) is Transition and op["transition_z"]._fused
+
     def _pack_block(self, i: int) -> dict:
         m = self.layers[i]
         return {"tri_mul_out": m.tri_mul_out.packed(), "tri_mul_in": m.tri_mul_in.packed(),
@@ -74,8 +83,7 @@ class PairMixerModule(PackedWeightsMixin, nn.Module):
 
     def forward_into(self, z_in: Tensor, z: Tensor, pair_mask: Tensor) -> Tensor:
         """The block loop ``z_in`` -> ``z`` (contiguous; ``z`` may be ``z_in``) in one native call; returns ``z``."""
-        if len(self.layers) == 0 or precision.use_ieee(None, z) or any(
-                m.tri_mul_out.matmul_precision == "ieee" or m.tri_mul_in.matmul_precision == "ieee" for m in self.layers):
+        if len(self.layers) == 0 or precision.use_ieee(None, z) or not all(self._native(m) for m in self.layers):
             if z is not z_in:
                 z.copy_(z_in)
             mask8 = F.mask_u8(pair_mask)
@@ -135,7 +143,11 @@ class PairMixerMSALayer(nn.Module):
             raise RuntimeError("bioemu2_b200 modules are inference-only: call .eval()")
         m = self.pair_weighted_averaging.forward_residual(m, z, token_mask)      # a new tensor
         self.msa_transition.forward_residual_(m)
-        z = self.outer_product_mean.forward_add(m, msa_mask, z)                  # a new tensor
+        if plain(self.outer_product_mean, OuterProductMean):
+            z = self.outer_product_mean.forward_add(m, msa_mask, z)              # a new tensor
+        else:
+            upd = self.outer_product_mean(m, msa_mask)
+            z = F.add_rows(z.contiguous(), upd) if z.dtype == torch.float32 else z + upd.to(z.dtype)
         mask8 = token_mask.to(torch.uint8).contiguous()
         self.tri_mul_out.forward_residual_(z, mask8)
         self.tri_mul_in.forward_residual_(z, mask8)

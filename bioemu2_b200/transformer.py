@@ -20,7 +20,7 @@ from . import _lib
 from . import functional as F
 from .attention_pair_bias import AttentionPairBias, AttentionPairBiasSlidingWindow
 from .transition import Transition
-from .triangle_multiplication import PackedWeightsMixin
+from .triangle_multiplication import PackedWeightsMixin, plain
 
 
 class AttentionLayer(nn.Module):
@@ -97,11 +97,10 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
         w_cond = pk.build(lin.weight.device).view(lin.weight.shape)
         b_cond = lin.bias.detach().float().contiguous()
         ln_w, ln_b = (None if p is None else p.detach().float().contiguous() for p in (ln.weight, ln.bias))
-        attn = self.attention.attention_layer.pair_bias_attn if self._windowed else self.attention.pair_bias_attn
-        tr = self.transition
+        attn, tr = self._native_attention(), self.transition
         native = None
-        if self.dim % 32 == 0 and lin.in_features % 8 == 0 and lin.in_features <= 1024 and not tr.use_norm and not attn.initial_norm \
-                and ln.eps == 1e-5 and tr.fc3.out_features == self.dim and (self._windowed or attn.c_z == 128):
+        if attn is not None and self.dim % 32 == 0 and lin.in_features % 8 == 0 and lin.in_features <= 1024 \
+                and not tr.use_norm and not attn.initial_norm and ln.eps == 1e-5 and tr.fc3.out_features == self.dim and (self._windowed or attn.c_z == 128):
             layer = _lib.CondLayer()
             ap, tp = attn.packed(), tr.packed()
             layer.dim, layer.dim_cond, layer.heads, layer.dim_pairwise = self.dim, lin.in_features, attn.num_heads, attn.c_z
@@ -119,12 +118,21 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
             native = (layer, (ap, tp, ln_w, ln_b))
         return w_cond, b_cond, native
 
+    def _native_attention(self):
+        """The attention module whose weights the native call takes, if it may stand for the sub-modules as they are now."""
+        attn = self.attention
+        if self._windowed:
+            attn = attn.attention_layer if plain(attn, SlidingWindowAttentionLayer) else None
+        attn = attn.pair_bias_attn if plain(attn, AttentionLayer) else None
+        own = AttentionPairBiasSlidingWindow if self._windowed else AttentionPairBias
+        return attn if plain(attn, own) and plain(self.transition, Transition) else None
+
     def forward(self, x: Tensor, pairs: Tensor, c: Tensor, mask: Tensor | None = None, multiplicity: int = 1) -> Tensor:
         if mask is None:  # full attention: pairs [B, T, T, .]; windowed: x [B*M, atoms, .]
             n = x.shape[1] if pairs.ndim == 5 else pairs.shape[1]
             mask = torch.ones(pairs.shape[0], n, dtype=torch.bool, device=x.device)
-        native = self.packed()[2]
-        if native is None:
+        native, attn = self.packed()[2], self._native_attention()
+        if native is None or attn is None:
             return self._forward(x, pairs, c, mask, multiplicity, self.attention)
         layer, B = native[0], pairs.shape[0]
         if self._windowed and x.ndim == 3 and mask.numel() == B * x.shape[1]:
@@ -143,7 +151,6 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
         else:
             if tuple(pairs.shape) != (B, N, N, 128):
                 raise ValueError(f"expected pairs[{B},{N},{N},128], got {tuple(pairs.shape)}")
-            attn = self.attention.pair_bias_attn
             if attn._bias_cache is not None:
                 bias = attn._bias_cache[0].lookup(attn._bias_cache[1], pairs)
         sized = _lib.CondLayer.from_buffer_copy(layer)  # the layer's own copy may be in use by another thread

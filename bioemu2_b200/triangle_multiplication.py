@@ -16,6 +16,12 @@ from . import functional as F
 from . import ieee, precision
 
 
+def plain(module, cls) -> bool:
+    """Whether calling ``module`` does what ``cls`` does and nothing besides (no subclass, no hook, no forward of its own), so
+    that a call which covers several modules may stand for it."""
+    return type(module) is cls and not module._forward_hooks and not module._forward_pre_hooks and "forward" not in module.__dict__
+
+
 def _watch_list(module: nn.Module):
     """Where a module tree keeps its parameters: (child dict, name, child) links and (parameter dict, name) slots."""
     links, slots, todo = [], [], [module]
@@ -147,3 +153,11 @@ class TriangleMultiplicationOutgoing(TriangleMultiplication):
 class TriangleMultiplicationIncoming(TriangleMultiplication):
     def __init__(self, dim: int = 128) -> None:
         super().__init__(dim=dim, mode="incoming")
+
+
+_OWN_TRIMUL = (TriangleMultiplication, TriangleMultiplicationOutgoing, TriangleMultiplicationIncoming)
+
+
+def native_trimul(module, mode: str) -> bool:
+    """A triangle multiplication of that direction that a trunk's native call may stand for."""
+    return type(module) in _OWN_TRIMUL and module.mode == mode and module.matmul_precision != "ieee"

@@ -93,3 +93,121 @@ def test_workspaces_of_threads_are_apart_and_go_back_together(monkeypatch):
     gc.collect()
     assert all(b is F._WORKSPACES.buffers for b in F._WORKSPACES.of_all_threads.values())  # the thread's went with it
     F.release_workspaces()
+
+
+class _Adds(torch.nn.Module):
+    """Stands where one of the package's modules stood."""
+
+    matmul_precision = None
+
+    def __init__(self, keeps=None):
+        super().__init__()
+        self.keeps, self._bias_cache, self._fused = keeps, None, False
+
+    def forward(self, x, *args):
+        return torch.ones_like(x)
+
+    def forward_residual(self, x, *args):
+        return x + 1
+
+    def forward_residual_(self, x, *args):
+        return x.add_(1)
+
+
+def _refuse(*args, **kwargs):
+    raise AssertionError("a native call")
+
+
+@pytest.mark.parametrize("keep", [False, True])
+def test_trunks_run_the_modules_that_were_put_into_them(monkeypatch, keep):
+    """``keep``: the stand-in holds the old module, so the parameters are the ones the stack knows."""
+    import bioemu2_b200 as b
+
+    monkeypatch.setattr(_lib, "raise_if_device_wait", lambda: None)
+    for name in ("trunk_", "trunk_blocks_"):
+        monkeypatch.setattr(F, name, _refuse)
+    s, z = torch.zeros(1, 4, 384), torch.zeros(1, 4, 4, 128)
+    tok = torch.ones(1, 4, dtype=torch.bool)
+    for trunk, mask in ((b.PairMixerModule(384, 128, 2), tok[:, :, None] & tok[:, None, :]), (b.PairformerModule(384, 128, 2), tok)):
+        trunk.eval()
+        trunk._pack_key()
+        updates = 0
+        for layer in trunk.layers:
+            for name, child in list(layer.named_children()):
+                updates += name not in ("attention", "transition_s")
+                setattr(layer, name, _Adds(child if keep else None))
+        with torch.no_grad():
+            got = trunk(s, z, mask)
+        assert torch.equal(got[1], torch.full_like(z, updates)) and not z.any()
+
+    layer = b.PairMixerLayer(384, 128).eval()
+    for name, child in list(layer.named_children()):
+        setattr(layer, name, _Adds())
+    assert torch.equal(layer(s, z, None)[1], z + 3)
+
+
+@pytest.mark.parametrize("change", ["mode", "width", "subclass"])
+def test_trunk_blocks_that_differ_run_by_themselves(monkeypatch, change):
+    import bioemu2_b200 as b
+
+    class Own(b.PairMixerLayer):
+        pass
+
+    trunk, ran = b.PairMixerModule(384, 128, 2).eval(), []
+    assert all(trunk._native(m) for m in trunk.layers)
+    if change == "mode":
+        trunk.layers[1].tri_mul_in = b.TriangleMultiplicationOutgoing(128)
+    elif change == "width":
+        trunk.layers[1].transition_z = b.Transition(128, 1024)
+    else:
+        trunk.layers[1] = Own(384, 128)
+    for name in ("trunk_", "trunk_blocks_"):
+        monkeypatch.setattr(F, name, _refuse)
+    monkeypatch.setattr(b.PairMixerLayer, "forward_", lambda self, z, mask: ran.append(self))
+    monkeypatch.setattr(_lib, "raise_if_device_wait", lambda: None)
+    trunk(None, torch.zeros(1, 4, 4, 128), torch.ones(1, 4, 4, dtype=torch.bool))
+    assert ran == list(trunk.layers)
+
+
+@pytest.mark.parametrize("windowed", [False, True])
+def test_conditioned_layer_runs_the_modules_that_were_put_into_it(monkeypatch, windowed):
+    import bioemu2_b200 as b
+
+    def layer():
+        kw = dict(is_sliding_window=True, window_queries=32, window_keys=128) if windowed else {}
+        m = b.ConditionedTransformerLayer(128, 16 if windowed else 128, 128, 4, 512, **kw)
+        kept = _lib.CondLayer()
+        kept.dim_cond, kept.window_queries, kept.window_keys, kept.dim_pairwise = 128, 32, 128, 16
+        monkeypatch.setattr(m, "packed", lambda: (None, None, (kept, ())))
+        monkeypatch.setattr(m, "_forward", lambda *args: "by modules")
+        return m
+
+    monkeypatch.setattr(F, "cond_layer", lambda *args: "one call")
+    pairs = torch.zeros(1, 1, 32, 128, 16) if windowed else torch.zeros(1, 32, 32, 128)
+    args = torch.zeros(1, 32, 128), pairs, torch.zeros(1, 32, 128)
+    assert layer()(*args) == "one call"
+    for hooked in ("transition", "attention", "attention.pair_bias_attn" if not windowed else "attention.attention_layer"):
+        m = layer()
+        handle = m.get_submodule(hooked).register_forward_hook(lambda *a: None)
+        assert m(*args) == "by modules"
+        handle.remove()
+        assert m(*args) == "one call"
+    m = layer()
+    m.transition = _Adds()
+    assert m(*args) == "by modules"
+    m = layer()
+    m.attention = _Adds()
+    assert m(*args) == "by modules"
+
+
+def test_msa_layer_runs_the_outer_product_mean_that_was_put_into_it(monkeypatch):
+    import bioemu2_b200 as b
+
+    monkeypatch.setattr(F, "add_rows", lambda x, y: x + y)
+    m = b.PairMixerMSALayer(384, 64, 128).eval()
+    for name, child in list(m.named_children()):
+        setattr(m, name, _Adds())
+    m.outer_product_mean.forward = lambda msa, mask: torch.full((1, 4, 4, 128), 7.0)
+    z = torch.zeros(1, 4, 4, 128)
+    _, got, _ = m(None, z, torch.zeros(1, 3, 4, 64), torch.ones(1, 4, 4), torch.ones(1, 3, 4))
+    assert torch.equal(got, z + 10)
