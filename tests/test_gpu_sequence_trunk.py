@@ -166,6 +166,28 @@ def test_sequence_trunk_encoders_are_called_like_the_reference():
     assert isinstance(mod, b.PairMixerSequenceEmbedder)
 
 
+@pytest.mark.parametrize("n,rows", [(256, 128), (100, 37)])
+def test_two_passes_are_equal(n, rows):
+    """Enough tiles that every CTA of a product reuses its staging tiles, whose stores have to be read out first."""
+    import bioemu2_b200 as b
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rand = lambda *s: torch.rand(*s, device="cuda", generator=g)  # noqa: E731
+    with torch.device("cuda"):
+        mod = b.PairMixerSequenceEmbedder(384, 128, 456, msa_s=64, msa_blocks=1, num_blocks=1).eval()
+    tok = torch.ones(1, n, dtype=torch.bool, device="cuda")
+    tok[:, n - 7:] = False
+    feats = {"msa": torch.nn.functional.one_hot((rand(1, rows, n) * 33).long(), 33).float(), "token_pad_mask": tok,
+             "msa_mask": tok[:, None] & (rand(1, rows, n) > 0.1), "has_deletion": (rand(1, rows, n) < 0.2).float(),
+             "deletion_value": rand(1, rows, n), "msa_paired": (rand(1, rows, n) < 0.5).float()}
+    x = rand(1, n, 456) - 0.5
+    with torch.no_grad():
+        first = mod(x, feats, num_steps_recycle=1)
+        for _ in range(8):
+            again = mod(x, feats, num_steps_recycle=1)
+            assert all(torch.equal(p, q) for p, q in zip(first, again))
+
+
 def test_sequence_trunk_argument_errors():
     case = C.CASES["sequence_trunk"]()
     mod = _embedder(case)

@@ -1,4 +1,6 @@
 """The trunk's two streams, and threads that share a stream."""
+import threading
+
 import pytest
 import torch
 
@@ -38,3 +40,36 @@ def test_a_call_that_fails_under_way_joins_its_side_stream():
     with torch.no_grad():
         again = trunk(s, z, mask)
     assert all(torch.equal(x, y) for x, y in zip(want, again))
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_threads_on_one_stream(shared):
+    """Two threads enqueue on the same stream at the same time, with a trunk each or with one between them: the results are those
+    of calls one after the other."""
+    trunks = [_trunk(2, 3)] * 2 if shared else [_trunk(2, 3), _trunk(2, 4)]
+    inputs = [_inputs(72, 5), _inputs(40, 6)]
+    with torch.no_grad():
+        want = [t(*x) for t, x in zip(trunks, inputs)]
+    torch.cuda.synchronize()
+    start, got, errors = threading.Barrier(2), [[], []], []
+
+    def work(i):
+        try:
+            with torch.no_grad():
+                start.wait(30)
+                for _ in range(20):
+                    got[i].append(trunks[i](*inputs[i]))
+        except Exception as exc:  # noqa: BLE001 - reported by the main thread
+            errors.append(exc)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    for w, runs in zip(want, got):
+        assert len(runs) == 20
+        for r in runs:
+            assert torch.equal(r[0], w[0]) and torch.equal(r[1], w[1])
