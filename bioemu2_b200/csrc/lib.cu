@@ -74,8 +74,14 @@ struct BmmLaunch {
 
 // Tile width by the estimated time of the busiest CTA.  A K block of 64 takes a 256-wide tile about 1.5 times as long as a
 // 128-wide one (48 against 32 KB through L2 for twice the product), the last tile's epilogue is exposed; in units of a
-// thousandth of a 128-wide block: 256 columns where they fill the waves, 128 where the narrow tile leaves fewer CTAs idle
-// (2816 x 768 columns for 2048 rows: 176 wide tiles in two waves, 24.0 us; 352 narrow ones, 20.9 us).
+// thousandth of a 128-wide block: 256 columns where they fill the waves, 128 where the narrow tile leaves fewer CTAs idle.
+// Against the better of the two widths, over 60 products of the trunk, the token and atom blocks, the contractions and the
+// outer product mean: within 2 % of it, once 5 % (rows x columns x K, us, 128 / 256 wide: 256 x 768 x 3072 12.2 / 18.8,
+// 2048 x 2816 x 768 12.2 / 13.5, 2048 x 6144 x 768 20.7 / 18.9, 3584 x 2816 x 768 17.9 / 18.6 where the estimate takes 256;
+// 128 batches of 384^3 21.8 / 25.7, of 512^3 42.5 / 38.7).
+// Products that run on a side stream underneath another's kernels go by the same estimate: wide tiles for those, since they
+// take less SM time, moved a trunk's time both ways (4 blocks, us, without / with: 144 tokens 890 / 902, 160 1024 / 1006,
+// 203 1144 / 1154, 256 1292 / 1322, 320 and more the same).
 static int bmm_tile_n(int M, int N, int K, int batch) {
   const int64_t tm = (M + 127) / 128, kb = (K + 63) / 64, sms = sm_count();
   auto cost = [&](int bn, int64_t per_block, int64_t tail) {
@@ -84,14 +90,6 @@ static int bmm_tile_n(int M, int N, int K, int batch) {
   };
   return cost(256, 1500, 5000) <= cost(128, 1000, 2500) ? 256 : 128;
 }
-
-// Set while a thread enqueues products that run underneath another stream's kernels: there the SM time they take counts, not
-// how soon they end, so they take wide tiles (trunk N = 203: 1.24 ms, 1.31 with narrow ones).
-static thread_local bool t_background = false;
-struct BackgroundScope {
-  explicit BackgroundScope(bool on) { t_background = on; }
-  ~BackgroundScope() { t_background = false; }
-};
 
 static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   const int64_t c_batch = a.sc > 0 ? a.sc : a.ldc * int64_t(a.M);
@@ -104,7 +102,7 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   // for 65536 x 128 x 128).
   const bool add = bulk_c && a.residual && a.residual != a.C && a.out_f32 && a.batch == 1 && a.remap_n == 0 && !a.mul &&
                    !a.swiglu && aligned(a.residual, 16);
-  const int BN = a.mul || add ? 128 : a.split || a.gate_mask ? 256 : t_background ? (a.N % 256 == 0 || a.N > 1024 ? 256 : 128) : bmm_tile_n(a.M, a.N, a.parts ? 3 * a.K : a.K, a.batch);
+  const int BN = a.mul || add ? 128 : a.split || a.gate_mask ? 256 : bmm_tile_n(a.M, a.N, a.parts ? 3 * a.K : a.K, a.batch);
   CUtensorMap tmA, tmB;
   const bool a_shared = a.batch > 1 && a.sa == 0;  // one A for every batch item
   {
@@ -2123,7 +2121,6 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
       B200_CUDA(cudaEventRecord(ev[k], stream));
       B200_CUDA(cudaStreamWaitEvent(side, ev[k], 0));
     }
-    BackgroundScope background(two && N > 128);  // up to 128 tokens the pair track leaves SMs free
     if (int e = apb_run(s, nullptr, bias[k], Nk, token_mask, s, &w.attention, B, 1, N, c_s, heads, s_dtype, B200_DTYPE_F32,
                         true, side_workspace, side_bytes, side))
       return e;
