@@ -168,14 +168,6 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, ui
       "r"(c2)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_4d(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1,
-                                            int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
-      "[%2];" ::"r"(smem_u32(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
 __device__ __forceinline__ void tma_store_4d(const void* tmap, const void* smem_src, int c0, int c1, int c2, int c3) {
   asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
                    reinterpret_cast<uint64_t>(tmap)),
@@ -253,26 +245,6 @@ __device__ __forceinline__ void tc_fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; bf16 inputs, fp32 accumulate; one thread issues.
-__device__ __forceinline__ void umma_bf16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem].
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // The mbarrier receives one arrival once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -332,17 +304,6 @@ __device__ __forceinline__ void tmem_st_32x16_f(uint32_t taddr, const float* v) 
       "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld_32x8_f(uint32_t taddr, float* v) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st_32x8_f(uint32_t taddr, const float* v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-               ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-               : "memory");
-}
 // One fp32 column of 32 lanes (a per-row scalar kept in tensor memory).
 __device__ __forceinline__ float tmem_ld_32x1_f(uint32_t taddr) {
   float v;
@@ -375,18 +336,6 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&v
       "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
 }
-// 32 lanes x 32 fp32 columns from registers into TMEM.
-__device__ __forceinline__ void tmem_st_32x32_f(uint32_t taddr, const float* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]),
-      "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "f"(v[16]),
-      "f"(v[17]), "f"(v[18]), "f"(v[19]), "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]), "f"(v[24]), "f"(v[25]),
-      "f"(v[26]), "f"(v[27]), "f"(v[28]), "f"(v[29]), "f"(v[30]), "f"(v[31])
-      : "memory");
-}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // TMEM address of (lane, column) relative to an allocation base.
@@ -406,37 +355,20 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N) {
          | (uint32_t(M >> 4) << 24);      // M / 16
 }
 
-// Shared-memory operand descriptor, K-major rows of 128 B with the 128-byte
-// swizzle (what TMA SWIZZLE_128B writes): 8-row groups are 1024 B apart.
-// `smem_addr` is the shared-space byte address of the first row; the tile base
-// must be 1024-byte aligned, K offsets inside a row are added to the address.
-__device__ __forceinline__ uint64_t make_desc_k_sw128(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= uint64_t((smem_addr & 0x3FFFF) >> 4);  // start address, 16-byte units
-  d |= uint64_t(1) << 16;                     // leading byte offset (unused for swizzled K-major)
-  d |= uint64_t(1024 >> 4) << 32;             // stride byte offset between 8-row groups
-  d |= uint64_t(1) << 46;                     // descriptor version (Blackwell)
-  d |= uint64_t(2) << 61;                     // SWIZZLE_128B
-  return d;
-}
-// Same with 64-byte rows and the 64-byte swizzle (TMA SWIZZLE_64B): 8-row groups 512 B apart.
-__device__ __forceinline__ uint64_t make_desc_k_sw64(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= uint64_t((smem_addr & 0x3FFFF) >> 4);
-  d |= uint64_t(1) << 16;
-  d |= uint64_t(512 >> 4) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(4) << 61;  // SWIZZLE_64B
-  return d;
-}
-// The same descriptors as two 32-bit halves, for issue loops that step through K by adding to the low word
-// (a K step of 16 bf16 = 32 bytes is +2) and so spend one integer add per operand per MMA.
+// Shared-memory operand descriptors, K-major, as two 32-bit halves: issue loops step through K by adding to the low word (a K
+// step of 16 bf16 = 32 bytes is +2) and so spend one integer add per operand per MMA.
+//   low word    start address and leading byte offset, in 16-byte units
+//   high word   stride byte offset between 8-row groups, descriptor version (bit 14), swizzle mode (bits 29..)
+// Rows of 128 B with the 128-byte swizzle (what TMA SWIZZLE_128B writes) have their 8-row groups 1024 B apart and need a
+// 1024-byte aligned base; rows of 64 B with the 64-byte swizzle 512 B.  Without a swizzle the operand is 8-row x 16-byte core
+// matrices: the stride between consecutive 8-row groups, and in the low word the one between the two 16-byte K chunks of a step.
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes = 16) {
   return ((smem_addr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);
 }
 constexpr uint32_t kDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
 constexpr uint32_t kDescHiSw64 = (512u >> 4) | (1u << 14) | (4u << 29);
 __host__ __device__ constexpr uint32_t desc_hi_noswizzle(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14); }
+// D[tmem] (+)= A[smem] * B[smem]; bf16 inputs, fp32 accumulate; one thread issues.
 __device__ __forceinline__ void umma_bf16_ss2(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                               uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -448,6 +380,7 @@ __device__ __forceinline__ void umma_bf16_ss2(uint32_t d_tmem, uint32_t a_lo, ui
       ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem].
 __device__ __forceinline__ void umma_bf16_ts2(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                                               uint32_t accumulate) {
   asm volatile(
@@ -457,16 +390,6 @@ __device__ __forceinline__ void umma_bf16_ts2(uint32_t d_tmem, uint32_t a_tmem, 
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
       : "memory");
-}
-// K-major operand without swizzle: 8-row x 16-byte core matrices, `sbo` bytes between consecutive 8-row groups,
-// `lbo` bytes between the two 16-byte K chunks of one MMA step.
-__device__ __forceinline__ uint64_t make_desc_k_noswizzle(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= uint64_t((smem_addr & 0x3FFFF) >> 4);
-  d |= uint64_t((lbo >> 4) & 0x3FFF) << 16;
-  d |= uint64_t((sbo >> 4) & 0x3FFF) << 32;
-  d |= uint64_t(1) << 46;
-  return d;
 }
 
 // Byte offset of 16-byte chunk `chunk` (0..7) of row `row` inside a 128B-swizzled
@@ -512,8 +435,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-// 2^lo, 2^hi of two fp32 exponents as packed bf16: one conversion and ONE exponential instruction for the pair
-// (the bf16x2 form of ex2 runs at the same instruction rate as the fp32 one, so it does twice the work).
+// 2^lo, 2^hi of two fp32 exponents as packed bf16: one conversion and one exponential instruction for the pair (an issue slot
+// instead of two; the pipe is busy for 19 clocks a warp, about as long as with two fp32 ones).
 __device__ __forceinline__ uint32_t exp2_bf16x2(float lo, float hi) {
   uint32_t d;
   asm("{ .reg .b32 t; cvt.rn.bf16x2.f32 t, %2, %1; ex2.approx.ftz.bf16x2 %0, t; }" : "=r"(d) : "f"(lo), "f"(hi));
@@ -525,8 +448,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
-
-
 
 // hi = bf16(v), lo = bf16(v - hi) of two neighbours.
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {

@@ -624,17 +624,6 @@ def cond_layer(layer: "_lib.CondLayer", x: Tensor, pairs: Tensor | None, bias: T
     return out
 
 
-def swiglu(h12: Tensor) -> Tensor:
-    """``silu(h12[..., :H]) * h12[..., H:]`` for bf16 ``h12[..., 2H]``."""
-    H = h12.shape[-1] // 2
-    h12 = h12.contiguous()
-    out = torch.empty(h12.shape[:-1] + (H,), dtype=torch.bfloat16, device=h12.device)
-    if out.numel() == 0:
-        return out
-    _lib.check(lib.b200_swiglu_fwd(h12.data_ptr(), out.data_ptr(), h12.numel() // (2 * H), H, _stream()))
-    return out
-
-
 def adaln(x: Tensor, cond: Tensor, alpha_col: int, beta_col: int, lns: float) -> Tensor:
     """``lns * (LN(x) * (1 + alpha) + beta)`` as bf16; alpha/beta are column blocks of fp32 ``cond[rows, cw]``."""
     xd = _zdtype(x)

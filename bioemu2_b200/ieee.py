@@ -120,7 +120,7 @@ def transition(x: Tensor, norm, fc1, fc2, fc3, ws: SplitWeights, add_residual: b
     rows, cols = x2.shape
     if out is not None and not (out.is_contiguous() and out.dtype == torch.float32):
         return out.copy_(transition(x, norm, fc1, fc2, fc3, ws, add_residual))
-    if getattr(ws, "native", False):
+    if ws.native:
         if out is None:
             out = torch.empty(shape[:-1] + (out_cols,), dtype=torch.float32, device=x.device)
         nbytes = lib.b200_accurate_transition_workspace_bytes(rows, cols, hidden)
@@ -148,8 +148,6 @@ def triangle_multiplication(x: Tensor, mask: Tensor, mod, ws: SplitWeights, add_
     B, N = x.shape[:2]
     if out is not None and not (out.is_contiguous() and out.dtype == torch.float32):
         return out.copy_(triangle_multiplication(x, mask, mod, ws, add_residual))
-    if not hasattr(ws, "norm_in_w"):
-        ws.norms(norm_in=mod.norm_in, norm_out=mod.norm_out)
     x, m8 = x.float().contiguous(), F.mask_u8(mask)
     if out is None:
         out = torch.empty_like(x)
