@@ -669,19 +669,20 @@ def run_b200(args) -> None:
             # q, k, g (N^2 x 384 bf16), V^T (N^2 x 128 bf16) read once, the gated output (N^2 x 128 bf16) written once,
             # the 4-head bias (4 N^2 bf16) read from L2
             core_bytes = P * (384 + 128 + 128) * 2 + 4 * P * 2
+            kernel = "flash_resident_kernel<32,32,2>" if N <= 512 else "flash_core_kernel<32,2>"
             roofline = {
-                "kernel": "flash_core_kernel<32,2> (triangle-attention core: QK^T + bias tile + online softmax + PV), "
+                "kernel": kernel + " (triangle-attention core: QK^T + bias tile + online softmax + PV), "
                           "launched alone on N rows x 4 heads x 32",
                 "bound": "tensor", "achieved": ach, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                 "frac": ach / pk["bf16_tflops"], "peak_source": pk["source"] + " burst (kernel timed alone)",
                 "algorithmic_flops_per_launch": core_flops, "algorithmic_bytes_per_launch": core_bytes,
                 "ms_per_launch": t["attention_core"],
-                # dram__bytes_read.sum + dram__bytes_write.sum of one launch at N=512 (ncu capture summarised in
-                # profiles/flash_core_triatt_n512.md); the operands scale with N^2, so other sizes are scaled from it
-                "traffic": 323.3e6 * (N / 512.0) ** 2,
-                "traffic_source": "ncu capture at N=512 (270.8 MB read + 52.5 MB written), scaled by (N/512)^2; the "
-                                  "algorithmic bytes of the launch are 337.6 MB at N=512 (four 67.1 MB operands read, one "
-                                  "67.1 MB result written, 2.1 MB of bias), so the kernel moves no byte twice",
+                # dram__bytes_read.sum + dram__bytes_write.sum of one launch (profiles/attention_core.md); captured at 512
+                # tokens only, and K and V^T are read once per query tile, so other sizes do not scale from it
+                "traffic": 733.6e6 if N == 512 else None,
+                "traffic_source": "ncu capture at N=512 (672.3 MB read + 61.3 MB written); every operand once would be "
+                                  "337.6 MB (four 67.1 MB operands read, one 67.1 MB result written, 2.1 MB of bias): K and "
+                                  "V^T are read once per tile of 128 queries, four times each" if N == 512 else None,
                 "note": "head dim 32 makes the core ex2-bound, not tensor-bound: N^3*4 exponentials at 16/clk/SM "
                         f"take {ex2_floor_ms:.3f} ms at the sampled clock; the tensor work alone would take "
                         f"{core_flops / (pk['bf16_tflops'] * 1e12) * 1e3:.3f} ms" if ex2_floor_ms else "",

@@ -83,7 +83,7 @@ class AttentionPairBiasSlidingWindow(AttentionPairBias):
     ``[B, heads, NW, W, H_keys]`` and shared by the ``multiplicity`` samples of a batch item.
 
     ``forward(s[B*M*NW, W, c_s], z[B, NW, W, H_keys, c_z], mask[B*NW, W], multiplicity)``.  The projections run on the
-    tensor cores in bf16; scores, softmax and the weighted sum are fp32.
+    tensor cores in bf16; scores and weighted sum accumulate in fp32, the softmax is fp32.
     """
 
     def __init__(self, c_s: int, c_z: int, num_heads: int, window_queries: int = 32, window_keys: int = 128,

@@ -9,9 +9,11 @@
 //   window_mma_kernel        windows of 16-query tiles and 128 keys: one CTA per (sample, window), a warp per head and 16
 //                            queries, scores and weighted sum by mma.sync (a tcgen05 tile of 128 rows would be three
 //                            quarters padding here).  fp32 softmax; the weights enter the second product as the sum of two
-//                            bf16 values, so they keep 16 bits
+//                            bf16 values, so they keep 16 bits: against fp64 the kernel's error is that of the CUDA-core
+//                            one, whose weights are fp32 (1.658e-3 for both at head dims 32 and 64, 1.661e-3 at 16: it
+//                            is the rounding of the bf16 result)
 //   window_attention_kernel  other shapes: fp32 CUDA cores, one thread per (head, query)
-// 4,096 atoms x 8 samples: window attention 115 us on CUDA cores (instruction-bound), bias 36 us (shuffles).
+// 4,096 atoms x 8 samples: window attention 115 us on CUDA cores (instruction-bound) -> 43 here, bias 36 us (shuffles) -> 10.
 #pragma once
 #include "elementwise.cuh"
 

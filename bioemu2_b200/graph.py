@@ -1,6 +1,6 @@
 """One CUDA-graph replay per forward for a trunk that is called again and again with tensors of one shape.
 
-A 48-block trunk is ~1,200 kernel launches; issued one by one from Python they cost a few milliseconds of host time
+A 48-block trunk is ~1,060 kernel launches; even enqueued by one native call they cost a few milliseconds of host time
 per forward that a serving loop does not need to pay.  ``trunk.graphed(s, z, mask)`` captures the block loop once on
 static device buffers; calling the result copies the new inputs into those buffers (from pinned host memory or from
 the device, asynchronously on the current stream), replays the graph and hands back the static output buffers, which

@@ -3,7 +3,8 @@
 ``fc3(silu(fc1(norm(x))) * fc2(norm(x)))``.  ``chunk_size`` exists in the reference to bound the
 memory of the hidden activations; the fused kernel never materialises them, so it is accepted and
 ignored.  The pair transition (dim 128, hidden up to 512) runs as one fused kernel; other widths (the single
-track: 384 -> 1536, 768 -> 4*768) run as LayerNorm, two tcgen05 GEMMs and a SwiGLU kernel.
+track: 384 -> 1536, 768 -> 4*768) run as LayerNorm and two tcgen05 GEMMs, the SwiGLU in the first one's epilogue where
+the hidden width is a multiple of 64 and as a kernel of its own otherwise.
 """
 from __future__ import annotations
 
