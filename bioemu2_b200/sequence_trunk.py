@@ -16,6 +16,7 @@ from torch import Tensor
 from . import functional as F
 from .pairmixer import PairMixerModule, PairMixerMSALayer
 from .transition import Transition
+from .triangle_multiplication import plain
 
 NUM_TOKENS = 33  # residue-token vocabulary of the reference (src/bioemu2/data_interface/const.py)
 
@@ -197,7 +198,8 @@ class PairMixerSequenceEmbedder(nn.Module):
         and a GEMM that adds ``x_init`` for the single track.  ``None``: the zeros of the first step, whose norm is the
         LayerNorm's bias in every row."""
         if x is None:
-            row = norm.bias.detach().to(torch.bfloat16).view(1, -1)
+            bias = norm.bias if norm.bias is not None else norm.weight.new_zeros(norm.normalized_shape)
+            row = bias.detach().to(torch.bfloat16).view(1, -1)
             return F.add_rows(x_init, F.linear_bf16(row, self._lin[name].weight(), out_dtype=torch.float32).view(-1))
         if x.shape[-1] == 128 and self._lin[name].linear.weight.shape == (128, 128):
             return F.ln_linear(x, None, norm.weight, norm.bias, self._lin[name].weight(), residual=x_init)
@@ -221,13 +223,15 @@ class PairMixerSequenceEmbedder(nn.Module):
         mask = feats["token_pad_mask"].bool()
         pair_mask = mask.unsqueeze(-1) & mask.unsqueeze(-2)
         # The MSA embedding is the same in every recycling step (the blocks leave their input alone).
-        m = self.msa_module.embed_msa(s_inputs, feats["msa"], feats["has_deletion"], feats["deletion_value"],
-                                      feats["msa_paired"])
+        once = {}
+        if plain(self.msa_module, PairMixerMSAModule):
+            once["embedded"] = self.msa_module.embed_msa(s_inputs, feats["msa"], feats["has_deletion"], feats["deletion_value"],
+                                                         feats["msa_paired"])
         s = z = None
         for _ in range(num_steps_recycle + 1):
             s = self._recycle(s, s_init, self.s_norm, "s_recycle")
             z = self._recycle(z, z_init, self.z_norm, "z_recycle")
             _, z = self.msa_module(None, z, s_inputs, feats["msa"], feats["msa_mask"], feats["has_deletion"],
-                                   feats["deletion_value"], feats["msa_paired"], feats["token_pad_mask"], embedded=m)
+                                   feats["deletion_value"], feats["msa_paired"], feats["token_pad_mask"], **once)
             s, z = self.pairmixer_module(s, z, pair_mask=pair_mask)
         return s, z

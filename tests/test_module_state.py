@@ -211,3 +211,36 @@ def test_msa_layer_runs_the_outer_product_mean_that_was_put_into_it(monkeypatch)
     z = torch.zeros(1, 4, 4, 128)
     _, got, _ = m(None, z, torch.zeros(1, 3, 4, 64), torch.ones(1, 4, 4), torch.ones(1, 3, 4))
     assert torch.equal(got, z + 10)
+
+
+@pytest.mark.parametrize("own", [False, True])
+def test_embedder_runs_the_msa_module_that_was_put_into_it(monkeypatch, own):
+    """The package's own module is handed the embedding of all recycling steps, another one the arguments it has always had."""
+    import bioemu2_b200 as b
+
+    calls, embedded = [], []
+
+    class Msa(torch.nn.Module):
+        def forward(self, s, z, emb, msa, msa_mask, has_deletion, deletion_value, msa_paired, token_pad_mask):
+            calls.append((msa, token_pad_mask))
+            return s, z
+
+    class Mixer(torch.nn.Module):
+        def forward(self, s, z, pair_mask):
+            return s, z
+
+    m = b.PairMixerSequenceEmbedder(64, 128, 16, msa_blocks=1, num_blocks=1).eval()
+    m.pairmixer_module = Mixer()
+    monkeypatch.setattr(m, "initial_embeddings", lambda s_inputs, feats: (torch.zeros(1, 4, 64), torch.zeros(1, 4, 4, 128)))
+    monkeypatch.setattr(m, "_recycle", lambda x, x_init, norm, name: x_init)
+    if own:
+        monkeypatch.setattr(m.msa_module, "embed_msa", lambda *args: embedded.append(args) or "m")
+        m.msa_module.layers = torch.nn.ModuleList([Msa()])
+        m.msa_module.layers[0].forward = lambda s, z, m, *args: calls.append(m) or (s, z, m)
+    else:
+        m.msa_module = Msa()
+    feats = {k: k for k in ("msa", "msa_mask", "has_deletion", "deletion_value", "msa_paired")}
+    feats["token_pad_mask"] = torch.ones(1, 4)
+    m(torch.zeros(1, 4, 16), feats, num_steps_recycle=2)
+    assert len(calls) == 3 and len(embedded) == own
+    assert calls == ["m"] * 3 if own else all(c[0] == "msa" and c[1] is feats["token_pad_mask"] for c in calls)
