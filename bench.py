@@ -672,7 +672,7 @@ def run_b200(args) -> None:
             kernel = "flash_resident_kernel<32,32,2>" if N <= 512 else "flash_core_kernel<32,2>"
             roofline = {
                 "kernel": kernel + " (triangle-attention core: QK^T + bias tile + online softmax + PV), "
-                          "launched alone on N rows x 4 heads x 32",
+                          "launched alone on N rows x 4 heads x 32, no key masked",
                 "bound": "tensor", "achieved": ach, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                 "frac": ach / pk["bf16_tflops"], "peak_source": pk["source"] + " burst (kernel timed alone)",
                 "algorithmic_flops_per_launch": core_flops, "algorithmic_bytes_per_launch": core_bytes,
@@ -683,7 +683,7 @@ def run_b200(args) -> None:
                 "traffic_source": "ncu capture at N=512 (672.3 MB read + 61.3 MB written); every operand once would be "
                                   "337.6 MB (four 67.1 MB operands read, one 67.1 MB result written, 2.1 MB of bias): K and "
                                   "V^T are read once per tile of 128 queries, four times each" if N == 512 else None,
-                "note": "head dim 32 makes the core ex2-bound, not tensor-bound: N^3*4 exponentials at 16/clk/SM "
+                "note": "at head dim 32 the exponentials, not the tensor work, set the floor: N^3*4 of them at 16/clk/SM "
                         f"take {ex2_floor_ms:.3f} ms at the sampled clock; the tensor work alone would take "
                         f"{core_flops / (pk['bf16_tflops'] * 1e12) * 1e3:.3f} ms" if ex2_floor_ms else "",
             }
