@@ -97,7 +97,7 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
         w_cond = pk.build(lin.weight.device).view(lin.weight.shape)
         b_cond = lin.bias.detach().float().contiguous()
         ln_w, ln_b = (None if p is None else p.detach().float().contiguous() for p in (ln.weight, ln.bias))
-        attn, tr = self._native_attention(), self.transition
+        attn, tr = self._native_attention(lambda m, cls: type(m) is cls), self.transition  # hooks may go again
         native = None
         if attn is not None and self.dim % 32 == 0 and lin.in_features % 8 == 0 and lin.in_features <= 1024 \
                 and not tr.use_norm and not attn.initial_norm and ln.eps == 1e-5 and tr.fc3.out_features == self.dim and (self._windowed or attn.c_z == 128):
@@ -118,14 +118,14 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
             native = (layer, (ap, tp, ln_w, ln_b))
         return w_cond, b_cond, native
 
-    def _native_attention(self):
+    def _native_attention(self, fits=plain):
         """The attention module whose weights the native call takes, if it may stand for the sub-modules as they are now."""
         attn = self.attention
         if self._windowed:
-            attn = attn.attention_layer if plain(attn, SlidingWindowAttentionLayer) else None
-        attn = attn.pair_bias_attn if plain(attn, AttentionLayer) else None
+            attn = attn.attention_layer if fits(attn, SlidingWindowAttentionLayer) else None
+        attn = attn.pair_bias_attn if fits(attn, AttentionLayer) else None
         own = AttentionPairBiasSlidingWindow if self._windowed else AttentionPairBias
-        return attn if plain(attn, own) and plain(self.transition, Transition) else None
+        return attn if fits(attn, own) and fits(self.transition, Transition) else None
 
     def forward(self, x: Tensor, pairs: Tensor, c: Tensor, mask: Tensor | None = None, multiplicity: int = 1) -> Tensor:
         if mask is None:  # full attention: pairs [B, T, T, .]; windowed: x [B*M, atoms, .]

@@ -193,6 +193,11 @@ def test_conditioned_layer_runs_the_modules_that_were_put_into_it(monkeypatch, w
         handle.remove()
         assert m(*args) == "one call"
     m = layer()
+    with m.transition.register_forward_hook(lambda *a: None):  # what is packed meanwhile serves both ways
+        monkeypatch.setattr(F, "_require_cuda", lambda *tensors: None)
+        monkeypatch.setattr(F._Pack, "build", lambda pk, device: torch.zeros(pk.size))
+        assert b.ConditionedTransformerLayer._build_packed(m)[2] is not None and m(*args) == "by modules"
+    m = layer()
     m.transition = _Adds()
     assert m(*args) == "by modules"
     m = layer()
