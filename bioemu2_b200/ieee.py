@@ -140,12 +140,13 @@ def transition(x: Tensor, norm, fc1, fc2, fc3, ws: SplitWeights, add_residual: b
 def triangle_multiplication(x: Tensor, mask: Tensor, mod, ws: SplitWeights, add_residual: bool = False,
                             out: Tensor | None = None) -> Tensor:
     """``out`` (fp32, contiguous): where the result goes; it may be ``x``."""
-    if x.ndim != 4 or x.shape[1] != x.shape[2] or x.shape[3] != 128:
-        raise ValueError(f"expected x[B,N,N,128], got {tuple(x.shape)}")
-    if mask.shape != x.shape[:3]:
-        raise ValueError(f"mask shape {tuple(mask.shape)} does not match x {tuple(x.shape)}")
+    shape = x.shape
+    if len(shape) != 4 or shape[1] != shape[2] or shape[3] != 128:
+        raise ValueError(f"expected x[B,N,N,128], got {tuple(shape)}")
+    if mask.shape != shape[:3]:
+        raise ValueError(f"mask shape {tuple(mask.shape)} does not match x {tuple(shape)}")
     F._require_cuda(x, mask)
-    B, N = x.shape[:2]
+    B, N = shape[0], shape[1]
     if out is not None and not (out.is_contiguous() and out.dtype == torch.float32):
         return out.copy_(triangle_multiplication(x, mask, mod, ws, add_residual))
     x, m8 = x.float().contiguous(), F.mask_u8(mask)
@@ -153,9 +154,10 @@ def triangle_multiplication(x: Tensor, mask: Tensor, mod, ws: SplitWeights, add_
         out = torch.empty_like(x)
     nbytes = lib.b200_accurate_trimul_workspace_bytes(N)
     buf, work = _workspace(nbytes, x.device)
+    xp, mp, op, pairs = x.data_ptr(), m8.data_ptr(), out.data_ptr(), N * N
     for b in range(B):
         _lib.check(lib.b200_accurate_trimul_fwd(
-            x[b].data_ptr(), m8[b].data_ptr(), out[b].data_ptr(), ws.w_in.data_ptr(), ws.w_p_out.data_ptr(),
+            xp + b * pairs * 512, mp + b * pairs, op + b * pairs * 512, ws.w_in.data_ptr(), ws.w_p_out.data_ptr(),
             ws.w_g_out.data_ptr(), ws.norm_in_w.data_ptr(), ws.norm_in_b.data_ptr(), ws.norm_out_w.data_ptr(),
             ws.norm_out_b.data_ptr(), N, 1 if mod.mode == "incoming" else 0, 1 if add_residual else 0, work, nbytes,
             _stream()))

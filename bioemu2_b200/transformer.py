@@ -120,12 +120,15 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
 
     def _native_attention(self, fits=plain):
         """The attention module whose weights the native call takes, if it may stand for the sub-modules as they are now."""
-        attn = self.attention
+        attn, own = self._modules["attention"], AttentionPairBias  # (on every pass: a module's own getattr is ten times a dict's)
         if self._windowed:
-            attn = attn.attention_layer if fits(attn, SlidingWindowAttentionLayer) else None
-        attn = attn.pair_bias_attn if fits(attn, AttentionLayer) else None
-        own = AttentionPairBiasSlidingWindow if self._windowed else AttentionPairBias
-        return attn if fits(attn, own) and fits(self.transition, Transition) else None
+            if not fits(attn, SlidingWindowAttentionLayer):
+                return None
+            attn, own = attn._modules["attention_layer"], AttentionPairBiasSlidingWindow
+        if not fits(attn, AttentionLayer):
+            return None
+        attn = attn._modules["pair_bias_attn"]
+        return attn if fits(attn, own) and fits(self._modules["transition"], Transition) else None
 
     def forward(self, x: Tensor, pairs: Tensor, c: Tensor, mask: Tensor | None = None, multiplicity: int = 1) -> Tensor:
         if mask is None:  # full attention: pairs [B, T, T, .]; windowed: x [B*M, atoms, .]
@@ -134,14 +137,16 @@ class ConditionedTransformerLayer(PackedWeightsMixin, nn.Module):
         native, attn = self.packed()[2], self._native_attention()
         if native is None or attn is None:
             return self._forward(x, pairs, c, mask, multiplicity, self.attention)
-        layer, B = native[0], pairs.shape[0]
-        if self._windowed and x.ndim == 3 and mask.numel() == B * x.shape[1]:
-            mask = mask.reshape(B, x.shape[1])  # it may come by query windows
-        if x.ndim != 3 or x.shape[0] != B * multiplicity or x.shape[2] != self.dim or tuple(mask.shape) != (B, x.shape[1]) \
-                or c.shape[-1] != layer.dim_cond or c.numel() != x.shape[0] * x.shape[1] * c.shape[-1]:
-            raise ValueError(f"x {tuple(x.shape)}, c {tuple(c.shape)}, pairs {tuple(pairs.shape)}, mask {tuple(mask.shape)}, "
+        layer, B, shape, mshape = native[0], pairs.shape[0], x.shape, mask.shape
+        N = shape[1] if len(shape) == 3 else -1
+        if self._windowed and mshape != (B, N) and mask.numel() == B * N:
+            mask = mask.reshape(B, N)  # it may come by query windows
+            mshape = mask.shape
+        if N < 0 or shape[0] != B * multiplicity or shape[2] != self.dim or mshape != (B, N) \
+                or c.shape[-1] != layer.dim_cond or c.numel() != shape[0] * N * layer.dim_cond:
+            raise ValueError(f"x {tuple(shape)}, c {tuple(c.shape)}, pairs {tuple(pairs.shape)}, mask {tuple(mshape)}, "
                              f"multiplicity={multiplicity}")
-        bias, N = None, x.shape[1]
+        bias = None
         if self._windowed:
             W, Hk = layer.window_queries, layer.window_keys
             if N % W:

@@ -19,7 +19,10 @@ from . import ieee, precision
 def plain(module, cls) -> bool:
     """Whether calling ``module`` does what ``cls`` does and nothing besides (no subclass, no hook, no forward of its own), so
     that a call which covers several modules may stand for it."""
-    return type(module) is cls and not module._forward_hooks and not module._forward_pre_hooks and "forward" not in module.__dict__
+    if type(module) is not cls:
+        return False
+    own = module.__dict__
+    return not own["_forward_hooks"] and not own["_forward_pre_hooks"] and "forward" not in own
 
 
 def _watch_list(module: nn.Module):
