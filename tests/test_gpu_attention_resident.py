@@ -63,3 +63,34 @@ def test_rows_that_start_low(rise_at, masked, dh):
     out = F.attention_core(q.cuda(), k.cuda(), v.cuda(), bias.cuda(), mask.cuda(), bias_div=lines)
     assert _lib.device_status() == 0
     assert_close(f"attention_core_low_{rise_at}_{masked}_dh{dh}", out, ref)
+
+
+@pytest.mark.parametrize("dh", [32, 48])
+@pytest.mark.parametrize("N", [1, 63, 65, 128, 150, 192, 203, 256, 449, 512, 700])
+@pytest.mark.parametrize("shift", [0.0, -90.0])
+def test_half_tiles_without_a_valid_key(N, shift, dh):
+    """Runs of masked keys that cover half tiles of 64 -- at the end, at the start, in the middle, everywhere -- with the rows'
+    reference at 0 and away from it.  Bound: P and V in bf16, 2^-9 each, as in the tests above."""
+    from bioemu2_b200 import _lib
+    from bioemu2_b200 import functional as F
+
+    g = torch.Generator().manual_seed(4000 + N)
+    lines, H = 7, 2
+    q, k, v = (torch.randn(lines, N, H, dh, generator=g).bfloat16() for _ in range(3))
+    bias = torch.randn(1, H, N, N, generator=g)
+    bias[:, :, ::3] += shift
+    mask = torch.ones(lines, N, dtype=torch.bool)
+    mask[0, N - N // 3:] = False            # padding
+    mask[1, :N // 2] = False                # nothing but masked keys at first, then valid ones
+    mask[2, N // 4:3 * N // 4] = False      # a hole
+    mask[3] = False
+    mask[4, 1:] = False                     # a single valid key
+    mask[5, :-1] = False
+    bias_bf = (bias * F.LOG2E).bfloat16().float() / F.LOG2E   # the kernel takes the bias in bf16, base 2
+    qs = (q.float() * (F.LOG2E / dh ** 0.5)).bfloat16().float() / F.LOG2E
+    logits = torch.einsum("bqhd,bkhd->bhqk", qs, k.float()) + bias_bf
+    logits = torch.where(mask[:, None, None, :], logits, torch.full_like(logits, -1e6))
+    ref = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(logits.double(), -1), v.double())
+    out = F.attention_core(q.cuda(), k.cuda(), v.cuda(), bias.cuda(), mask.cuda(), bias_div=lines)
+    assert _lib.device_status() == 0
+    assert_close(f"attention_core_runs_{N}_{shift}_dh{dh}", out, ref)
