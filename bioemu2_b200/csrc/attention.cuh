@@ -72,8 +72,8 @@ struct FlashCfg {
   static constexpr uint32_t K_OFF = 2 * G * Q_BYTES;
   static constexpr uint32_t V_OFF = K_OFF + K_STAGES * K_BYTES;
   static constexpr uint32_t BIAS_OFF = V_OFF + V_STAGES * V_BYTES;   // [G][2 slots] tiles x 32 KB
-  static constexpr uint32_t MASK_OFF = BIAS_OFF + 2 * G * kOperandTile;  // 2 x MAX_T x 8 words
-  static constexpr uint32_t XCH_OFF = MASK_OFF + 2 * MAX_T * 32;  // per group [tile parity][side][128] floats: row max exchange
+  static constexpr uint32_t MASK_OFF = BIAS_OFF + 2 * G * kOperandTile;  // 2 x MAX_T x 4 words
+  static constexpr uint32_t XCH_OFF = MASK_OFF + 2 * MAX_T * 16;  // per group [tile parity][side][128] floats: row max exchange
   // 16 x 16 identity (bf16) as an unswizzled K-major operand: two 16-byte K chunks of 16 rows each.
   static constexpr uint32_t IDENT_OFF = XCH_OFF + G * 2048;
   static constexpr uint32_t BAR_OFF = IDENT_OFF + 512;
@@ -122,9 +122,8 @@ flash_core_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint64_t* mask_full = bars + 30;    // [2] count 1 (mask warp)
   uint64_t* mask_empty = bars + 32;   // [2] count 256*G
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 34);
-  // Key-validity bits of a work item's mask row, two buffers of MAX_T x 8 words:
-  //   word t*8 + w      bit j <=> key t*128 + 32*w + j exists and is unmasked
-  //   word t*8 + 4 + w  bit j <=> key t*128 + 32*w + j exists
+  // Key-validity bits of a work item's mask row, two buffers of MAX_T x 4 words:
+  //   word t*4 + w      bit j <=> key t*128 + 32*w + j exists and is unmasked
   uint32_t* mask_bits = reinterpret_cast<uint32_t*>(smem + Cfg::MASK_OFF);
 
   const int warp = warp_index();
@@ -305,7 +304,7 @@ flash_core_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     for (int work = blockIdx.x; work < p.total_work; work += gridDim.x, ++w) {
       const int b = (work / p.nqg) / p.H;
       const uint8_t* mrow = p.mask + (long long)(b / p.mask_div) * p.mask_row_stride;
-      uint32_t* mb = mask_bits + (w & 1) * Cfg::MAX_T * 8;
+      uint32_t* mb = mask_bits + (w & 1) * Cfg::MAX_T * 4;
       mbar_wait(&mask_empty[w & 1], ((w >> 1) & 1) ^ 1, 74);
       for (int t = 0; t < T; ++t) {
         uint8_t mv[4];
@@ -316,13 +315,8 @@ flash_core_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const bool in = (t * 128 + u * 32 + lane) < p.N;
-          const uint32_t okb = __ballot_sync(0xffffffffu, in && mv[u] != 0);
-          const uint32_t inb = __ballot_sync(0xffffffffu, in);
-          if (lane == 0) {
-            mb[t * 8 + u] = okb;
-            mb[t * 8 + 4 + u] = inb;
-          }
+          const uint32_t okb = __ballot_sync(0xffffffffu, mv[u] != 0);
+          if (lane == 0) mb[t * 4 + u] = okb;
         }
       }
       __syncwarp();
