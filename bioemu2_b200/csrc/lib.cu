@@ -37,6 +37,47 @@ static int launch_window_attention(const WindowAttnParams& p, int BM, cudaStream
   return B200_OK;
 }
 
+// Whether window_pair_kernel takes these shapes: whole 16-query tiles, 128 keys, 16 pair channels, heads of 16 or 32 (with 64 it
+// spills 190 bytes) in boxes of 64 columns, two teams of warps within 512 threads and their K and V in shared memory; and the
+// windows in one wave of CTAs that have samples enough to pay for a bias phase of their own.  Three layers, heads 4 x 32, us as two
+// kernels / as one (windows x samples): 16 x 8 133 / 148, 32 x 4 135 / 147, 64 x 2 141 / 147, 32 x 6 156 / 157, 64 x 3 162 / 156,
+// 128 x 2 194 / 178, 128 x 8 425 / 384; 96 x 1 141 / 134, 148 x 1 161 / 143; 160 x 1 180 / 186, 160 x 4 340 / 361, 192 x 8 621 / 598.
+static bool window_pair_fits(const WindowAttnParams& p, int B, int head_dim, int c_z, const void* z) {
+  if ((head_dim != 16 && head_dim != 32) || p.W % 16 || p.W > p.Hk || p.Hk != kWindowMmaKeys || c_z != 16 || p.heads * (p.W / 16) > 8 ||
+      p.qkv_pitch % 8 || p.gate_pitch % 2 || p.heads * head_dim % 64 || !aligned(z, 32))
+    return false;
+  const int64_t windows = int64_t(B) * p.NW;
+  if (windows > sm_count() || (p.M == 1 ? windows < 96 : windows * p.M < 192)) return false;
+  const uint32_t smem = head_dim == 16 ? WindowPairCfg<16>::smem_bytes(p.heads, p.W) : WindowPairCfg<32>::smem_bytes(p.heads, p.W);
+  return smem <= 227 * 1024;
+}
+
+template <int DH>
+static int launch_window_pair(WindowPairParams p, int B, bool f32, cudaStream_t st) {
+  // A window's samples go to `chunks` CTAs, each of which computes the bias: as many as make the estimated time shortest (a wave's
+  // bias takes about as long as one and a half samples of a team).
+  const int windows = B * p.a.NW, most = (p.a.M + 1) / 2, sms = sm_count();
+  int64_t best = INT64_MAX;
+  p.chunks = 1;
+  for (int c = 1; c <= most; ++c) {
+    const int64_t waves = (int64_t(windows) * c + sms - 1) / sms, rounds = (p.a.M + 2 * c - 1) / (2 * c);
+    const int64_t cost = waves * (3 + 2 * rounds);
+    if (cost < best) best = cost, p.chunks = c;
+  }
+  CUtensorMap tmKV;
+  {
+    const uint64_t dims[3] = {uint64_t(3 * p.a.heads * DH), uint64_t(p.a.NW) * p.a.W, uint64_t(B) * p.a.M};
+    const uint64_t str[2] = {uint64_t(p.a.qkv_pitch) * 2, uint64_t(p.a.NW) * p.a.W * p.a.qkv_pitch * 2};
+    const uint32_t box[3] = {64, kWindowMmaKeys, 1};
+    if (int e = make_tmap_bf16(&tmKV, p.a.qkv, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+  }
+  const int threads = 2 * p.a.heads * (p.a.W / 16) * 32;
+  const uint32_t smem = WindowPairCfg<DH>::smem_bytes(p.a.heads, p.a.W);
+  if (f32) B200_LAUNCH((window_pair_kernel<true, DH>), windows * p.chunks, threads, smem, st, tmKV, p);
+  else B200_LAUNCH((window_pair_kernel<false, DH>), windows * p.chunks, threads, smem, st, tmKV, p);
+  return B200_OK;
+}
+
 static int grid_for(int64_t work_items, int per_block) {
   int64_t blocks = (work_items + per_block - 1) / per_block;
   const int64_t cap = int64_t(sm_count()) * 16;
@@ -1481,6 +1522,35 @@ static int window_attention_run(const void* qkv, int qkv_pitch, const void* gate
   return launch_window_attention<64>(p, B * M, st);
 }
 
+// The pair bias and the attention of all samples: one kernel where it serves the shapes, else by way of `bias`.
+static int window_pair_run(const void* qkv, int qkv_pitch, const void* gate, int gate_pitch, const void* z, const float* ln_w,
+                           const float* ln_b, const float* w_z, const uint8_t* mask, void* out, float* bias, int B, int M, int NW,
+                           int W, int Hk, int heads, int head_dim, int c_z, int z_dtype, cudaStream_t st) {
+  const WindowPairParams p{{static_cast<const __nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(gate), qkv_pitch, gate_pitch, nullptr,
+                            mask, static_cast<__nv_bfloat16*>(out), NW, W, Hk, heads, M, 1.0f / sqrtf(float(head_dim))},
+                           z, ln_w, ln_b, w_z, 1e-5f, 1};
+  const bool args = qkv && gate && z && ln_w && w_z && mask && out && B > 0 && M > 0 && NW > 0 && W > 0 && heads > 0 &&
+                    (z_dtype | 1) == 1 && aligned(qkv, 16) && aligned(gate, 16) && aligned(out, 16);
+  if (!args || !window_pair_fits(p.a, B, head_dim, c_z, z)) {  // the two calls check their arguments
+    if (int e = b200_window_bias_fwd(z, ln_w, ln_b, w_z, bias, int64_t(B) * NW, W, Hk, c_z, heads, z_dtype, st)) return e;
+    return window_attention_run(qkv, qkv_pitch, gate, gate_pitch, bias, mask, out, B, M, NW, W, Hk, heads, head_dim, st);
+  }
+  const bool f32 = z_dtype == B200_DTYPE_F32;
+  return head_dim == 16 ? launch_window_pair<16>(p, B, f32, st) : launch_window_pair<32>(p, B, f32, st);
+}
+
+int b200_window_pair_attention_fwd(const void* qkv, int qkv_pitch, const void* gate, int gate_pitch, const void* z,
+                                   const float* ln_w, const float* ln_b, const float* w_z, const uint8_t* mask, void* out,
+                                   float* bias, int B, int M, int NW, int W, int Hk, int heads, int head_dim, int c_z,
+                                   int z_dtype, b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(qkv_pitch >= 3 * heads * head_dim && gate_pitch >= heads * head_dim && qkv_pitch % 8 == 0 && gate_pitch % 8 == 0,
+                 "pitches must be multiples of 8 and hold a row");
+  B200_CHECK_ARG(bias, "bias is NULL");
+  return window_pair_run(qkv, qkv_pitch, gate, gate_pitch, z, ln_w, ln_b, w_z, mask, out, bias, B, M, NW, W, Hk, heads, head_dim,
+                         c_z, z_dtype, static_cast<cudaStream_t>(stream));
+}
+
 int b200_window_attention_fwd(const void* qkv, const void* gate, const float* bias, const uint8_t* mask, void* out, int B,
                               int M, int NW, int W, int Hk, int heads, int head_dim, b200_stream_t stream) {
   if (int e = b200_check_device()) return e;
@@ -2019,8 +2089,9 @@ int b200_cond_layer_fwd(const b200_cond_layer* l, const void* x, const void* pai
       a.bias = l->b_qkvg;
       if (int e = launch_bmm(a, stream)) return e;
     }
-    if (int e = b200_window_bias_fwd(pairs, l->ln_z_w, l->ln_z_b, l->w_z, wb, int64_t(l->B) * NW, W, Hk, l->dim_pairwise, l->heads, pairs_dtype, stream)) return e;
-    if (int e = window_attention_run(qkvg, 4 * D, qkvg + 3 * D, 4 * D, wb, mask, og, l->B, l->M, NW, W, Hk, l->heads, D / l->heads, stream)) return e;
+    if (int e = window_pair_run(qkvg, 4 * D, qkvg + 3 * D, 4 * D, pairs, l->ln_z_w, l->ln_z_b, l->w_z, mask, og, wb, l->B, l->M, NW, W, Hk,
+                                l->heads, D / l->heads, l->dim_pairwise, pairs_dtype, stream))
+      return e;
     BmmLaunch a{og, l->w_o, out, 1, int(rows), D, D, D, D, D, 0, 0, 0};
     a.residual = out;
     a.out_f32 = xf32;

@@ -12,6 +12,7 @@
 //                            bf16 values, so they keep 16 bits: against fp64 the kernel's error is that of the CUDA-core
 //                            one, whose weights are fp32 (1.658e-3 for both at head dims 32 and 64, 1.661e-3 at 16: it
 //                            is the rounding of the bf16 result)
+//   window_pair_kernel       the bias (c_z = 16) and window_mma_kernel's attention of all samples of a window in one CTA
 //   window_attention_kernel  other shapes: fp32 CUDA cores, one thread per (head, query)
 // 4,096 atoms x 8 samples: window attention 115 us on CUDA cores (instruction-bound) -> 43 here, bias 36 us (shuffles) -> 10.
 #pragma once
@@ -431,6 +432,312 @@ window_mma_kernel(WindowAttnParams p) {
       const float y0 = o[d][half * 2] * inv / (1.0f + __expf(-bf16lo(gv)));
       const float y1 = o[d][half * 2 + 1] * inv / (1.0f + __expf(-bf16hi(gv)));
       *reinterpret_cast<uint32_t*>(dst + d * 8) = pack_bf16x2(y0, y1);
+    }
+  }
+}
+
+
+// ---- the pair bias and all samples of a window in one kernel
+struct WindowPairParams {
+  WindowAttnParams a;  // a.bias unused
+  const void* z;       // [B][NW][W][128][16]
+  const float* ln_w;   // [16]
+  const float* ln_b;   // [16] or nullptr
+  const float* w_z;    // [heads][16]
+  float eps;
+  int chunks;          // CTAs of a window: each takes every chunks-th share of the samples
+};
+
+template <int DH>
+struct WindowPairCfg {
+  static constexpr int HK = kWindowMmaKeys;
+  static constexpr int BIAS_PITCH = HK + 8;  // floats: four rows of a fragment's 8-byte loads fall on different banks
+  // K or V of a window: boxes of 64 columns, [128 keys][128 B] each, swizzled as TMA writes them
+  __host__ __device__ static constexpr uint32_t kv_bytes(int heads) { return uint32_t(heads * DH / 64) * kOperandHalf; }
+  __host__ __device__ static constexpr uint32_t bias_bytes(int heads, int W) { return uint32_t(heads) * W * BIAS_PITCH * 4; }
+  __host__ __device__ static constexpr uint32_t smem_bytes(int heads, int W) {
+    return 4 * kv_bytes(heads) + bias_bytes(heads, W) + uint32_t(heads) * 17 * 4 + 64 + 1024;
+  }
+};
+
+// window_mma_kernel for pair tensors of 16 channels, with the bias projected here: a CTA owns a window, computes its bias once
+// into shared memory (fp32) and walks its samples.  Two teams of warps (a warp per head and 16 queries in each) take the samples
+// in turn, so that one team's loads run under the other's products; inside a team the next sample's K, queries and gate are
+// asked for as soon as the scores are done, its V^T after the weighted sum.
+// 4,096 atoms x 8 samples, 128 windows: 33 us, 11 of them the bias (its pair rows from DRAM, beside the write-back of what the
+// layer wrote before), 5 a pair of samples, which the two teams' issue slots bound.  As two kernels the bias went through global
+// memory and came back once per sample (64 KB a window, as much as K and V), and nothing covered a CTA's loads: 11.4 + 43 us.
+template <bool F32, int DH>
+__global__ void __launch_bounds__(512, 1)
+window_pair_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ WindowPairParams pp) {
+  using Cfg = WindowPairCfg<DH>;
+  constexpr int HK = Cfg::HK, BP = Cfg::BIAS_PITCH;
+  const WindowAttnParams& p = pp.a;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int c_s = p.heads * DH;
+  const uint32_t kv = Cfg::kv_bytes(p.heads);
+  float* bias = reinterpret_cast<float*>(smem + 4 * kv);
+  float* wz = bias + p.heads * p.W * BP;   // [heads][16] projection rows times the LayerNorm weight / score scale
+  float* wz0 = wz + p.heads * 16;          // [heads] what the LayerNorm bias adds
+  uint64_t* bars = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(wz0 + p.heads) + 7) & ~uintptr_t(7));
+  const int chunk = blockIdx.x % pp.chunks, bw = blockIdx.x / pp.chunks;
+  const int b = bw / p.NW, w = bw - b * p.NW;
+  const int L = p.NW * p.W;
+  const int a0 = w * p.W - (HK - p.W) / 2;  // atom index of key 0 (may be negative)
+  const int team_threads = blockDim.x >> 1;
+  const int team = threadIdx.x >= team_threads ? 1 : 0;
+  const int warp = (threadIdx.x - team * team_threads) >> 5, lane = threadIdx.x & 31;
+  uint8_t* Ks = smem + team * 2 * kv;
+  uint8_t* Vs = Ks + kv;
+  uint64_t* k_full = bars + team * 2;
+  uint64_t* v_full = k_full + 1;
+  const int step = 2 * pp.chunks;
+  const int m_first = chunk * 2 + team;
+  const bool loader = threadIdx.x == team * team_threads;  // the team's thread that issues its loads
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 4; ++i) mbar_init(&bars[i], 1);
+    fence_mbar_init();
+    prefetch_tmap(&tmKV);
+  }
+  __syncthreads();
+  pdl_wait();
+
+  auto load_rows = [&](uint8_t* dst, uint64_t* bar, int m, int col) {  // zero rows outside the sequence, as the zero-padded unfold gives
+    mbar_arrive_expect_tx(bar, kv);
+    for (int c = 0; c < c_s / 64; ++c) tma_load_3d(dst + c * kOperandHalf, &tmKV, bar, col + c * 64, a0, b * p.M + m);
+  };
+  const int tiles = p.W >> 4;
+  const int h = warp / tiles, q0 = (warp - h * tiles) * 16;
+  const int gr = lane >> 2, gc = (lane & 3) * 2;  // this lane's accumulator rows gr, gr + 8 and columns gc, gc + 1
+  uint32_t qf[DH / 16][4];
+  auto load_q = [&](int m) {  // fragments straight from global memory: rows gr / gr + 8, 16 dims per step
+    const __nv_bfloat16* r0 = p.qkv + ((long long)(b * p.M + m) * L + w * p.W + q0 + gr) * p.qkv_pitch + h * DH + gc;
+    const __nv_bfloat16* r1 = r0 + 8ll * p.qkv_pitch;
+#pragma unroll
+    for (int k = 0; k < DH / 16; ++k) {
+      qf[k][0] = *reinterpret_cast<const uint32_t*>(r0 + k * 16);
+      qf[k][1] = *reinterpret_cast<const uint32_t*>(r1 + k * 16);
+      qf[k][2] = *reinterpret_cast<const uint32_t*>(r0 + k * 16 + 8);
+      qf[k][3] = *reinterpret_cast<const uint32_t*>(r1 + k * 16 + 8);
+    }
+  };
+  if (loader && m_first < p.M) {  // the first sample's rows come while the bias is computed
+    load_rows(Ks, k_full, m_first, c_s);
+    load_rows(Vs, v_full, m_first, 2 * c_s);
+  }
+
+  // ---- bias, divided by the score scale: it is where the score accumulators start
+  if (threadIdx.x < p.heads * 16) {  // whole warps: the number of heads is even
+    const float wv = pp.w_z[threadIdx.x];
+    wz[threadIdx.x] = wv * pp.ln_w[lane & 15] / p.scale;
+    float t = pp.ln_b ? pp.ln_b[lane & 15] * wv : 0.f;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((lane & 15) == 0) wz0[threadIdx.x >> 4] = t / p.scale;
+  }
+  __syncthreads();
+  {
+    // Two pairs of a thread at a time, the next two on their way.
+    const int pairs = p.W * HK, stride = blockDim.x;
+    const uint8_t* zrow = static_cast<const uint8_t*>(pp.z) + (long long)bw * pairs * 16 * zbytes<F32>();
+    auto load = [&](int base, uint64_t (&x)[2][8]) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int ij = base + u * stride;
+        const uint8_t* row = zrow + (long long)(ij < pairs ? ij : 0) * 16 * zbytes<F32>();
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          float v[8];
+          load8<F32>(row, k * 8, v);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[u][k * 4 + e] = pack_f32x2(v[2 * e], v[2 * e + 1]);
+        }
+      }
+    };
+    auto project = [&](int base, uint64_t (&x)[2][8]) {
+      float rstd[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        uint64_t s[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[e] = add2(x[u][e], x[u][e + 4]);
+        float s0, s1;
+        unpack_f32x2(add2(add2(s[0], s[1]), add2(s[2], s[3])), s0, s1);
+        const float mean = (s0 + s1) * (-1.0f / 16);
+        const uint64_t mean2 = pack_f32x2(mean, mean);
+        uint64_t q[2] = {0, 0};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          x[u][e] = add2(x[u][e], mean2);
+          q[e & 1] = fma2(x[u][e], x[u][e], q[e & 1]);
+        }
+        unpack_f32x2(add2(q[0], q[1]), s0, s1);
+        rstd[u] = rsqrtf((s0 + s1) * (1.0f / 16) + pp.eps);
+      }
+      for (int hh = 0; hh < p.heads; hh += 2) {  // an even number: heads fill boxes of 64 columns
+        uint64_t acc[2][2] = {{0, 0}, {0, 0}};
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(wz + (hh + k) * 16 + e * 2);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) acc[k][u] = fma2(x[u][e + 1], wv.y, fma2(x[u][e], wv.x, acc[k][u]));
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int ij = base + u * stride;
+          float* dst = bias + (hh * p.W + ij / HK) * BP + ij % HK;
+          if (ij < pairs) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              float s0, s1;
+              unpack_f32x2(acc[k][u], s0, s1);
+              dst[k * p.W * BP] = fmaf(s0 + s1, rstd[u], wz0[hh + k]);
+            }
+          }
+        }
+      }
+    };
+    uint64_t xa[2][8], xb[2][8];
+    int base = threadIdx.x;
+    load(base, xa);
+    while (base < pairs) {
+      load(base + 2 * stride, xb);
+      project(base, xa);
+      base += 2 * stride;
+      if (base >= pairs) break;
+      load(base + 2 * stride, xa);
+      project(base, xb);
+      base += 2 * stride;
+    }
+  }
+  // validity of this lane's keys n * 8 + gc, n * 8 + gc + 1: bits 2n, 2n + 1
+  uint32_t ok = 0;
+#pragma unroll
+  for (int u = 0; u < HK / 32; ++u) {
+    const int a = a0 + u * 32 + lane;
+    const uint32_t word = __ballot_sync(0xffffffffu, a >= 0 && a < L && p.mask[(long long)b * L + a] != 0);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) ok |= ((word >> (n * 8 + gc)) & 3u) << (2 * (u * 4 + n));
+  }
+  const bool all_ok = __all_sync(0xffffffffu, ok == 0xffffffffu);
+  if (m_first < p.M) load_q(m_first);
+  __syncthreads();
+
+  const float c2 = p.scale * 1.4426950408889634f;  // to base-2 logits, in the exponent's multiply-add
+  const float masked = kWindowMasked / p.scale;
+  const int head_box = h * DH / 64, head_unit = (h * DH % 64) / 8;  // the head's 64-column box, its first 16-byte unit there
+  uint32_t phase = 0;
+  for (int m = m_first; m < p.M; m += step, phase ^= 1) {
+    const bool more = m + step < p.M;
+    float s[HK / 8][4];
+    const float* brow = bias + (h * p.W + q0 + gr) * BP + gc;
+#pragma unroll
+    for (int n = 0; n < HK / 8; ++n) {
+      const float2 b0 = *reinterpret_cast<const float2*>(brow + n * 8), b1 = *reinterpret_cast<const float2*>(brow + 8 * BP + n * 8);
+      s[n][0] = b0.x, s[n][1] = b0.y, s[n][2] = b1.x, s[n][3] = b1.y;
+    }
+    mbar_wait(k_full, phase, 82);
+    // scores: 16 queries x 128 keys
+#pragma unroll
+    for (int k = 0; k < DH / 16; ++k) {
+#pragma unroll
+      for (int n = 0; n < HK / 8; n += 2) {  // two 8-key tiles x 16 dims per load
+        uint32_t kf[4];
+        ldmatrix_x4(kf, Ks + head_box * kOperandHalf + sw128_offset(n * 8 + (lane & 7) + ((lane >> 4) << 3), head_unit + k * 2 + ((lane >> 3) & 1)));
+        mma_bf16(s[n], qf[k], kf[0], kf[1]);
+        mma_bf16(s[n + 1], qf[k], kf[2], kf[3]);
+      }
+    }
+    named_bar_sync(1 + team, team_threads);  // the team has read K
+    if (more) {
+      if (loader) load_rows(Ks, k_full, m + step, c_s);
+      load_q(m + step);
+    }
+    const long long atom = (long long)(b * p.M + m) * L + w * p.W + q0 + gr;
+    const __nv_bfloat16* gs = p.gate + atom * p.gate_pitch + h * DH + gc;
+    uint32_t gv[2][DH / 8];
+#pragma unroll
+    for (int d = 0; d < DH / 8; ++d) {
+      gv[0][d] = *reinterpret_cast<const uint32_t*>(gs + d * 8);
+      gv[1][d] = *reinterpret_cast<const uint32_t*>(gs + 8ll * p.gate_pitch + d * 8);
+    }
+    float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+    for (int n = 0; n < HK / 8; ++n) {
+      if (!all_ok) {
+        const bool ok0 = (ok >> (2 * n)) & 1u, ok1 = (ok >> (2 * n + 1)) & 1u;
+        s[n][0] = ok0 ? s[n][0] : masked;
+        s[n][1] = ok1 ? s[n][1] : masked;
+        s[n][2] = ok0 ? s[n][2] : masked;
+        s[n][3] = ok1 ? s[n][3] : masked;
+      }
+      m0 = max3(m0, s[n][0], s[n][1]);
+      m1 = max3(m1, s[n][2], s[n][3]);
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+      m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    }
+    mbar_wait(v_full, phase, 83);
+    const float n0 = -m0 * c2, n1 = -m1 * c2;
+    float l0 = 0.f, l1 = 0.f;
+    float o[DH / 8][4];
+#pragma unroll
+    for (int d = 0; d < DH / 8; ++d)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[d][e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < HK / 16; ++k) {  // 16 keys per step: the weights of two score tiles are the A operand
+      float e[8];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        e[u * 4 + 0] = exp2_approx(fmaf(s[2 * k + u][0], c2, n0));
+        e[u * 4 + 1] = exp2_approx(fmaf(s[2 * k + u][1], c2, n0));
+        e[u * 4 + 2] = exp2_approx(fmaf(s[2 * k + u][2], c2, n1));
+        e[u * 4 + 3] = exp2_approx(fmaf(s[2 * k + u][3], c2, n1));
+        l0 += e[u * 4 + 0] + e[u * 4 + 1];
+        l1 += e[u * 4 + 2] + e[u * 4 + 3];
+      }
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {  // register u: (row gr | gr + 8) of the first, then of the second tile
+        const float x0 = e[u * 2], x1 = e[u * 2 + 1];
+        hi[u] = pack_bf16x2(x0, x1);
+        lo[u] = pack_bf16x2(x0 - bf16lo(hi[u]), x1 - bf16hi(hi[u]));
+      }
+#pragma unroll
+      for (int d = 0; d < DH / 8; d += 2) {  // 16 keys x two 8-dim tiles per load
+        uint32_t vf[4];
+        ldmatrix_x4_trans(vf, Vs + head_box * kOperandHalf + sw128_offset(k * 16 + (lane & 15), head_unit + d + (lane >> 4)));
+        mma_bf16(o[d], hi, vf[0], vf[1]);
+        mma_bf16(o[d + 1], hi, vf[2], vf[3]);
+        mma_bf16(o[d], lo, vf[0], vf[1]);
+        mma_bf16(o[d + 1], lo, vf[2], vf[3]);
+      }
+    }
+    named_bar_sync(1 + team, team_threads);  // the team has read V
+    if (more && loader) load_rows(Vs, v_full, m + step, 2 * c_s);
+#pragma unroll
+    for (int x = 1; x < 4; x <<= 1) {
+      l0 += __shfl_xor_sync(0xffffffffu, l0, x);
+      l1 += __shfl_xor_sync(0xffffffffu, l1, x);
+    }
+    const float i0 = 1.0f / l0, i1 = 1.0f / l1;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      __nv_bfloat16* dst = p.out + (atom + half * 8) * c_s + h * DH + gc;
+      const float inv = half ? i1 : i0;
+#pragma unroll
+      for (int d = 0; d < DH / 8; ++d) {
+        const float y0 = __fdividef(o[d][half * 2] * inv, 1.0f + __expf(-bf16lo(gv[half][d])));
+        const float y1 = __fdividef(o[d][half * 2 + 1] * inv, 1.0f + __expf(-bf16hi(gv[half][d])));
+        *reinterpret_cast<uint32_t*>(dst + d * 8) = pack_bf16x2(y0, y1);
+      }
     }
   }
 }

@@ -593,13 +593,12 @@ def window_attention_pair_bias(s: Tensor, z: Tensor, mask: Tensor, w: WindowApbP
     qkvg = linear_bf16(sn, w.w_qkvg, bias_f32=w.b_qkvg)
     z = z.contiguous()
     bias = torch.empty(B, NW, w.H, W, Hk, dtype=torch.float32, device=s.device)
-    _lib.check(lib.b200_window_bias_fwd(z.data_ptr(), w.ln_z_w.data_ptr(), _ptr(w.ln_z_b), w.w_z.data_ptr(), bias.data_ptr(),
-                                        B * NW, W, Hk, c_z, w.H, _zdtype(z), _stream()))
     og = torch.empty(folded, W, c_s, dtype=torch.bfloat16, device=s.device)
     m8 = mask_u8(mask).contiguous()
-    _lib.check(lib.b200_window_attention_pitched_fwd(qkvg.data_ptr(), 4 * c_s, qkvg.data_ptr() + 6 * c_s, 4 * c_s,
-                                                     bias.data_ptr(), m8.data_ptr(), og.data_ptr(), B, M, NW, W, Hk, w.H, w.dh,
-                                                     _stream()))
+    _lib.check(lib.b200_window_pair_attention_fwd(qkvg.data_ptr(), 4 * c_s, qkvg.data_ptr() + 6 * c_s, 4 * c_s, z.data_ptr(),
+                                                  w.ln_z_w.data_ptr(), _ptr(w.ln_z_b), w.w_z.data_ptr(), m8.data_ptr(),
+                                                  og.data_ptr(), bias.data_ptr(), B, M, NW, W, Hk, w.H, w.dh, c_z, _zdtype(z),
+                                                  _stream()))
     return linear_bf16(og, w.w_o, out_dtype=s.dtype)
 
 

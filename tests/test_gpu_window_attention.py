@@ -39,6 +39,11 @@ def test_window_attention_golden(name):
     (1, 1, 5, 32, 128, 64, 16, 4, torch.float32),      # head dim 16
     (1, 2, 4, 32, 128, 128, 24, 2, torch.bfloat16),    # head dim 64, bf16 streams
     (1, 2, 9, 16, 48, 128, 16, 4, torch.float32),      # other window sizes
+    (2, 3, 48, 32, 128, 128, 16, 4, torch.float32),    # bias and samples in one kernel: odd and even numbers of samples,
+    (1, 4, 64, 32, 128, 128, 16, 4, torch.bfloat16),   # several CTAs a window, a team without a sample, head dim 16,
+    (1, 1, 96, 32, 128, 128, 16, 4, torch.float32),    # the last window of a wave, four heads on 16-query windows
+    (1, 9, 22, 32, 128, 64, 16, 4, torch.float32),
+    (1, 2, 148, 16, 128, 64, 16, 2, torch.bfloat16),
 ])
 def test_window_attention_vs_oracle(B, M, NW, W, Hk, c_s, c_z, heads, dtype):
     g = torch.Generator().manual_seed(1000 + NW * W + c_s)
