@@ -170,6 +170,8 @@ SIGNATURES = {
     "b200_add_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_void_p]),
     "b200_ln_linear_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int,
                                    c_void_p]),
+    "b200_pair_cond_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int,
+                                   c_void_p]),
     "b200_swiglu_transition_workspace_bytes": (c_size_t, [c_int64, c_int, c_int64]),
     "b200_swiglu_transition_fwd": (c_int, [c_void_p, c_void_p, POINTER(SwigluWeights), c_int64, c_int, c_int, c_int, c_int,
                                            c_void_p, c_size_t, c_void_p]),

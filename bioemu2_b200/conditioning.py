@@ -2,9 +2,10 @@
 (src/bioemu2/biomoa/modules/diffusion.py:464-534).
 
 ``z = Linear(LayerNorm(cat(z_trunk, token_rel_pos_feats)))`` followed by ``z = Transition(z) + z`` per transition.
-No pair talks to another pair: the module is three HBM-bound passes over the pair tensor.  At the model's widths (128 + 128
--> 128) LayerNorm and projection are one kernel (``F.ln_linear``); otherwise the LayerNorm kernel reads the two sources
-without materialising the concatenation and a tcgen05 GEMM follows.  Every transition adds its residual in its final store.
+No pair talks to another pair: at the model's widths (128 + 128 -> 128, hidden 256) the module is one pass over the pair tensor
+(``F.pair_cond``).  Otherwise LayerNorm and projection are one kernel at 128 channels (``F.ln_linear``) or the LayerNorm kernel
+reads the two sources without materialising the concatenation and a tcgen05 GEMM follows, and every transition adds its residual
+in its final store.
 """
 from __future__ import annotations
 
@@ -13,10 +14,12 @@ import torch.nn as nn
 from torch import Tensor
 
 from . import functional as F
+from . import precision
 from .transition import Transition
+from .triangle_multiplication import PackedWeightsMixin
 
 
-class PairwiseConditioning(nn.Module):
+class PairwiseConditioning(PackedWeightsMixin, nn.Module):
     def __init__(self, token_z: int, dim_token_rel_pos_feats: int, a_z: int | None = None, num_transitions: int = 2,
                  transition_expansion_factor: int = 2, transition_chunk_size: int | None = None) -> None:
         super().__init__()
@@ -41,6 +44,17 @@ class PairwiseConditioning(nn.Module):
             self._w_version = w._version
         return self._w_bf16
 
+    def _build_packed(self):
+        ln, proj = self.dim_pairwise_init_proj
+        return F.PairCondPacked(ln.weight, ln.bias, proj.weight, [
+            (t.norm.weight, t.norm.bias, t.fc1.weight, t.fc2.weight, t.fc3.weight) for t in self.transitions])
+
+    @staticmethod
+    def _native(t) -> bool:
+        """Whether the one-pass call covers a transition: 256 hidden units or less, a LayerNorm, not the accurate form (z is fp32)."""
+        return type(t) is Transition and t._fused and t.use_norm and t.hidden <= 256 and t.norm.bias is not None and \
+            not precision.use_ieee(None)
+
     def forward(self, z_trunk: Tensor, token_rel_pos_feats: Tensor) -> Tensor:
         """``z_trunk[B, N, N, token_z]``, ``token_rel_pos_feats[B, N, N, rel]`` -> fp32 ``[B, N, N, a_z]``."""
         if self.training:
@@ -53,7 +67,10 @@ class PairwiseConditioning(nn.Module):
         if token_rel_pos_feats.dtype != z_trunk.dtype:
             token_rel_pos_feats = token_rel_pos_feats.to(z_trunk.dtype)
         ln = self.dim_pairwise_init_proj[0]
-        if self.token_z == self.dim_token_rel_pos_feats == self.a_z == 128:
+        at_128 = self.token_z == self.dim_token_rel_pos_feats == self.a_z == 128
+        if at_128 and len(self.transitions) in (1, 2) and ln.bias is not None and all(self._native(t) for t in self.transitions):
+            return F.pair_cond(z_trunk, token_rel_pos_feats, self.packed())
+        if at_128:
             z = F.ln_linear(z_trunk, token_rel_pos_feats, ln.weight, ln.bias, self._weight())
         else:
             zn = F.rows2_to_bf16(z_trunk, token_rel_pos_feats, ln.weight, ln.bias)

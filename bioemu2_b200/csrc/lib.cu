@@ -11,6 +11,7 @@
 #include "trimul.cuh"
 #include "transition.cuh"
 #include "ln_linear.cuh"
+#include "pair_cond.cuh"
 #include "elementwise.cuh"
 #include "accurate.cuh"
 #include "opm.cuh"
@@ -859,6 +860,54 @@ int b200_ln_linear_fwd(const void* x1, const void* x2, const float* ln_w, const 
   const bool f32 = x_dtype == B200_DTYPE_F32;
   if (x2) return f32 ? launch_ln_linear<true, 2>(p, w, out, st) : launch_ln_linear<false, 2>(p, w, out, st);
   return f32 ? launch_ln_linear<true, 1>(p, w, out, st) : launch_ln_linear<false, 1>(p, w, out, st);
+}
+
+int b200_pair_cond_fwd(const void* x1, const void* x2, const float* ln_w, const float* ln_b, const void* w,
+                       const b200_transition_weights* transitions, int n_transitions, float* out, int64_t rows, int x_dtype,
+                       b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(x1 && x2 && w && transitions && out, "x1/x2/w/transitions/out is NULL");
+  B200_CHECK_ARG(n_transitions > 0 && n_transitions <= kPairCondMaxTransitions, "n_transitions=%d must be 1..%d", n_transitions,
+                 kPairCondMaxTransitions);
+  B200_CHECK_ARG(rows >= 0 && rows < (int64_t(1) << 31), "rows out of range");
+  B200_CHECK_ARG((x_dtype | 1) == 1, "unknown dtype");
+  B200_CHECK_ARG(aligned(x1, 32) && aligned(x2, 32) && aligned(w, 16) && aligned(out, 32),
+                 "x1/x2/out must be 32-byte aligned, w 16-byte aligned");
+  for (int t = 0; t < n_transitions; ++t) {
+    const b200_transition_weights& tw = transitions[t];
+    B200_CHECK_ARG(tw.hidden == 256 && tw.w13 && tw.w3 && aligned(tw.w13, 16) && aligned(tw.w3, 16), "transition %d: bad weights", t);
+    B200_CHECK_ARG(tw.ln_w && tw.ln_b, "transition %d: bad LayerNorm", t);
+  }
+  if (rows == 0) return B200_OK;
+  PairCondMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  PairCondParams p{x1, x2, ln_w, ln_b, {}, {}, rows, int((rows + 127) / 128), n_transitions, 1e-5f};
+  {
+    const uint64_t dims[2] = {256, 128};
+    const uint64_t str[1] = {512};
+    const uint32_t box[2] = {64, 128};
+    if (int e = make_tmap_bf16(&maps.w0, w, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+  }
+  for (int t = 0; t < n_transitions; ++t) {
+    const uint64_t dims13[2] = {128, 512}, dims3[2] = {256, 128};
+    const uint64_t str13[1] = {256}, str3[1] = {512};
+    const uint32_t box[2] = {64, 128};
+    if (int e = make_tmap_bf16(&maps.w13[t], transitions[t].w13, 2, dims13, str13, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+    if (int e = make_tmap_bf16(&maps.w3[t], transitions[t].w3, 2, dims3, str3, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+    p.t_ln_w[t] = transitions[t].ln_w;
+    p.t_ln_b[t] = transitions[t].ln_b;
+  }
+  {
+    const uint64_t dims[2] = {uint64_t(kD), uint64_t(rows)};
+    const uint64_t str[1] = {uint64_t(kD) * 4};
+    const uint32_t box[2] = {32, 128};
+    if (int e = make_tmap(&maps.out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+  }
+  const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (x_dtype == B200_DTYPE_F32) B200_LAUNCH(pair_cond_kernel<true>, grid, pair_cond::THREADS, pair_cond::SMEM_BYTES, st, maps, p);
+  else B200_LAUNCH(pair_cond_kernel<false>, grid, pair_cond::THREADS, pair_cond::SMEM_BYTES, st, maps, p);
+  return B200_OK;
 }
 
 // ------------------------------------------------------------------------------------------------ no-allocation variant

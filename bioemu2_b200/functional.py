@@ -219,6 +219,17 @@ class TransitionPacked:
             raise ValueError("the fused pair-transition kernel is built for dim=128, hidden<=512")
         width = self.hidden = 256 if hidden <= 256 else 512
         pk = _Pack()
+        self.add(pk, fc1, fc2, fc3, width)
+        buf = pk.build(fc3.device)
+        self.w13, self.w3 = buf[:2 * width * 128].view(-1, 128), buf[2 * width * 128:].view(128, width)
+        self.norm_w = norm_w.detach().float().contiguous() if norm_w is not None else None
+        self.norm_b = norm_b.detach().float().contiguous() if norm_b is not None else None
+        self.struct = _lib.TransitionWeights(self.w13.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b),
+                                             width)
+
+    @staticmethod
+    def add(pk: _Pack, fc1, fc2, fc3, width: int) -> int:
+        hidden, off = fc1.shape[0], pk.size
         if hidden == width:  # chunks of [64 fc1 rows | 64 fc2 rows]
             pk.interleave((fc1, fc2), groups=width // 64)
         else:
@@ -230,12 +241,7 @@ class TransitionPacked:
                     else:
                         pk.add(None, count=64 * 128)
         pk.add(fc3, groups=128, pad_to=width)
-        buf = pk.build(fc3.device)
-        self.w13, self.w3 = buf[:2 * width * 128].view(-1, 128), buf[2 * width * 128:].view(128, width)
-        self.norm_w = norm_w.detach().float().contiguous() if norm_w is not None else None
-        self.norm_b = norm_b.detach().float().contiguous() if norm_b is not None else None
-        self.struct = _lib.TransitionWeights(self.w13.data_ptr(), self.w3.data_ptr(), _ptr(self.norm_w), _ptr(self.norm_b),
-                                             width)
+        return off
 
 
 def transition(x: Tensor, w: TransitionPacked, add_residual: bool = False, out: Tensor | None = None) -> Tensor:
@@ -511,6 +517,35 @@ def ln_linear(x1: Tensor, x2: Tensor | None, weight: Tensor | None, bias: Tensor
     b = bias.detach().float().contiguous() if bias is not None else None
     _lib.check(lib.b200_ln_linear_fwd(x1.data_ptr(), _ptr(x2), _ptr(w), _ptr(b), w_bf16.data_ptr(), _ptr(residual),
                                       out.data_ptr(), x1.numel() // 128, _zdtype(x1), _stream()))
+    return out
+
+
+class PairCondPacked:
+    """Weights of the pairwise conditioning as ``b200_pair_cond_fwd`` takes them, packed by one launch: 128 + 128 -> 128 channels,
+    transitions (norm weight, norm bias, fc1, fc2, fc3) of up to 256 hidden units."""
+
+    def __init__(self, norm_w, norm_b, w, transitions):
+        pk = _Pack()
+        pk.add(w)
+        offs = [TransitionPacked.add(pk, *t[2:], 256) for t in transitions]
+        self.buf = pk.build(w.device)
+        self.norms = [t.detach().float().contiguous() for t in (norm_w, norm_b, *(n for t in transitions for n in t[:2]))]
+        base = self.buf.data_ptr()
+        ptrs = [t.data_ptr() for t in self.norms]
+        self.args = ptrs[0], ptrs[1], base, (_lib.TransitionWeights * len(transitions))(
+            *((base + 2 * o, base + 2 * (o + 512 * 128), ptrs[2 + 2 * k], ptrs[3 + 2 * k], 256) for k, o in enumerate(offs))), len(offs)
+
+
+def pair_cond(x1: Tensor, x2: Tensor, w: PairCondPacked) -> Tensor:
+    """``z = LayerNorm(cat(x1, x2)) @ w.T`` and ``z += transition(z)`` for one or two transitions, as fp32, in one pass."""
+    _require_cuda(x1, x2)
+    x1, x2 = x1.contiguous(), x2.contiguous()
+    if x1.shape[-1] != 128 or x2.shape != x1.shape or x2.dtype != x1.dtype:
+        raise ValueError("pair_cond takes two sources of 128 channels and one type")
+    out = torch.empty(x1.shape, dtype=torch.float32, device=x1.device)
+    if out.numel() == 0:
+        return out
+    _lib.check(lib.b200_pair_cond_fwd(x1.data_ptr(), x2.data_ptr(), *w.args, out.data_ptr(), x1.numel() // 128, _zdtype(x1), _stream()))
     return out
 
 

@@ -547,6 +547,13 @@ typedef struct {
   int64_t hidden;
 } b200_transition_weights;
 
+/* The pairwise conditioning in one call: out[rows][128] (fp32) = W . LayerNorm(x1 | x2), then out += transition(out) for each of
+ * one or two transitions of 256 hidden units with a LayerNorm (their out is b200_transition_hidden_fwd's).  x1 / x2 and W as in
+ * b200_ln_linear_fwd. */
+int b200_pair_cond_fwd(const void* x1, const void* x2, const float* ln_w, const float* ln_b, const void* w,
+                       const b200_transition_weights* transitions, int n_transitions, float* out, int64_t rows, int x_dtype,
+                       b200_stream_t stream);
+
 typedef struct {
   const void* w12;
   const void* w3;

@@ -91,6 +91,31 @@ def test_pairwise_conditioning_vs_oracle(N):
     assert_close(f"pairwise_conditioning_N{N}", out, ref, atol=4e-2)
 
 
+@pytest.mark.parametrize("B,n_i,n_j,transitions,factor,dtype", [
+    (1, 1, 1, 2, 2, torch.float32),       # a single row
+    (1, 8, 16, 1, 2, torch.float32),      # one whole tile, one transition
+    (2, 9, 15, 2, 2, torch.bfloat16),     # a tile and a part of one
+    (1, 160, 148, 2, 2, torch.bfloat16),  # a second tile for some CTAs
+    (1, 290, 131, 2, 1, torch.float32),   # three tiles a CTA, hidden padded to 256
+    (1, 12, 12, 2, 4, torch.float32),     # hidden 512 and three transitions: the passes one by one
+    (1, 12, 12, 3, 2, torch.float32),
+])
+def test_pairwise_conditioning_shapes(B, n_i, n_j, transitions, factor, dtype):
+    import bioemu2_b200 as b
+    from bioemu2_b200 import _lib
+
+    g = torch.Generator().manual_seed(915 + n_i)
+    w = H.pairwise_conditioning_weights(g, num_transitions=transitions, factor=factor)
+    z, rel = (torch.randn(B, n_i, n_j, 128, generator=g).to(dtype) for _ in range(2))
+    ref = O.pairwise_conditioning(z.double(), rel.double(), {k: v.double() for k, v in w.items()}, transitions)
+    m = b.PairwiseConditioning(128, 128, num_transitions=transitions, transition_expansion_factor=factor).eval()
+    m.load_state_dict(w, strict=True)
+    with torch.no_grad():
+        out = m.cuda()(z.cuda(), rel.cuda())
+    assert _lib.device_status() == 0 and out.dtype == torch.float32
+    assert_close(f"pairwise_conditioning_{B}x{n_i}x{n_j}_{transitions}_{factor}_{dtype}", out, ref, atol=4e-2)
+
+
 # ------------------------------------------------------------------------------------------ MSA module, trunk
 def test_msa_module_golden():
     import bioemu2_b200 as b
