@@ -62,13 +62,13 @@ enum BmmEpilogue : int {
   kEpiMul = 2,
   kEpiAdd = 6,     // the same with fp32 addends: a residual that is not C itself
   kEpiSwiglu = 3,  // bulk bf16: the columns are pairs of 64-column blocks (a | b), C gets silu(a) * b, half as many columns
-  kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b, with expf and exact division
+  kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b
   // kEpiBulk with eight epilogue warps, each group of four draining half of the tile's columns: a short product's tile is
   // its epilogue (K = 128: 2 K blocks of 64 against 128 columns of TMEM reads, staging and stores a lane).
   kEpiBulkWide = 7,
   // Gated operands of the accurate triangle contraction, from split operands: the weights' 256 rows are p and g of 128
   // channels and take the M side, so a lane is a channel and its columns are consecutive pairs -- the order in which the
-  // contraction reads them.  C gets hi and lo of p * sigmoid(g) (expf, exact division; masked pairs zero) as rows part *
+  // contraction reads them.  C gets hi and lo of p * sigmoid(g) (masked pairs zero) as rows part *
   // 128 + channel of column tile tn.  (Projection to fp32 and a gate kernel over it: 26 + 33 us for 40000 pairs.)
   kEpiGateSplit = 8,
   kEpiOuter = 5,   // outer products of 32 x 32, one pair's 2 KB in one piece
@@ -96,7 +96,7 @@ struct BmmCfg {
   static constexpr uint32_t OUT_OFFSET = BAR_OFFSET + 2048;        // [128 rows][128 B] tiles for bulk output
   static constexpr int OUT_TILES = kTwoGroups<EPI> ? 4 : 2;
   static constexpr uint32_t SMEM_BYTES = OUT_OFFSET + OUT_TILES * 16384 + 1024;  // + alignment slack
-  // The split SwiGLU's expf and division keep four warps busy for longer than the product (40000 x 1024 x 384: 105 us): it
+  // The split SwiGLU's arithmetic keeps four warps busy for longer than the product (40000 x 1024 x 384: 105 us): it
   // has eight, each group of four with one of the tile's two 64-column groups.
   static constexpr int EPI_THREADS = kTwoGroups<EPI> ? 256 : 128;
   static constexpr int GROUPS = EPI_THREADS / 128;
@@ -326,7 +326,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
 #pragma unroll
           for (int e = 0; e < 32; ++e) {
             const float a = __uint_as_float(va[e]);
-            va[e] = __float_as_uint(a / (1.f + expf(-a)) * __uint_as_float(vb[e]));
+            va[e] = __float_as_uint(times_sigmoid(a, a) * __uint_as_float(vb[e]));
           }
           if (c == 0) {
             if (leader) tma_store_wait_read0();  // the stores that last used the staging tiles have read them
@@ -371,7 +371,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           }
 #pragma unroll
           for (int e = 0; e < 32; ++e)
-            va[e] = (keep[c] >> e) & 1 ? __float_as_uint(__uint_as_float(va[e]) / (1.f + expf(-__uint_as_float(vb[e])))) : 0u;
+            va[e] = (keep[c] >> e) & 1 ? __float_as_uint(times_sigmoid(__uint_as_float(va[e]), __uint_as_float(vb[e]))) : 0u;
           if (c == 0) {
             if (leader) tma_store_wait_read0();  // the stores that last used the staging tiles have read them
             named_bar_sync(1 + grp, 128);

@@ -429,6 +429,10 @@ __device__ __forceinline__ float exp2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// num * sigmoid(x) = num / (1 + 2^(-x log2 e)) for the fp32-accurate forms: hardware exponential and reciprocal, about 2^-21
+// relative each, where the split operands around it carry 2^-16 (with expf and exact division, some twenty instructions more per
+// element, the two products of 40000 rows that have it in their epilogue take 63 and 37 us instead of 39 and 26).
+__device__ __forceinline__ float times_sigmoid(float num, float x) { return __fdividef(num, 1.0f + exp2_approx(-1.4426950408889634f * x)); }
 // Packed fp32 pair add (one FMA-pipe instruction for two lanes' worth of values) and three-input maximum.
 __device__ __forceinline__ void add_f32x2(float& a0, float& a1, float b0, float b1) {
   asm("{ .reg .b64 ra, rb; mov.b64 ra, {%0, %1}; mov.b64 rb, {%2, %3}; add.rn.f32x2 ra, ra, rb; mov.b64 {%0, %1}, ra; }"
