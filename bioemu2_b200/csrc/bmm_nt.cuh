@@ -28,11 +28,8 @@ struct BmmParams {
   // Outer-product store: with opm_ntok > 0, C row r = (i, c) and column q = (j, d) (c, d < 32) go to
   // C[((i * opm_ntok + j) * 32 + c) * 32 + d]: every pair (i, j) gets its 32x32 outer product contiguous.
   int opm_ntok;
-  // Residual and transposed pair store (output projection of triangle attention): with residual != nullptr
-  // the value read from it at the destination offset is added; with remap_n > 0 row r = line * remap_n + pos
-  // (line < remap_m) is stored as row pos * remap_m + line.
+  // With residual != nullptr the value read from it at the destination offset is added.
   const void* residual;
-  int remap_n, remap_m;
   // Bulk output: the scaled (+ bias) tile leaves through 16 KB staging tiles ([128 rows][128 B]: 32 fp32 or 64
   // bf16 columns) and the C tensor map, 1 = stored, 2 = added into C (the residual is C itself, which the
   // epilogue then never reads), 3 = stored with the rows as groups of 32, {column, row in group, group, batch}.
@@ -48,7 +45,7 @@ struct BmmParams {
   const uint8_t* mask;
   int mask_pitch, mask_n;
   long long mask_line, mask_pos;
-  int a_shared;              // 1: every batch item multiplies the same A (the A tensor map has a single batch slice)
+  int a_shared, b_shared;    // 1: every batch item multiplies the same A / B (its tensor map has a single batch slice)
 };
 
 // The epilogues are separate instantiations: with all of them in one kernel the plain one, which triangle multiplication's
@@ -160,7 +157,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           mbar_arrive_expect_tx(&full[stage], Cfg::STAGE_BYTES);
           int ka = kb < p.a_fold ? kb : kb - p.a_fold, kbb = kb < p.b_fold ? kb : kb - p.b_fold;
-          int ab = p.a_shared ? 0 : b, bb = b;
+          int ab = p.a_shared ? 0 : b, bb = p.b_shared ? 0 : b;
           if (p.part_blocks > 0) {
             const int part = kb / p.part_blocks;
             ka = kbb = kb - part * p.part_blocks;
@@ -400,11 +397,7 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         // 32 columns at a time into one of two swizzled staging tiles; warp 2's first lane sends each tile off.
         const int r = quarter * 32 + lane;
         const bool leader = (threadIdx.x & 127) == 64;
-        int c1 = tm * 128, c2 = b;  // tensor map {column, row, batch}, or {column, line, pos} when remapped
-        if (p.remap_n > 0) {
-          c1 = (tm * 128) / p.remap_n;
-          c2 = tm * 128 - c1 * p.remap_n;
-        }
+        const int c1 = tm * 128, c2 = b;  // tensor map {column, row, batch}
         const int cps = p.out_f32 ? 1 : 2;  // 32-column chunks per staging tile
         uint32_t va[32], vb[32];
         constexpr int CHUNKS = GCOLS / 32;
@@ -547,7 +540,6 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
                                         : nullptr;
       auto chunk_off = [&](int c) -> long long {  // element offset of (row, first column of chunk c)
         const int col0 = tn * BN + c * 32;
-        if (p.remap_n > 0) return ((long long)(row % p.remap_n) * p.remap_m + row / p.remap_n) * p.ldc + col0;
         return (long long)row * p.ldc + col0;
       };
       auto load_res = [&](int c, float (&rz)[32]) {

@@ -99,7 +99,7 @@ struct BmmLaunch {
   int out_f32 = 0;
   int opm_ntok = 0;
   const void* residual = nullptr;
-  int remap_n = 0, remap_m = 0;
+  bool b_shared = false;  // one B for every batch item
   const float* mul = nullptr;  // bulk output: per-element fp32 factor, row pitch mul_pitch
   int mul_pitch = 0;
   bool swiglu = false;  // bulk bf16 output: N columns are 64-wide (a | b) block pairs, C has N / 2 columns of silu(a) * b
@@ -138,11 +138,10 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   const int c_esz = a.out_f32 ? 4 : 2;
   // Bulk output through the C tensor map where the layout allows it (the map clips the last column group): the
   // residual (if any) being C itself, and for the transposed pair store lines that are whole row tiles.
-  const bool bulk_c = a.opm_ntok == 0 && (a.ldc * c_esz) % 16 == 0 && (c_batch * c_esz) % 16 == 0 && aligned(a.C, 16) &&
-                      (a.remap_n == 0 || (a.remap_n % 128 == 0 && a.batch == 1 && a.M == a.remap_n * (a.remap_m > 0 ? a.remap_m : a.remap_n)));
+  const bool bulk_c = a.opm_ntok == 0 && (a.ldc * c_esz) % 16 == 0 && (c_batch * c_esz) % 16 == 0 && aligned(a.C, 16);
   // An fp32 residual elsewhere comes by TMA tiles, as a gate's factors do (read by the lanes from their rows: 11 us against 7
   // for 65536 x 128 x 128).
-  const bool add = bulk_c && a.residual && a.residual != a.C && a.out_f32 && a.batch == 1 && a.remap_n == 0 && !a.mul &&
+  const bool add = bulk_c && a.residual && a.residual != a.C && a.out_f32 && a.batch == 1 && !a.mul &&
                    !a.swiglu && aligned(a.residual, 16);
   const int BN = a.mul || add ? 128 : a.split || a.gate_mask ? 256 : bmm_tile_n(a.M, a.N, a.parts ? 3 * a.K : a.K, a.batch);
   CUtensorMap tmA, tmB;
@@ -154,7 +153,7 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
     if (int e = make_tmap_bf16(&tmA, a.A, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   {
-    const uint64_t dims[3] = {uint64_t(a.b_fold ? a.b_fold * 128 : a.K), uint64_t(a.b_rows ? a.b_rows : a.N), uint64_t(a.parts ? 2 * a.batch : a.batch)};
+    const uint64_t dims[3] = {uint64_t(a.b_fold ? a.b_fold * 128 : a.K), uint64_t(a.b_rows ? a.b_rows : a.N), uint64_t(a.b_shared ? 1 : a.parts ? 2 * a.batch : a.batch)};
     const uint64_t str[2] = {uint64_t(a.ldb) * 2, uint64_t(a.sb > 0 ? a.sb : a.ldb * (a.b_rows ? a.b_rows : a.N)) * 2};
     const uint32_t box[3] = {64, uint32_t(BN), 1};
     if (int e = make_tmap_bf16(&tmB, a.B, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
@@ -182,9 +181,8 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   p.out_f32 = a.out_f32;
   p.opm_ntok = a.opm_ntok;
   p.residual = a.residual;
-  p.remap_n = a.remap_n;
-  p.remap_m = a.remap_m > 0 ? a.remap_m : a.remap_n;
   p.a_shared = a_shared ? 1 : 0;
+  p.b_shared = a.b_shared ? 1 : 0;
   p.a_fold = a.a_fold ? a.a_fold : INT_MAX;
   p.b_fold = a.b_fold ? a.b_fold : INT_MAX;
   p.tma_c = 0;
@@ -209,15 +207,9 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
     uint32_t box[3];
     dims[0] = uint64_t(a.swiglu && !a.split ? a.N / 2 : a.N);
     box[0] = uint32_t(c_cols);
-    if (a.remap_n > 0) {  // {column, line, pos}: pair (line, pos) lives in row pos * remap_m + line
-      dims[1] = uint64_t(p.remap_m), dims[2] = uint64_t(a.remap_n);
-      str[0] = uint64_t(a.ldc) * c_esz, str[1] = uint64_t(a.ldc) * c_esz * uint64_t(p.remap_m);
-      box[1] = 1, box[2] = 128;
-    } else {
-      dims[1] = uint64_t(a.M), dims[2] = uint64_t(a.batch);
-      str[0] = uint64_t(a.ldc) * c_esz, str[1] = uint64_t(c_batch) * c_esz;
-      box[1] = 128, box[2] = 1;
-    }
+    dims[1] = uint64_t(a.M), dims[2] = uint64_t(a.batch);
+    str[0] = uint64_t(a.ldc) * c_esz, str[1] = uint64_t(c_batch) * c_esz;
+    box[1] = 128, box[2] = 1;
     if (int e = make_tmap(&tmC, a.out_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.C, 3, dims,
                           str, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return e;
@@ -1434,11 +1426,17 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
     if (int e = launch_flash(a, 32, stream)) return e;
   }
   {
+    // Pair (line, pos) of the ending node lives in row pos * lines + line: a batch item per line, its rows a line of pairs apart, so
+    // that lines of any length leave by TMA tiles (stored by the lanes where a line is not whole tiles of 128: 20 us against 10 for
+    // 203 tokens).
     BmmLaunch a{og, w->w_o, out, 1, lines * pos, kD, kD, kD, kD, kD, 0, 0, 0};
+    if (ending) {
+      a.batch = lines, a.M = pos, a.ldc = int64_t(lines) * kD;
+      a.sa = int64_t(pos) * kD, a.sc = kD;
+      a.b_shared = true;
+    }
     a.out_f32 = f32;
     a.residual = add_residual ? z : nullptr;
-    a.remap_n = ending ? pos : 0;
-    a.remap_m = ending ? lines : 0;
     if (int e = launch_bmm(a, stream)) return e;
   }
   return B200_OK;
