@@ -12,6 +12,7 @@
 #include "transition.cuh"
 #include "ln_linear.cuh"
 #include "pair_cond.cuh"
+#include "cond_block.cuh"
 #include "elementwise.cuh"
 #include "accurate.cuh"
 #include "opm.cuh"
@@ -2079,6 +2080,60 @@ size_t b200_cond_layer_workspace_bytes(const b200_cond_layer* l) {
   return pl.total;
 }
 
+// The two kernels around the attention of a windowed block of 128 channels; maps and launch.
+static int cond_rows_map(CUtensorMap* m, const void* base, bool f32, int64_t rows, int cols) {
+  const uint64_t dims[2] = {uint64_t(cols), uint64_t(rows)};
+  const uint64_t str[1] = {uint64_t(cols) * (f32 ? 4 : 2)};
+  const uint32_t box[2] = {f32 ? 32u : 64u, 128};
+  return make_tmap(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, 2, dims, str, box,
+                   CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+static bool cond_block_fits(const b200_cond_layer* l, int x_dtype) {
+  const int64_t hidden = l->transition_fused.hidden;
+  return l->window_queries && l->dim == 128 && l->dim_cond == 128 && x_dtype == B200_DTYPE_F32 && l->transition_fused.w13 &&
+         l->transition_fused.w3 && (hidden == 256 || hidden == 512);
+}
+
+static CondBlockParams cond_block_params(const b200_cond_layer* l, const void* c, int64_t rows) {
+  return CondBlockParams{c, l->ln_c_w, l->ln_c_b, l->b_cond, l->b_qkvg, rows, int((rows + 127) / 128),
+                         int(l->transition_fused.hidden / 64), l->lns_scale, 1e-5f};
+}
+
+static int launch_cond_in(const b200_cond_layer* l, const void* x, const void* c, int c_dtype, void* qkvg, int64_t rows,
+                          cudaStream_t stream) {
+  CondInMaps m;
+  memset(&m, 0, sizeof(m));
+  if (int e = cond_rows_map(&m.w_cond, l->w_cond, false, 768, 128)) return e;
+  if (int e = cond_rows_map(&m.w_qkvg, l->w_qkvg, false, 512, 128)) return e;
+  if (int e = cond_rows_map(&m.x, x, true, rows, 128)) return e;
+  if (int e = cond_rows_map(&m.qkvg, qkvg, false, rows, 512)) return e;
+  const CondBlockParams p = cond_block_params(l, c, rows);
+  const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
+  if (c_dtype == B200_DTYPE_F32) B200_LAUNCH(cond_in_kernel<true>, grid, cond_block::THREADS, cond_block::InLayout::SMEM_BYTES, stream, m, p);
+  else B200_LAUNCH(cond_in_kernel<false>, grid, cond_block::THREADS, cond_block::InLayout::SMEM_BYTES, stream, m, p);
+  return B200_OK;
+}
+
+static int launch_cond_out(const b200_cond_layer* l, const void* x, const void* c, int c_dtype, const void* og, void* out, int64_t rows,
+                           cudaStream_t stream) {
+  CondOutMaps m;
+  memset(&m, 0, sizeof(m));
+  const int hidden = int(l->transition_fused.hidden);
+  if (int e = cond_rows_map(&m.w_cond, l->w_cond, false, 768, 128)) return e;
+  if (int e = cond_rows_map(&m.w_o, l->w_o, false, 128, 128)) return e;
+  if (int e = cond_rows_map(&m.w13, l->transition_fused.w13, false, 2 * hidden, 128)) return e;
+  if (int e = cond_rows_map(&m.w3, l->transition_fused.w3, false, 128, hidden)) return e;
+  if (int e = cond_rows_map(&m.og, og, false, rows, 128)) return e;
+  if (int e = cond_rows_map(&m.x, x, true, rows, 128)) return e;
+  if (int e = cond_rows_map(&m.out, out, true, rows, 128)) return e;
+  const CondBlockParams p = cond_block_params(l, c, rows);
+  const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
+  if (c_dtype == B200_DTYPE_F32) B200_LAUNCH(cond_out_kernel<true>, grid, cond_block::THREADS, cond_block::OutLayout::SMEM_BYTES, stream, m, p);
+  else B200_LAUNCH(cond_out_kernel<false>, grid, cond_block::THREADS, cond_block::OutLayout::SMEM_BYTES, stream, m, p);
+  return B200_OK;
+}
+
 int b200_cond_layer_fwd(const b200_cond_layer* l, const void* x, const void* pairs, const void* bias, int64_t bias_pitch,
                         const void* c, const uint8_t* mask, void* out, int x_dtype, int c_dtype, int pairs_dtype,
                         void* workspace, size_t workspace_bytes, b200_stream_t stream_) {
@@ -2104,6 +2159,20 @@ int b200_cond_layer_fwd(const b200_cond_layer* l, const void* x, const void* pai
   uint8_t* rest = ws + pl.off_rest;
   const int D = l->dim, CW = 6 * D;
   const bool xf32 = x_dtype == B200_DTYPE_F32;
+  if (cond_block_fits(l, x_dtype)) {
+    const int W = l->window_queries, Hk = l->window_keys, NW = l->N / W;
+    B200_CHECK_ARG(l->N % W == 0, "N=%d is not a multiple of the query window %d", l->N, W);
+    B200_CHECK_ARG(pairs && l->w_qkvg && l->b_qkvg && l->w_o && l->ln_z_w && l->w_z, "a window weight pointer is NULL");
+    B200_CHECK_ARG(D % l->heads == 0, "dim=%d is not a multiple of heads=%d", D, l->heads);
+    __nv_bfloat16* qkvg = reinterpret_cast<__nv_bfloat16*>(rest);
+    __nv_bfloat16* og = reinterpret_cast<__nv_bfloat16*>(rest + round_up_1k(size_t(rows) * 4 * D * 2));
+    float* wb = reinterpret_cast<float*>(rest + round_up_1k(size_t(rows) * 4 * D * 2) + round_up_1k(size_t(rows) * D * 2));
+    if (int e = launch_cond_in(l, x, c, c_dtype, qkvg, rows, stream)) return e;
+    if (int e = window_pair_run(qkvg, 4 * D, qkvg + 3 * D, 4 * D, pairs, l->ln_z_w, l->ln_z_b, l->w_z, mask, og, wb, l->B, l->M, NW, W, Hk,
+                                l->heads, D / l->heads, l->dim_pairwise, pairs_dtype, stream))
+      return e;
+    return launch_cond_out(l, x, c, c_dtype, og, out, rows, stream);
+  }
   // alpha1 | beta1 | gamma1 | alpha2 | beta2 | gamma2 = Linear(silu(LayerNorm(c)))
   if (int e = launch_rows_to_bf16(c, c_dtype == B200_DTYPE_F32, cn, l->ln_c_w, l->ln_c_b, rows, l->dim_cond, true, stream, true)) return e;
   {

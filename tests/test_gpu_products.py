@@ -97,6 +97,38 @@ def test_conditioned_layer_native_against_its_parts(windowed, dim, n, B, M, hidd
     _close(got, want)
 
 
+@pytest.mark.parametrize("n,B,M,hidden,c_dtype,lns", [
+    (32, 1, 1, 256, F32, 1.0),      # a quarter of a tile of tokens
+    (96, 1, 3, 200, BF16, 0.5),     # two tiles and a part of one, hidden units padded to 256
+    (4800, 1, 8, 256, F32, 0.25),   # three tiles for some CTAs
+    (2432, 2, 4, 512, BF16, 1.0),   # eight chunks of hidden units, two tiles for some
+])
+def test_atom_layer_between_its_attention(n, B, M, hidden, c_dtype, lns):
+    """The kernels on either side of the window attention at 128 channels, in place and not, against the layer's modules.  Bound: bf16
+    operands, as for the other products."""
+    import bioemu2_b200 as b
+    from bioemu2_b200 import _lib
+    from bioemu2_b200 import functional as F
+
+    g = _gen(n, B, M)
+    layer = _fill(b.ConditionedTransformerLayer(128, 16, 128, 4, hidden, is_sliding_window=True, window_queries=32, window_keys=128,
+                                                lns_scale=lns), n)
+    x, c = 3.0 + torch.randn(B * M, n, 128, generator=g).cuda(), torch.randn(B * M, n, 128, generator=g).to(c_dtype).cuda()
+    pairs = torch.randn(B, n // 32, 32, 128, 16, generator=g).cuda()
+    mask = (torch.rand(B, n, generator=g) > 0.1).cuda()
+    kept = x.clone()
+    with torch.no_grad():
+        got = layer(x, pairs, c, mask, M)
+        assert torch.equal(x, kept)
+        want = layer._forward(x, pairs, c, mask, M, layer.attention)
+        sized = _lib.CondLayer.from_buffer_copy(layer.packed()[2][0])
+        sized.B, sized.M, sized.N, sized.lns_scale = B, M, n, lns
+        F.cond_layer(sized, x, pairs, None, c, mask, out=x)
+    assert _lib.device_status() == 0
+    assert torch.equal(x, got)
+    _close(got - kept, want - kept)
+
+
 @pytest.mark.parametrize("S,n,H,c_m", [(1, 1, 1, 8), (3, 37, 8, 64), (5, 130, 6, 64), (2, 264, 16, 72)])
 def test_pwa_values(S, n, H, c_m):
     from bioemu2_b200 import functional as F
