@@ -697,7 +697,8 @@ static int trimul_fwd_impl(const void* z, const uint8_t* mask, void* out, const 
     if (int e = launch_trimul_project(zb, mask + size_t(bi) * N * N, a_buf, b_buf, w, gin, f32, stream, copy ? ob - zb : 0)) return e;
     {
       const int64_t plane_el = int64_t(Np) * Np;
-      BmmLaunch a{a_buf, b_buf, t_buf, kD, Np, Np, Np, Np, Np, Np, plane_el, plane_el, plane_el};
+      const int K = (N + 63) / 64 * 64;  // whole K blocks: the positions beyond N are zero
+      BmmLaunch a{a_buf, b_buf, t_buf, kD, Np, Np, K, Np, Np, Np, plane_el, plane_el, plane_el};
       if (int e = launch_bmm(a, stream)) return e;
     }
     if (int e = launch_trimul_output(copy ? ob : zb, ob, t_buf, w, gout, add_residual != 0, f32, stream)) return e;
