@@ -663,10 +663,12 @@ static bool trimul_weights_ok(const b200_trimul_weights* w) {
          aligned(w->w_out, 16);
 }
 
-// Argument checks and the three launches of triangle multiplication; the callers have checked the device.
+// Argument checks and the three launches of triangle multiplication; the callers have checked the device.  z_read: an event on another
+// stream after which out may be written.
 static int trimul_fwd_impl(const void* z, const uint8_t* mask, void* out, const b200_trimul_weights* w, int B, int N,
                            int incoming, int add_residual, int z_dtype, void* workspace, size_t workspace_bytes,
-                           b200_stream_t stream_) {
+                           b200_stream_t stream_,
+                           cudaEvent_t z_read = nullptr) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   B200_CHECK_ARG(z && mask && out && w, "z/mask/out/w is NULL");
   B200_CHECK_ARG(trimul_weights_ok(w), "a weight pointer is NULL or not 16-byte aligned");
@@ -701,6 +703,7 @@ static int trimul_fwd_impl(const void* z, const uint8_t* mask, void* out, const 
       BmmLaunch a{a_buf, b_buf, t_buf, kD, Np, Np, K, Np, Np, Np, plane_el, plane_el, plane_el};
       if (int e = launch_bmm(a, stream)) return e;
     }
+    if (z_read && bi == 0) B200_CUDA(cudaStreamWaitEvent(stream, z_read, 0));
     if (int e = launch_trimul_output(copy ? ob : zb, ob, t_buf, w, gout, add_residual != 0, f32, stream)) return e;
   }
   return B200_OK;
@@ -1846,7 +1849,7 @@ size_t b200_trunk_side_workspace_bytes(const b200_trunk_block* blocks, int n_blo
 // The events that order the two streams of a trunk call: two "bias ready", two "bias read", one for the joins.  Kept per
 // host thread and device -- an event may be recorded again as soon as the waits on it have been enqueued.
 struct TrunkEvents {
-  cudaEvent_t ev[5] = {};
+  cudaEvent_t ev[6] = {};
   int dev = -1;
   void drop() {
     for (cudaEvent_t& e : ev) {
@@ -2285,9 +2288,15 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
   const bool zf32 = z_dtype == B200_DTYPE_F32, sf32 = s_dtype == B200_DTYPE_F32;
   const size_t zsz = zf32 ? 4 : 2;
   const int Nk = (N + 7) / 8 * 8;
+  // The pair bias of a block reads z, which the next block writes for the first time two kernels on: where it and that block's first
+  // projection leave each other SMs, a tile each, it runs on the side stream beside them (4 blocks, us, on the main stream / beside: 24 tokens 450 / 441, 64 469 / 461; with 80
+  // tokens and more the two would take turns).
+  const bool beside = two && 2 * N <= sm_count();
   for (int i = 0; i < n_blocks; ++i) {
     const b200_trunk_block& w = blocks[i];
-    if (int e = trimul_fwd_impl(i == 0 ? z_in : z, pair_mask, z, &w.tri_mul_out, B, N, 0, 1, z_dtype, ws, scratch, stream)) return e;
+    if (int e = trimul_fwd_impl(i == 0 ? z_in : z, pair_mask, z, &w.tri_mul_out, B, N, 0, 1, z_dtype, ws, scratch, stream,
+                                beside && i > 0 ? ev[5] : nullptr))
+      return e;
     if (int e = trimul_fwd_impl(z, pair_mask, z, &w.tri_mul_in, B, N, 1, 1, z_dtype, ws, scratch, stream)) return e;
     if (has_triatt(w)) {
       if (int e = b200_triatt_fwd(z, pair_mask, z, &w.tri_att_start, B, N, 0, 1, z_dtype, ws, scratch, stream)) return e;
@@ -2299,20 +2308,26 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
       return e;
     if (!single) continue;
     const int k = i & 1;
-    if (two && i >= 2) B200_CUDA(cudaStreamWaitEvent(stream, ev[2 + k], 0));  // block i - 2 has read this bias buffer
+    if (two && !beside && i >= 2) B200_CUDA(cudaStreamWaitEvent(stream, ev[2 + k], 0));  // block i - 2 has read this bias buffer
+    if (beside) {
+      B200_CUDA(cudaEventRecord(ev[k], stream));
+      B200_CUDA(cudaStreamWaitEvent(side, ev[k], 0));
+    }
     for (int b = 0; b < B; ++b)
       if (int e = launch_pair_bias(static_cast<const uint8_t*>(z) + size_t(b) * N * N * kD * zsz, zf32, w.attention.ln_z_w,
                                    w.attention.ln_z_b, w.attention.w_z, bias[k] + size_t(b) * heads * N * Nk, N, N,
-                                   (long long)N * kD * zsz, (long long)kD * zsz, (long long)N * Nk, Nk, heads, stream))
+                                   (long long)N * kD * zsz, (long long)kD * zsz, (long long)N * Nk, Nk, heads, beside ? side : stream))
         return e;
-    if (two) {
+    if (beside) {
+      B200_CUDA(cudaEventRecord(ev[5], side));
+    } else if (two) {
       B200_CUDA(cudaEventRecord(ev[k], stream));
       B200_CUDA(cudaStreamWaitEvent(side, ev[k], 0));
     }
     if (int e = apb_run(s, nullptr, bias[k], Nk, token_mask, s, &w.attention, B, 1, N, c_s, heads, s_dtype, B200_DTYPE_F32,
                         true, side_workspace, side_bytes, side))
       return e;
-    if (two) B200_CUDA(cudaEventRecord(ev[2 + k], side));
+    if (two && !beside) B200_CUDA(cudaEventRecord(ev[2 + k], side));
     if (int e = swiglu_transition(s, sf32, s, sf32, true, nullptr, 0, w.transition_s, int64_t(B) * N, c_s, c_s,
                                   static_cast<uint8_t*>(side_workspace), side))
       return e;
