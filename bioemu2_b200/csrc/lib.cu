@@ -18,6 +18,7 @@
 #include "opm.cuh"
 #include "attention.cuh"
 #include "attention_resident.cuh"
+#include "attention_line.cuh"
 #include "pair_bias.cuh"
 #include "triatt.cuh"
 #include "window_attention.cuh"
@@ -373,6 +374,35 @@ static int launch_flash(const FlashLaunch& a, int DH, cudaStream_t stream) {
     return tiles <= FlashResidentCfg<32, 32, 2>::NB ? launch_flash_resident<32, 32, 2>(a, stream) : launch_flash_core<32, 2>(a, stream);
   if (a.p.dh_out <= 48 && tiles <= FlashResidentCfg<64, 48, 2>::NB) return launch_flash_resident<64, 48, 2>(a, stream);
   return launch_flash_core<64, 1>(a, stream);
+}
+
+// Lines that line_attention_kernel takes: one tile of queries and keys, four heads of 32, one wave of CTAs (a line each), the update
+// added in place.
+static bool line_attention_fits(const FlashLaunch& a) { return a.p.N <= 128 && a.p.H == 4 && a.p.dh_out == 32 && a.p.Bt <= sm_count(); }
+
+// out: pair (line, pos) at out + line * line_stride + pos * pos_stride elements.
+static int launch_line_attention(const FlashLaunch& a, const void* w_o, void* out, bool f32, int64_t line_stride, int64_t pos_stride,
+                                 cudaStream_t stream) {
+  CUtensorMap tmQ, tmV, tmB, tmW, tmO;
+  if (int e = flash_maps(a, 32, 32, &tmQ, &tmV, &tmB)) return e;
+  {
+    const uint64_t dims[2] = {128, 128};
+    const uint64_t str[1] = {256};
+    const uint32_t box[2] = {64, 128};
+    if (int e = make_tmap_bf16(&tmW, w_o, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+  }
+  {
+    const uint64_t esz = f32 ? 4 : 2;
+    const uint64_t dims[3] = {uint64_t(kD), uint64_t(a.p.N), uint64_t(a.p.Bt)};
+    const uint64_t str[2] = {uint64_t(pos_stride) * esz, uint64_t(line_stride) * esz};
+    const uint32_t box[3] = {f32 ? 32u : 64u, 128, 1};
+    if (int e = make_tmap(&tmO, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out, 3, dims, str, box,
+                          CU_TENSOR_MAP_SWIZZLE_128B))
+      return e;
+  }
+  if (f32) B200_LAUNCH(line_attention_kernel<true>, a.p.Bt, line_attention::THREADS, line_attention::SMEM_BYTES, stream, tmQ, tmV, tmB, tmW, tmO, a.p);
+  else B200_LAUNCH(line_attention_kernel<false>, a.p.Bt, line_attention::THREADS, line_attention::SMEM_BYTES, stream, tmQ, tmV, tmB, tmW, tmO, a.p);
+  return 0;
 }
 
 static int launch_pair_bias(const void* z, bool f32, const float* ln_w, const float* ln_b, const void* w_z,
@@ -1428,6 +1458,8 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
     p.q_col0 = 0;
     p.k_col0 = 128;
     p.v_row0 = 0;
+    if (add_residual && out == z && line_attention_fits(a))
+      return launch_line_attention(a, w->w_o, out, f32, line_b / esz, pos_b / esz, stream);
     if (int e = launch_flash(a, 32, stream)) return e;
   }
   {

@@ -57,3 +57,38 @@ def test_triatt_residual_inplace_and_padding(ending):
         upd_p = m(xp.cuda(), mp.cuda())[:, :N, :N]
     valid = (tok[:, :, None] & tok[:, None, :]).cuda()
     torch.testing.assert_close(upd_p[valid], upd[valid], atol=2e-3, rtol=0)
+
+
+@pytest.mark.parametrize("N,B", [(1, 1), (7, 2), (63, 1), (64, 1), (65, 1), (100, 2), (127, 1), (128, 1), (129, 1)])
+@pytest.mark.parametrize("ending", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("scale", [1.0, 60.0])
+def test_short_lines_in_place_are_the_update_added(N, B, ending, dtype, scale):
+    """Lines of up to 128 positions are attended to and projected in one kernel when the update is added in place: the same bits as the
+    update by itself, added in fp32 (one rounding of the sum in bf16).  Masks with padding, holes and lines without a valid key;
+    logits in the range of a row's reference and far outside it."""
+    import bioemu2_b200 as b
+    from bioemu2_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(3000 + N)
+    with torch.device("cuda"):
+        m = b.TriangleAttention(ending=ending).eval()
+    with torch.no_grad():
+        for name, p in m.named_parameters():
+            if p.ndim >= 2:
+                p.uniform_(-128 ** -0.5, 128 ** -0.5, generator=g)
+        m.linear_b.weight.mul_(scale)
+        z = torch.randn(B, N, N, 128, device="cuda", generator=g).to(dtype)
+        mask = torch.rand(B, N, N, device="cuda", generator=g) > 0.2
+        mask[:, :, N - N // 4:] = False
+        mask[:, :, N // 3:N // 2] = False
+        mask[:, N - N // 5:] = False
+        mask[:, :1] = True
+        want = z.float() + m(z, mask).float()
+        got = z.clone()
+        m.forward_residual_(got, mask)
+    assert _lib.device_status() == 0
+    if dtype == torch.float32:
+        assert torch.equal(got, want)
+    else:
+        torch.testing.assert_close(got.float(), want, rtol=2 ** -8, atol=2 ** -9 * want.abs().max().item())
