@@ -648,8 +648,8 @@ static int launch_trimul_output(const void* z, void* out, const __nv_bfloat16* t
   {
     const uint64_t dims[3] = {uint64_t(g.pos_pitch), uint64_t(g.lines_alloc), uint64_t(kD)};
     const uint64_t str[2] = {uint64_t(g.pos_pitch) * 2, uint64_t(g.pos_pitch) * g.lines_alloc * 2};
-    const uint32_t box[3] = {128, 1, 128};
-    if (int e = make_tmap_bf16(&tmT, t_buf, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE)) return e;
+    const uint32_t box[3] = {64, 1, 128};
+    if (int e = make_tmap_bf16(&tmT, t_buf, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   // Output tiles [128 pairs][128 B of channels]; the dimension with the smaller stride comes first.
   CUtensorMap tmO;
