@@ -123,16 +123,23 @@ struct BmmLaunch {
 // outer product mean: within 2 % of it, once 5 % (rows x columns x K, us, 128 / 256 wide: 256 x 768 x 3072 12.2 / 18.8,
 // 2048 x 2816 x 768 12.2 / 13.5, 2048 x 6144 x 768 20.7 / 18.9, 3584 x 2816 x 768 17.9 / 18.6 where the estimate takes 256;
 // 128 batches of 384^3 21.8 / 25.7, of 512^3 42.5 / 38.7).
+// 64 columns where even the narrow tiles are few: a K block of 64 is then bound by shared memory (24 KB written and 24 read, against
+// 32 and 32), and twice the SMs share the epilogues.  Token layers x 4 (rows, us with 128-wide tiles at the least / with 64): 32 280 /
+// 263, 256 289 / 268, 512 297 / 286, 800 354 / 341, 1600 434 / 433, 2048 the same tiles.
 // Products that run on a side stream underneath another's kernels go by the same estimate: wide tiles for those, since they
 // take less SM time, moved a trunk's time both ways (4 blocks, us, without / with: 144 tokens 890 / 902, 160 1024 / 1006,
 // 203 1144 / 1154, 256 1292 / 1322, 320 and more the same).
-static int bmm_tile_n(int M, int N, int K, int batch) {
+static int bmm_tile_n(int M, int N, int K, int batch, int narrowest, int widest) {
   const int64_t tm = (M + 127) / 128, kb = (K + 63) / 64, sms = sm_count();
   auto cost = [&](int bn, int64_t per_block, int64_t tail) {
     const int64_t tiles = tm * ((N + bn - 1) / bn) * batch;
     return (tiles + sms - 1) / sms * (kb * per_block + 700) + tail;
   };
-  return cost(256, 1500, 5000) <= cost(128, 1000, 2500) ? 256 : 128;
+  int bn = 128;
+  int64_t best = cost(128, 1000, 2500);
+  if (widest > 128 && cost(256, 1500, 5000) <= best) bn = 256, best = cost(256, 1500, 5000);
+  if (narrowest < 128 && cost(64, 760, 1250) < best) bn = 64;
+  return bn;
 }
 
 static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
@@ -145,7 +152,11 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   // for 65536 x 128 x 128).
   const bool add = bulk_c && a.residual && a.residual != a.C && a.out_f32 && a.batch == 1 && !a.mul &&
                    !a.swiglu && aligned(a.residual, 16);
-  const int BN = a.mul || add ? 128 : a.split || a.gate_mask ? 256 : bmm_tile_n(a.M, a.N, a.parts ? 3 * a.K : a.K, a.batch);
+  // 64-wide tiles: bulk output of whole rows
+  const bool narrow = bulk_c && (add || a.residual == nullptr || a.residual == a.C) && (a.bias == nullptr || aligned(a.bias, 16)) &&
+                      !a.swiglu && a.opm_ntok == 0 && a.row_groups == 0;
+  const int BN = a.split || a.gate_mask ? 256
+                                        : bmm_tile_n(a.M, a.N, a.parts ? 3 * a.K : a.K, a.batch, narrow ? 64 : 128, a.mul || add ? 128 : 256);
   CUtensorMap tmA, tmB;
   const bool a_shared = a.batch > 1 && a.sa == 0;  // one A for every batch item
   {
@@ -244,8 +255,11 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   };
   if (a.gate_mask) return go(std::integral_constant<int, 256>(), std::integral_constant<int, kEpiGateSplit>());
   if (a.split) return go(std::integral_constant<int, 256>(), std::integral_constant<int, kEpiSwigluSplit>());
-  if (add && p.tma_c) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiAdd>());
-  if (a.mul) return go(std::integral_constant<int, 128>(), std::integral_constant<int, kEpiMul>());
+  const auto bn64 = std::integral_constant<int, 64>();
+  const auto bn128 = std::integral_constant<int, 128>();
+  if (add && p.tma_c) return BN == 64 ? go(bn64, std::integral_constant<int, kEpiAdd>()) : go(bn128, std::integral_constant<int, kEpiAdd>());
+  if (a.mul) return BN == 64 ? go(bn64, std::integral_constant<int, kEpiMul>()) : go(bn128, std::integral_constant<int, kEpiMul>());
+  if (BN == 64) return go(bn64, std::integral_constant<int, kEpiBulk>());
   return BN == 256 ? pick(std::integral_constant<int, 256>()) : pick(std::integral_constant<int, 128>());
 }
 
