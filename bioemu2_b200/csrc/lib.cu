@@ -603,7 +603,14 @@ struct TriMulGeom {
   int n_lines, n_pos, lines_alloc, pos_pitch;
   long long z_line_stride, z_pos_stride;  // bytes
   long long m_line_stride, m_pos_stride;  // bytes
+  int half_tiles;  // of 64 positions a line: those that hold one, or the whole pitch where a caller's product reads it
 };
+
+// Half tiles of a line of the two kernels: an odd number has them cut tiles across lines.  In one wave a tile a line takes no longer,
+// and is spared the second division and store (PairMixer of 4 blocks, 48 tokens: 219 us, cut 223).
+static int trimul_half_tiles(int n_lines, int n_pos, int pos_pitch) {
+  return n_lines * (pos_pitch / 128) <= sm_count() ? pos_pitch / 64 : (n_pos + 63) / 64;
+}
 
 static int launch_trimul_project(const void* z, const uint8_t* mask, __nv_bfloat16* a_buf, __nv_bfloat16* b_buf,
                                  const b200_trimul_weights* w, const TriMulGeom& g, bool f32, cudaStream_t stream,
@@ -637,17 +644,17 @@ static int launch_trimul_project(const void* z, const uint8_t* mask, __nv_bfloat
   pi.z_pos_stride = g.z_pos_stride;
   pi.m_line_stride = g.m_line_stride;
   pi.m_pos_stride = g.m_pos_stride;
-  pi.num_tiles = g.n_lines * (g.pos_pitch / 128);
+  pi.half_tiles = g.half_tiles;
+  pi.num_tiles = (g.n_lines * g.half_tiles + 1) / 2;
   pi.eps = 1e-5f;
   const int grid = pi.num_tiles < sm_count() ? pi.num_tiles : sm_count();
-  if (z_copy_delta) {
-    if (f32) B200_LAUNCH(trimul_in_kernel<true, true>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
-    else B200_LAUNCH(trimul_in_kernel<false, true>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
-  } else {
-    if (f32) B200_LAUNCH(trimul_in_kernel<true, false>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
-    else B200_LAUNCH(trimul_in_kernel<false, false>, grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
-  }
-  return 0;
+  auto go = [&](auto copy, auto half) -> int {
+    if (f32) B200_LAUNCH((trimul_in_kernel<true, copy.value, half.value>), grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
+    else B200_LAUNCH((trimul_in_kernel<false, copy.value, half.value>), grid, trimul_in::THREADS, trimul_in::SMEM_BYTES, stream, tmWin, tmA, tmB, pi);
+    return 0;
+  };
+  if (g.half_tiles & 1) return z_copy_delta ? go(std::true_type(), std::true_type()) : go(std::false_type(), std::true_type());
+  return z_copy_delta ? go(std::true_type(), std::false_type()) : go(std::false_type(), std::false_type());
 }
 
 static int launch_trimul_output(const void* z, void* out, const __nv_bfloat16* t_buf, const b200_trimul_weights* w,
@@ -673,7 +680,8 @@ static int launch_trimul_output(const void* z, void* out, const __nv_bfloat16* t
     const uint64_t dims[3] = {uint64_t(kD), pos_first ? np : nl, pos_first ? nl : np};
     const uint64_t str[2] = {uint64_t(pos_first ? g.z_pos_stride : g.z_line_stride),
                              uint64_t(pos_first ? g.z_line_stride : g.z_pos_stride)};
-    const uint32_t box[3] = {f32 ? 32u : 64u, pos_first ? 128u : 1u, pos_first ? 1u : 128u};
+    const uint32_t run = g.half_tiles & 1 ? 64 : 128;
+    const uint32_t box[3] = {f32 ? 32u : 64u, pos_first ? run : 1u, pos_first ? 1u : run};
     if (int e = make_tmap(&tmO, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out, 3, dims,
                           str, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return e;
@@ -691,15 +699,17 @@ static int launch_trimul_output(const void* z, void* out, const __nv_bfloat16* t
   po.z_line_stride = g.z_line_stride;
   po.z_pos_stride = g.z_pos_stride;
   po.pos_is_dim1 = pos_first ? 1 : 0;
-  po.num_tiles = g.n_lines * (g.pos_pitch / 128);
+  po.half_tiles = g.half_tiles;
+  po.num_tiles = (g.n_lines * g.half_tiles + 1) / 2;
   po.add_residual = add_residual ? 1 : 0;
   po.eps = 1e-5f;
   const int grid = po.num_tiles < sm_count() ? po.num_tiles : sm_count();
-  if (f32)
-    B200_LAUNCH(trimul_out_kernel<true>, grid, trimul_out::THREADS, trimul_out::SMEM_BYTES, stream, tmWout, tmT, tmO, po);
-  else
-    B200_LAUNCH(trimul_out_kernel<false>, grid, trimul_out::THREADS, trimul_out::SMEM_BYTES, stream, tmWout, tmT, tmO, po);
-  return 0;
+  auto go = [&](auto half) -> int {
+    if (f32) B200_LAUNCH((trimul_out_kernel<true, half.value>), grid, trimul_out::THREADS, trimul_out::SMEM_BYTES, stream, tmWout, tmT, tmO, po);
+    else B200_LAUNCH((trimul_out_kernel<false, half.value>), grid, trimul_out::THREADS, trimul_out::SMEM_BYTES, stream, tmWout, tmT, tmO, po);
+    return 0;
+  };
+  return g.half_tiles & 1 ? go(std::true_type()) : go(std::false_type());
 }
 
 static bool trimul_weights_ok(const b200_trimul_weights* w) {
@@ -732,8 +742,9 @@ static int trimul_fwd_impl(const void* z, const uint8_t* mask, void* out, const 
   __nv_bfloat16* t_buf = b_buf + plane;
   const long long row_b = (long long)N * kD * esz, col_b = (long long)kD * esz;
   // projection walks rows (outgoing) or columns (incoming); the output stage always walks rows
-  TriMulGeom gin{N, N, Np, Np, incoming ? col_b : row_b, incoming ? row_b : col_b, incoming ? 1 : N, incoming ? N : 1};
-  TriMulGeom gout{N, N, Np, Np, row_b, col_b, 0, 0};
+  const int halves = trimul_half_tiles(N, N, Np);
+  TriMulGeom gin{N, N, Np, Np, incoming ? col_b : row_b, incoming ? row_b : col_b, incoming ? 1 : N, incoming ? N : 1, halves};
+  TriMulGeom gout{N, N, Np, Np, row_b, col_b, 0, 0, halves};
   for (int bi = 0; bi < B; ++bi) {
     const uint8_t* zb = static_cast<const uint8_t*>(z) + size_t(bi) * N * N * kD * esz;
     uint8_t* ob = static_cast<uint8_t*>(out) + size_t(bi) * N * N * kD * esz;
@@ -780,7 +791,7 @@ int b200_trimul_project(const void* z, const uint8_t* mask, void* a_out, void* b
   const long long esz = f32 ? 4 : 2;
   const long long row_b = z_row_stride * esz, col_b = kD * esz;
   TriMulGeom g{n_lines, n_pos, n_lines, pos_pitch, incoming ? col_b : row_b, incoming ? row_b : col_b,
-               incoming ? 1 : mask_row_stride, incoming ? mask_row_stride : 1};
+               incoming ? 1 : mask_row_stride, incoming ? mask_row_stride : 1, pos_pitch / 64};
   return launch_trimul_project(z, mask, static_cast<__nv_bfloat16*>(a_out), static_cast<__nv_bfloat16*>(b_out), w, g, f32,
                                static_cast<cudaStream_t>(stream));
 }
@@ -801,7 +812,8 @@ int b200_trimul_output(const void* t, const void* z, void* out, const b200_trimu
   const bool f32 = z_dtype == B200_DTYPE_F32;
   const long long esz = f32 ? 4 : 2;
   const long long row_b = z_row_stride * esz, col_b = kD * esz;
-  TriMulGeom g{n_lines, n_pos, n_lines, pos_pitch, transposed_t ? col_b : row_b, transposed_t ? row_b : col_b, 0, 0};
+  TriMulGeom g{n_lines, n_pos, n_lines, pos_pitch, transposed_t ? col_b : row_b, transposed_t ? row_b : col_b, 0, 0,
+               trimul_half_tiles(n_lines, n_pos, pos_pitch)};
   return launch_trimul_output(z, out, static_cast<const __nv_bfloat16*>(t), w, g, add_residual != 0, f32,
                               static_cast<cudaStream_t>(stream));
 }

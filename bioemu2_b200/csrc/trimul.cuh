@@ -10,7 +10,7 @@
 //                      reading t channel-major and writing the pair-major result.
 //
 // "line/pos": outgoing contracts the column index, a[d][i][k] = ab[i,k,d]; incoming contracts the
-// row index, a[d][i][k] = ab[k,i,d].  A tile is 128 consecutive `pos` on one `line`.
+// row index, a[d][i][k] = ab[k,i,d].  A tile is two runs of 64 consecutive `pos`, each on one `line`.
 #pragma once
 #include "row_tile.cuh"
 
@@ -32,8 +32,47 @@ struct TriMulInParams {
   int lines_alloc, pos_pitch;  // pos_pitch: multiple of 128 >= n_pos
   long long z_line_stride, z_pos_stride;
   long long m_line_stride, m_pos_stride;
-  int num_tiles;           // n_lines * pos_pitch/128
+  int half_tiles;          // a line's half tiles of 64 positions; a tile is two consecutive ones, of one line or of two
+  int num_tiles;           // ceil(n_lines * half_tiles / 2)
   float eps;
+};
+
+// The two runs of 64 positions of a tile.  HALF: two consecutive half tiles, of one line or of two -- a line's last half tile need
+// not bring a second one of padding along: 160 positions are three halves, not four.  Else both of one line: one division and one
+// store a tile, for lines of an even number of halves.  PairMixer of 4 blocks, us, whole / half tiles: 160 tokens 398 / 357, 192 417 /
+// 368, 290 797 / 758, 320 874 / 844; with an even number 203 456 / 466, 256 549 / 568, 384 1032 / 1050.
+template <bool HALF>
+struct TileRuns {
+  int line[2], pos0[2];
+  bool there1;
+  __device__ __forceinline__ TileRuns(int tile, int half_tiles, int n_lines) {
+    if (HALF) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        line[k] = (2 * tile + k) / half_tiles;
+        pos0[k] = (2 * tile + k - line[k] * half_tiles) << 6;
+      }
+      there1 = line[1] < n_lines;
+    } else {
+      const int per_line = half_tiles >> 1;
+      line[0] = line[1] = tile / per_line;
+      pos0[0] = (tile - line[0] * per_line) << 7;
+      pos0[1] = pos0[0] + 64;
+      there1 = true;
+    }
+  }
+  __device__ __forceinline__ int line_of(int k) const { return HALF && k ? line[1] : line[0]; }
+  __device__ __forceinline__ int pos_of(int k) const { return HALF ? (k ? pos0[1] : pos0[0]) : pos0[0] + 64 * k; }
+  // Address of tile row r of a tensor of pair rows, nullptr where there is none.
+  __device__ __forceinline__ auto rows(const void* z, int n_pos, long long line_stride, long long pos_stride) const {
+    const uint8_t* base0 = static_cast<const uint8_t*>(z) + line[0] * line_stride + pos0[0] * pos_stride;
+    const uint8_t* base1 = HALF ? static_cast<const uint8_t*>(z) + line[1] * line_stride + (pos0[1] - 64) * pos_stride : base0;
+    const int left0 = n_pos - pos0[0], left1 = HALF ? (there1 ? n_pos - pos0[1] + 64 : 0) : left0;
+    return [=](int r) -> const void* {
+      if (!HALF) return r < left0 ? base0 + r * pos_stride : nullptr;
+      return r < 64 ? (r < left0 ? base0 + r * pos_stride : nullptr) : (r < left1 ? base1 + r * pos_stride : nullptr);
+    };
+  }
 };
 
 namespace trimul_in {
@@ -56,7 +95,7 @@ constexpr int THREADS = 512;  // warps 0-3 epilogue of pairs 0-63, 4-7 of pairs 
 // had to wait for its own drain, a tile was a chain of products, drain and store: 78.5 us at N = 512).
 // COPY: the producers also store the raw rows at z_copy_delta from their source.  The first op of a stack that leaves its
 // input alone gets its working copy this way, for the write alone (N = 384: 26 us as a copy of its own before the stack).
-template <bool F32, bool COPY>
+template <bool F32, bool COPY, bool HALF>
 __global__ void __launch_bounds__(512, 1)
 trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
                  const __grid_constant__ CUtensorMap tmB, TriMulInParams p) {
@@ -74,7 +113,6 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
-  const int tiles_per_line = p.pos_pitch >> 7;
 
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
@@ -115,17 +153,13 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     rows.step = 14;
     const int groups = issuer ? 1 : G;
     uint8_t mreg = 0;
-    auto row_ptr = [&](int tile) {
-      const int line = tile / tiles_per_line;
-      const int pos0 = (tile - line * tiles_per_line) << 7;
-      const uint8_t* base = static_cast<const uint8_t*>(p.z) + line * line_stride + pos0 * pos_stride;
-      const int left = p.n_pos - pos0 < 128 ? p.n_pos - pos0 : 128;
-      return [=](int r) -> const void* { return r < left ? base + r * pos_stride : nullptr; };
-    };
+    auto row_ptr = [&](int tile) { return TileRuns<HALF>(tile, p.half_tiles, p.n_lines).rows(p.z, p.n_pos, line_stride, pos_stride); };
     auto load_mask = [&](int tile) {
-      const int line = tile / tiles_per_line;
-      const int pos = ((tile - line * tiles_per_line) << 7) + pt;
-      if (pt < 128) mreg = (pos < p.n_pos) ? p.mask[line * mline_stride + pos * mpos_stride] : 0;
+      if (pt < 128) {
+        const TileRuns<HALF> t(tile, p.half_tiles, p.n_lines);
+        const int k = pt >> 6, pos = t.pos_of(k) + (pt & 63);
+        mreg = (k == 0 || t.there1) && pos < p.n_pos ? p.mask[t.line_of(k) * mline_stride + pos * mpos_stride] : 0;
+      }
     };
     // Tile number `it` into its operand stage, and the loads of the block's next tile on their way.
     auto produce = [&](int tile, int it) {
@@ -202,8 +236,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     const uint32_t acc_addr = tmem_addr(tmem_base, (warp & 3) * 32, grp * 64);
     int it = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
-      const int line = tile / tiles_per_line;
-      const int pos0 = ((tile - line * tiles_per_line) << 7) + grp * 64;
+      const TileRuns<HALF> t(tile, p.half_tiles, p.n_lines);
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         mbar_wait(&acc_full[half], it & 1, 14);
@@ -250,7 +283,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         fence_proxy_async_smem();
         named_bar_sync(1 + grp, 128);
         if (d == 0) {
-          tma_store_3d(half ? &tmB : &tmA, stage, pos0, line, 0);
+          if (grp == 0 || t.there1) tma_store_3d(half ? &tmB : &tmA, stage, t.pos_of(grp), t.line_of(grp), 0);
           tma_store_commit();
         }
       }
@@ -279,7 +312,7 @@ struct TriMulOutParams {
   const float* ln_out_b;
   int n_lines, n_pos, pos_pitch;
   long long z_line_stride, z_pos_stride;
-  int num_tiles;           // n_lines * pos_pitch/128
+  int half_tiles, num_tiles;  // as in TriMulInParams
   int add_residual;
   int pos_is_dim1;         // the output tensor map is {channel, pos, line} (1) or {channel, line, pos} (0)
   float eps;
@@ -297,7 +330,7 @@ constexpr uint32_t SMEM_BYTES = STAGE_OFF + 2 * kOperandHalf + 1024;
 constexpr int THREADS = 512;  // warps 0-3 epilogue (thread 0 also issues the TMA loads and MMAs), 4-7 t transformers, 8-15 z producers
 }  // namespace trimul_out
 
-template <bool F32>
+template <bool F32, bool HALF>
 __global__ void __launch_bounds__(512, 1)
 trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmT,
                   const __grid_constant__ CUtensorMap tmO, TriMulOutParams p) {
@@ -317,7 +350,6 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
-  const int tiles_per_line = p.pos_pitch >> 7;
 
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
@@ -448,13 +480,8 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     load_gamma_beta(p.ln_in_w, p.ln_in_b, pt, gamma, beta);
     RowTile<256> regs;
     auto load_tile = [&](int tile) {
-      const int line = tile / tiles_per_line;
-      const int pos0 = (tile - line * tiles_per_line) << 7;
-      const uint8_t* base = static_cast<const uint8_t*>(p.z) + line * p.z_line_stride + pos0 * p.z_pos_stride;
       regs.template load<F32, true, 8>(
-          pt,
-          [&](int r) -> const void* { return (pos0 + r) < p.n_pos ? base + r * p.z_pos_stride : nullptr; },
-          gamma, beta, p.eps);
+          pt, TileRuns<HALF>(tile, p.half_tiles, p.n_lines).rows(p.z, p.n_pos, p.z_line_stride, p.z_pos_stride), gamma, beta, p.eps);
     };
     int it = 0;
     int tile = blockIdx.x;
@@ -485,11 +512,11 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     const uint32_t a1_s = smem_u32(smem + A1_OFF);
     const uint32_t a2_s = smem_u32(smem + A2_OFF);
     auto issue_t = [&](int tile, int s) {
-      const int line = tile / tiles_per_line;
-      const int pos0 = (tile - line * tiles_per_line) << 7;
       mbar_arrive_expect_tx(&t_full[s], kOperandTile);
-      tma_load_3d(smem + T_OFF + s * kOperandTile, &tmT, &t_full[s], pos0, line, 0);
-      tma_load_3d(smem + T_OFF + s * kOperandTile + kOperandHalf, &tmT, &t_full[s], pos0 + 64, line, 0);
+      const TileRuns<HALF> t(tile, p.half_tiles, p.n_lines);
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        tma_load_3d(smem + T_OFF + s * kOperandTile + k * kOperandHalf, &tmT, &t_full[s], t.pos_of(k), t.line_of(k), 0);
     };
     int my_tiles = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x) ++my_tiles;
@@ -532,11 +559,14 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       if (step == 0) continue;
       const int it = step - 1;
       const int tile = blockIdx.x + it * gridDim.x;
-      const int line = tile / tiles_per_line;
-      const int pos0 = (tile - line * tiles_per_line) << 7;
+      const TileRuns<HALF> t(tile, p.half_tiles, p.n_lines);
+      const int run = HALF ? r >> 6 : 0;  // the lane's
+      const int line = run ? t.line[1] : t.line[0], pos0 = run ? t.pos0[1] : t.pos0[0];
+      const bool sender = (r & (HALF ? 63 : 127)) == 0;  // sends its run's rows off
       const int acc = it & 1;
-      const bool valid = (pos0 + r) < p.n_pos;
-      const uint8_t* zrow = static_cast<const uint8_t*>(p.z) + line * p.z_line_stride + (pos0 + r) * p.z_pos_stride;
+      const int pos = HALF ? pos0 + (r & 63) : pos0 + r;
+      const bool valid = (run == 0 || t.there1) && pos < p.n_pos;
+      const uint8_t* zrow = static_cast<const uint8_t*>(p.z) + line * p.z_line_stride + pos * p.z_pos_stride;
       mbar_wait(&acc_full[acc], (it >> 1) & 1, 28);
       tc_fence_after_sync();
       const uint32_t p_addr = tmem_addr(tmem_base, warp * 32, acc * 256);
@@ -548,7 +578,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       for (int c = 0; c < 8; ++c) {
         uint8_t* stage = smem + STAGE_OFF + ((c / CPS) & 1) * kOperandHalf;
         if (c % CPS == 0) {  // the store that last used this staging tile has finished reading it
-          if (r == 0) tma_store_wait_read1();
+          if (sender) tma_store_wait_read1();
           named_bar_sync(1, 128);
         }
         uint32_t(&pv)[16] = (c & 1) ? pb : pa;
@@ -585,19 +615,21 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         if (c % CPS == CPS - 1) {
           fence_proxy_async_smem();
           named_bar_sync(1, 128);
-          if (r == 0) {
+          if (sender) {
             const int ch0 = (c / CPS) * (F32 ? 32 : 64);
             const int c1 = p.pos_is_dim1 ? pos0 : line, c2 = p.pos_is_dim1 ? line : pos0;
-            if (reduce)
-              tma_reduce_add_3d(&tmO, stage, ch0, c1, c2);
+            const uint8_t* rows = stage + run * (kOperandHalf / 2);
+            if (!valid) {  // (the run's first row is not there)
+            } else if (reduce)
+              tma_reduce_add_3d(&tmO, rows, ch0, c1, c2);
             else
-              tma_store_3d(&tmO, stage, ch0, c1, c2);
-            tma_store_commit();
+              tma_store_3d(&tmO, rows, ch0, c1, c2);
+            tma_store_commit();  // an empty group too: the waits count groups
           }
         }
       }
     }
-    if (r == 0) tma_store_wait0();
+    if ((r & (HALF ? 63 : 127)) == 0) tma_store_wait0();
   }
 
   tc_fence_before_sync();

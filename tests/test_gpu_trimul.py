@@ -49,6 +49,27 @@ def test_trimul_vs_oracle(mode, N, dtype):
     assert_close(f"trimul_{mode}_N{N}_{dtype}", out, ref)
 
 
+@pytest.mark.parametrize("mode", ["outgoing", "incoming"])
+@pytest.mark.parametrize("N,dtype", [(131, torch.bfloat16), (160, torch.float32), (192, torch.bfloat16), (319, torch.float32)])
+def test_lines_of_an_odd_number_of_half_tiles(mode, N, dtype):
+    """Tiles that hold the end of one line and the start of the next, the last of them without a second half (131, 319)."""
+    g = torch.Generator().manual_seed(700 + N)
+    w = H.trimul_weights(g)
+    x = torch.randn(1, N, N, 128, generator=g).to(dtype)
+    mask = torch.rand(1, N, N, generator=g) > 0.25
+    ref = O.triangle_multiplication(x.double(), mask, {k: v.double() for k, v in w.items()}, mode)
+    m = _module(w, mode)
+    with torch.no_grad():
+        out = m(x.cuda(), mask.cuda())
+        z = x.cuda()
+        m.forward_residual_(z, mask.cuda())
+    assert_close(f"half_tiles_{mode}_N{N}_{dtype}", out, ref)
+    # The same update added: one rounding of the update in `out`, and one or two (bfloat16: reduced in memory) of the sum.
+    eps = torch.finfo(dtype).eps
+    bound = 1.5 * eps * (x.cuda().float().abs() + out.float().abs()) + 1e-6
+    assert ((z.float() - (x.cuda().float() + out.float())).abs() <= bound).all()
+
+
 def test_trimul_residual_inplace_and_masked_poison():
     """z += update in place equals the separate add; poisoned masked entries do not leak
     (tests/biomoa/ops/test_triangle_multiplication.py:373-388 in the reference)."""
