@@ -608,7 +608,7 @@ struct TriMulGeom {
 
 // Half tiles of a line of the two kernels: an odd number has them cut tiles across lines.  In one wave a tile a line takes no longer,
 // and is spared the second division and store (PairMixer of 4 blocks, 48 tokens: 219 us, cut 223).
-static int trimul_half_tiles(int n_lines, int n_pos, int pos_pitch) {
+static int line_half_tiles(int n_lines, int n_pos, int pos_pitch) {
   return n_lines * (pos_pitch / 128) <= sm_count() ? pos_pitch / 64 : (n_pos + 63) / 64;
 }
 
@@ -742,7 +742,7 @@ static int trimul_fwd_impl(const void* z, const uint8_t* mask, void* out, const 
   __nv_bfloat16* t_buf = b_buf + plane;
   const long long row_b = (long long)N * kD * esz, col_b = (long long)kD * esz;
   // projection walks rows (outgoing) or columns (incoming); the output stage always walks rows
-  const int halves = trimul_half_tiles(N, N, Np);
+  const int halves = line_half_tiles(N, N, Np);
   TriMulGeom gin{N, N, Np, Np, incoming ? col_b : row_b, incoming ? row_b : col_b, incoming ? 1 : N, incoming ? N : 1, halves};
   TriMulGeom gout{N, N, Np, Np, row_b, col_b, 0, 0, halves};
   for (int bi = 0; bi < B; ++bi) {
@@ -813,7 +813,7 @@ int b200_trimul_output(const void* t, const void* z, void* out, const b200_trimu
   const long long esz = f32 ? 4 : 2;
   const long long row_b = z_row_stride * esz, col_b = kD * esz;
   TriMulGeom g{n_lines, n_pos, n_lines, pos_pitch, transposed_t ? col_b : row_b, transposed_t ? row_b : col_b, 0, 0,
-               trimul_half_tiles(n_lines, n_pos, pos_pitch)};
+               line_half_tiles(n_lines, n_pos, pos_pitch)};
   return launch_trimul_output(z, out, static_cast<const __nv_bfloat16*>(t), w, g, add_residual != 0, f32,
                               static_cast<cudaStream_t>(stream));
 }
@@ -1405,11 +1405,12 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
     const uint32_t box[2] = {64, 128};
     if (int e = make_tmap_bf16(&tmW, w->w_qkgv, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
-  CUtensorMap tmQKG, tmVT;  // [128 rows][64 values] boxes: pairs x channels of q|k|g, channels x keys of V^T
+  const int half_tiles = line_half_tiles(lines, pos, (pos + 127) / 128 * 128);
+  CUtensorMap tmQKG, tmVT;  // [128 rows][64 values] boxes: a tile's (or a run's 64) pairs x channels of q|k|g, channels x keys of V^T
   {
     const uint64_t dims[3] = {384, uint64_t(pos), uint64_t(lines)};
     const uint64_t str[2] = {768, uint64_t(pos) * 768};
-    const uint32_t box[3] = {64, 128, 1};
+    const uint32_t box[3] = {64, half_tiles & 1 ? 64u : 128u, 1};
     if (int e = make_tmap_bf16(&tmQKG, qkg, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
   }
   {
@@ -1437,7 +1438,8 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
   pp.Nk = pl.Nk;
   pp.z_line_stride = line_b;
   pp.z_pos_stride = pos_b;
-  pp.num_tiles = lines * ((pos + 127) / 128);
+  pp.half_tiles = half_tiles;
+  pp.num_tiles = (lines * half_tiles + 1) / 2;
   pp.eps = 1e-5f;
   // Without a bias from the caller the projection kernel writes the triangle bias of the same rows itself.
   pp.tri_bias = ext_bias ? nullptr : tb;
@@ -1445,12 +1447,12 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
   pp.bias_pitch = pl.Nk;
   pp.bias_scale = 1.4426950408889634f;
   const int grid = pp.num_tiles < sm_count() ? pp.num_tiles : sm_count();
-  if (f32)
-    B200_LAUNCH(triatt_proj_kernel<true>, grid, triatt_proj::THREADS, triatt_proj::SMEM_BYTES, stream, tmW, tmQKG, tmVT,
-                tmWB, pp);
-  else
-    B200_LAUNCH(triatt_proj_kernel<false>, grid, triatt_proj::THREADS, triatt_proj::SMEM_BYTES, stream, tmW, tmQKG, tmVT,
-                tmWB, pp);
+  auto go = [&](auto half) -> int {
+    if (f32) B200_LAUNCH((triatt_proj_kernel<true, half.value>), grid, triatt_proj::THREADS, triatt_proj::SMEM_BYTES, stream, tmW, tmQKG, tmVT, tmWB, pp);
+    else B200_LAUNCH((triatt_proj_kernel<false, half.value>), grid, triatt_proj::THREADS, triatt_proj::SMEM_BYTES, stream, tmW, tmQKG, tmVT, tmWB, pp);
+    return 0;
+  };
+  if (int e = half_tiles & 1 ? go(std::true_type()) : go(std::false_type())) return e;
   {
     FlashLaunch a;
     a.qk = qkg;

@@ -1,7 +1,7 @@
 // Triangle attention, projection stage: h = LN(x);  q | k | g = h Wq^T, h Wk^T, sigmoid(h Wg^T + b_g)  (pair-major,
 // bf16, row pitch 384) and V^T = Wv h^T (channel-major per line, bf16, pitch Nk), the layouts the flash
 // core reads.  x is the pair tensor for the starting node and its transpose for the ending node: a tile
-// is 128 consecutive `pos` on one `line`, pair (line, pos) = z[line][pos] or z[pos][line].
+// is two runs of 64 consecutive `pos`, each on one `line`, pair (line, pos) = z[line][pos] or z[pos][line].
 //
 //   warps 0-3   epilogue: q, k (lane = pair), then g (lane = pair) and V^T (lane = channel)
 //   warps 4-11  producers: load rows, LayerNorm, write the shared operand tile (A for q/k/g, B for V^T)
@@ -32,7 +32,8 @@ struct TriAttProjParams {
   float bias_scale;         // log2(e)
   int n_lines, n_pos, Nk;
   long long z_line_stride, z_pos_stride;  // bytes; starting node: line = row, ending node: line = column
-  int num_tiles;         // n_lines * ceil(n_pos/128)
+  int half_tiles;        // of a line; an odd number (HALF) has the tiles cut across lines
+  int num_tiles;         // ceil(n_lines * half_tiles / 2)
   float eps;
 };
 
@@ -47,7 +48,7 @@ constexpr uint32_t SMEM_BYTES = WB_OFF + 2048;       // exactly the 227 KB an SM
 constexpr int THREADS = 416;
 }  // namespace triatt_proj
 
-template <bool F32>
+template <bool F32, bool HALF>
 __global__ void __launch_bounds__(416, 1)
 triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQKG,
                    const __grid_constant__ CUtensorMap tmVT, const __grid_constant__ CUtensorMap tmWB,
@@ -72,7 +73,6 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
-  const int tiles_per_line = (p.n_pos + 127) >> 7;
 
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
@@ -164,13 +164,7 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     constexpr int G = 2;
     RowStream<F32, G, 4> rows;
     rows.place(pt);
-    auto row_ptr = [&](int tile) {
-      const int line = tile / tiles_per_line;
-      const int pos0 = (tile - line * tiles_per_line) << 7;
-      const uint8_t* base = static_cast<const uint8_t*>(p.z) + line * line_stride + pos0 * pos_stride;
-      const int left = p.n_pos - pos0 < 128 ? p.n_pos - pos0 : 128;
-      return [=](int r) -> const void* { return r < left ? base + r * pos_stride : nullptr; };
-    };
+    auto row_ptr = [&](int tile) { return TileRuns<HALF>(tile, p.half_tiles, p.n_lines).rows(p.z, p.n_pos, line_stride, pos_stride); };
     int it = 0;
     int tile = blockIdx.x;
     if (tile < p.num_tiles) {
@@ -193,8 +187,7 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const int r = warp * 32 + lane;  // TMEM lane: pair of the tile for q/k/g, channel for V^T
     int it = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
-      const int line = tile / tiles_per_line;
-      const int pos0 = (tile - line * tiles_per_line) << 7;
+      const TileRuns<HALF> t(tile, p.half_tiles, p.n_lines);
       // The 512 accumulator columns leave as eight [128 rows][64 values] bf16 tiles through two swizzled
       // staging tiles and TMA stores: q, k (4 tiles) and g + bias (2 tiles) with lane = pair into the pair-major
       // rows, V^T (2 tiles) with lane = channel into the line's channel-major plane.  TMEM is read 32 columns
@@ -220,8 +213,9 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             uint32_t bv[16];
             tmem_ld_32x16(tmem_addr(tmem_base, warp * 32, 0), bv);
             tmem_ld_wait();
-            if (pos0 + r < p.n_pos) {
-              __nv_bfloat16* dstb = p.tri_bias + (long long)line * p.bias_pitch + pos0 + r;
+            const int run = r >> 6, pos = t.pos_of(run) + (r & 63);
+            if ((run == 0 || t.there1) && pos < p.n_pos) {
+              __nv_bfloat16* dstb = p.tri_bias + (long long)t.line_of(run) * p.bias_pitch + pos;
 #pragma unroll
               for (int h = 0; h < 4; ++h) dstb[h * p.bias_plane] = __float2bfloat16(__uint_as_float(bv[h]) * p.bias_scale);
             }
@@ -260,10 +254,12 @@ triatt_proj_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           fence_proxy_async_smem();
           named_bar_sync(1, 128);
           if (leader) {
-            if (c < 12)
-              tma_store_3d(&tmQKG, stage, (c >> 1) * 64, pos0, line);
-            else
-              tma_store_3d(&tmVT, stage, pos0 + ((c >> 1) - 6) * 64, 0, line);
+            if (c < 12) {
+              tma_store_3d(&tmQKG, stage, (c >> 1) * 64, t.pos0[0], t.line[0]);
+              if (HALF && t.there1) tma_store_3d(&tmQKG, stage + kOperandHalf / 2, (c >> 1) * 64, t.pos0[1], t.line[1]);
+            } else if (c < 14 || t.there1) {
+              tma_store_3d(&tmVT, stage, t.pos_of((c >> 1) - 6), 0, t.line_of((c >> 1) - 6));
+            }
             tma_store_commit();
           }
         }

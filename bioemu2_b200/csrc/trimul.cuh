@@ -37,44 +37,6 @@ struct TriMulInParams {
   float eps;
 };
 
-// The two runs of 64 positions of a tile.  HALF: two consecutive half tiles, of one line or of two -- a line's last half tile need
-// not bring a second one of padding along: 160 positions are three halves, not four.  Else both of one line: one division and one
-// store a tile, for lines of an even number of halves.  PairMixer of 4 blocks, us, whole / half tiles: 160 tokens 398 / 357, 192 417 /
-// 368, 290 797 / 758, 320 874 / 844; with an even number 203 456 / 466, 256 549 / 568, 384 1032 / 1050.
-template <bool HALF>
-struct TileRuns {
-  int line[2], pos0[2];
-  bool there1;
-  __device__ __forceinline__ TileRuns(int tile, int half_tiles, int n_lines) {
-    if (HALF) {
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        line[k] = (2 * tile + k) / half_tiles;
-        pos0[k] = (2 * tile + k - line[k] * half_tiles) << 6;
-      }
-      there1 = line[1] < n_lines;
-    } else {
-      const int per_line = half_tiles >> 1;
-      line[0] = line[1] = tile / per_line;
-      pos0[0] = (tile - line[0] * per_line) << 7;
-      pos0[1] = pos0[0] + 64;
-      there1 = true;
-    }
-  }
-  __device__ __forceinline__ int line_of(int k) const { return HALF && k ? line[1] : line[0]; }
-  __device__ __forceinline__ int pos_of(int k) const { return HALF ? (k ? pos0[1] : pos0[0]) : pos0[0] + 64 * k; }
-  // Address of tile row r of a tensor of pair rows, nullptr where there is none.
-  __device__ __forceinline__ auto rows(const void* z, int n_pos, long long line_stride, long long pos_stride) const {
-    const uint8_t* base0 = static_cast<const uint8_t*>(z) + line[0] * line_stride + pos0[0] * pos_stride;
-    const uint8_t* base1 = HALF ? static_cast<const uint8_t*>(z) + line[1] * line_stride + (pos0[1] - 64) * pos_stride : base0;
-    const int left0 = n_pos - pos0[0], left1 = HALF ? (there1 ? n_pos - pos0[1] + 64 : 0) : left0;
-    return [=](int r) -> const void* {
-      if (!HALF) return r < left0 ? base0 + r * pos_stride : nullptr;
-      return r < 64 ? (r < left0 ? base0 + r * pos_stride : nullptr) : (r < left1 ? base1 + r * pos_stride : nullptr);
-    };
-  }
-};
-
 namespace trimul_in {
 constexpr uint32_t W_OFF = 0;                       // 4 M-tiles x 32 KB
 constexpr uint32_t X_OFF = 4 * kOperandTile;        // 2 stages x 32 KB

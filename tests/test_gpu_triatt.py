@@ -35,6 +35,26 @@ def test_triatt_vs_oracle(ending, N, dtype):
 
 
 @pytest.mark.parametrize("ending", [False, True])
+@pytest.mark.parametrize("N,dtype", [(131, torch.float32), (160, torch.bfloat16), (192, torch.float32), (319, torch.bfloat16)])
+def test_lines_of_an_odd_number_of_half_tiles(ending, N, dtype):
+    """Projection tiles that hold the end of one line and the start of the next, the last without a second half (131, 319); in place
+    the result is the update added, with a rounding of the update in `out` and one of the sum."""
+    g = torch.Generator().manual_seed(800 + N)
+    w = H.triatt_weights(g)
+    x = torch.randn(1, N, N, 128, generator=g).to(dtype)
+    mask = torch.rand(1, N, N, generator=g) > 0.2
+    ref = O.triangle_attention(x.double(), mask, {k: v.double() for k, v in w.items()}, 4, ending)
+    m = _module(w, ending)
+    with torch.no_grad():
+        out = m(x.cuda(), mask.cuda())
+        z = x.cuda()
+        m.forward_residual_(z, mask.cuda())
+    assert_close(f"half_tiles_{'end' if ending else 'start'}_N{N}_{dtype}", out, ref)
+    bound = 1.5 * torch.finfo(dtype).eps * (x.cuda().float().abs() + out.float().abs()) + 1e-6
+    assert ((z.float() - (x.cuda().float() + out.float())).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("ending", [False, True])
 def test_triatt_residual_inplace_and_padding(ending):
     N, P = 70, 6
     g = torch.Generator().manual_seed(77)
