@@ -28,7 +28,7 @@
 // exponentials at 16 per clock and SM that is 0.44 of the floor at 256 keys, 0.49 at 384 and 0.56 at 512.  K and V^T come once
 // per query tile: at 512 keys 672 MB are read from DRAM where every operand once would be 270 MB, 0.5 of the copy bandwidth.
 // One launch of triangle attention, 4 heads of 32 (ms, flash_core_kernel before -> here): N = 64 0.0143 -> 0.0082,
-// 128 0.0184 -> 0.0105, 203 0.0410 -> 0.0349, 256 0.0454 -> 0.0345, 512 0.263 -> 0.209.  For longer rows (a ring of bias tiles
+// 128 0.0184 -> 0.0105, 203 0.0410 -> 0.0323, 256 0.0454 -> 0.0339, 512 0.263 -> 0.208.  For longer rows (a ring of bias tiles
 // shared by the groups) this form drew enough power to pull the SM clock from 1.95 to 1.59 GHz and was slower (N = 1536: 6.1
 // against 5.3 ms), so those keep flash_core_kernel.  Tried without gain: part of the exponentials as a polynomial on the FMA
 // pipe, two threads per row, alternating the groups' exponential phases.

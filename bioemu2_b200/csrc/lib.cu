@@ -2349,8 +2349,8 @@ int b200_trunk_fwd(const b200_trunk_block* blocks, int n_blocks, const void* z_i
   const size_t zsz = zf32 ? 4 : 2;
   const int Nk = (N + 7) / 8 * 8;
   // The pair bias of a block reads z, which the next block writes for the first time two kernels on: where it and that block's first
-  // projection leave each other SMs, a tile each, it runs on the side stream beside them (4 blocks, us, on the main stream / beside: 24 tokens 450 / 441, 64 469 / 461; with 80
-  // tokens and more the two would take turns).
+  // projection leave each other SMs, a tile each, it runs on the side stream beside them (4 blocks, us, on the main stream / beside:
+  // 24 tokens 450 / 441, 64 469 / 461; with 80 tokens and more the two would take turns).
   const bool beside = two && 2 * N <= sm_count();
   for (int i = 0; i < n_blocks; ++i) {
     const b200_trunk_block& w = blocks[i];

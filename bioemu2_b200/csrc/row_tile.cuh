@@ -321,7 +321,7 @@ __device__ __forceinline__ void umma_k128(uint32_t d_tmem, uint32_t a_smem, uint
 // The two runs of 64 positions of a tile.  HALF: two consecutive half tiles, of one line or of two -- a line's last half tile need
 // not bring a second one of padding along: 160 positions are three halves, not four.  Else both of one line: one division and one
 // store a tile, for lines of an even number of halves.  PairMixer of 4 blocks, us, whole / half tiles: 160 tokens 398 / 357, 192 417 /
-// 368, 290 797 / 758, 320 874 / 844; with an even number 203 456 / 466, 256 549 / 568, 384 1032 / 1050; the
+// 368, 290 797 / 758, 320 874 / 844; with an even number 203 456 / 466, 256 549 / 568, 384 1032 / 1050.  The
 // projections of triangle attention take 30 and 40 us off a trunk of 4 blocks of 160 and 192 tokens (901 / 871, 960 / 920).
 template <bool HALF>
 struct TileRuns {
