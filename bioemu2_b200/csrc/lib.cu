@@ -1693,6 +1693,21 @@ int b200_pair_outer_sum(const float* a, const float* c, const float* extra, floa
   return B200_OK;
 }
 
+int b200_msa_features(const float* msa, const float* has_deletion, const float* deletion_value, const float* paired, void* out,
+                      int64_t rows, int nt, int pitch, b200_stream_t stream) {
+  if (int e = b200_check_device()) return e;
+  B200_CHECK_ARG(msa && has_deletion && deletion_value && out, "msa/has_deletion/deletion_value/out is NULL");
+  B200_CHECK_ARG(rows >= 0 && nt > 0 && pitch % 8 == 0 && pitch >= int64_t(nt) + (paired ? 3 : 2),
+                 "need nt > 0 and a pitch that is a multiple of 8 and holds every feature (nt=%d, pitch=%d)", nt, pitch);
+  B200_CHECK_ARG(aligned(msa, 4) && aligned(has_deletion, 4) && aligned(deletion_value, 4) && (!paired || aligned(paired, 4)) &&
+                     aligned(out, 16),
+                 "out must be 16-byte aligned");
+  if (rows == 0) return B200_OK;
+  B200_LAUNCH(msa_features_kernel, grid_for(rows * (pitch / 8), 256), 256, 0, static_cast<cudaStream_t>(stream), msa, has_deletion,
+              deletion_value, paired, static_cast<__nv_bfloat16*>(out), rows, nt, pitch);
+  return B200_OK;
+}
+
 int b200_add_rows(const float* x, const void* y, float* out, int64_t rows, int64_t period, int cols, int y_dtype,
                   b200_stream_t stream) {
   if (int e = b200_check_device()) return e;

@@ -569,6 +569,27 @@ def pair_outer_sum(a: Tensor, c: Tensor, extra: Tensor | None = None) -> Tensor:
     return z
 
 
+def msa_features(msa: Tensor, has_deletion: Tensor, deletion_value: Tensor, paired: Tensor | None = None) -> Tensor:
+    """``cat(msa, has_deletion, deletion_value[, paired])`` as bf16 rows zero-padded to a multiple of 8 columns.  One kernel for
+    contiguous fp32 features of one shape, copies for what else can be assigned to the columns."""
+    nt, extra = msa.shape[-1], [has_deletion, deletion_value] + ([] if paired is None else [paired])
+    pitch = (nt + len(extra) + 7) // 8 * 8
+    if all(t.dtype == torch.float32 and t.is_contiguous() and t.device == msa.device for t in (msa, *extra)) and msa.is_cuda \
+            and all(t.shape == msa.shape[:-1] for t in extra):
+        out = torch.empty(msa.shape[:-1] + (pitch,), dtype=torch.bfloat16, device=msa.device)
+        if out.numel():
+            _lib.check(lib.b200_msa_features(msa.data_ptr(), has_deletion.data_ptr(), deletion_value.data_ptr(),
+                                             None if paired is None else paired.data_ptr(), out.data_ptr(), out.numel() // pitch,
+                                             nt, pitch, _stream()))
+        return out
+    # one-hot rows and 0/1 flags are exact in bf16
+    out = torch.zeros(msa.shape[:-1] + (pitch,), dtype=torch.bfloat16, device=msa.device)
+    out[..., :nt] = msa
+    for i, t in enumerate(extra):
+        out[..., nt + i] = t
+    return out
+
+
 def add_rows(x: Tensor, y: Tensor, out: Tensor | None = None) -> Tensor:
     """``x + y`` for fp32 ``x[..., cols]`` where ``y`` (fp32 or bf16) has x's shape or only its trailing axes (it is
     then broadcast over the leading ones); ``out`` may be ``x``."""

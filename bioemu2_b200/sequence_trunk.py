@@ -96,18 +96,12 @@ class PairMixerMSAModule(nn.Module):
         """``msa_proj(cat(msa, has_deletion, deletion_value[, msa_paired])) + s_proj(emb)[:, None]`` as fp32
         ``[B, R, T, msa_s]`` (pairmixer.py:590-599).  ``tokens`` selects the token block a context-parallel rank holds:
         the MSA tensors then cover that block only, ``emb`` stays whole."""
-        B, R, T = msa.shape[:3]
+        B = msa.shape[0]
         width = self.msa_proj.in_features
-        # the MSA features as one zero-padded bf16 operand (one-hot rows and 0/1 flags are exact in bf16)
-        feat = torch.zeros(B, R, T, (width + 7) // 8 * 8, dtype=torch.bfloat16, device=msa.device)
         nt = msa.shape[-1]
-        feat[..., :nt] = msa
-        feat[..., nt] = has_deletion
-        feat[..., nt + 1] = deletion_value
-        if self.use_paired_feature:
-            feat[..., nt + 2] = msa_paired
         if nt + 2 + int(self.use_paired_feature) != width:
             raise ValueError(f"msa has {nt} feature columns, msa_proj expects {width - 2 - int(self.use_paired_feature)}")
+        feat = F.msa_features(msa, has_deletion, deletion_value, msa_paired if self.use_paired_feature else None)
         m = self._msa_proj(feat)                                    # fp32 [B, R, T, msa_s]
         e = self._s_proj(self._s_proj.operand(emb))                 # fp32 [B, tokens, msa_s]
         if tokens is not None:

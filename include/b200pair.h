@@ -398,6 +398,8 @@ int b200_gated_residual_fwd(void* x, const void* h, const float* cond, int cond_
  * b200_add_rows         out[r][:] = x[r][:] + y[r % period][:], x/out fp32 (out may be x), y fp32 or bf16: the residual
  *                       of the unconditional branch (pairmixer.py:268) with period = rows, and the broadcast of
  *                       s_proj(emb) over the MSA rows (pairmixer.py:598) with period = tokens.
+ * b200_msa_features     out[r][pitch] = msa[r][0..nt) | has_deletion[r] | deletion_value[r] [| paired[r]] | zeros, bf16 from fp32:
+ *                       the operand of msa_proj (pairmixer.py:590-597).  paired may be NULL.
  * b200_rows2_to_bf16    y = LN(x1[r] | x2[r]) * w + b as bf16 [rows][cols1 + cols2]: LayerNorm over the concatenation
  *                       of two row sources that is never materialised - cat(z_trunk, token_rel_pos_feats) of
  *                       PairwiseConditioning.forward (src/bioemu2/biomoa/modules/diffusion.py:526-529).
@@ -406,6 +408,8 @@ int b200_gated_residual_fwd(void* x, const void* h, const float* cond, int cond_
  * ------------------------------------------------------------------------------------------------- */
 int b200_pair_outer_sum(const float* a, const float* c, const float* extra, float* z, int n_i, int n_j, int cols,
                         b200_stream_t stream);
+int b200_msa_features(const float* msa, const float* has_deletion, const float* deletion_value, const float* paired, void* out,
+                      int64_t rows, int nt, int pitch, b200_stream_t stream);
 int b200_add_rows(const float* x, const void* y, float* out, int64_t rows, int64_t period, int cols, int y_dtype,
                   b200_stream_t stream);
 int b200_rows2_to_bf16(const void* x1, int cols1, const void* x2, int cols2, void* y, const float* w, const float* b,

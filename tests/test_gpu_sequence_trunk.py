@@ -44,6 +44,25 @@ def test_add_rows_plain_and_broadcast():
     assert F.add_rows(x, yb, out=x) is x and torch.equal(x, x0 + yb)
 
 
+@pytest.mark.parametrize("shape,nt", [((1, 1, 1), 33), ((2, 3, 37), 33), ((1, 5, 64), 5), ((1, 7, 11), 6), ((1, 0, 4), 33)])
+@pytest.mark.parametrize("paired", [False, True])
+def test_msa_features_are_the_rounded_concatenation(shape, nt, paired):
+    """Whole columns (5 + 3, 6 + 2) and padded ones; fp32 features, and forms that go by copies, give the same bits."""
+    from bioemu2_b200 import functional as F
+
+    g = torch.Generator().manual_seed(910)
+    msa = torch.randn(*shape, nt, generator=g).cuda()
+    cols = [torch.randn(*shape, generator=g).cuda() for _ in range(2 + paired)]
+    want = torch.cat([msa] + [c[..., None] for c in cols], -1).bfloat16()
+    got = F.msa_features(msa, *cols)
+    width = nt + len(cols)
+    assert got.shape == (*shape, (width + 7) // 8 * 8) and got.dtype == torch.bfloat16
+    assert torch.equal(got[..., :width], want) and not got[..., width:].any()
+    for other in (F.msa_features(msa.transpose(0, 2).contiguous().transpose(0, 2), *cols),
+                  F.msa_features(msa, cols[0].bfloat16().double(), *cols[1:])):
+        assert torch.equal(other, got)
+
+
 def test_two_source_layernorm_matches_the_concatenation():
     from bioemu2_b200 import functional as F
 
