@@ -96,11 +96,12 @@ class PairMixerMSAModule(nn.Module):
         """``msa_proj(cat(msa, has_deletion, deletion_value[, msa_paired])) + s_proj(emb)[:, None]`` as fp32
         ``[B, R, T, msa_s]`` (pairmixer.py:590-599).  ``tokens`` selects the token block a context-parallel rank holds:
         the MSA tensors then cover that block only, ``emb`` stays whole."""
-        B = msa.shape[0]
+        B, nt = msa.shape[0], msa.shape[-1]
         width = self.msa_proj.in_features
-        nt = msa.shape[-1]
         if nt + 2 + int(self.use_paired_feature) != width:
             raise ValueError(f"msa has {nt} feature columns, msa_proj expects {width - 2 - int(self.use_paired_feature)}")
+        if self.use_paired_feature and msa_paired is None:  # ``msa_features`` takes None for "no such column"
+            raise TypeError("use_paired_feature=True needs the msa_paired feature")
         feat = F.msa_features(msa, has_deletion, deletion_value, msa_paired if self.use_paired_feature else None)
         m = self._msa_proj(feat)                                    # fp32 [B, R, T, msa_s]
         e = self._s_proj(self._s_proj.operand(emb))                 # fp32 [B, tokens, msa_s]

@@ -7,6 +7,7 @@ import torch
 from bioemu2_b200 import _lib
 from bioemu2_b200 import functional as F
 from bioemu2_b200 import ieee
+from bioemu2_b200.sequence_trunk import PairMixerMSAModule
 
 
 @pytest.mark.parametrize("shape,mask,exc", [
@@ -53,6 +54,23 @@ class _OnDevice(torch.Tensor):
 def test_one_tensor_on_the_host(call):
     with pytest.raises(RuntimeError, match="CUDA tensors"):
         call(lambda *s: torch.zeros(s).as_subclass(_OnDevice), lambda *s: torch.zeros(s))
+
+
+def _msa(paired: bool, **kw):
+    m = PairMixerMSAModule(64, 64, 128, 16, 1, use_paired_feature=paired)
+    feats = dict(emb=torch.zeros(1, 5, 16), msa=torch.zeros(1, 3, 5, 33), has_deletion=torch.zeros(1, 3, 5),
+                 deletion_value=torch.zeros(1, 3, 5), msa_paired=torch.zeros(1, 3, 5) if paired else None)
+    return m.embed_msa(**{**feats, **kw})
+
+
+@pytest.mark.parametrize("tokens", [None, slice(0, 5)])
+def test_msa_embedding_without_its_paired_feature(tokens):
+    """With 33 token columns both widths are padded to 40, so the product alone would not notice."""
+    with pytest.raises(TypeError, match="msa_paired"):
+        _msa(True, msa_paired=None, tokens=tokens)
+    for paired in (True, False):
+        with pytest.raises(RuntimeError, match="CUDA tensors"):
+            _msa(paired, tokens=tokens)
 
 
 @pytest.mark.parametrize("width,heads", [(768, 16), (192, 16), (384, 8)])
