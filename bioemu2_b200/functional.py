@@ -574,8 +574,11 @@ def msa_features(msa: Tensor, has_deletion: Tensor, deletion_value: Tensor, pair
     contiguous fp32 features of one shape, copies for what else can be assigned to the columns."""
     nt, extra = msa.shape[-1], [has_deletion, deletion_value] + ([] if paired is None else [paired])
     pitch = (nt + len(extra) + 7) // 8 * 8
-    if all(t.dtype == torch.float32 and t.is_contiguous() and t.device == msa.device for t in (msa, *extra)) and msa.is_cuda \
-            and all(t.shape == msa.shape[:-1] for t in extra):
+
+    def rows(t, shape) -> bool:
+        return isinstance(t, Tensor) and t.dtype == torch.float32 and t.device == msa.device and t.shape == shape and t.is_contiguous()
+
+    if msa.is_cuda and rows(msa, msa.shape) and all(rows(t, msa.shape[:-1]) for t in extra):
         out = torch.empty(msa.shape[:-1] + (pitch,), dtype=torch.bfloat16, device=msa.device)
         if out.numel():
             _lib.check(lib.b200_msa_features(msa.data_ptr(), has_deletion.data_ptr(), deletion_value.data_ptr(),

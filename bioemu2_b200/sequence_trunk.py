@@ -96,6 +96,8 @@ class PairMixerMSAModule(nn.Module):
         """``msa_proj(cat(msa, has_deletion, deletion_value[, msa_paired])) + s_proj(emb)[:, None]`` as fp32
         ``[B, R, T, msa_s]`` (pairmixer.py:590-599).  ``tokens`` selects the token block a context-parallel rank holds:
         the MSA tensors then cover that block only, ``emb`` stays whole."""
+        if msa.dim() != 4:
+            raise ValueError(f"msa must be [batch, rows, tokens, columns], got {tuple(msa.shape)}")
         B, nt = msa.shape[0], msa.shape[-1]
         width = self.msa_proj.in_features
         if nt + 2 + int(self.use_paired_feature) != width:

@@ -73,6 +73,19 @@ def test_msa_embedding_without_its_paired_feature(tokens):
             _msa(paired, tokens=tokens)
 
 
+@pytest.mark.parametrize("shape", [(3, 5, 33), (1, 1, 3, 5, 33)])
+def test_msa_embedding_of_another_rank(shape):
+    with pytest.raises(ValueError, match="msa must be"):
+        _msa(False, msa=torch.zeros(shape), has_deletion=torch.zeros(shape[:-1]), deletion_value=torch.zeros(shape[:-1]))
+
+
+def test_msa_feature_columns_given_as_numbers_or_rows():
+    msa = torch.randn(2, 3, 5, 6)
+    got = F.msa_features(msa, True, torch.full((5,), 0.5), 0.25)
+    want = torch.cat([msa, torch.tensor([1.0, 0.5, 0.25]).expand(2, 3, 5, 3), torch.zeros(2, 3, 5, 7)], -1)
+    assert torch.equal(got, want.bfloat16())
+
+
 @pytest.mark.parametrize("width,heads", [(768, 16), (192, 16), (384, 8)])
 def test_trunk_single_track_of_another_width(width, heads):
     w = F.TrunkPacked([])
