@@ -4,8 +4,7 @@
 // (hi.hi + hi.lo + lo.hi) laid end to end along K: one operand reads hi | hi | lo, the other hi | lo | hi.  Activations whose
 // hi part is whole K blocks of 64 are stored once as (hi | lo) and the operands of the triangle contraction, whose K is the
 // token count, as hi and lo planes; the product's loads read hi twice.  All arithmetic here is fp32 with expf and exact
-// division (in the products' epilogues, which they would bind, times_sigmoid).  Every kernel is bound by memory: each reads its
-// input once, 16 bytes a lane, and writes its output once.
+// division.  Every kernel is bound by memory: each reads its input once, 16 bytes a lane, and writes its output once.
 #pragma once
 #include "elementwise.cuh"
 

@@ -59,14 +59,17 @@ enum BmmEpilogue : int {
   kEpiMul = 2,
   kEpiAdd = 6,     // the same with fp32 addends: a residual that is not C itself
   kEpiSwiglu = 3,  // bulk bf16: the columns are pairs of 64-column blocks (a | b), C gets silu(a) * b, half as many columns
-  kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b
+  kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b, see kEpiGateSplit
   // kEpiBulk with eight epilogue warps, each group of four draining half of the tile's columns: a short product's tile is
   // its epilogue (K = 128: 2 K blocks of 64 against 128 columns of TMEM reads, staging and stores a lane).
   kEpiBulkWide = 7,
   // Gated operands of the accurate triangle contraction, from split operands: the weights' 256 rows are p and g of 128
   // channels and take the M side, so a lane is a channel and its columns are consecutive pairs -- the order in which the
   // contraction reads them.  C gets hi and lo of p * sigmoid(g) (masked pairs zero) as rows part *
-  // 128 + channel of column tile tn.  (Projection to fp32 and a gate kernel over it: 26 + 33 us for 40000 pairs.)
+  // 128 + channel of column tile tn.  (Projection to fp32 and a gate kernel over it: 26 + 33 us for 40000 pairs.)  Both split
+  // epilogues keep fp32: expf and the refined quotient.  Transition of 40000 rows / triangle multiplication of 200 tokens, us:
+  // with the compiler's division, whose rare cases are a branch per value, 98 / 117, refined 82 / 108, with the hardware's
+  // exponential and reciprocal alone 79 / 104 (a rounded argument costs the exponential 2^-18 of its value at 64).
   kEpiGateSplit = 8,
   kEpiOuter = 5,   // outer products of 32 x 32, one pair's 2 KB in one piece
 };
@@ -367,8 +370,8 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             mbar_arrive(&acc_empty[acc]);
           }
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            va[e] = (keep[c] >> e) & 1 ? __float_as_uint(times_sigmoid(__uint_as_float(va[e]), __uint_as_float(vb[e]))) : 0u;
+          for (int e = 0; e < 32; ++e)  // an AND masks: a selection would be a branch around each value (114 us for the op)
+            va[e] = __float_as_uint(times_sigmoid(__uint_as_float(va[e]), __uint_as_float(vb[e]))) & (0u - ((keep[c] >> e) & 1u));
           if (c == 0) {
             if (leader) tma_store_wait_read0();  // the stores that last used the staging tiles have read them
             named_bar_sync(1 + grp, 128);

@@ -429,10 +429,19 @@ __device__ __forceinline__ float exp2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// num * sigmoid(x) = num / (1 + 2^(-x log2 e)) for the fp32-accurate forms: hardware exponential and reciprocal, about 2^-21
-// relative each, where the split operands around it carry 2^-16 (with expf and exact division, some twenty instructions more per
-// element, the two products of 40000 rows that have it in their epilogue take 63 and 37 us instead of 39 and 26).
-__device__ __forceinline__ float times_sigmoid(float num, float x) { return __fdividef(num, 1.0f + exp2_approx(-1.4426950408889634f * x)); }
+// num / den for 1 <= den <= inf: the hardware's reciprocal (within an ulp) and one refinement of the quotient by its remainder, which
+// a fused multiply-add gives exactly (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990).  The division's result but for about one quotient in four million, whose neighbour it is; six instructions in a straight
+// line, where the division's rare cases keep a loop's iterations from overlapping.
+__device__ __forceinline__ float quotient(float num, float den) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(den));
+  const float q = num * r;
+  const float refined = fmaf(fmaf(-q, den, num), r, q);
+  return den < INFINITY ? refined : q;  // no remainder of an infinity
+}
+// num * sigmoid(x) for the fp32-accurate forms.
+__device__ __forceinline__ float times_sigmoid(float num, float x) { return quotient(num, 1.0f + expf(-x)); }
 // Packed fp32 pair add (one FMA-pipe instruction for two lanes' worth of values) and three-input maximum.
 __device__ __forceinline__ void add_f32x2(float& a0, float& a1, float b0, float b1) {
   asm("{ .reg .b64 ra, rb; mov.b64 ra, {%0, %1}; mov.b64 rb, {%2, %3}; add.rn.f32x2 ra, ra, rb; mov.b64 {%0, %1}, ra; }"

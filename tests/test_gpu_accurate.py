@@ -57,3 +57,35 @@ def test_transition(rows, dim, hidden, out, norm):
         assert _rel(got, want) < 5e-5
         if out == dim:
             torch.testing.assert_close(m.forward_residual_(x.clone()), x + got, atol=1e-5, rtol=1e-5)
+
+
+def test_swiglu_keeps_fp32_where_the_gate_is_nearly_shut():
+    """silu(a) * b far below zero, where an exponential whose argument is rounded to a multiple of 2^-17 shows.  What the output
+    keeps of a value is its (hi | lo): lo is at most half a unit of hi's eighth bit and is rounded to eight bits itself, 2^-17
+    of the value at the most and, over evenly spread significands, 0.32 * 2^-17 = 2.4e-6 in the root mean square."""
+    import bioemu2_b200 as b
+
+    rows = 4096
+    m = b.Transition(128, 64, 64, use_norm=False).eval().cuda()
+    with torch.no_grad():
+        for p in m.parameters():
+            p.zero_()
+        m.fc1.weight[:, 0] = 1.0
+        m.fc2.weight[:, 1] = 1.0
+        m.fc3.weight.copy_(torch.eye(64))
+    g = torch.Generator().manual_seed(61)
+    a = (-40.0 - 40.0 * torch.rand(rows, generator=g)).cuda()
+    hi = a.bfloat16()
+    a = hi.float() + (a - hi.float()).bfloat16().float()  # what the product's split operands hold
+    x = torch.zeros(rows + 5, 128, device="cuda")
+    x[:rows, 0], x[:, 1] = a, 2.0 ** 60
+    x[rows:, 0] = torch.tensor([-88.0, -89.0, -3.0e5, 0.0, float("nan")])
+    x[rows + 3, 1] = 3.0
+    with torch.no_grad(), b.precision.matmul_precision("ieee"):
+        got = m(x).double()
+    assert torch.equal(got[:-1, :1].expand(-1, 64), got[:-1])
+    want = a.double() * torch.sigmoid(a.double()) * 2.0 ** 60
+    rel = (got[:rows, 0] - want) / want
+    assert rel.abs().max() <= 2.0 ** -17 + 2.0 ** -21
+    assert rel.square().mean().sqrt() < 2.6e-6
+    assert got[rows, 0] != 0 and not got[rows + 1:rows + 4].any() and not torch.isnan(got[:-1]).any() and torch.isnan(got[-1]).all()
