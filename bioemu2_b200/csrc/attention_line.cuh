@@ -1,6 +1,7 @@
 // Triangle attention of short lines with the output projection: a CTA takes one line of up to 128 positions, all four heads of 32, and adds
 // the projected update into the pair tensor.  Attention and gate as in flash_resident_kernel; a head's gated output goes to shared
-// memory as the operand of  out += og W_o^T  instead of through global memory and a product of its own.
+// memory as the operand of  out += og W_o^T  instead of through global memory and a product of its own.  An fp32 pair tensor gets the
+// sum from the memory (reduce-add); a bf16 one is read, added in fp32 and rounded once, which a reduction in bf16 would do twice.
 //
 //   warps 0-7    two groups of four softmax warps, heads g and g + 2 one after the other; then 64 output channels each
 //   warps 8, 9   MMA issuers of the groups (8 also of the output projection)
@@ -53,6 +54,7 @@ line_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint64_t* s_empty = gb + 3;     // count 128: the scores have been read
   uint64_t* p_full = gb + 4;      // count 128
   uint64_t* pv_done = gb + 5;     // commit: O; V^T may be loaded again
+  uint64_t* z_full = gb + 6;      // TMA: the pair tensor's rows (bf16)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
@@ -60,7 +62,7 @@ line_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     mbar_init(out_full, 1);
     for (int i = 0; i < 2; ++i) {
       uint64_t* x = bars + 4 + i * 8;
-      for (int j = 0; j < 6; ++j) mbar_init(&x[j], (j == 3 || j == 4) ? 128 : 1);
+      for (int j = 0; j < 7; ++j) mbar_init(&x[j], (j == 3 || j == 4) ? 128 : 1);
     }
     fence_mbar_init();
     prefetch_tmap(&tmQ);
@@ -110,6 +112,11 @@ line_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           tma_load_2d(smem + W_OFF, &tmW, w_full, 0, 0);
           tma_load_2d(smem + W_OFF + kOperandHalf, &tmW, w_full, 64, 0);
         }
+      }
+      if (!F32) {
+        mbar_wait(s_full, 1, 181);  // the second head's bias tile has been multiplied
+        mbar_arrive_expect_tx(z_full, kOperandHalf);
+        tma_load_3d(smem + BIAS_OFF + g * kOperandTile, &tmO, z_full, g * 64, 0, b);
       }
     }
   } else if (warp >= 8) {
@@ -297,17 +304,25 @@ line_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         *reinterpret_cast<float4*>(stage + (q >> 3) * kOperandHalf + sw128_offset(r, q & 7)) =
             make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
     } else {
+      mbar_wait(z_full, 0, 182);
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<uint4*>(stage + sw128_offset(r, q)) =
-            make_uint4(pack_bf16x2(v[q * 8], v[q * 8 + 1]), pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]), pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]),
-                       pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]));
+      for (int q = 0; q < 8; ++q) {
+        uint4* unit = reinterpret_cast<uint4*>(stage + sw128_offset(r, q));
+        uint32_t w[4] = {unit->x, unit->y, unit->z, unit->w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = pack_bf16x2(v[q * 8 + 2 * e] + bf16lo(w[e]), v[q * 8 + 2 * e + 1] + bf16hi(w[e]));
+        *unit = make_uint4(w[0], w[1], w[2], w[3]);
+      }
     }
     fence_proxy_async_smem();
     named_bar_sync(1 + g, 128);
     if ((threadIdx.x & 127) == 0) {
-      tma_reduce_add_3d(&tmO, stage, g * 64, 0, b);
-      if (F32) tma_reduce_add_3d(&tmO, stage + kOperandHalf, g * 64 + 32, 0, b);
+      if (F32) {
+        tma_reduce_add_3d(&tmO, stage, g * 64, 0, b);
+        tma_reduce_add_3d(&tmO, stage + kOperandHalf, g * 64 + 32, 0, b);
+      } else {
+        tma_store_3d(&tmO, stage, g * 64, 0, b);
+      }
       tma_store_commit();
       tma_store_wait0();
     }

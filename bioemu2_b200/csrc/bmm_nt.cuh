@@ -57,7 +57,7 @@ enum BmmEpilogue : int {
   // come by TMA during the product's K loop (read by the lanes from their rows: 16 against 9 us without the gate for
   // 2048 x 768 x 768, 23 against 13 for K = 3072).
   kEpiMul = 2,
-  kEpiAdd = 6,     // the same with fp32 addends: a residual that is not C itself
+  kEpiAdd = 6,     // the same with addends of C's type: an fp32 residual that is not C itself, or a bf16 C that is to be rounded once
   kEpiSwiglu = 3,  // bulk bf16: the columns are pairs of 64-column blocks (a | b), C gets silu(a) * b, half as many columns
   kEpiSwigluSplit = 4,  // the same from split operands: C gets (hi | lo) of silu(a) * b, see kEpiGateSplit
   // kEpiBulk with eight epilogue warps, each group of four draining half of the tile's columns: a short product's tile is
@@ -224,6 +224,13 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     auto load_factors = [&](int tile) {
       const int rem = tile % tiles_per_batch;
       const int tm = rem / p.tiles_n, tn = rem - tm * p.tiles_n;
+      if (EPI == kEpiAdd && !p.out_f32) {  // [128 rows][64 columns] of C itself
+        mbar_arrive_expect_tx(mul_full, Cfg::MUL_BYTES / 2);
+#pragma unroll
+        for (int c = 0; c < BN / 64; ++c)
+          tma_load_3d(smem + Cfg::MUL_OFFSET + c * 16384, &tmM, mul_full, tn * BN + c * 64, tm * 128, tile / tiles_per_batch);
+        return;
+      }
       mbar_arrive_expect_tx(mul_full, Cfg::MUL_BYTES);
 #pragma unroll
       for (int c = 0; c < BN / 32; ++c)
@@ -463,6 +470,12 @@ bmm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
                 const float4 m1 = *reinterpret_cast<const float4*>(factors + sw128_offset(r, g * 2 + 1));
                 x[0] *= m0.x; x[1] *= m0.y; x[2] *= m0.z; x[3] *= m0.w;
                 x[4] *= m1.x; x[5] *= m1.y; x[6] *= m1.z; x[7] *= m1.w;
+              }
+              if (EPI == kEpiAdd) {
+                const uint4 a4 = *reinterpret_cast<const uint4*>(smem + Cfg::MUL_OFFSET + (c >> 1) * 16384 + sw128_offset(r, (c & 1) * 4 + g));
+                const uint32_t aw[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[2 * e] += bf16lo(aw[e]), x[2 * e + 1] += bf16hi(aw[e]);
               }
               *reinterpret_cast<uint4*>(stage + sw128_offset(r, (c & 1) * 4 + g)) = make_uint4(
                   pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));

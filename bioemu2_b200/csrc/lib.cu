@@ -101,6 +101,7 @@ struct BmmLaunch {
   int out_f32 = 0;
   int opm_ntok = 0;
   const void* residual = nullptr;
+  bool round_once = false;  // bf16 residual in C itself: read, added in fp32 and rounded once, not reduced into memory in bf16
   bool b_shared = false;  // one B for every batch item
   const float* mul = nullptr;  // bulk output: per-element fp32 factor, row pitch mul_pitch
   int mul_pitch = 0;
@@ -146,12 +147,12 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   const int64_t c_batch = a.sc > 0 ? a.sc : a.ldc * int64_t(a.M);
   const int c_esz = a.out_f32 ? 4 : 2;
   // Bulk output through the C tensor map where the layout allows it (the map clips the last column group): the
-  // residual (if any) being C itself, and for the transposed pair store lines that are whole row tiles.
+  // residual (if any) being C itself.
   const bool bulk_c = a.opm_ntok == 0 && (a.ldc * c_esz) % 16 == 0 && (c_batch * c_esz) % 16 == 0 && aligned(a.C, 16);
   // An fp32 residual elsewhere comes by TMA tiles, as a gate's factors do (read by the lanes from their rows: 11 us against 7
-  // for 65536 x 128 x 128).
-  const bool add = bulk_c && a.residual && a.residual != a.C && a.out_f32 && a.batch == 1 && !a.mul &&
-                   !a.swiglu && aligned(a.residual, 16);
+  // for 65536 x 128 x 128), and so does a bf16 one that is rounded once.
+  const bool add = bulk_c && a.residual && !a.mul && !a.swiglu &&
+                   (a.out_f32 ? a.residual != a.C && a.batch == 1 && aligned(a.residual, 16) : a.residual == a.C && a.round_once);
   // 64-wide tiles: bulk output of whole rows
   const bool narrow = bulk_c && (add || a.residual == nullptr || a.residual == a.C) && (a.bias == nullptr || aligned(a.bias, 16)) &&
                       !a.swiglu && a.opm_ntok == 0 && a.row_groups == 0;
@@ -231,7 +232,7 @@ static int launch_bmm(const BmmLaunch& a, cudaStream_t stream) {
   if ((a.mul || a.swiglu) && (!p.tma_c || (a.mul && (!aligned(a.mul, 16) || a.mul_pitch % 4 || a.batch != 1))))
     return fail(B200_ERR_INVALID_ARGUMENT, "a gated product needs bulk output and 16-byte aligned factors");
   CUtensorMap tmM = tmC;
-  if (a.mul || add) {
+  if (a.mul || (add && a.out_f32)) {
     const uint64_t dims[2] = {uint64_t(a.N), uint64_t(a.M)};
     const uint64_t str[1] = {uint64_t(add ? a.ldc : a.mul_pitch) * 4};
     const uint32_t box[2] = {32, 128};
@@ -1493,7 +1494,9 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
   {
     // Pair (line, pos) of the ending node lives in row pos * lines + line: a batch item per line, its rows a line of pairs apart, so
     // that lines of any length leave by TMA tiles (stored by the lanes where a line is not whole tiles of 128: 20 us against 10 for
-    // 203 tokens).
+    // 203 tokens).  In bf16 those lines are read back and rounded once, 13 us.  The starting node's and lines of whole tiles are reduced
+    // into memory, with a rounding of the update and one of the sum: read back, a whole call takes 72 us instead of 66 at 256
+    // tokens and 316 instead of 300 at 512.
     BmmLaunch a{og, w->w_o, out, 1, lines * pos, kD, kD, kD, kD, kD, 0, 0, 0};
     if (ending) {
       a.batch = lines, a.M = pos, a.ldc = int64_t(lines) * kD;
@@ -1502,6 +1505,7 @@ static int triatt_slab(const void* z, const uint8_t* mask, const void* ext_bias,
     }
     a.out_f32 = f32;
     a.residual = add_residual ? z : nullptr;
+    a.round_once = ending && !f32 && pos % 128 != 0;
     if (int e = launch_bmm(a, stream)) return e;
   }
   return B200_OK;

@@ -112,3 +112,26 @@ def test_short_lines_in_place_are_the_update_added(N, B, ending, dtype, scale):
         assert torch.equal(got, want)
     else:
         torch.testing.assert_close(got.float(), want, rtol=2 ** -8, atol=2 ** -9 * want.abs().max().item())
+
+
+@pytest.mark.parametrize("N,B,ending", [(1, 1, True), (24, 1, False), (65, 2, True), (100, 1, True), (128, 1, False), (128, 1, True),
+                                        (129, 1, True), (150, 2, True), (203, 1, True), (300, 1, True)])
+def test_bf16_update_added_in_place_is_rounded_once(N, B, ending):
+    """Short lines, and ending-node lines that are not whole tiles of 128: the bf16 result is the rounding of what the same rows
+    give in fp32 (the projection's fp32 result rounded to bf16 before the sum would be off in 3 % to 7 % of the values)."""
+    import bioemu2_b200 as b
+    from bioemu2_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(3300 + N)
+    with torch.device("cuda"):
+        m = b.TriangleAttention(ending=ending).eval()
+    with torch.no_grad():
+        for p in m.parameters():
+            if p.ndim >= 2:
+                p.uniform_(-128 ** -0.5, 128 ** -0.5, generator=g)
+        z = torch.randn(B, N, N, 128, device="cuda", generator=g).bfloat16()
+        mask = torch.rand(B, N, N, device="cuda", generator=g) > 0.2
+        want = m.forward_residual_(z.float(), mask).bfloat16()
+        got = m.forward_residual_(z.clone(), mask)
+    assert _lib.device_status() == 0
+    assert torch.equal(got, want)
