@@ -8,7 +8,7 @@
 // All weights (64 KB and 192 KB a transition) stream from L2 through one ring of 16 KB units in the order in which the products
 // take them.
 //
-//   warps 0-7    two groups of four: LayerNorm of 64 channels of z each (the sums of a row's halves meet in shared memory), the
+//   warps 0-7    two groups of four: LayerNorm of 64 channels of z each (a row's halves meet in shared memory), the
 //                SwiGLU of the even / odd chunks of 64 hidden units, 64 channels of the finished tile to TMA
 //   warps 8-13   producers: LayerNorm of the next tile's source rows into the operand S
 //   warp  14     issues all products
@@ -52,7 +52,7 @@ constexpr int CHUNKS = 4, UNITS = 5;
 constexpr uint32_t S_OFF = 0;                                 // two sources x 32 KB
 constexpr uint32_t W_OFF = 2 * kOperandTile;                  // ring of units, [128 rows][64 K]
 constexpr uint32_t STAGE_OFF = W_OFF + UNITS * kOperandHalf;  // the finished tile, four times [128 rows][32 channels] fp32
-constexpr uint32_t XCH_OFF = STAGE_OFF + 2 * kOperandTile;    // sums of the LayerNorm, [2 groups][128 rows] x 2 fp32
+constexpr uint32_t XCH_OFF = STAGE_OFF + 2 * kOperandTile;    // mean and squares of the rows' halves, [2 groups][128 rows] x 2 fp32
 constexpr uint32_t LN_OFF = XCH_OFF + 2048;                     // the transitions' weight and half bias, [128] fp32 each
 constexpr uint32_t BAR_OFF = LN_OFF + kPairCondMaxTransitions * 1024;
 constexpr uint32_t SMEM_BYTES = BAR_OFF + 512 + 1024;
@@ -324,23 +324,27 @@ pair_cond_kernel(const __grid_constant__ PairCondMaps maps, const __grid_constan
           tmem_ld_32x32_f(z_addr, v);
           tmem_ld_32x32_f(z_addr + 32, v + 32);
           tmem_ld_wait();
-          // Sum and sum of squares together, one exchange: in fp32 the variance then errs by about 1e-7 (1 + mean^2 / var).
+          // A half's sum of squares about its own mean, then one exchange: mean and variance of the row are those of its halves, d on
+          // either side of the mean (T. Chan, G. Golub, R. LeVeque, "Updating formulae and a pairwise algorithm for computing sample
+          // variances", 1979).  The mean of the squares less the square of the mean has no digits left where a row's mean is a
+          // thousand times its deviation.
           float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, q0[4] = {0.f, 0.f, 0.f, 0.f}, q1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
+          for (int e = 0; e < 64; e += 2) add_f32x2(s0[(e >> 1) & 3], s1[(e >> 1) & 3], v[e], v[e + 1]);
+          const float mu = (((s0[0] + s1[0]) + (s0[1] + s1[1])) + ((s0[2] + s1[2]) + (s0[3] + s1[3]))) * (1.0f / 64);
+#pragma unroll
           for (int e = 0; e < 64; e += 2) {
-            add_f32x2(s0[(e >> 1) & 3], s1[(e >> 1) & 3], v[e], v[e + 1]);
+            add_f32x2(v[e], v[e + 1], -mu, -mu);
             fma_f32x2(q0[(e >> 1) & 3], q1[(e >> 1) & 3], v[e], v[e + 1], v[e], v[e + 1], q0[(e >> 1) & 3], q1[(e >> 1) & 3]);
           }
-          float sum = 0.f, sq = 0.f;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) sum += s0[e] + s1[e], sq += q0[e] + q1[e];
-          xch[grp * 128 + r] = make_float2(sum, sq);
+          const float sq = ((q0[0] + q1[0]) + (q0[1] + q1[1])) + ((q0[2] + q1[2]) + (q0[3] + q1[3]));
+          xch[grp * 128 + r] = make_float2(mu, sq);
           named_bar_sync(3, COMPUTE);
           const float2 other = xch[(grp ^ 1) * 128 + r];
-          const float mean = (sum + other.x) * (1.0f / kD);
+          const float d = 0.5f * (other.x - mu);
           // half of the LayerNorm: see the SwiGLU below
-          const float rstd = 0.5f * rsqrtf(fmaxf((sq + other.y) * (1.0f / kD) - mean * mean, 0.f) + p.eps);
-          const float shift = -mean * rstd;
+          const float rstd = 0.5f * rsqrtf((sq + other.y) * (1.0f / kD) + d * d + p.eps);
+          const float shift = -d * rstd;
           mbar_wait(x_empty, (n & 1) ^ 1, 130);
           tc_fence_after_sync();
           const float4* gw = reinterpret_cast<const float4*>(ln + t * 256 + grp * 64);

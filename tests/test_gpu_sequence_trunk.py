@@ -135,6 +135,26 @@ def test_pairwise_conditioning_shapes(B, n_i, n_j, transitions, factor, dtype):
     assert_close(f"pairwise_conditioning_{B}x{n_i}x{n_j}_{transitions}_{factor}_{dtype}", out, ref, atol=4e-2)
 
 
+@pytest.mark.parametrize("transitions", [1, 2, 3])
+def test_pairwise_conditioning_of_rows_far_from_zero(transitions):
+    """Rows of z whose mean is two thousand times their deviation: the LayerNorms in between have to find the deviation (three
+    transitions go pass by pass).  Channel 0 of the input's LayerNorm is constant and adds 1024 to all of z, exactly; z itself then
+    has 2^-13 of a unit, the operands bf16's 2^-9 as ever."""
+    import bioemu2_b200 as b
+
+    g = torch.Generator().manual_seed(917)
+    w = H.pairwise_conditioning_weights(g, num_transitions=transitions)
+    w["dim_pairwise_init_proj.0.weight"][0], w["dim_pairwise_init_proj.0.bias"][0] = 0.0, 2.0
+    w["dim_pairwise_init_proj.1.weight"][:, 0] = 512.0
+    z, rel = (torch.randn(1, 20, 13, 128, generator=g) for _ in range(2))
+    ref = O.pairwise_conditioning(z.double(), rel.double(), {k: v.double() for k, v in w.items()}, transitions)
+    m = b.PairwiseConditioning(128, 128, num_transitions=transitions).eval()
+    m.load_state_dict(w, strict=True)
+    with torch.no_grad():
+        out = m.cuda()(z.cuda(), rel.cuda())
+    assert_close(f"pairwise_conditioning_far_{transitions}", out.double() - 1024, ref - 1024, atol=4e-2)
+
+
 # ------------------------------------------------------------------------------------------ MSA module, trunk
 def test_msa_module_golden():
     import bioemu2_b200 as b
