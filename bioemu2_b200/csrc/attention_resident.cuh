@@ -401,7 +401,7 @@ flash_resident_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             if ((wa | wb) == 0 && (only_masked || first || !shifted)) {
               if (first) {
                 only_masked = shifted = true;
-              rare = 3u;
+                rare = 3u;
                 m_ref = kNegMasked;
               }
               const int ones = only_masked ? p.N - (t * 128 + h * 64) : 0;

@@ -1925,8 +1925,9 @@ size_t b200_trunk_side_workspace_bytes(const b200_trunk_block* blocks, int n_blo
   return need;
 }
 
-// The events that order the two streams of a trunk call: two "bias ready", two "bias read", one for the joins.  Kept per
-// host thread and device -- an event may be recorded again as soon as the waits on it have been enqueued.
+// The events that order the two streams of a trunk call: two "bias ready", two "bias read", one for the joins, and one for z
+// read by a pair bias on the side stream.  Kept per host thread and device -- an event may be recorded again as soon as the
+// waits on it have been enqueued.
 struct TrunkEvents {
   cudaEvent_t ev[6] = {};
   int dev = -1;
