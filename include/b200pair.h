@@ -436,8 +436,9 @@ int b200_window_attention_fwd(const void* qkv, const void* gate, const float* bi
 int b200_window_attention_pitched_fwd(const void* qkv, int qkv_pitch, const void* gate, int gate_pitch, const float* bias,
                                       const uint8_t* mask, void* out, int B, int M, int NW, int W, int Hk, int heads,
                                       int head_dim, b200_stream_t stream);
-/* Both calls in one: the bias of z as b200_window_bias_fwd computes it, then the attention.  `bias` holds
- * B*NW*heads*W*Hk floats of scratch for the shapes that go by way of it (all but 16-query tiles, 128 keys, c_z = 16). */
+/* Both calls in one: the bias of z as b200_window_bias_fwd computes it, then the attention.  `bias` must always hold
+ * B*NW*heads*W*Hk floats: whether the bias goes by way of it depends on the number of windows and samples, on the heads and on
+ * the alignment of z too, not on the window alone. */
 int b200_window_pair_attention_fwd(const void* qkv, int qkv_pitch, const void* gate, int gate_pitch, const void* z,
                                    const float* ln_w, const float* ln_b, const float* w_z, const uint8_t* mask, void* out,
                                    float* bias, int B, int M, int NW, int W, int Hk, int heads, int head_dim, int c_z,

@@ -107,3 +107,43 @@ def test_window_attention_shape_errors():
         mod(s, torch.zeros(1, 2, 32, 96, 16).cuda(), torch.ones(2, 32, dtype=torch.bool).cuda())
     with pytest.raises(ValueError, match="inconsistent shapes"):
         mod(s, torch.zeros(1, 3, 32, 128, 16).cuda(), torch.ones(3, 32, dtype=torch.bool).cuda())
+
+
+@pytest.mark.parametrize("B,M,NW,heads,dh,offset", [
+    (1, 8, 16, 4, 32, 0),    # too few windows and samples for the one kernel
+    (1, 8, 32, 4, 32, 0),    # the one kernel
+    (1, 8, 32, 4, 32, 4),    # the same, but for a pair tensor that starts off 32 bytes
+    (1, 8, 32, 2, 64, 0),    # head dim 64
+    (2, 3, 75, 4, 32, 0),    # more windows than SMs
+])
+def test_window_pair_attention_scratch(B, M, NW, heads, dh, offset):
+    """The C entry with as much scratch as its header asks for, whichever way the bias goes: what lies around it stays as it was."""
+    from bioemu2_b200 import _lib
+    from bioemu2_b200._lib import lib
+
+    W, Hk, c_z, D = 32, 128, 16, heads * dh
+    g = torch.Generator(device="cuda").manual_seed(1103 + NW)
+
+    def randn(*shape):
+        return torch.randn(*shape, device="cuda", generator=g)
+
+    qkvg = randn(B * M, NW * W, 4 * D).bfloat16()
+    z = randn(B * NW * W * Hk * c_z + offset)[offset:]
+    ln_w, ln_b, w_z = randn(c_z), randn(c_z), randn(heads, c_z)
+    mask = (torch.rand(B, NW * W, device="cuda", generator=g) > 0.1).to(torch.uint8)
+    n, guard = B * NW * heads * W * Hk, 4096
+    scratch = torch.full((n + 2 * guard,), 7.0, device="cuda")
+    out, want = (torch.empty(B * M, NW * W, D, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    bias = torch.empty(n, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    q, gate = qkvg.data_ptr(), qkvg.data_ptr() + 6 * D
+    _lib.check(lib.b200_window_pair_attention_fwd(q, 4 * D, gate, 4 * D, z.data_ptr(), ln_w.data_ptr(), ln_b.data_ptr(), w_z.data_ptr(),
+                                                  mask.data_ptr(), out.data_ptr(), scratch.data_ptr() + 4 * guard, B, M, NW, W, Hk,
+                                                  heads, dh, c_z, 0, st))
+    _lib.check(lib.b200_window_bias_fwd(z.data_ptr(), ln_w.data_ptr(), ln_b.data_ptr(), w_z.data_ptr(), bias.data_ptr(), B * NW, W, Hk,
+                                        c_z, heads, 0, st))
+    _lib.check(lib.b200_window_attention_pitched_fwd(q, 4 * D, gate, 4 * D, bias.data_ptr(), mask.data_ptr(), want.data_ptr(), B, M, NW,
+                                                     W, Hk, heads, dh, st))
+    assert _lib.device_status() == 0
+    assert (scratch[:guard] == 7).all() and (scratch[-guard:] == 7).all()
+    assert_close(f"window_pair_scratch_{NW}_{heads}_{offset}", out, want)
