@@ -79,3 +79,24 @@ def test_two_stream_trunk_loop_equals_the_serial_loop():
         s2, z2 = trunk.forward_(s.clone(), z.clone(), tok, pm, overlap=False)
         torch.cuda.synchronize()
     assert torch.equal(z1, z2) and torch.equal(s1, s2)
+
+
+@pytest.mark.parametrize("N", [24, 72, 74, 75])
+def test_pair_bias_beside_the_next_block_equals_the_serial_loop(N):
+    """Up to 74 tokens (a tile each on half of the SMs) a block's pair bias is read from z on the side stream while the next block's
+    first projection runs, and that block's output waits for it; with 75 it runs on the main stream.  Two pair tensors, of which only
+    the first waits; five blocks, so that both bias buffers come round again; other inputs in every pass."""
+    import bioemu2_b200 as b
+
+    torch.manual_seed(46)
+    trunk = b.PairformerModule(384, 128, 5).eval().cuda()
+    g = torch.Generator().manual_seed(47 + N)
+    tok = torch.ones(2, N, dtype=torch.bool, device="cuda")
+    tok[0, N - 5:] = False
+    pm = (tok[:, :, None] & tok[:, None, :]).to(torch.uint8)
+    with torch.no_grad():
+        for _ in range(6):
+            s, z = torch.randn(2, N, 384, generator=g).cuda(), torch.randn(2, N, N, 128, generator=g).cuda()
+            s1, z1 = trunk.forward_(s.clone(), z.clone(), tok, pm, overlap=True)
+            s2, z2 = trunk.forward_(s.clone(), z.clone(), tok, pm, overlap=False)
+            assert torch.equal(z1, z2) and torch.equal(s1, s2)
