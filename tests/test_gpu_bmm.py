@@ -8,12 +8,17 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("batch,M,N,K", [
-    (1, 128, 128, 64),      # one tile, one K slab
-    (3, 128, 128, 256),     # batching, K loop
-    (2, 256, 384, 192),     # several tiles, BN=128
-    (1, 384, 512, 1024),    # BN=256 path, ring wraps
+    (1, 128, 128, 64),      # 64 wide: one K slab
+    (3, 128, 128, 256),     # 64 wide: batching, K loop
+    (2, 256, 384, 192),     # 64 wide: several tiles
+    (1, 384, 512, 1024),    # 64 wide: the ring wraps
     (2, 100, 72, 40),       # ragged M/N/K: TMA zero fill and store bounds
-    (130, 128, 256, 128),   # more tiles than CTAs can hold at once for one wave of channels
+    (130, 128, 256, 128),   # 128 wide, two groups of epilogue warps, more tiles than CTAs
+    (140, 128, 120, 640),   # 128 wide, one group, ragged N, the ring wraps
+    (40, 256, 384, 1024),   # 128 wide, one group, two tiles for some CTAs
+    (140, 100, 248, 576),   # 256 wide, one group, ragged M and N, the ring wraps
+    (160, 130, 256, 576),   # 256 wide, one group, three tiles for some CTAs
+    (520, 120, 256, 128),   # 256 wide, two groups, four tiles a CTA
 ])
 def test_bmm_nt(batch, M, N, K):
     from bioemu2_b200 import functional as F

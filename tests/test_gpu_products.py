@@ -77,7 +77,7 @@ def test_transition_widths(rows, dim, hidden, dtype):
         _close(m.forward_residual_(x.clone()), x.double() + want)
 
 
-@pytest.mark.parametrize("windowed,dim,n,B,M,hidden", [(False, 768, 40, 1, 1, 1536), (False, 384, 136, 2, 3, 768),
+@pytest.mark.parametrize("windowed,dim,n,B,M,hidden", [(False, 768, 40, 1, 1, 1536), (False, 384, 136, 2, 3, 768), (False, 96, 136, 1, 2, 192),
                                                        (True, 128, 64, 2, 2, 256), (True, 128, 32, 1, 5, 512), (True, 64, 96, 1, 1, 128)])
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_conditioned_layer_native_against_its_parts(windowed, dim, n, B, M, hidden, dtype):
