@@ -16,8 +16,10 @@
 // 32,768 tokens: as nine kernels (LayerNorm of c, the projection to 100 MB of conditioning, two adaptive LayerNorms, the products, the
 // transition, two gated residuals) 104 us beside the attention, most of it reading and writing the conditioning; here 24 + 34.
 // Bound by the chain of a tile (about 16 and 22
-// thousand clocks) with at most two tiles a CTA to overlap, the first behind its own loads.  Tried: twelve rows of c a thread on
-// their way at once (spills: 297 us for three layers instead of 277), the output projections through one staging tile a group (284).
+// thousand clocks) with at most two tiles a CTA to overlap, the first behind its own loads.  At 128 registers a thread both spill (the
+// 64 channels of a row a thread beside alpha and beta): 136 bytes in cond_in, 116 in cond_out for an fp32 c, 76 and 84 for bf16.
+// Tried: twelve rows of c a thread on their way at once (more spills: 297 us for three layers instead of 277), the output
+// projections through one staging tile a group (284).
 #pragma once
 #include "row_tile.cuh"
 

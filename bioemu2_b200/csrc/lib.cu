@@ -41,7 +41,7 @@ static int launch_window_attention(const WindowAttnParams& p, int BM, cudaStream
 }
 
 // Whether window_pair_kernel takes these shapes: whole 16-query tiles, 128 keys, 16 pair channels, heads of 16 or 32 (with 64 it
-// spills 190 bytes) in boxes of 64 columns, two teams of warps within 512 threads and their K and V in shared memory; and the
+// spills 190 bytes, with 32 36) in boxes of 64 columns, two teams of warps within 512 threads and their K and V in shared memory; and the
 // windows in one wave of CTAs that have samples enough to pay for a bias phase of their own.  Three layers, heads 4 x 32, us as two
 // kernels / as one (windows x samples): 16 x 8 133 / 148, 32 x 4 135 / 147, 64 x 2 141 / 147, 32 x 6 156 / 157, 64 x 3 162 / 156,
 // 128 x 2 194 / 178, 128 x 8 425 / 384; 96 x 1 141 / 134, 148 x 1 161 / 143; 160 x 1 180 / 186, 160 x 4 340 / 361, 192 x 8 621 / 598.

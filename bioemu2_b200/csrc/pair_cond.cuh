@@ -20,6 +20,7 @@
 // operands there reads at its full 128 bytes a clock: with X and H in shared memory every wait for an access of the other warps was
 // longer (123 us).  Tried: 16 warps on the LayerNorm and SwiGLU at 80 registers (126 us: the producers then have one row a thread in
 // flight), a warp a source row (142: more shuffles, which share the shared memory's path), the output stored by the lanes (110).
+// At 128 registers a thread it spills 140 bytes for fp32 sources and 168 for bf16.
 #pragma once
 #include "row_tile.cuh"
 

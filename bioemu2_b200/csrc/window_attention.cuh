@@ -467,6 +467,7 @@ struct WindowPairCfg {
 // 4,096 atoms x 8 samples, 128 windows: 33 us, 11 of them the bias (its pair rows from DRAM, beside the write-back of what the
 // layer wrote before), 5 a pair of samples, which the two teams' issue slots bound.  As two kernels the bias went through global
 // memory and came back once per sample (64 KB a window, as much as K and V), and nothing covered a CTA's loads: 11.4 + 43 us.
+// At 128 registers a thread it spills 36 bytes with heads of 32, 8 with 16.
 template <bool F32, int DH>
 __global__ void __launch_bounds__(512, 1)
 window_pair_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ WindowPairParams pp) {
