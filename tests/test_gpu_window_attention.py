@@ -139,9 +139,9 @@ def test_window_pair_attention_scratch(B, M, NW, heads, dh, offset):
     q, gate = qkvg.data_ptr(), qkvg.data_ptr() + 6 * D
     _lib.check(lib.b200_window_pair_attention_fwd(q, 4 * D, gate, 4 * D, z.data_ptr(), ln_w.data_ptr(), ln_b.data_ptr(), w_z.data_ptr(),
                                                   mask.data_ptr(), out.data_ptr(), scratch.data_ptr() + 4 * guard, B, M, NW, W, Hk,
-                                                  heads, dh, c_z, 0, st))
+                                                  heads, dh, c_z, _lib.DTYPE_F32, st))
     _lib.check(lib.b200_window_bias_fwd(z.data_ptr(), ln_w.data_ptr(), ln_b.data_ptr(), w_z.data_ptr(), bias.data_ptr(), B * NW, W, Hk,
-                                        c_z, heads, 0, st))
+                                        c_z, heads, _lib.DTYPE_F32, st))
     _lib.check(lib.b200_window_attention_pitched_fwd(q, 4 * D, gate, 4 * D, bias.data_ptr(), mask.data_ptr(), want.data_ptr(), B, M, NW,
                                                      W, Hk, heads, dh, st))
     assert _lib.device_status() == 0
