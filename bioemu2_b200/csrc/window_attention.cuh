@@ -735,8 +735,8 @@ window_pair_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_consta
       const float inv = half ? i1 : i0;
 #pragma unroll
       for (int d = 0; d < DH / 8; ++d) {
-        const float y0 = __fdividef(o[d][half * 2] * inv, 1.0f + __expf(-bf16lo(gv[half][d])));
-        const float y1 = __fdividef(o[d][half * 2 + 1] * inv, 1.0f + __expf(-bf16hi(gv[half][d])));
+        const float y0 = quotient(o[d][half * 2] * inv, 1.0f + __expf(-bf16lo(gv[half][d])));
+        const float y1 = quotient(o[d][half * 2 + 1] * inv, 1.0f + __expf(-bf16hi(gv[half][d])));
         *reinterpret_cast<uint32_t*>(dst + d * 8) = pack_bf16x2(y0, y1);
       }
     }
