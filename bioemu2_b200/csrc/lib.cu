@@ -43,8 +43,11 @@ static int launch_window_attention(const WindowAttnParams& p, int BM, cudaStream
 // Whether window_pair_kernel takes these shapes: whole 16-query tiles, 128 keys, 16 pair channels, heads of 16 or 32 (with 64 it
 // spills 190 bytes, with 32 36) in boxes of 64 columns, two teams of warps within 512 threads and their K and V in shared memory; and the
 // windows in one wave of CTAs that have samples enough to pay for a bias phase of their own.  Three layers, heads 4 x 32, us as two
-// kernels / as one (windows x samples): 16 x 8 133 / 148, 32 x 4 135 / 147, 64 x 2 141 / 147, 32 x 6 156 / 157, 64 x 3 162 / 156,
-// 128 x 2 194 / 178, 128 x 8 425 / 384; 96 x 1 141 / 134, 148 x 1 161 / 143; 160 x 1 180 / 186, 160 x 4 340 / 361, 192 x 8 621 / 598.
+// kernels / as one (windows x samples): 16 x 8 118 / 131, 32 x 4 121 / 131, 64 x 2 126 / 132, 32 x 6 131 / 132, 64 x 3 136 / 132, 64 x 8
+// 173 / 154, 95 x 3 147 / 142, 96 x 1 132 / 125, 128 x 2 151 / 134, 128 x 8 317 / 274, 148 x 1 141 / 125, 148 x 8 343 / 281; beyond a
+// wave 149 x 1 149 / 160, 149 x 8 402 / 419, 160 x 4 277 / 285.  Of 72 pairs of 16 to 192 windows and 1 to 8 samples it takes the slower
+// of the two by more than 1 % in these: 80 x 3 139 / 142 as one; as two 80 x 1 128 / 124, 80 x 2 138 / 132, 95 x 1 132 / 125, 95 x 2 143
+// / 132, 176 x 2 194 / 185, 192 x 1 166 / 164, 192 x 2 199 / 188, 192 x 6 348 / 344, 192 x 8 457 / 436 (149 x 3 within the spread).
 static bool window_pair_fits(const WindowAttnParams& p, int B, int head_dim, int c_z, const void* z) {
   if ((head_dim != 16 && head_dim != 32) || p.W % 16 || p.W > p.Hk || p.Hk != kWindowMmaKeys || c_z != 16 || p.heads * (p.W / 16) > 8 ||
       p.qkv_pitch % 8 || p.gate_pitch % 2 || p.heads * head_dim % 64 || !aligned(z, 32))
@@ -126,7 +129,10 @@ struct BmmLaunch {
 // 128 batches of 384^3 21.8 / 25.7, of 512^3 42.5 / 38.7).
 // 64 columns where even the narrow tiles are few: a K block of 64 is then bound by shared memory (24 KB written and 24 read, against
 // 32 and 32), and twice the SMs share the epilogues.  Token layers x 4 (rows, us with 128-wide tiles at the least / with 64): 32 280 /
-// 263, 256 289 / 268, 512 297 / 286, 800 354 / 341, 1600 434 / 433, 2048 the same tiles.
+// 263, 256 289 / 268, 512 297 / 286, 800 354 / 341, 1600 434 / 433, 2048 the same tiles.  Of 261 products (24 to 20000 rows,
+// widths of the trunk, the token and atom blocks, contractions; one after the other in a graph) it is taken for 186: 185 are 6 to 20 %
+// shorter than with the 128-wide tiles' best (1024 x 384 x 384 5.3 / 4.3), short K among them although wider tiles then have eight
+// epilogue warps; 128 batches of 128 x 128 x 64 take 3.69 us instead of 3.59.
 // Products that run on a side stream underneath another's kernels go by the same estimate: wide tiles for those, since they
 // take less SM time, moved a trunk's time both ways (4 blocks, us, without / with: 144 tokens 890 / 902, 160 1024 / 1006,
 // 203 1144 / 1154, 256 1292 / 1322, 320 and more the same).
